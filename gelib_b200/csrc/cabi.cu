@@ -221,6 +221,8 @@ int run_product(const char* fn, bool diag, int mode, int nr, const gelib_tensor5
   if (mode == 0) {
     st = -1;
     if (c.dense_channels && !c.r_bcast && !fp64) {
+      if (col_enabled()) st = launch_col_fwd(c, s);
+      if (st != -1) return st;
       if (diag) {
         st = launch_diag_fwd(c, s);
       } else {
@@ -233,6 +235,8 @@ int run_product(const char* fn, bool diag, int mode, int nr, const gelib_tensor5
   }
   st = -1;
   if (c.dense_channels && !fp64) {
+    if (col_enabled()) st = launch_col_bwd(c, s);
+    if (st != -1) return st;
     if (diag) {
       st = launch_diag_bwd(c, s);
     } else {

@@ -1,0 +1,85 @@
+// Column kernels: products in which every channel of the output has its own pair of input columns -- the diagonal
+// product, and the full product when x has one channel (the spherical harmonics of a first layer).  With "column" =
+// (cell, channel) both are
+//
+//   r_l[m] (+)= sum_{m1} C_l[m1, m-m1] x_l1[m1] y_l2[m-m1]
+//   G[m1,m2] = sum_l C_l[m1,m2] g_l[m1+m2];   xg[m1] += G conj(y[m2]);   yg[m2] += G conj(x[m1])
+//
+// and a lane that owns a column needs nothing from any other lane.
+//
+// Organisation.  A warp owns 32 lanes of columns (two adjacent channels per lane where alignment allows, else one) and
+// walks the (l1,l2) pairs; the part with the smaller l is the pair's "a" side, the other its "b" side.  The rows of the
+// b part at work, and their gradients, sit in shared memory in slots that belong to the lane; up to eleven a rows (a
+// block) and their gradients sit in registers.  The pair is walked by output row m: entry i of a step multiplies a[i]
+// with b[m - m1(i)].  The gradients of the b rows that a step touches are a window of registers that moves by one row per
+// step (the body is instantiated per block size, so everything in registers is indexed statically); a row is added to its
+// slot when it leaves the window.  There are no atomics in shared memory, no shuffles and no barriers in the loop, and one
+// read-modify-write per row and block instead of one per band entry.
+// Everything a warp reads from global memory -- b rows, a rows, the gradient rows g -- arrives through one stream of rows
+// (cp.async, 8 or 16 bytes per lane) in a ring of kColRing rows, whose order is the order of use: taking k rows requests
+// the k rows that come kColRing later, so the bytes in flight do not depend on how short the steps are.  What the warps
+// of a block share is the walk itself: a chunk (row addresses, step records, coefficients stored twice for the packed
+// multiply-adds) is copied to shared memory one chunk ahead.
+// Why this form: diag_bwd_cell_kernel spends its time in four shared-memory atomics (compare-and-swap loops) per band
+// entry, which a lane that owns its column does not need.  Measured, backward of the diagonal product: maxl 8 x 128
+// channels, batch 2048 10.5 -> 5.9 ms; maxl 6 x 33, batch 4000 4.3 -> 1.1 ms; maxl 3 x 12, batch 500 49 -> 18 us (forward 32 ->
+// 15 us).  Bound by instruction issue at two to three warps per scheduler: 475 k warp instructions per 64 columns at maxl
+// 8, 0.33 issued per cycle, the largest stalls instruction fetch (the unrolled bodies) and fixed-latency dependencies.
+#pragma once
+#include "plan.h"
+
+namespace gelib_b200 {
+
+constexpr int kColRing = 16;                    // rows in flight per warp (a power of two)
+constexpr int kColMaxNl = 10;                   // output l per step; pairs with more are walked twice
+constexpr int kColMaxLa = 8;                    // largest l of an a side
+constexpr int kColBlockBwd = 11;                // a rows per block, backward (registers: a, its gradient, the window)
+constexpr int kColBlockFwd = 17;                // a rows per block, forward
+constexpr int kColChunkBytes = 13312;           // capacity of a chunk buffer
+constexpr int kColMaxSmem = 232448;
+constexpr int kColSlots = 3 * kMaxParts;        // x parts, y parts, r (g) parts
+
+// Row (slot, v) of a column: base + v * unit + cell * cell_stride + channel * ch_stride, all in bytes.
+struct ColPart {
+  float* base;
+  unsigned unit, cell_stride;
+};
+
+struct ColArgs {
+  ColPart part[kColSlots];         // x: 0.., y: kMaxParts.., r or g: 2 kMaxParts..  (v = row for x, y; complex offset for r)
+  ColPart grad[2 * kMaxParts];     // xg: 0.., yg: kMaxParts..  (v = row)
+  unsigned ch_stride[3];           // bytes between channels of x, y, r: 8, or 0 for an operand of one channel
+  int nx, ny, nr;
+  unsigned n, nlanes;              // lanes per cell (channels / columns per lane), lanes in all
+  int b_rows;                      // rows of the largest b part
+  int accumulate;                  // forward: add to r instead of storing
+  const int4* blob;
+  const int* chunks;               // per split {first chunk, number of chunks, first record of the ring prologue}, then
+                                   // per chunk {offset, size} in int4 units
+  int nsplits;
+};
+
+struct ColPlan {
+  DevicePlan* dev;
+  int max_la;     // largest l of an a side
+  int max_block;  // a rows of the largest block
+  int cpl;        // columns per lane
+};
+
+// Bits of a segment record.
+enum { kColFirstOfB = 1, kColLastOfB = 2, kColLastOfChunk = 4, kColLast = 8, kColDrain = 16, kColHalf1 = 32 };
+
+// Warps per block, at most `most`: an SM holds one block, so when one wave of blocks is enough its warps are spread over
+// all SMs instead of filling some of them.
+inline int col_block_warps(unsigned warps, int splits, int most) {
+  const long long total = (long long)warps * splits;
+  if (total >= 148LL * most) return most;
+  const long long nw = (total + 147) / 148;
+  return (int)(nw < 2 ? 2 : nw);
+}
+
+// Returns false when the call is not one the column kernels take; otherwise fills args and
+// plan (plan->dev == nullptr on a CUDA error).
+bool col_setup(const VecCall& c, bool backward, int warps_resident, ColArgs* a, ColPlan* plan);
+
+}  // namespace gelib_b200

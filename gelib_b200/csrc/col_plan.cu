@@ -1,0 +1,352 @@
+// Host side of the column kernels: which calls they take, and the walk (col.h).
+#include <algorithm>
+#include <cstring>
+#include <map>
+
+#include "col.h"
+
+namespace gelib_b200 {
+
+namespace {
+
+// Stride in floats between consecutive cells (b, g0, g1), or -1 when the view is not an arithmetic progression.
+long long cell_stride(const PartView& p, const CellGrid& cg) {
+  long long st = 0;
+  bool any = false;
+  const long long dims[3] = {cg.G1, cg.G0, cg.B}, strides[3] = {p.sg1, p.sg0, p.sb};
+  long long inner = 1;
+  for (int d = 0; d < 3; d++) {
+    if (dims[d] == 1) continue;
+    if (!any) st = strides[d];
+    else if (strides[d] != st * inner) return -1;
+    any = true;
+    inner *= dims[d];
+  }
+  return any ? st : 0;
+}
+
+struct Step {
+  int m, nl, lo, hi;  // output row, output l, first and last entry of the band
+};
+struct Segment {
+  int half, ai, bi, la, lb, mlo, kb;  // mlo, kb: first m1 and number of rows of the a block
+  std::vector<Step> steps;
+  std::vector<const Triple*> ls;      // the triples of the pair's l group, ascending l
+  int flags = 0;
+  double cost = 0;
+};
+
+int nl_padded(int nl) { return (nl + 1) / 2 * 2; }
+
+struct Builder {
+  const std::vector<PartSig>& rs;
+  bool backward, do_x, do_y;
+  std::vector<int2> rows;  // the stream, in order of use
+
+  bool do_a(int half) const { return backward && (half == 0 ? do_x : do_y); }
+  bool do_b(int half) const { return backward && (half == 0 ? do_y : do_x); }
+  bool need_a(int half) const { return !backward || do_b(half); }
+  bool need_b(int half) const { return !backward || do_a(half); }
+
+  int2 r_row(const Segment& s, const Step& st, int j) const {
+    const Triple& t = *s.ls[s.ls.size() - st.nl + j];
+    return make_int2(2 * kMaxParts + t.ri, (st.m + t.l) * rs[t.ri].n + t.offs);
+  }
+  void emit_rows(const Segment& s) {
+    if ((s.flags & kColFirstOfB) && need_b(s.half))
+      for (int r = 0; r <= 2 * s.lb; r++) rows.push_back(make_int2((s.half == 0 ? kMaxParts : 0) + s.bi, r));
+    if (need_a(s.half))
+      for (int i = 0; i < s.kb; i++) rows.push_back(make_int2((s.half == 0 ? 0 : kMaxParts) + s.ai, s.mlo + s.la + i));
+    if (backward)
+      for (const Step& st : s.steps)
+        for (int j = 0; j < st.nl; j++) rows.push_back(r_row(s, st, j));
+  }
+  // int4 units of a segment in a chunk, and how many of them are address records
+  int units(const Segment& s, int* recs) {
+    const size_t n0 = rows.size();
+    emit_rows(s);
+    *recs = (int)(rows.size() - n0);
+    rows.resize(n0);
+    int u = 2 + ((int)s.steps.size() + 3) / 4;
+    for (const Step& st : s.steps) {
+      u += s.kb * nl_padded(st.nl) / 2;
+      if (!backward) *recs += st.nl;
+    }
+    return u + *recs;
+  }
+};
+
+void build(DevicePlan& p, const std::vector<PartSig>& xs, const std::vector<PartSig>& ys, const std::vector<PartSig>& rs,
+           bool diag, bool backward, bool do_x, bool do_y, int splits) {
+  build_schedule(xs, ys, rs, diag, false, &p.sched);
+  Builder B{rs, backward, do_x, do_y};
+  std::map<std::pair<int, int>, std::vector<const Triple*>> pairs;
+  for (const Triple& t : p.sched.triples) pairs[{t.xi, t.yi}].push_back(&t);
+  const int cap = kColChunkBytes / 16, max_block = backward ? kColBlockBwd : kColBlockFwd;
+
+  // all segments in order: half, b part, a part, block of a rows, group of l, piece of m
+  std::vector<Segment> all;
+  for (int half = 0; half < 2; half++) {
+    const auto& as = half == 0 ? xs : ys;
+    const auto& bs = half == 0 ? ys : xs;
+    for (size_t bi = 0; bi < bs.size(); bi++)
+      for (size_t ai = 0; ai < as.size(); ai++) {
+        const int la = as[ai].l, lb = bs[bi].l;
+        if (half == 0 ? la > lb : la >= lb) continue;
+        const auto it = pairs.find(half == 0 ? std::make_pair((int)ai, (int)bi) : std::make_pair((int)bi, (int)ai));
+        if (it == pairs.end()) continue;
+        std::vector<const Triple*> ts = it->second;
+        std::sort(ts.begin(), ts.end(), [](const Triple* u, const Triple* v) { return u->l < v->l; });
+        const int nblocks = (2 * la + max_block) / max_block;
+        int mlo = -la;
+        for (int k = 0; k < nblocks; k++) {
+          const int kb = (2 * la + 1 + nblocks - 1 - k) / nblocks;  // sizes that differ by at most one
+          for (size_t g0 = 0; g0 < ts.size(); g0 += kColMaxNl) {
+            Segment s;
+            s.half = half;
+            s.ai = (int)ai;
+            s.bi = (int)bi;
+            s.la = la;
+            s.lb = lb;
+            s.mlo = mlo;
+            s.kb = kb;
+            s.ls.assign(ts.begin() + g0, ts.begin() + std::min(ts.size(), g0 + kColMaxNl));
+            int room = 0;
+            for (int m = -s.ls.back()->l; m <= s.ls.back()->l; m++) {
+              Step st{m, 0, std::max(0, m - lb - mlo), std::min(kb - 1, m + lb - mlo)};
+              for (const Triple* t : s.ls) st.nl += t->l >= std::abs(m);
+              if (st.hi < st.lo || st.nl == 0) continue;
+              const int need = 1 + kb * nl_padded(st.nl) / 2 + st.nl;
+              if (need > room || s.steps.empty() || st.m != s.steps.back().m + 1) {  // a new piece
+                if (!s.steps.empty()) all.push_back(s);
+                s.steps.clear();
+                s.cost = 0;
+                room = cap - 4 - kb - (2 * lb + 1) - 1;
+              }
+              room -= need;
+              s.cost += (st.hi - st.lo + 1) * (1.5 * st.nl + 9) + 60 + 8 * st.nl;
+              s.steps.push_back(st);
+            }
+            if (!s.steps.empty()) all.push_back(s);
+          }
+          mlo += kb;
+        }
+      }
+  }
+  double total = 0;
+  for (const auto& s : all) total += s.cost;
+
+  // splits: contiguous runs of about equal cost
+  std::vector<std::vector<Segment>> runs;
+  double done = 0;
+  size_t next = 0;
+  for (int sp = 0; sp < splits && next < all.size(); sp++) {
+    std::vector<Segment> run;
+    const double until = total * (sp + 1) / splits;
+    while (next < all.size() && (run.empty() || sp + 1 == splits || done + 0.5 * all[next].cost <= until)) {
+      done += all[next].cost;
+      run.push_back(all[next++]);
+    }
+    runs.push_back(std::move(run));
+  }
+
+  std::vector<int> split_table, chunk_table;
+  int nchunks = 0;
+  for (auto& run : runs) {
+    auto same_b = [](const Segment& s, const Segment& t) { return s.half == t.half && s.bi == t.bi; };
+    for (size_t k = 0; k < run.size(); k++) {
+      Segment& s = run[k];
+      if (k == 0 || !same_b(run[k - 1], s)) s.flags |= kColFirstOfB;
+      if (k + 1 == run.size() || !same_b(run[k + 1], s)) s.flags |= kColLastOfB;
+      if (s.half) s.flags |= kColHalf1;
+      if (k + 1 == run.size()) s.flags |= kColLast;
+    }
+    struct Chunk { size_t from, to, row_begin; };
+    std::vector<Chunk> chunks;
+    B.rows.clear();
+    for (size_t k = 0; k < run.size();) {
+      Chunk c{k, k, B.rows.size()};
+      int used = 2;
+      while (k < run.size()) {
+        int recs = 0;
+        const int need = B.units(run[k], &recs);
+        if (k > c.from && used + need > cap) break;
+        used += need;
+        B.emit_rows(run[k++]);
+      }
+      c.to = k;
+      run[k - 1].flags |= kColLastOfChunk;
+      // the rows requested during the chunk push the copy of the next one out of the pending groups, or it is waited for
+      if ((int)(B.rows.size() - c.row_begin) < kColRing + 12) run[k - 1].flags |= kColDrain;
+      chunks.push_back(c);
+    }
+    auto rec = [&](size_t i) {
+      if (B.rows.empty()) return make_int4(2 * kMaxParts, 0, 0, 0);
+      const int2 r = B.rows[std::min(i, B.rows.size() - 1)];  // past the end: the last row again, never taken
+      return make_int4(r.x, r.y, 0, 0);
+    };
+    split_table.push_back(nchunks);
+    split_table.push_back((int)chunks.size());
+    split_table.push_back((int)p.h_items.size());
+    for (int j = 0; j < kColRing; j++) p.h_items.push_back(rec(j));
+    for (size_t ci = 0; ci < chunks.size(); ci++) {
+      const Chunk& c = chunks[ci];
+      const size_t row_end = ci + 1 < chunks.size() ? chunks[ci + 1].row_begin : B.rows.size();
+      std::vector<int4> v(2);
+      for (size_t i = c.row_begin; i < row_end; i++) v.push_back(rec(i + kColRing));
+      const int store_at = (int)v.size();
+      if (!backward)
+        for (size_t q = c.from; q < c.to; q++)
+          for (const Step& st : run[q].steps)
+            for (int j = 0; j < st.nl; j++) {
+              const int2 r = B.r_row(run[q], st, j);
+              v.push_back(make_int4(r.x, r.y, 0, 0));
+            }
+      const int nrec = (int)v.size() - 2;
+      const int seg_at = (int)v.size();
+      for (size_t q = c.from; q < c.to; q++) {
+        const Segment& s = run[q];
+        v.push_back(make_int4(s.kb | (s.flags << 8) | ((int)s.steps.size() << 16), s.steps[0].m - s.mlo, s.mlo + s.la, s.ai));
+        v.push_back(make_int4(s.bi, s.lb, 0, 0));
+        std::vector<int> w;
+        for (const Step& st : s.steps) w.push_back(st.nl | (st.lo << 8) | (st.hi << 16));
+        while (w.size() % 4) w.push_back(0);
+        for (size_t i = 0; i < w.size(); i += 4) v.push_back(make_int4(w[i], w[i + 1], w[i + 2], w[i + 3]));
+      }
+      const int coef_at = (int)v.size();
+      std::vector<float> cf;
+      for (size_t q = c.from; q < c.to; q++) {
+        const Segment& s = run[q];
+        for (const Step& st : s.steps)
+          for (int i = 0; i < s.kb; i++)
+            for (int j = 0; j < nl_padded(st.nl); j++) {
+              float x = 0.f;
+              if (i >= st.lo && i <= st.hi && j < st.nl) {
+                const Triple& t = *s.ls[s.ls.size() - st.nl + j];
+                const int ma = s.mlo + i, mb = st.m - ma;
+                x = (float)(s.half == 0 ? cg_coefficient(t.l1, t.l2, t.l, ma, mb) : cg_coefficient(t.l1, t.l2, t.l, mb, ma));
+              }
+              cf.push_back(x);
+              cf.push_back(x);
+            }
+      }
+      for (size_t i = 0; i < cf.size(); i += 4) {
+        int4 q;
+        memcpy(&q, &cf[i], 16);
+        v.push_back(q);
+      }
+      v[0] = make_int4(16 * 2, 16 * store_at, 16 * seg_at, 16 * coef_at);
+      v[1] = make_int4(nrec, 0, 0, 0);
+      chunk_table.push_back((int)p.h_items.size());
+      chunk_table.push_back((int)v.size());
+      p.h_items.insert(p.h_items.end(), v.begin(), v.end());
+      nchunks++;
+    }
+  }
+  p.h_jobs = split_table;
+  p.h_jobs.insert(p.h_jobs.end(), chunk_table.begin(), chunk_table.end());
+  p.h_jobs.push_back((int)runs.size());  // the last word: splits that were built
+}
+
+bool fill_part(const PartView& p, const CellGrid& cg, long long extra_floats, bool rows, ColPart* out) {
+  const long long cs = cell_stride(p, cg);
+  const long long unit = rows ? p.sm : 2;
+  if (cs < 0 || 4 * cs > 0xffffffffLL || unit < 0 || 4 * unit > 0xffffffffLL) return false;
+  out->base = p.base + extra_floats;
+  out->unit = (unsigned)(4 * unit);
+  out->cell_stride = (unsigned)(4 * cs);
+  return true;
+}
+
+}  // namespace
+
+bool col_setup(const VecCall& c, bool backward, int warps_resident, ColArgs* a, ColPlan* plan) {
+  if (c.x.empty() || c.y.empty() || c.r.empty() || !c.dense_channels || c.sph) return false;
+  if (c.x.size() > (size_t)kMaxParts || c.y.size() > (size_t)kMaxParts || c.r.size() > (size_t)kMaxParts) return false;
+  const int n = c.y[0].n, nx = c.diag ? n : 1;
+  for (const auto& p : c.x) if (p.n != nx || p.l > 63) return false;
+  for (const auto& p : c.y) if (p.n != n || p.l > 63) return false;
+  if (n < 1 || (long long)n * c.cg.ncells > 0x7fffffffLL) return false;
+  const bool do_x = !c.xg.empty(), do_y = !c.yg.empty();
+  if (backward && !c.diag && do_x && n > 1) return false;  // the gradient of the one channel is a sum over columns
+  int max_la = 0, max_lb = 0;
+  for (const auto& p : c.x)
+    for (const auto& q : c.y) {
+      max_la = std::max(max_la, std::min(p.l, q.l));
+      max_lb = std::max(max_lb, std::max(p.l, q.l));
+    }
+  if (max_la > kColMaxLa || max_lb > 40) return false;
+  plan->max_la = max_la;
+  // Calls that the other kernels do faster (measured, us, other kernel / this one):
+  //   diagonal forward: with l >= 6 and full 64-channel slices diag_fwd_cell_kernel, which shares its operands between the
+  //     warps of a block, fits more warps on an SM: maxl 8 x 128 channels, batch 2048 3018 / 3820; maxl 6 x 64 608 / 835,
+  //     maxl 6 x 128 1208 / 1265; but maxl 5 x 128 711 / 661, maxl 8 x 48, batch 1000 821 / 652.
+  //   one-channel x: cg_narrow_fwd_kernel when it fills the chip and wastes no lanes (its rows are padded to a power of two):
+  //     30000 cells, maxl 4 x 32 channels 900 / 1174; 16000, maxl 6 x 16 1274 / 1362; but 4096 cells 467 / 367, 1000 cells
+  //     357 / 151; 40000 cells, maxl 6 x 24 5043 / 4281.
+  //   its gradient of y: cg_narrow1_bwd_kernel under the same conditions and l >= 6: 65536 cells, maxl 6 x 16 5418 / 5609;
+  //     but maxl 4 x 32, 5000 cells 356 / 331; 60000 cells, maxl 2 x 16 247 / 189; 4096 cells, maxl 6 x 16 638 / 370.
+  if (c.diag) {
+    const int slices = (n + 63) / 64;
+    if (!backward && max_la >= 6 && 8 * n >= 7 * 64 * slices) return false;
+  } else if (n > 1 && n <= 32) {
+    int cw = 1;
+    while (cw < n) cw *= 2;
+    const long long narrow_warps = c.cg.ncells * cw / 32;
+    if (!backward && narrow_warps >= 148 * 16 && !(max_la >= 4 && 4 * n <= 3 * cw)) return false;
+    if (backward && narrow1_enabled() && narrow_warps >= 148 * 32 && max_la >= 6 && 4 * n > 3 * cw) return false;
+  }
+  const int max_rows = backward ? kColBlockBwd : kColBlockFwd;
+  plan->max_block = 2 * max_la + 1 <= max_rows ? 2 * max_la + 1 : max_rows;
+  a->b_rows = 2 * max_lb + 1;
+  for (size_t i = 0; i < c.x.size(); i++)
+    if (!fill_part(c.x[i], c.cg, 0, true, &a->part[i])) return false;
+  for (size_t i = 0; i < c.y.size(); i++)
+    if (!fill_part(c.y[i], c.cg, 0, true, &a->part[kMaxParts + i])) return false;
+  for (size_t i = 0; i < c.r.size(); i++) {
+    if (c.r[i].sm != 2LL * c.r[i].n) return false;  // the walk holds offsets of dense rows
+    if ((2LL * c.r[i].l + 1) * c.r[i].n > 0x7fffffffLL) return false;
+    if (!fill_part(c.r[i], c.cg, 2LL * c.offs_extra, false, &a->part[2 * kMaxParts + i])) return false;
+    a->part[2 * kMaxParts + i].unit = 8;
+  }
+  for (size_t i = 0; i < c.xg.size(); i++)
+    if (!fill_part(c.xg[i], c.cg, 0, true, &a->grad[i])) return false;
+  for (size_t i = 0; i < c.yg.size(); i++)
+    if (!fill_part(c.yg[i], c.cg, 0, true, &a->grad[kMaxParts + i])) return false;
+  // two columns per lane: every access is 16 bytes (8 for an operand of one channel, which both columns share)
+  const bool x_shared = nx == 1 && n > 1;
+  bool two = n % 2 == 0 && c.offs_extra % 2 == 0;
+  for (auto* v : {&c.y, &c.r, &c.yg, x_shared ? &c.y : &c.x, x_shared ? &c.y : &c.xg})
+    for (const auto& p : *v)
+      if ((uintptr_t)p.base % 16 || p.sb % 4 || p.sg0 % 4 || p.sg1 % 4 || p.sm % 4) two = false;
+  // two columns share the records, coefficients and control of a step; with few columns warps matter more
+  const long long columns = c.cg.ncells * n;
+  plan->cpl = two && columns >= 64 * 148 * 4 ? 2 : 1;
+  a->ch_stride[0] = x_shared ? 0 : 8 * plan->cpl;
+  a->ch_stride[1] = a->ch_stride[2] = 8 * plan->cpl;
+  a->nx = (int)c.x.size();
+  a->ny = (int)c.y.size();
+  a->nr = (int)c.r.size();
+  a->n = (unsigned)(n / plan->cpl);
+  a->nlanes = (unsigned)(c.cg.ncells * a->n);
+  // with fewer warps than the chip holds, the walk is cut into runs of pairs that different blocks take
+  const long long warps = (a->nlanes + 31) / 32;
+  int splits = 1;
+  while (splits < 16 && warps * splits * 2 <= warps_resident) splits *= 2;
+  a->accumulate = (c.flags & GELIB_OVERWRITE) ? 0 : 1;
+
+  std::vector<int> key = {20 /*family*/, backward, do_x, do_y, splits, c.diag, (int)c.x.size(), (int)c.y.size(), (int)c.r.size(), n};
+  for (const auto& p : c.x) key.push_back(p.l);
+  for (const auto& p : c.y) key.push_back(p.l);
+  for (const auto& p : c.r) { key.push_back(p.l); key.push_back(p.n); }
+  const auto xs = sig_of(c.x), ys = sig_of(c.y), rs = sig_of(c.r);
+  const bool diag = c.diag;
+  plan->dev = get_plan(key, [&](DevicePlan& p) { build(p, xs, ys, rs, diag, backward, do_x, do_y, splits); });
+  if (!plan->dev) return true;
+  a->blob = plan->dev->items;
+  a->chunks = plan->dev->jobs;
+  a->nsplits = plan->dev->h_jobs.back();
+  return true;
+}
+
+}  // namespace gelib_b200

@@ -43,6 +43,9 @@ bool narrow1_enabled();  // option "narrow1" (default on): tests compare the two
 int launch_cg_narrow_fwd(const VecCall& c, cudaStream_t s);  // x with at most 4 channels; -1 when the call does not qualify
 int launch_cg_strided(const VecCall& c, int mode, cudaStream_t s);  // mode 0 fwd, 1 back0, 2 back1
 int launch_cg_strided_static(const VecCall& c, cudaStream_t s);  // forward, tables in a static device array: no allocation
+int launch_col_fwd(const VecCall& c, cudaStream_t s);  // diagonal products and one-channel x; -1 when the call does not qualify
+int launch_col_bwd(const VecCall& c, cudaStream_t s);  // likewise
+bool col_enabled();  // option "col" (default on): tests compare the kernels
 int launch_diag_fwd(const VecCall& c, cudaStream_t s);
 int launch_diag_bwd(const VecCall& c, cudaStream_t s);
 int launch_diag_fwd_fast(const VecCall& c, cudaStream_t s);  // -1 when the call does not qualify

@@ -175,7 +175,7 @@ __global__ void __launch_bounds__(256, 2) cg_bwd_kernel(const __grid_constant__ 
 #pragma unroll
   for (int u = 0; u < TBU; u++) yo[u] = 2 * ((u ^ cp) * WB + lb) * UB;
 
-  for (int it = warp; it < A.nitems; it += nwarps) {
+  for (int it = blockIdx.y * nwarps + warp; it < A.nitems; it += nwarps * gridDim.y) {
     const int4 i0 = __ldg(&A.items[2 * it]), i1 = __ldg(&A.items[2 * it + 1]);
     const int ri = i0.x & 15, xi = (i0.x >> 4) & 15, yi = (i0.x >> 8) & 15;
     const int l = i0.y & 0xfff, m = (i0.y >> 12) - l;
@@ -322,6 +322,9 @@ struct BwdCfg {
 };
 constexpr BwdCfg kCfgs[] = {
     {4, 4, 8, 4},  // 32 x 32 channels (16 without vector loads), 1 cell per warp
+    {4, 2, 4, 4},  // 16 x 16, 2 cells
+    {4, 2, 2, 2},  //  8 x  8, 8 cells
+    {2, 2, 4, 2},  //  8 x  8, 4 cells
     {2, 2, 4, 4},  //  8 x 16, 2 cells
     {1, 2, 1, 4},  //  1 x 16, 8 cells
     {2, 1, 2, 2},  //  4 x  4, 8 cells
@@ -330,7 +333,7 @@ constexpr BwdCfg kCfgs[] = {
 constexpr int kNumCfgs = sizeof(kCfgs) / sizeof(kCfgs[0]);
 
 template <int TA, int TBU, int WA, int WB>
-cudaError_t launch_cfg(const BwdArgs& a, unsigned grid, int threads, size_t smem, bool vec, cudaStream_t s) {
+cudaError_t launch_cfg(const BwdArgs& a, dim3 grid, int threads, size_t smem, bool vec, cudaStream_t s) {
   auto k = vec ? cg_bwd_kernel<TA, TBU, WA, WB, true> : cg_bwd_kernel<TA, TBU, WA, WB, false>;
   cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e != cudaSuccess) return e;
@@ -362,17 +365,46 @@ int launch_cg_bwd(const VecCall& c, cudaStream_t s) {
   }
   const bool vec = c.vec_ok;
   const int UB = vec ? 2 : 1;
-  int n1 = 1, n2 = 1;
-  for (const auto& p : c.x) n1 = std::max(n1, p.n);
-  for (const auto& p : c.y) n2 = std::max(n2, p.n);
   for (const auto& p : c.x) if (p.l > 2047 || p.n > 65535) return -1;
   for (const auto& p : c.y) if (p.l > 2047 || p.n > 65535) return -1;
   for (const auto& p : c.r) if (p.l > 2047) return -1;
+  // The lane layout whose warps execute the fewest instructions for the call.  Per band entry: 8 multiply-adds per
+  // complex number of the slab, the operand loads, the butterflies' shuffles and adds, and about five instructions per
+  // shared-memory atomic (they are compare-and-swap loops); per slab its loads.  The layouts differ in the padding of
+  // the channel counts and in how many multiply-adds share a butterfly; the work is spread over the warps the call can
+  // fill.  Measured (maxl 4 x 16 channels, batch 1000): 689 us with 8 x 16 channels per warp, 418 us with 16 x 16.
+  Schedule sched;
+  build_schedule(sig_of(c.x), sig_of(c.y), sig_of(c.r), false, false, &sched);
+  auto halving = [](int n, int e, int w, int* own) {  // shuffles of butterfly<n, e, w>, elements left per lane
+    int sh = 0;
+    for (int s = 1; s < w; s *= 2) {
+      if (n > 1) n /= 2;
+      sh += n * e;
+    }
+    *own = n * e;
+    return sh;
+  };
   int best = 0;
   double best_cost = 1e300;
   for (int i = 0; i < kNumCfgs; i++) {
-    const int ta = kCfgs[i].TA * kCfgs[i].WA, tb = kCfgs[i].TBU * UB * kCfgs[i].WB;
-    const double cost = (double)ceil_div(n1, ta) * ta * ceil_div(n2, tb) * tb;
+    const BwdCfg& f = kCfgs[i];
+    const int ta = f.TA * f.WA, tb = f.TBU * UB * f.WB;
+    const int wc = 32 / (f.WA * f.WB);
+    size_t floats = 0;
+    for (const auto& p : c.x) floats += align4(2 * (2 * p.l + 1) * ceil_div(p.n, ta) * ta);
+    for (const auto& p : c.y) floats += align4(2 * (2 * p.l + 1) * ceil_div(p.n, tb) * tb);
+    if ((6 * kMaxParts + 2 * floats) * wc * sizeof(float) > 220 * 1024) continue;
+    int own_x, own_y;
+    const int sh = halving(f.TA, 2, f.WB, &own_x) + halving(f.TBU, 2 * UB, f.WA, &own_y);
+    const double entry = 8.0 * f.TA * f.TBU * UB + f.TA + f.TBU + 2 * sh + 6 * (own_x + own_y) + 12, slab = 3.0 * f.TA * f.TBU + 30;
+    double cost = 0, items = 0;
+    for (const Triple& t : sched.triples) {
+      const double tiles = (double)ceil_div(c.x[t.xi].n, ta) * ceil_div(c.y[t.yi].n, tb);
+      cost += tiles * (band_size(t.l1, t.l2, t.l) * entry + (2 * t.l + 1) * slab);
+      items += tiles * (2 * t.l + 1);
+    }
+    const double groups = (double)((c.cg.ncells + wc - 1) / wc);
+    cost *= groups / std::min(groups * std::min(128.0, std::max(8.0, items / 2)), 148.0 * 16);
     if (cost < best_cost * 0.999) {
       best_cost = cost;
       best = i;
@@ -451,19 +483,27 @@ int launch_cg_bwd(const VecCall& c, cudaStream_t s) {
   a.offs_extra = c.offs_extra;
   a.do_x = c.xg.empty() ? 0 : 1;
   a.do_y = c.yg.empty() ? 0 : 1;
-  a.x_atomic = c.xg_bcast ? 1 : 0;
-  a.y_atomic = c.yg_bcast ? 1 : 0;
-
   const long long groups = (c.cg.ncells + WC - 1) / WC;
+  // Few cells: several blocks share a group of cells, each takes every splits-th round of slabs, and the rows are added
+  // to global memory with atomics.  A block should still have two rounds.
+  int splits = 1;
+  while (splits < 16 && groups * splits * 2 <= 2 * 148 && a.nitems >= 2 * nwarps * splits * 2) splits *= 2;
+  a.x_atomic = c.xg_bcast || splits > 1 ? 1 : 0;
+  a.y_atomic = c.yg_bcast || splits > 1 ? 1 : 0;
+
   if (groups > 0x7fffffffLL) return fail(GELIB_SKIPPED, fn, "number of cells exceeds 2^31-1");
   cudaError_t e = cudaSuccess;
   const int threads = nwarps * 32;
+  const dim3 grid((unsigned)groups, (unsigned)splits);
   switch (best) {
-    case 0: e = launch_cfg<4, 4, 8, 4>(a, (unsigned)groups, threads, smem, vec, s); break;
-    case 1: e = launch_cfg<2, 2, 4, 4>(a, (unsigned)groups, threads, smem, vec, s); break;
-    case 2: e = launch_cfg<1, 2, 1, 4>(a, (unsigned)groups, threads, smem, vec, s); break;
-    case 3: e = launch_cfg<2, 1, 2, 2>(a, (unsigned)groups, threads, smem, vec, s); break;
-    default: e = launch_cfg<4, 1, 4, 1>(a, (unsigned)groups, threads, smem, vec, s); break;
+    case 0: e = launch_cfg<4, 4, 8, 4>(a, grid, threads, smem, vec, s); break;
+    case 1: e = launch_cfg<4, 2, 4, 4>(a, grid, threads, smem, vec, s); break;
+    case 2: e = launch_cfg<4, 2, 2, 2>(a, grid, threads, smem, vec, s); break;
+    case 3: e = launch_cfg<2, 2, 4, 2>(a, grid, threads, smem, vec, s); break;
+    case 4: e = launch_cfg<2, 2, 4, 4>(a, grid, threads, smem, vec, s); break;
+    case 5: e = launch_cfg<1, 2, 1, 4>(a, grid, threads, smem, vec, s); break;
+    case 6: e = launch_cfg<2, 1, 2, 2>(a, grid, threads, smem, vec, s); break;
+    default: e = launch_cfg<4, 1, 4, 1>(a, grid, threads, smem, vec, s); break;
   }
   if (e != cudaSuccess) return check_cuda(e, fn, "backward kernel launch");
   count_launch();

@@ -196,7 +196,10 @@ struct TileCfg {
 constexpr TileCfg kCfgs[] = {
     {4, 4, 8},  // 16 x 32 channels, 1 cell per warp
     {2, 4, 8},  //  8 x 32, 1 cell
+    {4, 4, 4},  // 16 x 16, 2 cells
     {1, 1, 4},  //  1 x 16, 8 cells
+    {4, 2, 2},  //  8 x  8, 8 cells
+    {2, 4, 2},  //  8 x  8, 4 cells
     {2, 2, 2},  //  4 x  8, 8 cells
     {1, 1, 1},  //  1 x  4, 32 cells
     {4, 4, 1},  // 16 x  4, 8 cells
@@ -235,15 +238,34 @@ int launch_cg_fwd(const VecCall& c, cudaStream_t s) {
     if (rc != -1) return rc;
     if (mode == kFwdTcStrict) return fail(GELIB_INVALID, fn, "the call does not qualify for the tcgen05 kernel");
   }
-  // ---- choose the lane layout: least padded work on the dominant channel counts, then the widest tile
-  int n1 = 1, n2 = 1;
-  for (const auto& p : c.x) n1 = std::max(n1, p.n);
-  for (const auto& p : c.y) n2 = std::max(n2, p.n);
+  // ---- choose the lane layout by an estimate of its time.  Per band entry a warp issues 16 multiply-adds and 2
+  // multiplies for each of its TA rows, half a load per row and about 7 others; per output row it issues 2 TA stores (4 TA
+  // of half the size without 16-byte alignment), each of which occupies the load/store unit, which four schedulers share,
+  // once per 128-byte line it touches.  The work is spread over the warps the call can fill.  Layouts differ in the padding
+  // of the channel counts, in how many multiply-adds share the loads and in how many lines a store touches.  Measured
+  // (maxl 4 x 16 channels, batch 1000): 521 us with 1 x 16 channels per warp row, 247 us with 16 x 16.
+  Schedule sched;
+  build_schedule(sig_of(c.x), sig_of(c.y), sig_of(c.r), false, false, &sched);
+  int cell_floats = 0;
+  for (auto* v : {&c.x, &c.y})
+    for (const auto& p : *v) cell_floats += 2 * (2 * p.l + 1) * (ceil_div(p.n, 4) * 4);
+  // floats; tiles may read up to 128 past the last row
+  auto smem_floats = [&](int WC) { return (size_t)cell_floats * WC + 128 + 2 * WC * kMaxParts; };
   int best = 0;
   double best_cost = 1e300;
   for (int i = 0; i < kNumCfgs; i++) {
-    const int ta = kCfgs[i].TA * kCfgs[i].WA, tb = 4 * kCfgs[i].NBL;
-    const double cost = (double)ceil_div(n1, ta) * ta * ceil_div(n2, tb) * tb;
+    const TileCfg& f = kCfgs[i];
+    const int ta = f.TA * f.WA, tb = 4 * f.NBL, wc = 32 / (f.WA * f.NBL);
+    if (smem_floats(wc) * sizeof(float) > 200 * 1024) continue;
+    const double entry = 18.5 * f.TA + 7, row = 6.0 * f.TA + 12 + 4.0 * (c.vec_ok ? 2 : 4) * f.TA * wc * f.WA;
+    double cost = 0, items = 0;
+    for (const Triple& t : sched.triples) {
+      const double tiles = (double)ceil_div(c.x[t.xi].n, ta) * ceil_div(c.y[t.yi].n, tb);
+      cost += tiles * (band_size(t.l1, t.l2, t.l) * entry + (2 * t.l + 1) * row);
+      items += tiles;
+    }
+    const double groups = (double)((c.cg.ncells + wc - 1) / wc);
+    cost *= groups / std::min(groups * std::min(64.0, std::max(4.0, items)), 148.0 * 16);
     if (cost < best_cost * 0.999) {
       best_cost = cost;
       best = i;
@@ -273,7 +295,7 @@ int launch_cg_fwd(const VecCall& c, cudaStream_t s) {
   a.ny = (int)c.y.size();
   a.nr = (int)c.r.size();
   a.cell_floats = off;
-  const size_t smem = ((size_t)off * WC + 128 + 2 * WC * kMaxParts) * sizeof(float);  // +128 floats: tiles may read past the last row
+  const size_t smem = smem_floats(WC) * sizeof(float);
   if (smem > 200 * 1024) return -1;                             // caller falls back to the strided kernel
 
   // ---- jobs: enough CTAs to fill the machine several times over
@@ -327,9 +349,12 @@ int launch_cg_fwd(const VecCall& c, cudaStream_t s) {
   switch (best) {
     case 0: e = launch_cfg<4, 4, 8>(a, grid, smem, c.vec_ok, s); break;
     case 1: e = launch_cfg<2, 4, 8>(a, grid, smem, c.vec_ok, s); break;
-    case 2: e = launch_cfg<1, 1, 4>(a, grid, smem, c.vec_ok, s); break;
-    case 3: e = launch_cfg<2, 2, 2>(a, grid, smem, c.vec_ok, s); break;
-    case 4: e = launch_cfg<1, 1, 1>(a, grid, smem, c.vec_ok, s); break;
+    case 2: e = launch_cfg<4, 4, 4>(a, grid, smem, c.vec_ok, s); break;
+    case 3: e = launch_cfg<1, 1, 4>(a, grid, smem, c.vec_ok, s); break;
+    case 4: e = launch_cfg<4, 2, 2>(a, grid, smem, c.vec_ok, s); break;
+    case 5: e = launch_cfg<2, 4, 2>(a, grid, smem, c.vec_ok, s); break;
+    case 6: e = launch_cfg<2, 2, 2>(a, grid, smem, c.vec_ok, s); break;
+    case 7: e = launch_cfg<1, 1, 1>(a, grid, smem, c.vec_ok, s); break;
     default: e = launch_cfg<4, 4, 1>(a, grid, smem, c.vec_ok, s); break;
   }
   if (e != cudaSuccess) return check_cuda(e, fn, "forward kernel launch");

@@ -12,7 +12,17 @@ from .gelib_common import common_batch
 from .SO3part import SO3part, SO3partArr
 
 
+# Inside the functions below attributes of the operands are read without the tensor classes' __torch_function__, whose
+# Python handler costs several microseconds per access: a small product is bound by the host.
+_plain = torch._C.DisableTorchFunctionSubclass
+
+
 def _vec_forward(ctx, k1, k2, maxl, args, diag, part_cls):
+    with _plain():
+        return _vec_forward_plain(ctx, k1, k2, maxl, args, diag, part_cls)
+
+
+def _vec_forward_plain(ctx, k1, k2, maxl, args, diag, part_cls):
     ctx.k1, ctx.k2, ctx.diag = k1, k2, diag
     ctx.save_for_backward(*args)
     xs, ys = [a.detach() for a in args[0:k1]], [a.detach() for a in args[k1:k1 + k2]]
@@ -35,12 +45,27 @@ def _vec_forward(ctx, k1, k2, maxl, args, diag, part_cls):
 
 
 def _vec_backward(ctx, gargs):
+    with _plain():
+        return _vec_backward_plain(ctx, gargs)
+
+
+def zeros_like_all(tensors):
+    """One zero tensor per tensor and of its class, filled by one launch."""
+    r = [torch.empty_like(t) for t in tensors]
+    if r:
+        torch._foreach_zero_(r)
+    return [z if type(t) is torch.Tensor else z.as_subclass(type(t)) for z, t in zip(r, tensors)]
+
+
+def _vec_backward_plain(ctx, gargs):
     k1, k2 = ctx.k1, ctx.k2
     saved = ctx.saved_tensors
     need = ctx.needs_input_grad[3:]
     need_x, need_y = any(need[0:k1]), any(need[k1:k1 + k2])
     # a side that needs no gradient (spherical harmonics of fixed points, say) is not computed at all
-    grads = [torch.zeros_like(t) if (need_x if i < k1 else need_y) else None for i, t in enumerate(saved)]
+    grads = [None] * len(saved)
+    first, last = 0 if need_x else k1, k1 + k2 if need_y else k1
+    grads[first:last] = zeros_like_all(saved[first:last])
     x, y = gb.SO3vec.view(list(saved[0:k1])), gb.SO3vec.view(list(saved[k1:k1 + k2]))
     g = gb.SO3vec.view([a.as_subclass(torch.Tensor) for a in gargs])
     if need_x and need_y:
@@ -163,9 +188,10 @@ class _VecBase:
 
     def __init__(self, *args):
         self.parts = {}
-        for x in args:
-            assert isinstance(x, torch.Tensor)
-            self.parts[(x.size(-2) - 1) // 2] = x
+        with _plain():
+            for x in args:
+                assert isinstance(x, torch.Tensor)
+                self.parts[(x.size(-2) - 1) // 2] = x
 
     @classmethod
     def zeros_like(cls, x):

@@ -5,8 +5,10 @@ the library are raw pointers, sizes and strides.  There is no CPU or pure-PyTorc
 the shared library is missing, importing a product fails with instructions to build it, and a
 product on CPU tensors raises.
 """
+import contextlib
 import ctypes
 import os
+import struct
 import sys
 
 import torch
@@ -144,12 +146,13 @@ def _fuse(dims, strides):
     return n, keep[-1][1]
 
 
-def descriptor(t, real=False):
-    """``gelib_tensor5`` of a torch tensor in the reference's 5-D canonical form (core/Gpart.hpp:450-469).
+# One gelib_tensor5 in native layout.  Packing it in one call and reading the tensor's attributes once is what the cost of
+# a small product is made of: a field-by-field ctypes structure took 8 us per tensor, this takes about 1.
+_TENSOR5 = struct.Struct("@P5i5q")
+assert _TENSOR5.size == ctypes.sizeof(Tensor5)
 
-    Complex tensors (b, [grid...], 2l+1, n) are viewed as interleaved floats, so strides double
-    (cuda/GPUtensor.hpp:31-38).  ``real=True`` is for the (b, [grid...], 3, n) float input of spharm.
-    """
+
+def _pack(buf, at, t, real):
     if not t.is_cuda:
         raise RuntimeError("gelib_b200 computes on CUDA tensors only (this build has no CPU path); got a %s tensor"
                            % t.device.type)
@@ -161,44 +164,59 @@ def descriptor(t, real=False):
         if t.dtype != torch.complex64:
             raise RuntimeError("expected a complex64 tensor (an SO3part)")
         scale = 2
-    d = t.dim()
+    D, S = t.shape, t.stride()
+    d = len(D)
+    if d == 3:
+        _TENSOR5.pack_into(buf, at, t.data_ptr(), D[0], 1, 1, D[1], D[2], scale * S[0], 0, 0, scale * S[1], scale * S[2])
+        return
     if d < 3:
         raise RuntimeError("an SO3part has at least 3 dimensions (batch, 2l+1, channels)")
-    dims, strides = list(t.shape), [s * scale for s in t.stride()]
-    if d == 3:
-        D = [dims[0], 1, 1, dims[1], dims[2]]
-        S = [strides[0], 0, 0, strides[1], strides[2]]
-    elif d == 4:
-        D = [dims[0], dims[1], 1, dims[2], dims[3]]
-        S = [strides[0], strides[1], 0, strides[2], strides[3]]
-    elif d == 5:
-        D, S = dims, strides
-    else:
-        g, s = _fuse(dims[1:d - 2], strides[1:d - 2])
-        D = [dims[0], g, 1, dims[d - 2], dims[d - 1]]
-        S = [strides[0], s, 0, strides[d - 2], strides[d - 1]]
+    S = [scale * s for s in S]
+    if d == 4:
+        D = (D[0], D[1], 1, D[2], D[3])
+        S = (S[0], S[1], 0, S[2], S[3])
+    elif d > 5:
+        g, s = _fuse(D[1:d - 2], S[1:d - 2])
+        D = (D[0], g, 1, D[d - 2], D[d - 1])
+        S = (S[0], s, 0, S[d - 2], S[d - 1])
+    _TENSOR5.pack_into(buf, at, t.data_ptr(), *D, *S)
+
+
+def descriptor(t, real=False):
+    """``gelib_tensor5`` of a torch tensor in the reference's 5-D canonical form (core/Gpart.hpp:450-469).
+
+    Complex tensors (b, [grid...], 2l+1, n) are viewed as interleaved floats, so strides double
+    (cuda/GPUtensor.hpp:31-38).  ``real=True`` is for the (b, [grid...], 3, n) float input of spharm.
+    """
     out = Tensor5()
-    out.base = t.data_ptr()
-    for i in range(5):
-        out.dims[i] = D[i]
-        out.strides[i] = S[i]
+    with torch._C.DisableTorchFunctionSubclass():
+        _pack(out, 0, t, real)
     return out
 
 
 def descriptor_array(tensors, real=False):
     arr = (Tensor5 * max(1, len(tensors)))()
-    for i, t in enumerate(tensors):
-        arr[i] = descriptor(t, real)
+    at = 0
+    with torch._C.DisableTorchFunctionSubclass():
+        for t in tensors:
+            _pack(arr, at, t, real)
+            at += _TENSOR5.size
     return arr
+
+
+_SAME_DEVICE = contextlib.nullcontext()
 
 
 def device_guard(t):
     """Context manager making t's device current; raises for anything that is not a CUDA tensor."""
-    if not t.is_cuda:
-        raise RuntimeError("gelib_b200 computes on CUDA tensors only (this build has no CPU path); got a %s tensor"
-                           % t.device.type)
-    return torch.cuda.device(t.device)
+    with torch._C.DisableTorchFunctionSubclass():
+        if not t.is_cuda:
+            raise RuntimeError("gelib_b200 computes on CUDA tensors only (this build has no CPU path); got a %s tensor"
+                               % t.device.type)
+        index = t.get_device()
+    return _SAME_DEVICE if torch.cuda.current_device() == index else torch.cuda.device(index)
 
 
 def stream_of(t):
-    return ctypes.c_void_p(torch.cuda.current_stream(t.device).cuda_stream)
+    with torch._C.DisableTorchFunctionSubclass():
+        return ctypes.c_void_p(torch._C._cuda_getCurrentRawStream(t.get_device()))

@@ -8,6 +8,7 @@ keyword-only or new names: ``overwrite=`` on the forward products, the fused ``*
 ``SO3vec.add_spharm``.
 """
 import ctypes
+import functools
 
 import torch
 
@@ -26,10 +27,25 @@ def _flags(overwrite, fp64):
 def _one_device(*tensors):
     """The reference asserts that the operands of a product live on one device (SO3/SO3part.hpp:351,
     core/CGproduct.hpp:47-49); here a tensor on another GPU would be dereferenced as a raw pointer."""
-    dev = tensors[0].device
-    for t in tensors:
-        if t.device != dev:
-            raise RuntimeError("GElib error: operands on different devices (%s and %s)." % (dev, t.device))
+    with torch._C.DisableTorchFunctionSubclass():
+        dev = tensors[0].device
+        for t in tensors:
+            if t.device != dev:
+                raise RuntimeError("GElib error: operands on different devices (%s and %s)." % (dev, t.device))
+
+
+@functools.lru_cache(maxsize=256)
+def _product_type(x, y, maxl, diag):
+    """((l, channels), ...) of the product of two types given the same way."""
+    xl, xn = [l for l, _ in x], [n for _, n in x]
+    yl, yn = [l for l, _ in y], [n for _, n in y]
+    cap = (max(xl) + max(yl) + 1) if xl and yl else 1
+    ol, on = (ctypes.c_int * cap)(), (ctypes.c_int * cap)()
+    k = lib().gelib_SO3type_CGproduct(len(xl), _ints(xl), _ints(xn), len(yl), _ints(yl), _ints(yn), maxl,
+                                      1 if diag else 0, cap, ol, on)
+    if k < 0:
+        raise RuntimeError("GElib error: product type does not fit")
+    return tuple((ol[i], on[i]) for i in range(k))
 
 
 class SO3type:
@@ -59,15 +75,7 @@ class SO3type:
         return dict(self.parts)
 
     def _product(self, y, maxl, diag):
-        xl, xn = list(self.parts.keys()), list(self.parts.values())
-        yl, yn = list(y.parts.keys()), list(y.parts.values())
-        cap = (max(xl) + max(yl) + 1) if xl and yl else 1
-        ol, on = (ctypes.c_int * cap)(), (ctypes.c_int * cap)()
-        k = lib().gelib_SO3type_CGproduct(len(xl), _ints(xl), _ints(xn), len(yl), _ints(yl), _ints(yn), maxl,
-                                          1 if diag else 0, cap, ol, on)
-        if k < 0:
-            raise RuntimeError("GElib error: product type does not fit")
-        return SO3type({ol[i]: on[i] for i in range(k)})
+        return SO3type(dict(_product_type(tuple(self.parts.items()), tuple(y.parts.items()), maxl, diag)))
 
     def CGproduct(self, y, maxl=-1):
         return self._product(y, maxl, False)
@@ -329,10 +337,12 @@ class SO3vec:
     def view(parts):
         if isinstance(parts, dict):
             return SO3vec(dict(sorted((int(l), t) for l, t in parts.items())))
-        return SO3vec(dict(sorted(((t.size(-2) - 1) // 2, t) for t in parts)))
+        with torch._C.DisableTorchFunctionSubclass():
+            return SO3vec(dict(sorted(((t.size(-2) - 1) // 2, t) for t in parts)))
 
     def get_tau(self):
-        return SO3type({l: t.size(-1) for l, t in self.parts.items()})
+        with torch._C.DisableTorchFunctionSubclass():
+            return SO3type({l: t.size(-1) for l, t in self.parts.items()})
 
     def _tensors(self):
         return list(self.parts.values())

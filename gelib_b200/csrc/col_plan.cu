@@ -277,25 +277,6 @@ bool col_setup(const VecCall& c, bool backward, int warps_resident, ColArgs* a, 
     }
   if (max_la > kColMaxLa || max_lb > 40) return false;
   plan->max_la = max_la;
-  // Calls that the other kernels do faster (measured, us, other kernel / this one):
-  //   diagonal forward: with l >= 6 and full 64-channel slices diag_fwd_cell_kernel, which shares its operands between the
-  //     warps of a block, fits more warps on an SM: maxl 8 x 128 channels, batch 2048 3018 / 3820; maxl 6 x 64 608 / 835,
-  //     maxl 6 x 128 1208 / 1265; but maxl 5 x 128 711 / 661, maxl 8 x 48, batch 1000 821 / 652.
-  //   one-channel x: cg_narrow_fwd_kernel when it fills the chip and wastes no lanes (its rows are padded to a power of two):
-  //     30000 cells, maxl 4 x 32 channels 900 / 1174; 16000, maxl 6 x 16 1274 / 1362; but 4096 cells 467 / 367, 1000 cells
-  //     357 / 151; 40000 cells, maxl 6 x 24 5043 / 4281.
-  //   its gradient of y: cg_narrow1_bwd_kernel under the same conditions and l >= 6: 65536 cells, maxl 6 x 16 5418 / 5609;
-  //     but maxl 4 x 32, 5000 cells 356 / 331; 60000 cells, maxl 2 x 16 247 / 189; 4096 cells, maxl 6 x 16 638 / 370.
-  if (c.diag) {
-    const int slices = (n + 63) / 64;
-    if (!backward && max_la >= 6 && 8 * n >= 7 * 64 * slices) return false;
-  } else if (n > 1 && n <= 32) {
-    int cw = 1;
-    while (cw < n) cw *= 2;
-    const long long narrow_warps = c.cg.ncells * cw / 32;
-    if (!backward && narrow_warps >= 148 * 16 && !(max_la >= 4 && 4 * n <= 3 * cw)) return false;
-    if (backward && narrow1_enabled() && narrow_warps >= 148 * 32 && max_la >= 6 && 4 * n > 3 * cw) return false;
-  }
   const int max_rows = backward ? kColBlockBwd : kColBlockFwd;
   plan->max_block = 2 * max_la + 1 <= max_rows ? 2 * max_la + 1 : max_rows;
   a->b_rows = 2 * max_lb + 1;
@@ -322,6 +303,27 @@ bool col_setup(const VecCall& c, bool backward, int warps_resident, ColArgs* a, 
   // two columns share the records, coefficients and control of a step; with few columns warps matter more
   const long long columns = c.cg.ncells * n;
   plan->cpl = two && columns >= 64 * 148 * 4 ? 2 : 1;
+  // Calls that the other kernels do faster (measured, us, other kernel / this one):
+  //   diagonal forward: with l >= 6 and full 64-channel slices diag_fwd_cell_kernel, which shares its operands between the
+  //     warps of a block, fits more warps on an SM: maxl 8 x 128 channels, batch 2048 3018 / 3820; maxl 6 x 64 608 / 835,
+  //     maxl 6 x 128 1208 / 1265; but maxl 5 x 128 711 / 661, maxl 8 x 48, batch 1000 821 / 652.
+  //   one-channel x: cg_narrow_fwd_kernel when it fills the chip and wastes no lanes (its rows are padded to a power of two):
+  //     30000 cells, maxl 4 x 32 channels 900 / 1174; 16000, maxl 6 x 16 1274 / 1362; but 4096 cells 467 / 367, 1000 cells
+  //     357 / 151; 40000 cells, maxl 6 x 24 5043 / 4281.
+  //   its gradient of y: cg_narrow1_bwd_kernel under the same conditions and l >= 6: 65536 cells, maxl 6 x 16 5418 / 5609;
+  //     but maxl 4 x 32, 5000 cells 356 / 331; 60000 cells, maxl 2 x 16 247 / 189; 4096 cells, maxl 6 x 16 638 / 370.
+  // One column per lane (an odd channel count) does without what two share, so padding has to cost more before these win.
+  if (c.diag) {
+    const int slices = (n + 63) / 64;
+    if (!backward && max_la >= 6 && 8 * n >= 7 * 64 * slices) return false;
+  } else if (n > 1 && n <= 32) {
+    int cw = 1;
+    while (cw < n) cw *= 2;
+    const long long narrow_warps = c.cg.ncells * cw / 32;
+    const bool padded = plan->cpl == 2 ? 4 * n <= 3 * cw : 5 * n <= 3 * cw;
+    if (!backward && narrow_warps >= 148 * 16 && !(max_la >= 4 && padded)) return false;
+    if (backward && narrow1_enabled() && narrow_warps >= 148 * 32 && (max_la >= 6 || plan->cpl == 1) && !padded) return false;
+  }
   a->ch_stride[0] = x_shared ? 0 : 8 * plan->cpl;
   a->ch_stride[1] = a->ch_stride[2] = 8 * plan->cpl;
   a->nx = (int)c.x.size();

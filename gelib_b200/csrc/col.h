@@ -22,9 +22,9 @@
 // multiply-adds) is copied to shared memory one chunk ahead.
 // Why this form: diag_bwd_cell_kernel spends its time in four shared-memory atomics (compare-and-swap loops) per band
 // entry, which a lane that owns its column does not need.  Measured, backward of the diagonal product: maxl 8 x 128
-// channels, batch 2048 10.5 -> 5.9 ms; maxl 6 x 33, batch 4000 4.3 -> 1.1 ms; maxl 3 x 12, batch 500 49 -> 18 us (forward 32 ->
-// 15 us).  Bound by instruction issue at two to three warps per scheduler: 475 k warp instructions per 64 columns at maxl
-// 8, 0.33 issued per cycle, the largest stalls instruction fetch (the unrolled bodies) and fixed-latency dependencies.
+// channels, batch 2048 10.5 -> 4.8 ms; maxl 6 x 33, batch 4000 4.3 -> 1.1 ms; maxl 3 x 12, batch 500 49 -> 18 us (forward 32 ->
+// 15 us).  Bound by instruction issue at two to three warps per scheduler: about 475 k warp instructions per 64 columns at
+// maxl 8; the largest stalls are instruction fetch (the unrolled bodies) and fixed-latency dependencies.
 #pragma once
 #include "plan.h"
 
@@ -33,11 +33,20 @@ namespace gelib_b200 {
 constexpr int kColRing = 16;                    // rows in flight per warp (a power of two)
 constexpr int kColMaxNl = 10;                   // output l per step; pairs with more are walked twice
 constexpr int kColMaxLa = 8;                    // largest l of an a side
-constexpr int kColBlockBwd = 11;                // a rows per block, backward (registers: a, its gradient, the window)
+constexpr int kColBlockBwd = 11;                // a rows per block, one gradient (registers: a or its gradient, the window)
+constexpr int kColBlockBoth = 11;               // a rows per block, both gradients
 constexpr int kColBlockFwd = 17;                // a rows per block, forward
 constexpr int kColChunkBytes = 13312;           // capacity of a chunk buffer
 constexpr int kColMaxSmem = 232448;
 constexpr int kColSlots = 3 * kMaxParts;        // x parts, y parts, r (g) parts
+
+// Output l that a step of nl is worked on with (zero coefficients beyond nl): the body of a step is instantiated per block
+// size and for each of these numbers.  With both gradients the bodies are long and fetching them is what costs most, so
+// large blocks have two instances, 6 and 10, that stay in the instruction cache: maxl 8 x 128 channels, batch 2048 5.9 ms
+// with 2, 4, .. 10, 4.8 ms with 6 and 10, 5.3 ms with 10 alone.  With one gradient, or
+// forward, the added multiply-adds cost more than that: one-channel x, maxl 4 x 32, 30000 cells 1.33 against 1.45 ms;
+// forward, maxl 8 x 128 3.8 against 4.3 ms.
+constexpr int col_nl_padded(int nl, int kb, bool both) { return !both || kb < 6 ? (nl + 1) / 2 * 2 : nl <= 6 ? 6 : 10; }
 
 // Row (slot, v) of a column: base + v * unit + cell * cell_stride + channel * ch_stride, all in bytes.
 struct ColPart {

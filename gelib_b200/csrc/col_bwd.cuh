@@ -21,7 +21,7 @@ __device__ __forceinline__ Row<CPL> to_row(const float2 (&v)[CPL]) {
 }
 
 // One step: an output row of a pair against the a block.  Entry i pairs a[i] with the b row at bptr - i rows.
-template <int K, int CPL, bool DOA, bool DOB, int NL>
+template <int K, int CPL, bool DOA, bool DOB, int NL, int NLMIN = NL - 1>
 __device__ __forceinline__ void bwd_step(Walk<CPL>& W, int st, const float2 (&a)[K][CPL], float2 (&ag)[K][CPL], float2 (&bg)[K][CPL],
                                          uint32_t bptr) {
   cp_wait<kColRing - NL>();
@@ -31,7 +31,7 @@ __device__ __forceinline__ void bwd_step(Walk<CPL>& W, int st, const float2 (&a)
   for (int j = 0; j < NL; j++) {
     const Row<CPL> r = W.row(j);
 #pragma unroll
-    for (int c = 0; c < CPL; c++) g[j][c] = j < NL - 1 || nl == NL ? r.c[c] : 0ull;  // beyond nl: a row of a later step
+    for (int c = 0; c < CPL; c++) g[j][c] = j < NLMIN || j < nl ? r.c[c] : 0ull;  // beyond nl: a row of a later step
   }
   W.template refill<NL>(nl);
   const unsigned span = hi - lo;
@@ -108,13 +108,18 @@ __device__ __forceinline__ void bwd_segment(Walk<CPL>& W, const int4 h, int lb, 
   for (int s = 0; s < nsteps; s++, br++) {
     const int st = next;
     next = *reinterpret_cast<const int*>(W.smem + steps + 4 * s + 4);  // past the last one: another word of the chunk
-    const int nl2 = ((st & 255) + 1) >> 1;
     const uint32_t bptr = bval + kRow * br;
-    if (nl2 == 1) bwd_step<K, CPL, DOA, DOB, 2>(W, st, a, ag, bg, bptr);
-    if constexpr (NLMAX >= 4) if (nl2 == 2) bwd_step<K, CPL, DOA, DOB, 4>(W, st, a, ag, bg, bptr);
-    if constexpr (NLMAX >= 6) if (nl2 == 3) bwd_step<K, CPL, DOA, DOB, 6>(W, st, a, ag, bg, bptr);
-    if constexpr (NLMAX >= 8) if (nl2 == 4) bwd_step<K, CPL, DOA, DOB, 8>(W, st, a, ag, bg, bptr);
-    if constexpr (NLMAX >= 10) if (nl2 == 5) bwd_step<K, CPL, DOA, DOB, 10>(W, st, a, ag, bg, bptr);
+    const int nl = st & 255, nl2 = (nl + 1) >> 1;
+    if constexpr (DOA && DOB && K >= 6) {  // the instances of col_nl_padded
+      if (nl <= 6) bwd_step<K, CPL, DOA, DOB, 6, 1>(W, st, a, ag, bg, bptr);
+      else bwd_step<K, CPL, DOA, DOB, 10, 7>(W, st, a, ag, bg, bptr);
+    } else {
+      if (nl2 == 1) bwd_step<K, CPL, DOA, DOB, 2>(W, st, a, ag, bg, bptr);
+      if constexpr (NLMAX >= 4) if (nl2 == 2) bwd_step<K, CPL, DOA, DOB, 4>(W, st, a, ag, bg, bptr);
+      if constexpr (NLMAX >= 6) if (nl2 == 3) bwd_step<K, CPL, DOA, DOB, 6>(W, st, a, ag, bg, bptr);
+      if constexpr (NLMAX >= 8) if (nl2 == 4) bwd_step<K, CPL, DOA, DOB, 8>(W, st, a, ag, bg, bptr);
+      if constexpr (NLMAX >= 10) if (nl2 == 5) bwd_step<K, CPL, DOA, DOB, 10>(W, st, a, ag, bg, bptr);
+    }
     if (DOB) {  // the row that leaves the window, then the window moves by one row
       leave(br - (K - 1), bg[K - 1]);
 #pragma unroll
@@ -211,9 +216,10 @@ cudaError_t launch_bwd(const ColArgs& a, cudaStream_t s) {
 
 template <bool DOX, bool DOY>
 cudaError_t launch_bwd_k(const ColArgs& a, const ColPlan& p, cudaStream_t s) {
-  if (p.cpl == 1) return launch_bwd<11, 1, DOX, DOY, 384>(a, s);
+  constexpr int KMAX = DOX && DOY ? kColBlockBoth : kColBlockBwd;
+  if (p.cpl == 1) return launch_bwd<KMAX, 1, DOX, DOY, 384>(a, s);
   if (p.max_block <= 5) return launch_bwd<5, 2, DOX, DOY, 512>(a, s);
-  return launch_bwd<11, 2, DOX, DOY, 256>(a, s);
+  return launch_bwd<KMAX, 2, DOX, DOY, 256>(a, s);
 }
 
 }  // namespace col

@@ -36,13 +36,12 @@ struct Segment {
   double cost = 0;
 };
 
-int nl_padded(int nl) { return (nl + 1) / 2 * 2; }
-
 struct Builder {
   const std::vector<PartSig>& rs;
   bool backward, do_x, do_y;
   std::vector<int2> rows;  // the stream, in order of use
 
+  int nlp(int nl, int kb) const { return col_nl_padded(nl, kb, backward && do_x && do_y); }
   bool do_a(int half) const { return backward && (half == 0 ? do_x : do_y); }
   bool do_b(int half) const { return backward && (half == 0 ? do_y : do_x); }
   bool need_a(int half) const { return !backward || do_b(half); }
@@ -69,7 +68,7 @@ struct Builder {
     rows.resize(n0);
     int u = 2 + ((int)s.steps.size() + 3) / 4;
     for (const Step& st : s.steps) {
-      u += s.kb * nl_padded(st.nl) / 2;
+      u += s.kb * nlp(st.nl, s.kb) / 2;
       if (!backward) *recs += st.nl;
     }
     return u + *recs;
@@ -82,7 +81,7 @@ void build(DevicePlan& p, const std::vector<PartSig>& xs, const std::vector<Part
   Builder B{rs, backward, do_x, do_y};
   std::map<std::pair<int, int>, std::vector<const Triple*>> pairs;
   for (const Triple& t : p.sched.triples) pairs[{t.xi, t.yi}].push_back(&t);
-  const int cap = kColChunkBytes / 16, max_block = backward ? kColBlockBwd : kColBlockFwd;
+  const int cap = kColChunkBytes / 16, max_block = !backward ? kColBlockFwd : do_x && do_y ? kColBlockBoth : kColBlockBwd;
 
   // all segments in order: half, b part, a part, block of a rows, group of l, piece of m
   std::vector<Segment> all;
@@ -116,7 +115,7 @@ void build(DevicePlan& p, const std::vector<PartSig>& xs, const std::vector<Part
               Step st{m, 0, std::max(0, m - lb - mlo), std::min(kb - 1, m + lb - mlo)};
               for (const Triple* t : s.ls) st.nl += t->l >= std::abs(m);
               if (st.hi < st.lo || st.nl == 0) continue;
-              const int need = 1 + kb * nl_padded(st.nl) / 2 + st.nl;
+              const int need = 1 + kb * B.nlp(st.nl, kb) / 2 + st.nl;
               if (need > room || s.steps.empty() || st.m != s.steps.back().m + 1) {  // a new piece
                 if (!s.steps.empty()) all.push_back(s);
                 s.steps.clear();
@@ -219,7 +218,7 @@ void build(DevicePlan& p, const std::vector<PartSig>& xs, const std::vector<Part
         const Segment& s = run[q];
         for (const Step& st : s.steps)
           for (int i = 0; i < s.kb; i++)
-            for (int j = 0; j < nl_padded(st.nl); j++) {
+            for (int j = 0; j < B.nlp(st.nl, s.kb); j++) {
               float x = 0.f;
               if (i >= st.lo && i <= st.hi && j < st.nl) {
                 const Triple& t = *s.ls[s.ls.size() - st.nl + j];
@@ -277,7 +276,7 @@ bool col_setup(const VecCall& c, bool backward, int warps_resident, ColArgs* a, 
     }
   if (max_la > kColMaxLa || max_lb > 40) return false;
   plan->max_la = max_la;
-  const int max_rows = backward ? kColBlockBwd : kColBlockFwd;
+  const int max_rows = !backward ? kColBlockFwd : do_x && do_y ? kColBlockBoth : kColBlockBwd;
   plan->max_block = 2 * max_la + 1 <= max_rows ? 2 * max_la + 1 : max_rows;
   a->b_rows = 2 * max_lb + 1;
   for (size_t i = 0; i < c.x.size(); i++)

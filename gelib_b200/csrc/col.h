@@ -20,6 +20,10 @@
 // the k rows that come kColRing later, so the bytes in flight do not depend on how short the steps are.  What the warps
 // of a block share is the walk itself: a chunk (row addresses, step records, coefficients stored twice for the packed
 // multiply-adds) is copied to shared memory one chunk ahead.
+// Gradient rows are added to global memory with red.  A row belongs to one lane of one block, so the sums have one order and
+// gradients are bitwise repeatable, except those of an operand that is broadcast over cells (stride 0).  Calls with few
+// columns split the walk over blocks; in the backward each of these takes everything that is added to one a block's rows
+// (an "owned" run, in which either part of a pair may be the larger one).
 // Why this form: diag_bwd_cell_kernel spends its time in four shared-memory atomics (compare-and-swap loops) per band
 // entry, which a lane that owns its column does not need.  Measured, backward of the diagonal product: maxl 8 x 128
 // channels, batch 2048 10.5 -> 4.8 ms; maxl 6 x 33, batch 4000 4.3 -> 1.1 ms; maxl 3 x 12, batch 500 49 -> 18 us (forward 32 ->
@@ -33,8 +37,7 @@ namespace gelib_b200 {
 constexpr int kColRing = 16;                    // rows in flight per warp (a power of two)
 constexpr int kColMaxNl = 10;                   // output l per step; pairs with more are walked twice
 constexpr int kColMaxLa = 8;                    // largest l of an a side
-constexpr int kColBlockBwd = 11;                // a rows per block, one gradient (registers: a or its gradient, the window)
-constexpr int kColBlockBoth = 11;               // a rows per block, both gradients
+constexpr int kColBlockBwd = 11;                // a rows per block, backward (registers: a and its gradient, the window)
 constexpr int kColBlockFwd = 17;                // a rows per block, forward
 constexpr int kColChunkBytes = 13312;           // capacity of a chunk buffer
 constexpr int kColMaxSmem = 232448;
@@ -73,6 +76,7 @@ struct ColPlan {
   int max_la;     // largest l of an a side
   int max_block;  // a rows of the largest block
   int cpl;        // columns per lane
+  bool owned;     // backward with few columns: one run per a block
 };
 
 // Bits of a segment record.
@@ -89,6 +93,6 @@ inline int col_block_warps(unsigned warps, int splits, int most) {
 
 // Returns false when the call is not one the column kernels take; otherwise fills args and
 // plan (plan->dev == nullptr on a CUDA error).
-bool col_setup(const VecCall& c, bool backward, int warps_resident, ColArgs* a, ColPlan* plan);
+bool col_setup(const VecCall& c, bool backward, ColArgs* a, ColPlan* plan);
 
 }  // namespace gelib_b200

@@ -144,14 +144,15 @@ __device__ __forceinline__ void bwd_segment(Walk<CPL>& W, const int4 h, int lb, 
   }
 }
 
-template <int KMAX, int CPL, bool DOX, bool DOY, int THREADS>
+// OWNED: a run of the walk holds everything that is added to the rows of one a block, and only those are computed.
+template <int KMAX, int CPL, bool DOX, bool DOY, int THREADS, bool OWNED>
 __global__ void __launch_bounds__(THREADS, 1) col_bwd_kernel(const __grid_constant__ ColArgs A) {
   extern __shared__ __align__(16) unsigned char smem[];
-  constexpr uint32_t kRow = Walk<CPL>::kRow;
+  constexpr uint32_t kRow = Walk<CPL>::kRow, kSets = OWNED ? 1 : 2;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nwarps = blockDim.x >> 5;
-  // [part table][two chunk buffers][rings][b rows and their gradients, per warp]
+  // [part table][two chunk buffers][rings][b rows and, unless OWNED, their gradients, per warp]
   const uint32_t bufs = 16 * kColSlots, rings = bufs + 2 * kColChunkBytes, slots = rings + nwarps * Walk<CPL>::kRing;
-  const uint32_t bval = slots + warp * 2 * kRow * A.b_rows + 8 * CPL * lane, bacc = bval + kRow * A.b_rows;
+  const uint32_t bval = slots + warp * kSets * kRow * A.b_rows + 8 * CPL * lane, bacc = bval + kRow * A.b_rows;
   Walk<CPL> W(A, smem);
   W.set_lane((blockIdx.x * nwarps + warp) * 32 + lane);
   W.start(0, bufs, rings + warp * Walk<CPL>::kRing);
@@ -161,7 +162,7 @@ __global__ void __launch_bounds__(THREADS, 1) col_bwd_kernel(const __grid_consta
     const int kb = h.x & 255, nb = 2 * h1.y + 1;
     f = (h.x >> 8) & 255;
     const bool half1 = (f & kColHalf1) != 0;
-    const bool do_a = half1 ? DOY : DOX, do_b = half1 ? DOX : DOY;
+    const bool do_a = OWNED || (half1 ? DOY : DOX), do_b = !OWNED && (half1 ? DOX : DOY);
     if (f & kColFirstOfB) {
       if (do_a) W.take_to(bval, nb);
       if (do_b) {
@@ -174,7 +175,8 @@ __global__ void __launch_bounds__(THREADS, 1) col_bwd_kernel(const __grid_consta
 #define GELIB_COL_CASE(N)                                                                        \
   if constexpr (N <= KMAX)                                                                       \
     if (kb == N) {                                                                               \
-      if (DOX == DOY || !half1) bwd_segment<N, CPL, DOX, DOY>(W, h, h1.y, bval, bacc);           \
+      if constexpr (OWNED) bwd_segment<N, CPL, true, false>(W, h, h1.y, bval, bacc);             \
+      else if (DOX == DOY || !half1) bwd_segment<N, CPL, DOX, DOY>(W, h, h1.y, bval, bacc);      \
       else bwd_segment<N, CPL, DOY, DOX>(W, h, h1.y, bval, bacc);                                \
     }
     if (kb <= 5) {
@@ -200,14 +202,15 @@ __global__ void __launch_bounds__(THREADS, 1) col_bwd_kernel(const __grid_consta
   cp_wait<0>();
 }
 
-template <int KMAX, int CPL, bool DOX, bool DOY, int THREADS>
+template <int KMAX, int CPL, bool DOX, bool DOY, int THREADS, bool OWNED = false>
 cudaError_t launch_bwd(const ColArgs& a, cudaStream_t s) {
-  const size_t fixed = 16 * kColSlots + 2 * kColChunkBytes, per_warp = Walk<CPL>::kRow * (kColRing + 2 * (size_t)a.b_rows);
+  const size_t fixed = 16 * kColSlots + 2 * kColChunkBytes;
+  const size_t per_warp = Walk<CPL>::kRow * (kColRing + (OWNED ? 1 : 2) * (size_t)a.b_rows);
   const unsigned warps = (a.nlanes + 31) / 32;
   int nw = (int)std::min<size_t>(THREADS / 32, (kColMaxSmem - fixed) / per_warp);
   nw = col_block_warps(warps, a.nsplits, nw);
   const size_t smem = fixed + nw * per_warp;
-  auto k = col_bwd_kernel<KMAX, CPL, DOX, DOY, THREADS>;
+  auto k = col_bwd_kernel<KMAX, CPL, DOX, DOY, THREADS, OWNED>;
   cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e != cudaSuccess) return e;
   k<<<dim3((warps + nw - 1) / nw, a.nsplits), nw * 32, smem, s>>>(a);
@@ -216,10 +219,9 @@ cudaError_t launch_bwd(const ColArgs& a, cudaStream_t s) {
 
 template <bool DOX, bool DOY>
 cudaError_t launch_bwd_k(const ColArgs& a, const ColPlan& p, cudaStream_t s) {
-  constexpr int KMAX = DOX && DOY ? kColBlockBoth : kColBlockBwd;
-  if (p.cpl == 1) return launch_bwd<KMAX, 1, DOX, DOY, 384>(a, s);
+  if (p.cpl == 1) return launch_bwd<kColBlockBwd, 1, DOX, DOY, 384>(a, s);
   if (p.max_block <= 5) return launch_bwd<5, 2, DOX, DOY, 512>(a, s);
-  return launch_bwd<KMAX, 2, DOX, DOY, 256>(a, s);
+  return launch_bwd<kColBlockBwd, 2, DOX, DOY, 256>(a, s);
 }
 
 }  // namespace col

@@ -160,7 +160,7 @@ int launch_col_fwd(const VecCall& c, cudaStream_t s) {
   static const char* fn = "SO3vec_addCGproduct";
   ColArgs a;
   ColPlan plan;
-  if (!col_setup(c, false, 148 * 12, &a, &plan)) return -1;
+  if (!col_setup(c, false, &a, &plan)) return -1;
   if (!plan.dev) return GELIB_CUDA_ERROR;
   if (a.nsplits == 0) return GELIB_OK;
   cudaError_t e;

@@ -38,12 +38,12 @@ struct Segment {
 
 struct Builder {
   const std::vector<PartSig>& rs;
-  bool backward, do_x, do_y;
+  bool backward, do_x, do_y, owned;
   std::vector<int2> rows;  // the stream, in order of use
 
-  int nlp(int nl, int kb) const { return col_nl_padded(nl, kb, backward && do_x && do_y); }
-  bool do_a(int half) const { return backward && (half == 0 ? do_x : do_y); }
-  bool do_b(int half) const { return backward && (half == 0 ? do_y : do_x); }
+  int nlp(int nl, int kb) const { return col_nl_padded(nl, kb, backward && do_x && do_y && !owned); }
+  bool do_a(int half) const { return backward && (owned || (half == 0 ? do_x : do_y)); }
+  bool do_b(int half) const { return backward && !owned && (half == 0 ? do_y : do_x); }
   bool need_a(int half) const { return !backward || do_b(half); }
   bool need_b(int half) const { return !backward || do_a(half); }
 
@@ -75,78 +75,137 @@ struct Builder {
   }
 };
 
+// Block sizes that the bodies are instantiated for (col_bwd.cuh, col_fwd.cu).
+std::vector<int> a_blocks(int rows, int most) {
+  std::vector<int> v;
+  if (rows <= 17) {  // sizes that differ by at most one
+    const int n = (rows + most - 1) / most;
+    for (int k = 0; k < n; k++) v.push_back((rows + n - 1 - k) / n);
+    return v;
+  }
+  // an a part with l > 8, on owned walks only: elevens, and what they leave in sizes of six rows and more (smaller bodies
+  // only hold the output l of a part that is no larger than they are)
+  static const std::vector<int> ends[11] = {{}, {6, 6}, {7, 6}, {7, 7}, {8, 7}, {8, 8}, {6}, {7}, {8}, {9}, {7, 7, 7}};
+  const std::vector<int>& end = ends[rows % 11];
+  v.assign(rows / 11 - (end.size() > 1 ? 1 : 0), 11);
+  v.insert(v.end(), end.begin(), end.end());
+  return v;
+}
+
+// The segments of a pair for one block of a rows: groups of l, pieces of m.
+void pair_segments(const Builder& B, const std::vector<const Triple*>& ts, Segment s, std::vector<Segment>* out) {
+  const int cap = kColChunkBytes / 16;
+  for (size_t g0 = 0; g0 < ts.size(); g0 += kColMaxNl) {
+    s.steps.clear();
+    s.cost = 0;
+    s.ls.assign(ts.begin() + g0, ts.begin() + std::min(ts.size(), g0 + kColMaxNl));
+    int room = 0;
+    for (int m = -s.ls.back()->l; m <= s.ls.back()->l; m++) {
+      Step st{m, 0, std::max(0, m - s.lb - s.mlo), std::min(s.kb - 1, m + s.lb - s.mlo)};
+      for (const Triple* t : s.ls) st.nl += t->l >= std::abs(m);
+      if (st.hi < st.lo || st.nl == 0) continue;
+      const int need = 1 + s.kb * B.nlp(st.nl, s.kb) / 2 + st.nl;
+      if (need > room || s.steps.empty() || st.m != s.steps.back().m + 1) {  // a new piece
+        if (!s.steps.empty()) out->push_back(s);
+        s.steps.clear();
+        s.cost = 0;
+        room = cap - 4 - s.kb - (2 * s.lb + 1) - 1;
+      }
+      room -= need;
+      s.cost += (st.hi - st.lo + 1) * (1.5 * st.nl + 9) + 60 + 8 * st.nl;
+      s.steps.push_back(st);
+    }
+    if (!s.steps.empty()) out->push_back(s);
+  }
+}
+
+double cost_of(const std::vector<Segment>& v) {
+  double c = 0;
+  for (const auto& s : v) c += s.cost;
+  return c;
+}
+
 void build(DevicePlan& p, const std::vector<PartSig>& xs, const std::vector<PartSig>& ys, const std::vector<PartSig>& rs,
-           bool diag, bool backward, bool do_x, bool do_y, int splits) {
+           bool diag, bool backward, bool do_x, bool do_y, int splits, bool owned) {
   build_schedule(xs, ys, rs, diag, false, &p.sched);
-  Builder B{rs, backward, do_x, do_y};
+  Builder B{rs, backward, do_x, do_y, owned};
   std::map<std::pair<int, int>, std::vector<const Triple*>> pairs;
   for (const Triple& t : p.sched.triples) pairs[{t.xi, t.yi}].push_back(&t);
-  const int cap = kColChunkBytes / 16, max_block = !backward ? kColBlockFwd : do_x && do_y ? kColBlockBoth : kColBlockBwd;
+  for (auto& kv : pairs)
+    std::sort(kv.second.begin(), kv.second.end(), [](const Triple* u, const Triple* v) { return u->l < v->l; });
+  const int cap = kColChunkBytes / 16, max_block = backward ? kColBlockBwd : kColBlockFwd;
+  auto segment = [&](int half, int ai, int bi) {
+    Segment s;
+    s.half = half;
+    s.ai = ai;
+    s.bi = bi;
+    s.la = (half == 0 ? xs : ys)[ai].l;
+    s.lb = (half == 0 ? ys : xs)[bi].l;
+    return s;
+  };
+  auto triples = [&](int half, int ai, int bi) -> const std::vector<const Triple*>* {
+    const auto it = pairs.find(half == 0 ? std::make_pair(ai, bi) : std::make_pair(bi, ai));
+    return it == pairs.end() ? nullptr : &it->second;
+  };
 
-  // all segments in order: half, b part, a part, block of a rows, group of l, piece of m
-  std::vector<Segment> all;
-  for (int half = 0; half < 2; half++) {
-    const auto& as = half == 0 ? xs : ys;
-    const auto& bs = half == 0 ? ys : xs;
-    for (size_t bi = 0; bi < bs.size(); bi++)
-      for (size_t ai = 0; ai < as.size(); ai++) {
-        const int la = as[ai].l, lb = bs[bi].l;
-        if (half == 0 ? la > lb : la >= lb) continue;
-        const auto it = pairs.find(half == 0 ? std::make_pair((int)ai, (int)bi) : std::make_pair((int)bi, (int)ai));
-        if (it == pairs.end()) continue;
-        std::vector<const Triple*> ts = it->second;
-        std::sort(ts.begin(), ts.end(), [](const Triple* u, const Triple* v) { return u->l < v->l; });
-        const int nblocks = (2 * la + max_block) / max_block;
-        int mlo = -la;
-        for (int k = 0; k < nblocks; k++) {
-          const int kb = (2 * la + 1 + nblocks - 1 - k) / nblocks;  // sizes that differ by at most one
-          for (size_t g0 = 0; g0 < ts.size(); g0 += kColMaxNl) {
-            Segment s;
-            s.half = half;
-            s.ai = (int)ai;
-            s.bi = (int)bi;
-            s.la = la;
-            s.lb = lb;
+  std::vector<std::vector<Segment>> runs;
+  if (owned) {
+    // a run per block of rows of a part whose gradient is wanted: every pair of that part, with it as the a side
+    for (int half = 0; half < 2; half++) {
+      if (half == 0 ? !do_x : !do_y) continue;
+      const auto& as = half == 0 ? xs : ys;
+      const auto& bs = half == 0 ? ys : xs;
+      for (int ai = 0; ai < (int)as.size(); ai++) {
+        int mlo = -as[ai].l;
+        for (int kb : a_blocks(2 * as[ai].l + 1, max_block)) {
+          std::vector<Segment> run;
+          for (int bi = 0; bi < (int)bs.size(); bi++) {
+            const auto* ts = triples(half, ai, bi);
+            if (!ts) continue;
+            Segment s = segment(half, ai, bi);
             s.mlo = mlo;
             s.kb = kb;
-            s.ls.assign(ts.begin() + g0, ts.begin() + std::min(ts.size(), g0 + kColMaxNl));
-            int room = 0;
-            for (int m = -s.ls.back()->l; m <= s.ls.back()->l; m++) {
-              Step st{m, 0, std::max(0, m - lb - mlo), std::min(kb - 1, m + lb - mlo)};
-              for (const Triple* t : s.ls) st.nl += t->l >= std::abs(m);
-              if (st.hi < st.lo || st.nl == 0) continue;
-              const int need = 1 + kb * B.nlp(st.nl, kb) / 2 + st.nl;
-              if (need > room || s.steps.empty() || st.m != s.steps.back().m + 1) {  // a new piece
-                if (!s.steps.empty()) all.push_back(s);
-                s.steps.clear();
-                s.cost = 0;
-                room = cap - 4 - kb - (2 * lb + 1) - 1;
-              }
-              room -= need;
-              s.cost += (st.hi - st.lo + 1) * (1.5 * st.nl + 9) + 60 + 8 * st.nl;
-              s.steps.push_back(st);
-            }
-            if (!s.steps.empty()) all.push_back(s);
+            pair_segments(B, *ts, s, &run);
           }
           mlo += kb;
+          if (!run.empty()) runs.push_back(std::move(run));
         }
       }
-  }
-  double total = 0;
-  for (const auto& s : all) total += s.cost;
-
-  // splits: contiguous runs of about equal cost
-  std::vector<std::vector<Segment>> runs;
-  double done = 0;
-  size_t next = 0;
-  for (int sp = 0; sp < splits && next < all.size(); sp++) {
-    std::vector<Segment> run;
-    const double until = total * (sp + 1) / splits;
-    while (next < all.size() && (run.empty() || sp + 1 == splits || done + 0.5 * all[next].cost <= until)) {
-      done += all[next].cost;
-      run.push_back(all[next++]);
     }
-    runs.push_back(std::move(run));
+    std::stable_sort(runs.begin(), runs.end(),  // the longest start first
+                     [](const std::vector<Segment>& u, const std::vector<Segment>& v) { return cost_of(u) > cost_of(v); });
+  } else {
+    // all segments in order: half, b part, a part, block of a rows, group of l, piece of m
+    std::vector<Segment> all;
+    for (int half = 0; half < 2; half++) {
+      const auto& as = half == 0 ? xs : ys;
+      const auto& bs = half == 0 ? ys : xs;
+      for (int bi = 0; bi < (int)bs.size(); bi++)
+        for (int ai = 0; ai < (int)as.size(); ai++) {
+          const auto* ts = triples(half, ai, bi);
+          Segment s = segment(half, ai, bi);
+          if (!ts || (half == 0 ? s.la > s.lb : s.la >= s.lb)) continue;
+          s.mlo = -s.la;
+          for (int kb : a_blocks(2 * s.la + 1, max_block)) {
+            s.kb = kb;
+            pair_segments(B, *ts, s, &all);
+            s.mlo += kb;
+          }
+        }
+    }
+    // splits: contiguous runs of about equal cost
+    const double total = cost_of(all);
+    double done = 0;
+    size_t next = 0;
+    for (int sp = 0; sp < splits && next < all.size(); sp++) {
+      std::vector<Segment> run;
+      const double until = total * (sp + 1) / splits;
+      while (next < all.size() && (run.empty() || sp + 1 == splits || done + 0.5 * all[next].cost <= until)) {
+        done += all[next].cost;
+        run.push_back(all[next++]);
+      }
+      runs.push_back(std::move(run));
+    }
   }
 
   std::vector<int> split_table, chunk_table;
@@ -259,7 +318,7 @@ bool fill_part(const PartView& p, const CellGrid& cg, long long extra_floats, bo
 
 }  // namespace
 
-bool col_setup(const VecCall& c, bool backward, int warps_resident, ColArgs* a, ColPlan* plan) {
+bool col_setup(const VecCall& c, bool backward, ColArgs* a, ColPlan* plan) {
   if (c.x.empty() || c.y.empty() || c.r.empty() || !c.dense_channels || c.sph) return false;
   if (c.x.size() > (size_t)kMaxParts || c.y.size() > (size_t)kMaxParts || c.r.size() > (size_t)kMaxParts) return false;
   const int n = c.y[0].n, nx = c.diag ? n : 1;
@@ -276,8 +335,7 @@ bool col_setup(const VecCall& c, bool backward, int warps_resident, ColArgs* a, 
     }
   if (max_la > kColMaxLa || max_lb > 40) return false;
   plan->max_la = max_la;
-  const int max_rows = !backward ? kColBlockFwd : do_x && do_y ? kColBlockBoth : kColBlockBwd;
-  plan->max_block = 2 * max_la + 1 <= max_rows ? 2 * max_la + 1 : max_rows;
+  plan->max_block = std::min(2 * max_la + 1, backward ? kColBlockBwd : kColBlockFwd);
   a->b_rows = 2 * max_lb + 1;
   for (size_t i = 0; i < c.x.size(); i++)
     if (!fill_part(c.x[i], c.cg, 0, true, &a->part[i])) return false;
@@ -330,19 +388,26 @@ bool col_setup(const VecCall& c, bool backward, int warps_resident, ColArgs* a, 
   a->nr = (int)c.r.size();
   a->n = (unsigned)(n / plan->cpl);
   a->nlanes = (unsigned)(c.cg.ncells * a->n);
-  // with fewer warps than the chip holds, the walk is cut into runs of pairs that different blocks take
+  // With fewer warps than the chip holds, the walk is cut into runs that different blocks take: forward into runs of pairs;
+  // backward into one run per a block (owned), so that every gradient row is added to by one lane and the sums have one
+  // order.  The owned walk combines the g rows once per side and not once per pair, so with both gradients the whole walk
+  // wins earlier.  us, owned / whole, diagonal product of 15 channels: both gradients, 282 warps maxl 1 8.3 / 8.9, maxl 3
+  // 26 / 35, maxl 8 386 / 591; 375 warps 9.8 / 9.0, 37 / 35, 505 / 582; 563 warps 12 / 9, 40 / 35, 657 / 608.  One gradient,
+  // 563 warps 7.8 / 8.1, 23 / 30, 354 / 610; 703 warps 8.7 / 8.3, 30 / 33, 438 / 665; 938 warps 14 / 9, 42 / 33, 604 / 686.
   const long long warps = (a->nlanes + 31) / 32;
   int splits = 1;
-  while (splits < 16 && warps * splits * 2 <= warps_resident) splits *= 2;
+  while (!backward && splits < 16 && warps * splits * 2 <= 148 * 12) splits *= 2;
+  plan->owned = backward && plan->cpl == 1 && warps <= (do_x && do_y ? 2 : 4) * 148;
   a->accumulate = (c.flags & GELIB_OVERWRITE) ? 0 : 1;
 
-  std::vector<int> key = {20 /*family*/, backward, do_x, do_y, splits, c.diag, (int)c.x.size(), (int)c.y.size(), (int)c.r.size(), n};
+  std::vector<int> key = {20 /*family*/, backward, do_x, do_y, splits, plan->owned, c.diag, (int)c.x.size(), (int)c.y.size(), (int)c.r.size(), n};
   for (const auto& p : c.x) key.push_back(p.l);
   for (const auto& p : c.y) key.push_back(p.l);
   for (const auto& p : c.r) { key.push_back(p.l); key.push_back(p.n); }
   const auto xs = sig_of(c.x), ys = sig_of(c.y), rs = sig_of(c.r);
   const bool diag = c.diag;
-  plan->dev = get_plan(key, [&](DevicePlan& p) { build(p, xs, ys, rs, diag, backward, do_x, do_y, splits); });
+  const bool owned = plan->owned;
+  plan->dev = get_plan(key, [&](DevicePlan& p) { build(p, xs, ys, rs, diag, backward, do_x, do_y, splits, owned); });
   if (!plan->dev) return true;
   a->blob = plan->dev->items;
   a->chunks = plan->dev->jobs;

@@ -142,3 +142,26 @@ def test_an_infinity_stays_in_its_band(G, oracle, l):
         wx = {l: np.zeros_like(np_c(x[l]))}
         oracle.vec_cg_back0(wx, {k: np_c(t) for k, t in g.items()}, {k: np_c(t) for k, t in y.items()}, True)
     assert (np.isfinite(np_c(xg[l])) == np.isfinite(wx[l])).all()
+
+
+@pytest.mark.parametrize("diag,B,tx,ty,maxl", [
+    (True, 16, U(4, 8), U(4, 8), 4), (True, 500, U(3, 12), U(3, 12), 3), (True, 30, U(8, 16), U(8, 16), 8), (True, 40, U(3, 40), U(5, 40), 5),
+    (True, 4, U(3, 4), {9: 4, 12: 4, 20: 4}, -1), (False, 33, U(6, 1), U(6, 16), 6), (False, 500, U(4, 1), U(4, 8), 4),
+])
+def test_gradients_are_repeatable(G, oracle, diag, B, tx, ty, maxl):
+    """Few columns: blocks share the walk, yet a gradient row is added to in one order."""
+    tr = oracle.cg_type(tx, ty, maxl, diag)
+    x, y, g = cuda(parts(1, B, tx)), cuda(parts(100, B, ty)), cuda(parts(200, B, tr))
+    x0, y0 = cuda(parts(300, B, tx)), cuda(parts(400, B, ty))
+    first = None
+    for _ in range(10):
+        xg, yg = {l: t.clone() for l, t in x0.items()}, {l: t.clone() for l, t in y0.items()}
+        y1 = {l: t.clone() for l, t in y0.items()}
+        if diag:
+            G.backend.SO3vec.addDiagCGproduct_back01(vec(G, xg), vec(G, yg), vec(G, g), vec(G, x), vec(G, y))
+            vec(G, y1).addDiagCGproduct_back1(vec(G, g), vec(G, x))
+        else:
+            vec(G, y1).addCGproduct_back1(vec(G, g), vec(G, x))
+        got = [torch.view_as_real(t) for d in (xg, yg, y1) for t in d.values()]
+        first = first or got
+        assert all(torch.equal(a, b) for a, b in zip(first, got))

@@ -131,6 +131,36 @@ int check_room(const char* fn, const std::vector<PartView>& x, const std::vector
   return GELIB_OK;
 }
 
+// The kernels that serve what the column kernels do not take.
+int run_kernels(const VecCall& c, int mode, bool fp64, cudaStream_t s) {
+  int st = -1;
+  if (mode == 0) {
+    if (c.dense_channels && !c.r_bcast && !fp64) {
+      if (c.diag) {
+        st = launch_diag_fwd(c, s);
+      } else {
+        st = launch_cg_narrow_fwd(c, s);
+        if (st == -1) st = launch_cg_fwd(c, s);
+      }
+    }
+    return st == -1 ? launch_cg_strided(c, 0, s) : st;
+  }
+  if (c.dense_channels && !fp64) {
+    if (c.diag) {
+      st = launch_diag_bwd(c, s);
+    } else {
+      st = launch_cg_narrow_bwd(c, s);
+      if (st == -1) st = launch_cg_bwd(c, s);
+    }
+  }
+  if (st == -1) {
+    st = GELIB_OK;
+    if (!c.xg.empty()) st = launch_cg_strided(c, 1, s);
+    if (st == GELIB_OK && !c.yg.empty()) st = launch_cg_strided(c, 2, s);
+  }
+  return st;
+}
+
 // mode 0: forward (out = r).  mode 1/2/3: gradient wrt x / y / both (r is g).
 int run_product(const char* fn, bool diag, int mode, int nr, const gelib_tensor5* r, int nx, const gelib_tensor5* x,
                 int ny, const gelib_tensor5* y, int nxg, const gelib_tensor5* xg, int nyg, const gelib_tensor5* yg,
@@ -218,38 +248,17 @@ int run_product(const char* fn, bool diag, int mode, int nr, const gelib_tensor5
     return st;
   }
   const bool fp64 = (flags & GELIB_FP64) != 0;  // double coefficients and sums: the general strided kernels
-  if (mode == 0) {
-    st = -1;
-    if (c.dense_channels && !c.r_bcast && !fp64) {
-      if (col_enabled()) st = launch_col_fwd(c, s);
-      if (st != -1) return st;
-      if (diag) {
-        st = launch_diag_fwd(c, s);
-      } else {
-        st = launch_cg_narrow_fwd(c, s);
-        if (st == -1) st = launch_cg_fwd(c, s);
-      }
-    }
-    if (st == -1) st = launch_cg_strided(c, 0, s);
-    return st;
-  }
   st = -1;
-  if (c.dense_channels && !fp64) {
-    if (col_enabled()) st = launch_col_bwd(c, s);
-    if (st != -1) return st;
-    if (diag) {
-      st = launch_diag_bwd(c, s);
-    } else {
-      st = launch_cg_narrow_bwd(c, s);
-      if (st == -1) st = launch_cg_bwd(c, s);
+  if (c.dense_channels && !(mode == 0 && c.r_bcast) && !fp64 && col_enabled()) {
+    bool plan_others = false;
+    st = mode == 0 ? launch_col_fwd(c, s, &plan_others) : launch_col_bwd(c, s, &plan_others);
+    if (plan_others) {  // should that fail, the call that needs the plan says so
+      VecCall other = c;
+      other.plan_only = true;
+      run_kernels(other, mode, fp64, s);
     }
   }
-  if (st == -1) {
-    st = GELIB_OK;
-    if (!c.xg.empty()) st = launch_cg_strided(c, 1, s);
-    if (st == GELIB_OK && !c.yg.empty()) st = launch_cg_strided(c, 2, s);
-  }
-  return st;
+  return st == -1 ? run_kernels(c, mode, fp64, s) : st;
 }
 
 int type_product(int nx, const int* xl, const int* xn, int ny, const int* yl, const int* yn, int maxl, bool diag,

@@ -344,6 +344,20 @@ cudaError_t launch_cfg(const BwdArgs& a, dim3 grid, int threads, size_t smem, bo
 inline int ceil_div(int a, int b) { return (a + b - 1) / b; }
 inline int align4(int v) { return (v + 3) / 4 * 4; }
 
+// Whether the operands and gradients of wc cells, padded to ta x tb tiles, fit shared memory and the items' 16 bits.
+bool fits(const std::vector<PartSig>& xs, const std::vector<PartSig>& ys, int ta, int tb, int wc) {
+  size_t floats = 0;
+  for (const auto& p : xs) {
+    if (ceil_div(p.n, ta) * ta > 65535) return false;
+    floats += align4(2 * (2 * p.l + 1) * (ceil_div(p.n, ta) * ta));
+  }
+  for (const auto& p : ys) {
+    if (ceil_div(p.n, tb) * tb > 65535) return false;
+    floats += align4(2 * (2 * p.l + 1) * (ceil_div(p.n, tb) * tb));
+  }
+  return (6 * kMaxParts + 2 * floats) * wc * sizeof(float) <= 220 * 1024;
+}
+
 }  // namespace
 
 int launch_cg_bwd(const VecCall& c, cudaStream_t s) {
@@ -368,51 +382,88 @@ int launch_cg_bwd(const VecCall& c, cudaStream_t s) {
   for (const auto& p : c.x) if (p.l > 2047 || p.n > 65535) return -1;
   for (const auto& p : c.y) if (p.l > 2047 || p.n > 65535) return -1;
   for (const auto& p : c.r) if (p.l > 2047) return -1;
-  // The lane layout whose warps execute the fewest instructions for the call.  Per band entry: 8 multiply-adds per
-  // complex number of the slab, the operand loads, the butterflies' shuffles and adds, and about five instructions per
-  // shared-memory atomic (they are compare-and-swap loops); per slab its loads.  The layouts differ in the padding of
-  // the channel counts and in how many multiply-adds share a butterfly; the work is spread over the warps the call can
-  // fill.  Measured (maxl 4 x 16 channels, batch 1000): 689 us with 8 x 16 channels per warp, 418 us with 16 x 16.
-  Schedule sched;
-  build_schedule(sig_of(c.x), sig_of(c.y), sig_of(c.r), false, false, &sched);
-  auto halving = [](int n, int e, int w, int* own) {  // shuffles of butterfly<n, e, w>, elements left per lane
-    int sh = 0;
-    for (int s = 1; s < w; s *= 2) {
-      if (n > 1) n /= 2;
-      sh += n * e;
+  // ---- plan: work lists of every lane layout that some batch size uses
+  std::vector<int> key = {3 /*family*/, vec ? 1 : 0, (int)c.x.size(), (int)c.y.size(), (int)c.r.size()};
+  for (const auto& p : c.x) { key.push_back(p.l); key.push_back(p.n); }
+  for (const auto& p : c.y) { key.push_back(p.l); key.push_back(p.n); }
+  for (const auto& p : c.r) key.push_back(p.l);
+  const auto xs = sig_of(c.x), ys = sig_of(c.y), rs = sig_of(c.r);
+  DevicePlan* plan = get_plan(key, [&](DevicePlan& p) {
+    build_schedule(xs, ys, rs, false, true, &p.sched);
+    std::vector<int> band;
+    for (const Triple& t : p.sched.triples) band.push_back(band_size(t.l1, t.l2, t.l));
+    // The estimate of a layout's time: the instructions its warps execute.  Per band entry: 8 multiply-adds per complex
+    // number of the slab, the operand loads, the butterflies' shuffles and adds, and about five instructions per
+    // shared-memory atomic (they are compare-and-swap loops); per slab its loads.  The layouts differ in the padding of
+    // the channel counts and in how many multiply-adds share a butterfly; the work is spread over the warps the call can
+    // fill.  Measured (maxl 4 x 16 channels, batch 1000): 689 us with 8 x 16 channels per warp, 418 us with 16 x 16.
+    auto halving = [](int n, int e, int w, int* own) {  // shuffles of butterfly<n, e, w>, elements left per lane
+      int sh = 0;
+      for (int s = 1; s < w; s *= 2) {
+        if (n > 1) n /= 2;
+        sh += n * e;
+      }
+      *own = n * e;
+      return sh;
+    };
+    for (const BwdCfg& f : kCfgs) {
+      const int ta = f.TA * f.WA, tb = f.TBU * UB * f.WB, wc = 32 / (f.WA * f.WB);
+      LayoutCost lc{0, 0, wc};
+      if (fits(xs, ys, ta, tb, wc)) {
+        int own_x, own_y;
+        const int sh = halving(f.TA, 2, f.WB, &own_x) + halving(f.TBU, 2 * UB, f.WA, &own_y);
+        const double entry = 8.0 * f.TA * f.TBU * UB + f.TA + f.TBU + 2 * sh + 6 * (own_x + own_y) + 12, slab = 3.0 * f.TA * f.TBU + 30;
+        double items = 0;
+        for (size_t i = 0; i < band.size(); i++) {
+          const Triple& t = p.sched.triples[i];
+          const double tiles = (double)ceil_div(xs[t.xi].n, ta) * ceil_div(ys[t.yi].n, tb);
+          lc.work += tiles * (band[i] * entry + (2 * t.l + 1) * slab);
+          items += tiles * (2 * t.l + 1);
+        }
+        lc.warps = std::min(128.0, std::max(8.0, items / 2));
+      }
+      p.cost.push_back(lc);
     }
-    *own = n * e;
-    return sh;
-  };
-  int best = 0;
-  double best_cost = 1e300;
-  for (int i = 0; i < kNumCfgs; i++) {
-    const BwdCfg& f = kCfgs[i];
-    const int ta = f.TA * f.WA, tb = f.TBU * UB * f.WB;
-    const int wc = 32 / (f.WA * f.WB);
-    size_t floats = 0;
-    for (const auto& p : c.x) floats += align4(2 * (2 * p.l + 1) * ceil_div(p.n, ta) * ta);
-    for (const auto& p : c.y) floats += align4(2 * (2 * p.l + 1) * ceil_div(p.n, tb) * tb);
-    if ((6 * kMaxParts + 2 * floats) * wc * sizeof(float) > 220 * 1024) continue;
-    int own_x, own_y;
-    const int sh = halving(f.TA, 2, f.WB, &own_x) + halving(f.TBU, 2 * UB, f.WA, &own_y);
-    const double entry = 8.0 * f.TA * f.TBU * UB + f.TA + f.TBU + 2 * sh + 6 * (own_x + own_y) + 12, slab = 3.0 * f.TA * f.TBU + 30;
-    double cost = 0, items = 0;
-    for (const Triple& t : sched.triples) {
-      const double tiles = (double)ceil_div(c.x[t.xi].n, ta) * ceil_div(c.y[t.yi].n, tb);
-      cost += tiles * (band_size(t.l1, t.l2, t.l) * entry + (2 * t.l + 1) * slab);
-      items += tiles * (2 * t.l + 1);
+    struct It { int4 v0, v1; int cost; };
+    p.tables.assign(2 * kNumCfgs, 0);  // per layout: {first entry of h_items, items}
+    for (int i : layouts_used(p.cost)) {
+      const int ta = kCfgs[i].TA * kCfgs[i].WA, tb = kCfgs[i].TBU * UB * kCfgs[i].WB;
+      std::vector<It> its;
+      for (const Triple& t : p.sched.triples) {
+        int cpos = t.coff;
+        const int xnp = ceil_div(xs[t.xi].n, ta) * ta, ynp = ceil_div(ys[t.yi].n, tb) * tb;
+        for (int m = -t.l; m <= t.l; m++) {
+          const int lo = std::max<int>(-t.l1, m - t.l2), hi = std::min<int>(t.l1, m + t.l2);
+          for (int a0 = 0; a0 < xs[t.xi].n; a0 += ta)
+            for (int b0 = 0; b0 < ys[t.yi].n; b0 += tb) {
+              const bool full = a0 + ta <= xs[t.xi].n && b0 + tb <= ys[t.yi].n;
+              its.push_back({make_int4(t.ri | (t.xi << 4) | (t.yi << 8) | (full ? (int)0x80000000 : 0),
+                                       t.l | ((m + t.l) << 12), a0 | (b0 << 16), cpos),
+                             make_int4(t.offs, t.l1 | (t.l2 << 12), xnp | (ynp << 16), 0), hi - lo + 2});
+            }
+          cpos += hi - lo + 1;
+        }
+      }
+      // longest first, dealt round robin to the warps: a balanced static schedule without barriers
+      std::stable_sort(its.begin(), its.end(), [](const It& u, const It& v) { return u.cost > v.cost; });
+      p.tables[2 * i] = (int)p.h_items.size();
+      p.tables[2 * i + 1] = (int)its.size();
+      for (const auto& it : its) {
+        p.h_items.push_back(it.v0);
+        p.h_items.push_back(it.v1);
+      }
     }
-    const double groups = (double)((c.cg.ncells + wc - 1) / wc);
-    cost *= groups / std::min(groups * std::min(128.0, std::max(8.0, items / 2)), 148.0 * 16);
-    if (cost < best_cost * 0.999) {
-      best_cost = cost;
-      best = i;
-    }
-  }
+  });
+  if (!plan) return GELIB_CUDA_ERROR;
+  if (plan->sched.triples.empty() || c.cg.ncells == 0) return GELIB_OK;
+  const int best = choose_layout(plan->cost, c.cg.ncells);
+  if (best < 0) return -1;  // caller falls back to the strided kernels
+  if (c.plan_only) return GELIB_OK;
   const BwdCfg cfg = kCfgs[best];
   const int WC = 32 / (cfg.WA * cfg.WB);
   const int tile_a = cfg.TA * cfg.WA, tile_b = cfg.TBU * UB * cfg.WB;
+  const int first_item = plan->tables[2 * best], nitems = plan->tables[2 * best + 1];
+  if (nitems == 0) return GELIB_OK;
 
   BwdArgs a;
   int off = 0;
@@ -435,50 +486,12 @@ int launch_cg_bwd(const VecCall& c, cudaStream_t s) {
   a.ny = (int)c.y.size();
   a.ng = (int)c.r.size();
   a.cell_floats = off;
-  for (size_t i = 0; i < c.x.size(); i++) if (a.xnp[i] > 65535) return -1;
-  for (size_t i = 0; i < c.y.size(); i++) if (a.ynp[i] > 65535) return -1;
   const size_t smem = ((size_t)6 * WC * kMaxParts + (size_t)2 * WC * off) * sizeof(float);
-  if (smem > 220 * 1024) return -1;  // caller falls back to the strided kernels
-
-  std::vector<int> key = {3 /*family*/, best, vec ? 1 : 0, (int)c.x.size(), (int)c.y.size(), (int)c.r.size()};
-  for (const auto& p : c.x) { key.push_back(p.l); key.push_back(p.n); }
-  for (const auto& p : c.y) { key.push_back(p.l); key.push_back(p.n); }
-  for (const auto& p : c.r) key.push_back(p.l);
-  const auto xs = sig_of(c.x), ys = sig_of(c.y), rs = sig_of(c.r);
-  const int* xnp = a.xnp;
-  const int* ynp = a.ynp;
-  DevicePlan* plan = get_plan(key, [&](DevicePlan& p) {
-    build_schedule(xs, ys, rs, false, true, &p.sched);
-    struct It { int4 v0, v1; int cost; };
-    std::vector<It> its;
-    for (const Triple& t : p.sched.triples) {
-      int cpos = t.coff;
-      for (int m = -t.l; m <= t.l; m++) {
-        const int lo = std::max<int>(-t.l1, m - t.l2), hi = std::min<int>(t.l1, m + t.l2);
-        for (int a0 = 0; a0 < xs[t.xi].n; a0 += tile_a)
-          for (int b0 = 0; b0 < ys[t.yi].n; b0 += tile_b) {
-            const bool full = a0 + tile_a <= xs[t.xi].n && b0 + tile_b <= ys[t.yi].n;
-            its.push_back({make_int4(t.ri | (t.xi << 4) | (t.yi << 8) | (full ? (int)0x80000000 : 0),
-                                     t.l | ((m + t.l) << 12), a0 | (b0 << 16), cpos),
-                           make_int4(t.offs, t.l1 | (t.l2 << 12), xnp[t.xi] | (ynp[t.yi] << 16), 0), hi - lo + 2});
-          }
-        cpos += hi - lo + 1;
-      }
-    }
-    // longest first, dealt round robin to the warps: a balanced static schedule without barriers
-    std::stable_sort(its.begin(), its.end(), [](const It& u, const It& v) { return u.cost > v.cost; });
-    for (const auto& it : its) {
-      p.h_items.push_back(it.v0);
-      p.h_items.push_back(it.v1);
-    }
-  });
-  if (!plan) return GELIB_CUDA_ERROR;
-  if (plan->nitems == 0 || c.cg.ncells == 0) return GELIB_OK;
 
   a.cg = c.cg;
   a.coeffs = plan->coeffs;
-  a.items = plan->items;
-  a.nitems = plan->nitems / 2;
+  a.items = plan->items + first_item;
+  a.nitems = nitems;
   // a warp per slab when a cell has fewer than eight: idle warps would only cost residency (l1 = l2 = l = 2, 32 channels,
   // batch 1024, five slabs per cell: 38 -> 32 us)
   const int nwarps = std::min(8, a.nitems);

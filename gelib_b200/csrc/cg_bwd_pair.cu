@@ -670,7 +670,7 @@ int launch_cg_bwd_pair(const VecCall& c, cudaStream_t s, int min_groups) {
     p.h_jobs.push_back((int)std::min<long long>(entries, 0x7fffffffLL));
   });
   if (!plan) return GELIB_CUDA_ERROR;
-  if (plan->nitems == 0 || c.cg.ncells == 0) return GELIB_OK;
+  if (plan->nitems == 0 || c.cg.ncells == 0 || c.plan_only) return GELIB_OK;
   // a cell with only a few groups does not fill the pipeline of 12 warps: the one-slab-per-warp kernel is faster there
   // Automatic choice: the kernel pays a fixed cost per group (handshake, slab loads into registers) that short bands
   // do not repay.  Measured against the kernel of cg_bwd.cu at 32 channels: maxl 4 (188 groups, 3.1 entries per

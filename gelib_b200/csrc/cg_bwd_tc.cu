@@ -545,7 +545,7 @@ int launch_cg_bwd_tc(const VecCall& c, cudaStream_t s) {
     }
   });
   if (!plan) return GELIB_CUDA_ERROR;
-  if (plan->nitems == 0 || c.cg.ncells == 0) return GELIB_OK;
+  if (plan->nitems == 0 || c.cg.ncells == 0 || c.plan_only) return GELIB_OK;
   if (c.cg.ncells > 0x3fffffffLL) return fail(GELIB_SKIPPED, fn, "number of cells exceeds 2^30-1");
 
   a.cg = c.cg;

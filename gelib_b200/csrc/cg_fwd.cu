@@ -205,6 +205,7 @@ constexpr TileCfg kCfgs[] = {
     {4, 4, 1},  // 16 x  4, 8 cells
 };
 constexpr int kNumCfgs = sizeof(kCfgs) / sizeof(kCfgs[0]);
+constexpr int kMaxJobs = 16;
 
 template <int TA, int WA, int NBL>
 cudaError_t launch_cfg(const FwdArgs& a, dim3 grid, size_t smem, bool vec, cudaStream_t s) {
@@ -238,42 +239,86 @@ int launch_cg_fwd(const VecCall& c, cudaStream_t s) {
     if (rc != -1) return rc;
     if (mode == kFwdTcStrict) return fail(GELIB_INVALID, fn, "the call does not qualify for the tcgen05 kernel");
   }
-  // ---- choose the lane layout by an estimate of its time.  Per band entry a warp issues 16 multiply-adds and 2
-  // multiplies for each of its TA rows, half a load per row and about 7 others; per output row it issues 2 TA stores (4 TA
-  // of half the size without 16-byte alignment), each of which occupies the load/store unit, which four schedulers share,
-  // once per 128-byte line it touches.  The work is spread over the warps the call can fill.  Layouts differ in the padding
-  // of the channel counts, in how many multiply-adds share the loads and in how many lines a store touches.  Measured
-  // (maxl 4 x 16 channels, batch 1000): 521 us with 1 x 16 channels per warp row, 247 us with 16 x 16.
-  Schedule sched;
-  build_schedule(sig_of(c.x), sig_of(c.y), sig_of(c.r), false, false, &sched);
+  // ---- plan: work lists and job tables of every lane layout that some batch size uses
   int cell_floats = 0;
   for (auto* v : {&c.x, &c.y})
     for (const auto& p : *v) cell_floats += 2 * (2 * p.l + 1) * (ceil_div(p.n, 4) * 4);
   // floats; tiles may read up to 128 past the last row
   auto smem_floats = [&](int WC) { return (size_t)cell_floats * WC + 128 + 2 * WC * kMaxParts; };
-  int best = 0;
-  double best_cost = 1e300;
-  for (int i = 0; i < kNumCfgs; i++) {
-    const TileCfg& f = kCfgs[i];
-    const int ta = f.TA * f.WA, tb = 4 * f.NBL, wc = 32 / (f.WA * f.NBL);
-    if (smem_floats(wc) * sizeof(float) > 200 * 1024) continue;
-    const double entry = 18.5 * f.TA + 7, row = 6.0 * f.TA + 12 + 4.0 * (c.vec_ok ? 2 : 4) * f.TA * wc * f.WA;
-    double cost = 0, items = 0;
-    for (const Triple& t : sched.triples) {
-      const double tiles = (double)ceil_div(c.x[t.xi].n, ta) * ceil_div(c.y[t.yi].n, tb);
-      cost += tiles * (band_size(t.l1, t.l2, t.l) * entry + (2 * t.l + 1) * row);
-      items += tiles;
+  std::vector<int> key = {1 /*family*/, c.vec_ok ? 1 : 0, (int)c.x.size(), (int)c.y.size(), (int)c.r.size()};
+  for (const auto& p : c.x) { key.push_back(p.l); key.push_back(p.n); }
+  for (const auto& p : c.y) { key.push_back(p.l); key.push_back(p.n); }
+  for (const auto& p : c.r) key.push_back(p.l);
+  const auto xs = sig_of(c.x), ys = sig_of(c.y), rs = sig_of(c.r);
+  const bool vec = c.vec_ok;
+  DevicePlan* plan = get_plan(key, [&](DevicePlan& p) {
+    build_schedule(xs, ys, rs, false, true, &p.sched);
+    std::vector<int> band;
+    for (const Triple& t : p.sched.triples) band.push_back(band_size(t.l1, t.l2, t.l));
+    // The estimate of a layout's time.  Per band entry a warp issues 16 multiply-adds and 2 multiplies for each of its TA
+    // rows, half a load per row and about 7 others; per output row it issues 2 TA stores (4 TA of half the size without
+    // 16-byte alignment), each of which occupies the load/store unit, which four schedulers share, once per 128-byte line
+    // it touches.  The work is spread over the warps the call can fill.  Layouts differ in the padding of the channel
+    // counts, in how many multiply-adds share the loads and in how many lines a store touches.  Measured (maxl 4 x 16
+    // channels, batch 1000): 521 us with 1 x 16 channels per warp row, 247 us with 16 x 16.
+    for (const TileCfg& f : kCfgs) {
+      const int ta = f.TA * f.WA, tb = 4 * f.NBL, wc = 32 / (f.WA * f.NBL);
+      LayoutCost lc{0, 0, wc};
+      if (smem_floats(wc) * sizeof(float) <= 200 * 1024) {
+        const double entry = 18.5 * f.TA + 7, row = 6.0 * f.TA + 12 + 4.0 * (vec ? 2 : 4) * f.TA * wc * f.WA;
+        double items = 0;
+        for (size_t i = 0; i < band.size(); i++) {
+          const Triple& t = p.sched.triples[i];
+          const double tiles = (double)ceil_div(xs[t.xi].n, ta) * ceil_div(ys[t.yi].n, tb);
+          lc.work += tiles * (band[i] * entry + (2 * t.l + 1) * row);
+          items += tiles;
+        }
+        lc.warps = std::min(64.0, std::max(4.0, items));
+      }
+      p.cost.push_back(lc);
     }
-    const double groups = (double)((c.cg.ncells + wc - 1) / wc);
-    cost *= groups / std::min(groups * std::min(64.0, std::max(4.0, items)), 148.0 * 16);
-    if (cost < best_cost * 0.999) {
-      best_cost = cost;
-      best = i;
+    // per layout: {first item, items, first of its job tables}; a job table for every number of jobs up to kMaxJobs
+    p.tables.assign(3 * kNumCfgs, 0);
+    for (int i : layouts_used(p.cost)) {
+      const int ta = kCfgs[i].TA * kCfgs[i].WA, tb = 4 * kCfgs[i].NBL;
+      const int first = (int)p.h_items.size();
+      std::vector<long long> cost;
+      for (size_t ti = 0; ti < p.sched.triples.size(); ti++) {
+        const Triple& t = p.sched.triples[ti];
+        for (int a0 = 0; a0 < xs[t.xi].n; a0 += ta)
+          for (int b0 = 0; b0 < ys[t.yi].n; b0 += tb) {
+            p.h_items.push_back(make_int4((int)ti, a0, b0, 0));
+            cost.push_back(band[ti] + 2 * (2 * t.l + 1));
+          }
+      }
+      p.tables[3 * i] = first;
+      p.tables[3 * i + 1] = (int)cost.size();
+      p.tables[3 * i + 2] = (int)p.h_jobs.size();
+      long long total = 0;
+      for (long long v : cost) total += v;
+      for (int nj = 1; nj <= kMaxJobs; nj++) {
+        const size_t begin = p.h_jobs.size();
+        p.h_jobs.push_back(0);
+        long long run = 0;
+        for (size_t k = 0; k < cost.size(); k++) {
+          run += cost[k];
+          const int done = (int)(p.h_jobs.size() - begin);
+          if (done < nj && run * nj >= total * (long long)done) p.h_jobs.push_back((int)k + 1);
+        }
+        p.h_jobs.resize(begin + nj + 1, (int)cost.size());
+        p.h_jobs.back() = (int)cost.size();
+      }
     }
-  }
+  });
+  if (!plan) return GELIB_CUDA_ERROR;
+  if (plan->sched.triples.empty() || c.cg.ncells == 0) return GELIB_OK;
+  const int best = choose_layout(plan->cost, c.cg.ncells);
+  if (best < 0) return -1;  // caller falls back to the strided kernel
+  if (c.plan_only) return GELIB_OK;
   const TileCfg cfg = kCfgs[best];
   const int WC = 32 / (cfg.WA * cfg.NBL);
-  const int tile_a = cfg.TA * cfg.WA, tile_b = 4 * cfg.NBL;
+  const int first_item = plan->tables[3 * best], nitems = plan->tables[3 * best + 1];
+  if (nitems == 0) return GELIB_OK;
 
   // ---- shared-memory layout of one cell
   FwdArgs a;
@@ -296,55 +341,23 @@ int launch_cg_fwd(const VecCall& c, cudaStream_t s) {
   a.nr = (int)c.r.size();
   a.cell_floats = off;
   const size_t smem = smem_floats(WC) * sizeof(float);
-  if (smem > 200 * 1024) return -1;                             // caller falls back to the strided kernel
 
   // ---- jobs: enough CTAs to fill the machine several times over
   const long long groups = (c.cg.ncells + WC - 1) / WC;
   int njobs = 1;
-  if (groups < 16384) njobs = (int)std::min<long long>(16, (16384 + groups - 1) / groups);
-
-  std::vector<int> key = {1 /*family*/, best, njobs, (int)c.x.size(), (int)c.y.size(), (int)c.r.size()};
-  for (const auto& p : c.x) { key.push_back(p.l); key.push_back(p.n); }
-  for (const auto& p : c.y) { key.push_back(p.l); key.push_back(p.n); }
-  for (const auto& p : c.r) key.push_back(p.l);
-  const auto xs = sig_of(c.x), ys = sig_of(c.y), rs = sig_of(c.r);
-  DevicePlan* plan = get_plan(key, [&](DevicePlan& p) {
-    build_schedule(xs, ys, rs, false, true, &p.sched);
-    std::vector<long long> cost;
-    for (size_t ti = 0; ti < p.sched.triples.size(); ti++) {
-      const Triple& t = p.sched.triples[ti];
-      const int T = band_size(t.l1, t.l2, t.l);
-      for (int a0 = 0; a0 < xs[t.xi].n; a0 += tile_a)
-        for (int b0 = 0; b0 < ys[t.yi].n; b0 += tile_b) {
-          p.h_items.push_back(make_int4((int)ti, a0, b0, 0));
-          cost.push_back(T + 2 * (2 * t.l + 1));
-        }
-    }
-    long long total = 0;
-    for (long long v : cost) total += v;
-    const int nj = std::max(1, std::min<int>(njobs, (int)p.h_items.size() / 4));
-    p.h_jobs.push_back(0);
-    long long run = 0;
-    for (size_t i = 0; i < cost.size(); i++) {
-      run += cost[i];
-      if ((int)p.h_jobs.size() < nj && run * nj >= total * (long long)p.h_jobs.size()) p.h_jobs.push_back((int)i + 1);
-    }
-    while ((int)p.h_jobs.size() < nj + 1) p.h_jobs.push_back((int)cost.size());
-    p.h_jobs.back() = (int)cost.size();
-  });
-  if (!plan) return GELIB_CUDA_ERROR;
-  if (plan->nitems == 0 || c.cg.ncells == 0) return GELIB_OK;
+  if (groups < 16384) njobs = (int)std::min<long long>(kMaxJobs, (16384 + groups - 1) / groups);
+  njobs = std::max(1, std::min(njobs, nitems / 4));
 
   a.cg = c.cg;
   a.triples = plan->triples;
   a.coeffs = plan->coeffs;
-  a.items = plan->items;
-  a.jobs = plan->jobs;
+  a.items = plan->items + first_item;
+  a.jobs = plan->jobs + plan->tables[3 * best + 2] + (njobs - 1) * (njobs + 2) / 2;
   a.offs_extra = c.offs_extra;
   a.accumulate = (c.flags & GELIB_OVERWRITE) ? 0 : 1;
 
   if (groups > 0x7fffffffLL) return fail(GELIB_SKIPPED, fn, "number of cells exceeds 2^31-1");
-  const dim3 grid((unsigned)groups, (unsigned)plan->njobs);
+  const dim3 grid((unsigned)groups, (unsigned)njobs);
   cudaError_t e = cudaSuccess;
   switch (best) {
     case 0: e = launch_cfg<4, 4, 8>(a, grid, smem, c.vec_ok, s); break;

@@ -463,7 +463,7 @@ int launch_cg_narrow_fwd(const VecCall& c, cudaStream_t s) {
   if (smem > 200 * 1024) return -1;
   DevicePlan* plan = narrow_plan(c);
   if (!plan) return GELIB_CUDA_ERROR;
-  if (plan->ntriples == 0 || c.cg.ncells == 0) return GELIB_OK;
+  if (plan->ntriples == 0 || c.cg.ncells == 0 || c.plan_only) return GELIB_OK;
   a.triples = plan->triples;
   a.coeffs = plan->coeffs;
   a.pairs = reinterpret_cast<const int2*>(plan->jobs);
@@ -501,7 +501,7 @@ int launch_cg_narrow_bwd(const VecCall& c, cudaStream_t s) {
   if (smem > 200 * 1024) return -1;
   DevicePlan* plan = narrow_plan(c);
   if (!plan) return GELIB_CUDA_ERROR;
-  if (plan->ntriples == 0 || c.cg.ncells == 0) return GELIB_OK;
+  if (plan->ntriples == 0 || c.cg.ncells == 0 || c.plan_only) return GELIB_OK;
   a.triples = plan->triples;
   a.coeffs = plan->coeffs;
   a.pairs = reinterpret_cast<const int2*>(plan->jobs);

@@ -322,7 +322,7 @@ int launch_cg_narrow1_bwd(const VecCall& c, cudaStream_t s) {
     if (!p.h_items.empty()) p.h_items[p.h_items.size() - kRec].x |= 0x10000;
   });
   if (!plan) return GELIB_CUDA_ERROR;
-  if (plan->nitems == 0 || c.cg.ncells == 0) return GELIB_OK;
+  if (plan->nitems == 0 || c.cg.ncells == 0 || c.plan_only) return GELIB_OK;
   a.cg = c.cg;
   a.recs = plan->items;
   a.ngroups = plan->nitems / kRec;

@@ -146,7 +146,7 @@ int launch_cg_strided(const VecCall& c, int mode, cudaStream_t s) {
     }
   });
   if (!plan) return GELIB_CUDA_ERROR;
-  if (plan->ntriples == 0 || c.cg.ncells == 0) return GELIB_OK;
+  if (plan->ntriples == 0 || c.cg.ncells == 0 || c.plan_only) return GELIB_OK;
   if (plan->ntriples > 65535) return fail(GELIB_SKIPPED, fn, "more than 65535 triples");
   if (c.cg.ncells > 0x7fffffffLL) return fail(GELIB_SKIPPED, fn, "number of cells exceeds 2^31-1");
 

@@ -73,10 +73,10 @@ struct ColArgs {
 
 struct ColPlan {
   DevicePlan* dev;
-  int max_la;     // largest l of an a side
   int max_block;  // a rows of the largest block
   int cpl;        // columns per lane
   bool owned;     // backward with few columns: one run per a block
+  bool plan_others;  // first use of a signature that goes to other kernels at other batch sizes: they should plan it too
 };
 
 // Bits of a segment record.

@@ -7,13 +7,14 @@ cudaError_t col_launch_bwd_x(const ColArgs& a, const ColPlan& p, cudaStream_t s)
 cudaError_t col_launch_bwd_y(const ColArgs& a, const ColPlan& p, cudaStream_t s);
 cudaError_t col_launch_bwd_owned(const ColArgs& a, cudaStream_t s);
 
-int launch_col_bwd(const VecCall& c, cudaStream_t s) {
+int launch_col_bwd(const VecCall& c, cudaStream_t s, bool* plan_others) {
   static const char* fn = "SO3vec_addCGproduct_back";
   ColArgs a;
   ColPlan plan;
   if (c.xg.empty() && c.yg.empty()) return -1;
   if (!col_setup(c, true, &a, &plan)) return -1;
   if (!plan.dev) return GELIB_CUDA_ERROR;
+  *plan_others = plan.plan_others;
   if (a.nsplits == 0) return GELIB_OK;
   const bool do_x = !c.xg.empty(), do_y = !c.yg.empty();
   const cudaError_t e = plan.owned     ? col_launch_bwd_owned(a, s)

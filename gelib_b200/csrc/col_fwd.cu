@@ -156,12 +156,13 @@ cudaError_t launch_fwd(const ColArgs& a, cudaStream_t s) {
 
 }  // namespace col
 
-int launch_col_fwd(const VecCall& c, cudaStream_t s) {
+int launch_col_fwd(const VecCall& c, cudaStream_t s, bool* plan_others) {
   static const char* fn = "SO3vec_addCGproduct";
   ColArgs a;
   ColPlan plan;
   if (!col_setup(c, false, &a, &plan)) return -1;
   if (!plan.dev) return GELIB_CUDA_ERROR;
+  *plan_others = plan.plan_others;
   if (a.nsplits == 0) return GELIB_OK;
   cudaError_t e;
   if (plan.cpl == 1) e = col::launch_fwd<17, 1, 512>(a, s);

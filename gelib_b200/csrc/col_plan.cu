@@ -25,6 +25,8 @@ long long cell_stride(const PartView& p, const CellGrid& cg) {
   return any ? st : 0;
 }
 
+constexpr int kMaxSplitLog = 4;  // forward: at most 16 runs
+
 struct Step {
   int m, nl, lo, hi;  // output row, output l, first and last entry of the band
 };
@@ -46,6 +48,13 @@ struct Builder {
   bool do_b(int half) const { return backward && !owned && (half == 0 ? do_y : do_x); }
   bool need_a(int half) const { return !backward || do_b(half); }
   bool need_b(int half) const { return !backward || do_a(half); }
+
+  // C_l[m1, m - m1], from the band table of the triple (m ascending, then m1 ascending)
+  float coefficient(const Schedule& sched, const Triple& t, int m, int m1) const {
+    int at = t.coff;
+    for (int k = -t.l; k < m; k++) at += std::min<int>(t.l1, k + t.l2) - std::max<int>(-t.l1, k - t.l2) + 1;
+    return sched.coeffs[at + m1 - std::max<int>(-t.l1, m - t.l2)];
+  }
 
   int2 r_row(const Segment& s, const Step& st, int j) const {
     const Triple& t = *s.ls[s.ls.size() - st.nl + j];
@@ -125,9 +134,10 @@ double cost_of(const std::vector<Segment>& v) {
   return c;
 }
 
-void build(DevicePlan& p, const std::vector<PartSig>& xs, const std::vector<PartSig>& ys, const std::vector<PartSig>& rs,
-           bool diag, bool backward, bool do_x, bool do_y, int splits, bool owned) {
-  build_schedule(xs, ys, rs, diag, false, &p.sched);
+// Appends one walk to the plan (whose schedule and coefficients are there): `splits` runs of pairs, or owned runs.  Its place
+// goes to p.tables: {first word in h_jobs, runs}.
+void build_walk(DevicePlan& p, const std::vector<PartSig>& xs, const std::vector<PartSig>& ys, const std::vector<PartSig>& rs,
+                bool backward, bool do_x, bool do_y, int splits, bool owned) {
   Builder B{rs, backward, do_x, do_y, owned};
   std::map<std::pair<int, int>, std::vector<const Triple*>> pairs;
   for (const Triple& t : p.sched.triples) pairs[{t.xi, t.yi}].push_back(&t);
@@ -281,8 +291,8 @@ void build(DevicePlan& p, const std::vector<PartSig>& xs, const std::vector<Part
               float x = 0.f;
               if (i >= st.lo && i <= st.hi && j < st.nl) {
                 const Triple& t = *s.ls[s.ls.size() - st.nl + j];
-                const int ma = s.mlo + i, mb = st.m - ma;
-                x = (float)(s.half == 0 ? cg_coefficient(t.l1, t.l2, t.l, ma, mb) : cg_coefficient(t.l1, t.l2, t.l, mb, ma));
+                const int ma = s.mlo + i;
+                x = B.coefficient(p.sched, t, st.m, s.half == 0 ? ma : st.m - ma);
               }
               cf.push_back(x);
               cf.push_back(x);
@@ -301,9 +311,23 @@ void build(DevicePlan& p, const std::vector<PartSig>& xs, const std::vector<Part
       nchunks++;
     }
   }
-  p.h_jobs = split_table;
+  p.tables.push_back((int)p.h_jobs.size());
+  p.tables.push_back((int)runs.size());
+  p.h_jobs.insert(p.h_jobs.end(), split_table.begin(), split_table.end());
   p.h_jobs.insert(p.h_jobs.end(), chunk_table.begin(), chunk_table.end());
-  p.h_jobs.push_back((int)runs.size());  // the last word: splits that were built
+}
+
+// The plan of a signature: every walk that a call of it, whatever its number of cells, may take.
+void build(DevicePlan& p, const std::vector<PartSig>& xs, const std::vector<PartSig>& ys, const std::vector<PartSig>& rs,
+           bool diag, bool backward, bool do_x, bool do_y) {
+  build_schedule(xs, ys, rs, diag, true, &p.sched);
+  if (backward) {
+    build_walk(p, xs, ys, rs, true, do_x, do_y, 1, false);
+    build_walk(p, xs, ys, rs, true, do_x, do_y, 1, true);
+  } else {
+    for (int k = 0; k <= kMaxSplitLog; k++) build_walk(p, xs, ys, rs, false, false, false, 1 << k, false);
+  }
+  p.sched.coeffs.clear();  // they are in the walks
 }
 
 bool fill_part(const PartView& p, const CellGrid& cg, long long extra_floats, bool rows, ColPart* out) {
@@ -334,7 +358,7 @@ bool col_setup(const VecCall& c, bool backward, ColArgs* a, ColPlan* plan) {
       max_lb = std::max(max_lb, std::max(p.l, q.l));
     }
   if (max_la > kColMaxLa || max_lb > 40) return false;
-  plan->max_la = max_la;
+  plan->plan_others = false;
   plan->max_block = std::min(2 * max_la + 1, backward ? kColBlockBwd : kColBlockFwd);
   a->b_rows = 2 * max_lb + 1;
   for (size_t i = 0; i < c.x.size(); i++)
@@ -373,14 +397,24 @@ bool col_setup(const VecCall& c, bool backward, ColArgs* a, ColPlan* plan) {
   if (c.diag) {
     const int slices = (n + 63) / 64;
     if (!backward && max_la >= 6 && 8 * n >= 7 * 64 * slices) return false;
-  } else if (n > 1 && n <= 32) {
+  }
+  std::vector<int> key = {20 /*family*/, backward, do_x, do_y, c.diag, (int)c.x.size(), (int)c.y.size(), (int)c.r.size(), n};
+  for (const auto& p : c.x) key.push_back(p.l);
+  for (const auto& p : c.y) key.push_back(p.l);
+  for (const auto& p : c.r) { key.push_back(p.l); key.push_back(p.n); }
+  const auto xs = sig_of(c.x), ys = sig_of(c.y), rs = sig_of(c.r);
+  const bool diag = c.diag;
+  plan->dev = get_plan(key, [&](DevicePlan& p) { build(p, xs, ys, rs, diag, backward, do_x, do_y); });
+  if (!c.diag && n > 1 && n <= 32) {  // reads the number of cells: another batch of the signature may go the other way
     int cw = 1;
     while (cw < n) cw *= 2;
     const long long narrow_warps = c.cg.ncells * cw / 32;
     const bool padded = plan->cpl == 2 ? 4 * n <= 3 * cw : 5 * n <= 3 * cw;
     if (!backward && narrow_warps >= 148 * 16 && !(max_la >= 4 && padded)) return false;
     if (backward && narrow1_enabled() && narrow_warps >= 148 * 32 && (max_la >= 6 || plan->cpl == 1) && !padded) return false;
+    plan->plan_others = plan->dev && plan->dev->first_use.exchange(false);
   }
+  if (!plan->dev) return true;
   a->ch_stride[0] = x_shared ? 0 : 8 * plan->cpl;
   a->ch_stride[1] = a->ch_stride[2] = 8 * plan->cpl;
   a->nx = (int)c.x.size();
@@ -395,23 +429,15 @@ bool col_setup(const VecCall& c, bool backward, ColArgs* a, ColPlan* plan) {
   // 26 / 35, maxl 8 386 / 591; 375 warps 9.8 / 9.0, 37 / 35, 505 / 582; 563 warps 12 / 9, 40 / 35, 657 / 608.  One gradient,
   // 563 warps 7.8 / 8.1, 23 / 30, 354 / 610; 703 warps 8.7 / 8.3, 30 / 33, 438 / 665; 938 warps 14 / 9, 42 / 33, 604 / 686.
   const long long warps = (a->nlanes + 31) / 32;
-  int splits = 1;
-  while (!backward && splits < 16 && warps * splits * 2 <= 148 * 12) splits *= 2;
+  int walk = 0;  // as build() orders them
+  while (!backward && walk < kMaxSplitLog && (warps << (walk + 1)) <= 148 * 12) walk++;
   plan->owned = backward && plan->cpl == 1 && warps <= (do_x && do_y ? 2 : 4) * 148;
+  if (plan->owned) walk = 1;
   a->accumulate = (c.flags & GELIB_OVERWRITE) ? 0 : 1;
 
-  std::vector<int> key = {20 /*family*/, backward, do_x, do_y, splits, plan->owned, c.diag, (int)c.x.size(), (int)c.y.size(), (int)c.r.size(), n};
-  for (const auto& p : c.x) key.push_back(p.l);
-  for (const auto& p : c.y) key.push_back(p.l);
-  for (const auto& p : c.r) { key.push_back(p.l); key.push_back(p.n); }
-  const auto xs = sig_of(c.x), ys = sig_of(c.y), rs = sig_of(c.r);
-  const bool diag = c.diag;
-  const bool owned = plan->owned;
-  plan->dev = get_plan(key, [&](DevicePlan& p) { build(p, xs, ys, rs, diag, backward, do_x, do_y, splits, owned); });
-  if (!plan->dev) return true;
   a->blob = plan->dev->items;
-  a->chunks = plan->dev->jobs;
-  a->nsplits = plan->dev->h_jobs.back();
+  a->chunks = plan->dev->jobs + plan->dev->tables[2 * walk];
+  a->nsplits = plan->dev->tables[2 * walk + 1];
   return true;
 }
 

@@ -3,6 +3,7 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include <atomic>
 #include <string>
 #include <vector>
 
@@ -89,6 +90,13 @@ void build_schedule(const std::vector<PartSig>& x, const std::vector<PartSig>& y
 double cg_coefficient(int l1, int l2, int l, int m1, int m2);
 int band_size(int l1, int l2, int l);  // number of (m1,m2) with |m1|<=l1, |m2|<=l2, |m1+m2|<=l
 
+// What the choice of a lane layout needs besides the number of cells.
+struct LayoutCost {
+  double work;  // warp instructions of one group of cells; 0: the layout does not fit shared memory
+  double warps; // warps that can share a group
+  int cells;    // cells of a group
+};
+
 // Device-resident copy of a plan's tables.  Owned by the per-device cache; never freed before exit.
 struct DevicePlan {
   Triple* triples = nullptr;
@@ -100,6 +108,9 @@ struct DevicePlan {
   std::vector<int4> h_items;
   std::vector<int> h_jobs;
   std::vector<float> h_floats;
+  std::vector<int> tables;        // host only: where the variants of a work list lie (kernel-specific)
+  std::vector<LayoutCost> cost;   // host only: per lane layout
+  std::atomic<bool> first_use{true};  // cleared by the first call that asks, to plan what other batch sizes will run
   Schedule sched;
 };
 

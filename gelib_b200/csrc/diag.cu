@@ -413,7 +413,7 @@ int launch_diag_fwd(const VecCall& c, cudaStream_t s) {
   int max_nl = 0;
   const int st = setup(c, a, &plan, &max_nl);
   if (st != GELIB_OK) return st;
-  if (plan->nitems == 0 || c.cg.ncells == 0) return GELIB_OK;
+  if (plan->nitems == 0 || c.cg.ncells == 0 || c.plan_only) return GELIB_OK;
   const size_t smem = (size_t)2 * a.WC * (a.xrows + a.yrows) * a.CW * sizeof(float);
   if (smem > 200 * 1024) return -1;
   const long long groups = (c.cg.ncells + a.WC - 1) / a.WC;
@@ -451,7 +451,7 @@ int launch_diag_bwd(const VecCall& c, cudaStream_t s) {
   int max_nl = 0;
   const int st = setup(c, a, &plan, &max_nl);
   if (st != GELIB_OK) return st;
-  if (plan->nitems == 0 || c.cg.ncells == 0) return GELIB_OK;
+  if (plan->nitems == 0 || c.cg.ncells == 0 || c.plan_only) return GELIB_OK;
   int lmax1 = 0, lmax2 = 0;
   for (const auto& p : c.x) lmax1 = std::max(lmax1, p.l);
   for (const auto& p : c.y) lmax2 = std::max(lmax2, p.l);

@@ -229,7 +229,7 @@ int launch_diag_bwd_fast(const VecCall& c, cudaStream_t s) {
   DevicePlan* plan = diag_cell_plan(c, xrow0, yrow0);
   if (!plan) return GELIB_CUDA_ERROR;
   const int nchunks = plan->h_jobs.empty() ? 0 : plan->h_jobs[0];
-  if (nchunks == 0 || c.cg.ncells == 0) return GELIB_OK;
+  if (nchunks == 0 || c.cg.ncells == 0 || c.plan_only) return GELIB_OK;
   a.cg = c.cg;
   a.coeffs = plan->coeffs;
   a.recs = plan->items;

@@ -2,8 +2,11 @@
 //
 // The reference looks its coefficient matrices up in an unordered_map on every launch and copies
 // them to "the" GPU on first use (SO3/SO3CGbank.hpp:33-49, single device only).  Here a plan is
-// keyed by (device, kernel family, tiling, part signature), built once under a mutex and kept in
-// device memory for the life of the process, so any number of devices can be used from one process.
+// keyed by (device, kernel family, part signature), built once under a mutex and kept in device
+// memory for the life of the process, so any number of devices can be used from one process.  The
+// number of cells is in no key: a plan holds the work lists of every variant that some batch size
+// takes, so a signature that has run once builds and uploads nothing more.
+#include <algorithm>
 #include <atomic>
 #include <cstdlib>
 #include <cstring>
@@ -176,6 +179,38 @@ bool device_has_tcgen05() {
     cc_major[dev] = v;
   }
   return cc_major[dev] == 10;
+}
+
+int choose_layout(const std::vector<LayoutCost>& cost, long long ncells) {
+  int shift = 0;
+  while ((ncells >> shift) >= 16) shift++;
+  const long long n = (ncells >> shift) << shift;
+  int best = -1;
+  double best_time = 0;
+  for (size_t i = 0; i < cost.size(); i++) {
+    if (cost[i].work <= 0) continue;
+    const double groups = (double)((n + cost[i].cells - 1) / cost[i].cells);
+    const double time = cost[i].work * groups / std::min(groups * cost[i].warps, 148.0 * 16);
+    if (best < 0 || time < best_time * 0.999) {
+      best = (int)i;
+      best_time = time;
+    }
+  }
+  return best;
+}
+
+std::vector<int> layouts_used(const std::vector<LayoutCost>& cost) {
+  std::vector<bool> used(cost.size(), false);
+  std::vector<int> v;
+  for (int shift = 0; shift < 40; shift++)
+    for (long long n = shift == 0 ? 1 : 8; n < 16; n++) {
+      const int i = choose_layout(cost, n << shift);
+      if (i >= 0 && !used[i]) {
+        used[i] = true;
+        v.push_back(i);
+      }
+    }
+  return v;
 }
 
 DevicePlan* get_plan(const std::vector<int>& key, const std::function<void(DevicePlan&)>& build) {

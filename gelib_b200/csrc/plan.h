@@ -22,6 +22,7 @@ struct VecCall {
   const float* sph = nullptr;  // fused first layer: x parts are the harmonics of these points (cell, 3), never read
   long long sph_sb = 0, sph_sm = 0;
   int sph_lmax = 0;
+  bool plan_only = false;  // build the plan, launch nothing
   bool in_vec_ok = true;       // 16-byte alignment of every x, y, xg, yg part (float4 access to the small operands)
 };
 
@@ -31,7 +32,13 @@ std::vector<PartSig> sig_of(const std::vector<PartView>& v);
 // `build` fills sched / h_items / h_jobs.  nullptr (with the error message set) on CUDA failure.
 DevicePlan* get_plan(const std::vector<int>& key, const std::function<void(DevicePlan&)>& build);
 
-// Kernel families (each returns a status code).
+// Layout of the least estimated time for a number of cells, -1 when none fits.  The number is cut to its four leading bits
+// (the estimate is no finer), so that layouts_used can name every layout some batch size will choose: a plan holds the work
+// lists of all of them, and no later call of the signature, whatever its batch, builds or uploads anything.
+int choose_layout(const std::vector<LayoutCost>& cost, long long ncells);
+std::vector<int> layouts_used(const std::vector<LayoutCost>& cost);
+
+// Kernel families (each returns a status code; with c.plan_only they build their plan and return).
 int launch_cg_fwd(const VecCall& c, cudaStream_t s);
 int launch_cg_fwd_tc(const VecCall& c, cudaStream_t s, int min_slabs);  // tcgen05 kernel; -1 when the call does not qualify or has fewer slabs per cell
 int launch_cg_bwd(const VecCall& c, cudaStream_t s);
@@ -43,8 +50,10 @@ bool narrow1_enabled();  // option "narrow1" (default on): tests compare the two
 int launch_cg_narrow_fwd(const VecCall& c, cudaStream_t s);  // x with at most 4 channels; -1 when the call does not qualify
 int launch_cg_strided(const VecCall& c, int mode, cudaStream_t s);  // mode 0 fwd, 1 back0, 2 back1
 int launch_cg_strided_static(const VecCall& c, cudaStream_t s);  // forward, tables in a static device array: no allocation
-int launch_col_fwd(const VecCall& c, cudaStream_t s);  // diagonal products and one-channel x; -1 when the call does not qualify
-int launch_col_bwd(const VecCall& c, cudaStream_t s);  // likewise
+// Diagonal products and one-channel x; -1 when the call does not qualify.  *plan_others: the signature goes to other kernels
+// at other batch sizes, and they have not planned it yet.
+int launch_col_fwd(const VecCall& c, cudaStream_t s, bool* plan_others);
+int launch_col_bwd(const VecCall& c, cudaStream_t s, bool* plan_others);
 bool col_enabled();  // option "col" (default on): tests compare the kernels
 int launch_diag_fwd(const VecCall& c, cudaStream_t s);
 int launch_diag_bwd(const VecCall& c, cudaStream_t s);

@@ -9,7 +9,7 @@ and the backward pass reads the upstream gradient once for both input gradients.
 import torch
 
 from . import backend as gb
-from .gelib_common import common_batch
+from .gelib_common import common_batch, of_class, plain
 from .SO3element import SO3element
 from .SO3irrep import SO3irrep
 
@@ -49,7 +49,7 @@ class SO3partArr_GatherFn(torch.autograd.Function):
     @staticmethod
     def forward(ctx, x, gmap, d):
         ctx.gmap, ctx.d = gmap, d
-        with _plain():
+        with plain():
             ctx.xshape = list(x.shape)
             shape = list(x.shape)
             shape[d + 1] = gmap.d_out()
@@ -59,7 +59,7 @@ class SO3partArr_GatherFn(torch.autograd.Function):
 
     @staticmethod
     def backward(ctx, rg):
-        with _plain():
+        with plain():
             xg = torch.zeros(ctx.xshape, dtype=torch.complex64, device=rg.device)
             gb.SO3part.view(xg).add_gather_back(rg.as_subclass(torch.Tensor).contiguous(), ctx.gmap, ctx.d)
         return xg, None, None
@@ -69,18 +69,13 @@ def _odot(x, y):
     return torch.sum(torch.mul(torch.view_as_real(x), torch.view_as_real(y))).as_subclass(torch.Tensor)
 
 
-# Inside the functions below attributes of the operands are read without the tensor classes' __torch_function__, whose
-# Python handler costs several microseconds per access: a small product is bound by the host.
-_plain = torch._C.DisableTorchFunctionSubclass
-
-
 def _product_forward(ctx, x, y, l, diag):
-    with _plain():
+    with plain():
         return _product_forward_plain(ctx, x, y, l, diag)
 
 
 def _product_backward(ctx, g):
-    with _plain():
+    with plain():
         return _product_backward_plain(ctx, g)
 
 
@@ -108,8 +103,8 @@ def _product_forward_plain(ctx, x, y, l, diag):
 def _product_backward_plain(ctx, g):
     x, y = ctx.saved_tensors
     need_x, need_y = ctx.needs_input_grad[0], ctx.needs_input_grad[1]
-    xg = torch.zeros_like(x).as_subclass(type(x)) if need_x else None
-    yg = torch.zeros_like(y).as_subclass(type(y)) if need_y else None
+    xg = of_class(torch.zeros_like(x), x) if need_x else None
+    yg = of_class(torch.zeros_like(y), y) if need_y else None
     gv, xv, yv = gb.SO3part.view(g), gb.SO3part.view(x), gb.SO3part.view(y)
     if need_x and need_y:
         f = gb.SO3part.add_DiagCGproduct_back01 if ctx.diag else gb.SO3part.add_CGproduct_back01

@@ -8,17 +8,12 @@ forward and one backward instead of one launch per triple (core/Gvec.hpp:311-389
 import torch
 
 from . import backend as gb
-from .gelib_common import common_batch
+from .gelib_common import common_batch, plain, zeros_like_all
 from .SO3part import SO3part, SO3partArr
 
 
-# Inside the functions below attributes of the operands are read without the tensor classes' __torch_function__, whose
-# Python handler costs several microseconds per access: a small product is bound by the host.
-_plain = torch._C.DisableTorchFunctionSubclass
-
-
 def _vec_forward(ctx, k1, k2, maxl, args, diag, part_cls):
-    with _plain():
+    with plain():
         return _vec_forward_plain(ctx, k1, k2, maxl, args, diag, part_cls)
 
 
@@ -45,16 +40,8 @@ def _vec_forward_plain(ctx, k1, k2, maxl, args, diag, part_cls):
 
 
 def _vec_backward(ctx, gargs):
-    with _plain():
+    with plain():
         return _vec_backward_plain(ctx, gargs)
-
-
-def zeros_like_all(tensors):
-    """One zero tensor per tensor and of its class, filled by one launch."""
-    r = [torch.empty_like(t) for t in tensors]
-    if r:
-        torch._foreach_zero_(r)
-    return [z if type(t) is torch.Tensor else z.as_subclass(type(t)) for z, t in zip(r, tensors)]
 
 
 def _vec_backward_plain(ctx, gargs):
@@ -188,7 +175,7 @@ class _VecBase:
 
     def __init__(self, *args):
         self.parts = {}
-        with _plain():
+        with plain():
             for x in args:
                 assert isinstance(x, torch.Tensor)
                 self.parts[(x.size(-2) - 1) // 2] = x

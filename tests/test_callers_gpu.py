@@ -238,3 +238,12 @@ def test_vec_times_weights_autograd(G):
         assert (o.as_subclass(torch.Tensor) - ref).abs().max() < 1e-5
         assert (p.grad - p2.grad).abs().max() < 1e-5
         assert (w_.grad - w2.grad).abs().max() < 1e-4
+
+
+def test_gradients_of_parameters_are_plain_tensors(G):
+    """A gradient that were a torch.nn.Parameter would register itself as a weight of the module it is assigned to."""
+    p = [torch.nn.Parameter(crandn(10 + l, 3, 2 * l + 1, 4).cuda()) for l in range(4)]
+    z = G.CGproduct(G.SO3vec(p[0], p[1]), G.SO3vec(p[2], p[3]), maxl=3)
+    out = [t.as_subclass(torch.Tensor) for t in list(z.parts.values()) + [G.SO3part_CGproductFn.apply(p[1], p[2], 2)]]
+    for got in torch.autograd.grad(out, p, grad_outputs=[torch.ones_like(t) for t in out]):
+        assert type(got) is torch.Tensor

@@ -246,3 +246,24 @@ def test_reference_python_package_imports_on_gelib_base():
     env = dict(os.environ, PYTHONPATH=root + os.pathsep + ref)
     r = subprocess.run([sys.executable, "-c", code], capture_output=True, text=True, env=env, timeout=300)
     assert r.returncode == 0 and "ok" in r.stdout, r.stdout + r.stderr
+
+
+def test_zeroed_gradients_have_the_class_that_zeros_like_gives():
+    import gelib_b200 as G
+    from gelib_b200.gelib_common import of_class, plain, zeros_like_all
+
+    class Mine(torch.Tensor):
+        pass
+
+    t = torch.randn(2, 3, 4, dtype=torch.complex64)
+    ts = [t, torch.nn.Parameter(t), G.SO3part(t), t.as_subclass(Mine), t.transpose(0, 2), t[:1].expand(5, 3, 4)]
+    with plain():
+        zs = zeros_like_all(ts)
+        singles = [of_class(torch.zeros_like(a), a) for a in ts]
+    for a, z, z1 in zip(ts, zs, singles):
+        want = torch.zeros_like(a)
+        for got in (z, z1):
+            assert type(got) is type(want)
+            assert got.shape == want.shape and got.stride() == want.stride() and not got.requires_grad
+            assert bool((got == 0).all())
+    assert zeros_like_all([]) == []

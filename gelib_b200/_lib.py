@@ -152,7 +152,7 @@ _TENSOR5 = struct.Struct("@P5i5q")
 assert _TENSOR5.size == ctypes.sizeof(Tensor5)
 
 
-def _pack(buf, at, t, real):
+def _pack(buf, at, t, real, written):
     if not t.is_cuda:
         raise RuntimeError("gelib_b200 computes on CUDA tensors only (this build has no CPU path); got a %s tensor"
                            % t.device.type)
@@ -164,6 +164,13 @@ def _pack(buf, at, t, real):
         if t.dtype != torch.complex64:
             raise RuntimeError("expected a complex64 tensor (an SO3part)")
         scale = 2
+        if t.is_conj():
+            # t.conj() only marks a view, and the kernels read memory.  The array keeps the copy until the call has been
+            # issued; after that the allocator hands its memory out in stream order.
+            if written:
+                raise RuntimeError("GElib error: a conjugated view cannot be written to.")
+            t = t.resolve_conj()
+            buf.__dict__.setdefault("copies", []).append(t)
     D, S = t.shape, t.stride()
     d = len(D)
     if d == 3:
@@ -182,24 +189,25 @@ def _pack(buf, at, t, real):
     _TENSOR5.pack_into(buf, at, t.data_ptr(), *D, *S)
 
 
-def descriptor(t, real=False):
+def descriptor(t, real=False, written=False):
     """``gelib_tensor5`` of a torch tensor in the reference's 5-D canonical form (core/Gpart.hpp:450-469).
 
     Complex tensors (b, [grid...], 2l+1, n) are viewed as interleaved floats, so strides double
-    (cuda/GPUtensor.hpp:31-38).  ``real=True`` is for the (b, [grid...], 3, n) float input of spharm.
+    (cuda/GPUtensor.hpp:31-38).  ``real=True`` is for the (b, [grid...], 3, n) float input of spharm, ``written=True`` for
+    a tensor that the call adds to or overwrites.
     """
     out = Tensor5()
     with torch._C.DisableTorchFunctionSubclass():
-        _pack(out, 0, t, real)
+        _pack(out, 0, t, real, written)
     return out
 
 
-def descriptor_array(tensors, real=False):
+def descriptor_array(tensors, real=False, written=False):
     arr = (Tensor5 * max(1, len(tensors)))()
     at = 0
     with torch._C.DisableTorchFunctionSubclass():
         for t in tensors:
-            _pack(arr, at, t, real)
+            _pack(arr, at, t, real, written)
             at += _TENSOR5.size
     return arr
 

@@ -177,6 +177,9 @@ def _gather(r, x, gmap, d, transposed):
         raise RuntimeError("gelib_b200: tensors must live on a CUDA device (there is no CPU path).")
     if not (r.is_contiguous() and x.is_contiguous()):
         raise RuntimeError("GElib error: add_gather needs contiguous tensors.")
+    if r.is_conj():
+        raise RuntimeError("GElib error: a conjugated view cannot be written to.")
+    x = x.resolve_conj()
     n_out, n_in = (gmap.n_in, gmap.n_out) if transposed else (gmap.n_out, gmap.n_in)
     if r.size(d + 1) != n_out or x.size(d + 1) != n_in:
         raise RuntimeError("GElib error: gather map does not match the array dimension.")
@@ -205,7 +208,7 @@ def mix_supported(x, w):
 def mix(x, w, adjoint=False):
     """x (.., n_in) times w (n_in, n_out), or with adjoint=True x (.., n_out) times w^H: a new dense tensor."""
     _one_device(x, w)
-    x, w = x.contiguous(), w.contiguous()
+    x, w = x.contiguous().resolve_conj(), w.contiguous().resolve_conj()
     n_in, n_out = w.size(0), w.size(1)
     rows = x.numel() // x.size(-1)
     r = torch.empty(list(x.shape[:-1]) + [n_in if adjoint else n_out], dtype=torch.complex64, device=x.device)
@@ -218,7 +221,7 @@ def mix(x, w, adjoint=False):
 def mix_back_w(x, g, n_in, n_out):
     """x^H g summed over all rows: the gradient of the weight matrix, (n_in, n_out)."""
     _one_device(x, g)
-    x, g = x.contiguous(), g.contiguous()
+    x, g = x.contiguous().resolve_conj(), g.contiguous().resolve_conj()
     rows = x.numel() // x.size(-1)
     wg = torch.zeros(n_in, n_out, dtype=torch.complex64, device=x.device)
     with device_guard(x):
@@ -252,7 +255,7 @@ class SO3part:
     def _call3(self, name, a, b, c, offs, flags=0):
         _one_device(a, b, c)
         with device_guard(a):
-            da, db, dc = descriptor(a), descriptor(b), descriptor(c)
+            da, db, dc = descriptor(a, written=True), descriptor(b), descriptor(c)
             return check(getattr(lib(), name)(ctypes.byref(da), ctypes.byref(db), ctypes.byref(dc), offs, flags,
                                               stream_of(a)))
 
@@ -279,7 +282,7 @@ class SO3part:
     def _back01(name, xg, yg, g, x, y, offs):
         _one_device(xg.t, yg.t, g.t, x.t, y.t)
         with device_guard(g.t):
-            d = [descriptor(v.t) for v in (xg, yg, g, x, y)]
+            d = [descriptor(v.t, written=v is xg or v is yg) for v in (xg, yg, g, x, y)]
             return check(getattr(lib(), name)(*[ctypes.byref(v) for v in d], offs, 0, stream_of(g.t)))
 
     @staticmethod
@@ -303,8 +306,8 @@ class SO3part:
         """self (+)= D x cell by cell; D a (2l+1, 2l+1) complex64 tensor on the same device."""
         _one_device(self.t, x.t, D)
         with device_guard(self.t):
-            dr, dx = descriptor(self.t), descriptor(x.t)
-            Dc = D.contiguous()
+            dr, dx = descriptor(self.t, written=True), descriptor(x.t)
+            Dc = D.contiguous().resolve_conj()
             return check(lib().gelib_SO3part_apply(ctypes.byref(dr), ctypes.byref(dx), Dc.data_ptr(),
                                                    GELIB_OVERWRITE if overwrite else 0, stream_of(self.t)))
 
@@ -314,7 +317,7 @@ class SO3part:
             X = X.unsqueeze(0)
         _one_device(self.t, X)
         with device_guard(self.t):
-            dr, dx = descriptor(self.t), descriptor(X, real=True)
+            dr, dx = descriptor(self.t, written=True), descriptor(X, real=True)
             check(lib().gelib_SO3part_addSPharm(ctypes.byref(dr), ctypes.byref(dx), GELIB_OVERWRITE if overwrite else 0,
                                                 stream_of(self.t)))
 
@@ -353,7 +356,7 @@ class SO3vec:
             return True
         _one_device(*(ta + tb + tc))
         with device_guard(ta[0]):
-            return check(getattr(lib(), name)(len(ta), descriptor_array(ta), len(tb), descriptor_array(tb), len(tc),
+            return check(getattr(lib(), name)(len(ta), descriptor_array(ta, written=True), len(tb), descriptor_array(tb), len(tc),
                                               descriptor_array(tc), flags, stream_of(ta[0])))
 
     def addCGproduct(self, x, y, *, overwrite=False, fp64=False):
@@ -370,7 +373,7 @@ class SO3vec:
         _one_device(*(tr + ty + [X]))
         with device_guard(tr[0]):
             dx = descriptor(X, real=True)
-            return check(lib().gelib_SO3vec_addCGproduct_spharm(len(tr), descriptor_array(tr), ctypes.byref(dx), lmax_x,
+            return check(lib().gelib_SO3vec_addCGproduct_spharm(len(tr), descriptor_array(tr, written=True), ctypes.byref(dx), lmax_x,
                                                                 len(ty), descriptor_array(ty),
                                                                 GELIB_OVERWRITE if overwrite else 0, stream_of(tr[0])))
 
@@ -380,7 +383,7 @@ class SO3vec:
         _one_device(*(tyg + tg + [X]))
         with device_guard(tg[0]):
             dx = descriptor(X, real=True)
-            return check(lib().gelib_SO3vec_addCGproduct_spharm_back1(len(tyg), descriptor_array(tyg), len(tg),
+            return check(lib().gelib_SO3vec_addCGproduct_spharm_back1(len(tyg), descriptor_array(tyg, written=True), len(tg),
                                                                       descriptor_array(tg), ctypes.byref(dx), lmax_x, 0,
                                                                       stream_of(tg[0])))
 
@@ -408,7 +411,8 @@ class SO3vec:
             raise RuntimeError("GElib error: gradient vectors must have the parts of x and y.")
         _one_device(*(txg + tyg + tg + tx + ty))
         with device_guard(tg[0]):
-            return check(getattr(lib(), name)(len(txg), descriptor_array(txg), len(tyg), descriptor_array(tyg),
+            return check(getattr(lib(), name)(len(txg), descriptor_array(txg, written=True), len(tyg),
+                                              descriptor_array(tyg, written=True),
                                               len(tg), descriptor_array(tg), descriptor_array(tx),
                                               descriptor_array(ty), 0, stream_of(tg[0])))
 
@@ -429,7 +433,7 @@ class SO3vec:
         _one_device(*(tr + [X]))
         with device_guard(tr[0]):
             dx = descriptor(X, real=True)
-            check(lib().gelib_SO3vec_addSPharm(len(tr), descriptor_array(tr), ctypes.byref(dx),
+            check(lib().gelib_SO3vec_addSPharm(len(tr), descriptor_array(tr, written=True), ctypes.byref(dx),
                                                GELIB_OVERWRITE if overwrite else 0, stream_of(tr[0])))
 
     def __repr__(self):

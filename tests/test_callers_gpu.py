@@ -247,3 +247,29 @@ def test_gradients_of_parameters_are_plain_tensors(G):
     out = [t.as_subclass(torch.Tensor) for t in list(z.parts.values()) + [G.SO3part_CGproductFn.apply(p[1], p[2], 2)]]
     for got in torch.autograd.grad(out, p, grad_outputs=[torch.ones_like(t) for t in out]):
         assert type(got) is torch.Tensor
+
+
+def test_conjugated_views_are_read_as_their_values(G):
+    """t.conj() only marks a view of t's memory: operands, weights and upstream gradients that are such views."""
+    x, y = crandn(1, 3, 3, 4).cuda(), crandn(2, 3, 5, 4).cuda()
+    w, D = crandn(3, 4, 4).cuda(), crandn(4, 3, 3).cuda()
+    gm = G.gather_map.sources_targets([0, 1, 1], [1, 0, 2], n_in=3, n_out=3)
+
+    def results(conj):
+        xc, yc, wc = conj(x), conj(y), conj(w)
+        out = [G.CGproduct(G.SO3part(xc), G.SO3part(yc), 2), G.DiagCGproduct(G.SO3part(xc), G.SO3part(yc), 2)]
+        out += list(G.CGproduct(G.SO3vec(xc, yc), G.SO3vec(yc), maxl=2).parts.values())
+        out += list((G.SO3vec(xc, yc) * G.SO3weights(wc, wc)).parts.values())
+        out += [G.gather(G.SO3partArr(conj(crandn(5, 2, 3, 5, 4).cuda())), gm, 0)]
+        r = torch.empty_like(x)
+        G.backend.SO3part.view(r).add_apply(G.backend.SO3part.view(xc), conj(D), overwrite=True)
+        leaves = [t.clone().requires_grad_() for t in (x, y, w)]
+        z = [G.CGproduct(G.SO3part(leaves[0]), G.SO3part(leaves[1]), 2)]
+        z += list(G.CGproduct(G.SO3vec(leaves[0]), G.SO3vec(leaves[1]), maxl=2).parts.values())
+        z += list((G.SO3vec(leaves[0]) * G.SO3weights(leaves[2])).parts.values())
+        z = [t.as_subclass(torch.Tensor) for t in z]
+        grads = torch.autograd.grad(z, leaves, grad_outputs=[conj(crandn(9, *t.shape).cuda()) for t in z])
+        return [t.as_subclass(torch.Tensor) for t in out + [r] + list(grads)]
+
+    for a, b in zip(results(torch.conj), results(torch.conj_physical)):
+        assert rel_err(a, b) < 1e-6

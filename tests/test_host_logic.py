@@ -134,6 +134,12 @@ def test_descriptor_canonical_form():
     assert list(d.strides)[0] == 0
     d = desc(torch.zeros(4, 3, 6), real=True)
     assert list(d.dims) == [4, 1, 1, 3, 6] and list(d.strides) == [18, 0, 0, 6, 1]
+    t = torch.randn(4, 5, 6, dtype=torch.complex64)
+    d = desc(t.conj())  # a lazily conjugated view: the kernels get memory with the conjugated values
+    got = np.ctypeslib.as_array(ctypes.cast(d.base, ctypes.POINTER(ctypes.c_float)), (4, 5, 6, 2))
+    assert (got[..., 0] == t.real.numpy()).all() and (got[..., 1] == -t.imag.numpy()).all()
+    with pytest.raises(RuntimeError):
+        desc(t.conj(), written=True)
     with pytest.raises(RuntimeError):
         desc(torch.zeros(4, 2, 3, 2, 5, 6, dtype=torch.complex64).transpose(1, 2))
     with pytest.raises(RuntimeError):

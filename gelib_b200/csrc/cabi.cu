@@ -249,7 +249,7 @@ int run_product(const char* fn, bool diag, int mode, int nr, const gelib_tensor5
   }
   const bool fp64 = (flags & GELIB_FP64) != 0;  // double coefficients and sums: the general strided kernels
   st = -1;
-  if (c.dense_channels && !(mode == 0 && c.r_bcast) && !fp64 && col_enabled()) {
+  if (c.dense_channels && !(mode == 0 && c.r_bcast) && !fp64 && col_mode() != kColOff) {
     bool plan_others = false;
     st = mode == 0 ? launch_col_fwd(c, s, &plan_others) : launch_col_bwd(c, s, &plan_others);
     if (plan_others) {  // should that fail, the call that needs the plan says so

@@ -383,7 +383,8 @@ int launch_cg_bwd(const VecCall& c, cudaStream_t s) {
   for (const auto& p : c.y) if (p.l > 2047 || p.n > 65535) return -1;
   for (const auto& p : c.r) if (p.l > 2047) return -1;
   // ---- plan: work lists of every lane layout that some batch size uses
-  std::vector<int> key = {3 /*family*/, vec ? 1 : 0, (int)c.x.size(), (int)c.y.size(), (int)c.r.size()};
+  const int pinned = pinned_layout(true);
+  std::vector<int> key = {3 /*family*/, pinned, vec ? 1 : 0, (int)c.x.size(), (int)c.y.size(), (int)c.r.size()};
   for (const auto& p : c.x) { key.push_back(p.l); key.push_back(p.n); }
   for (const auto& p : c.y) { key.push_back(p.l); key.push_back(p.n); }
   for (const auto& p : c.r) key.push_back(p.l);
@@ -426,7 +427,7 @@ int launch_cg_bwd(const VecCall& c, cudaStream_t s) {
     }
     struct It { int4 v0, v1; int cost; };
     p.tables.assign(2 * kNumCfgs, 0);  // per layout: {first entry of h_items, items}
-    for (int i : layouts_used(p.cost)) {
+    for (int i : layouts_used(p.cost, pinned)) {
       const int ta = kCfgs[i].TA * kCfgs[i].WA, tb = kCfgs[i].TBU * UB * kCfgs[i].WB;
       std::vector<It> its;
       for (const Triple& t : p.sched.triples) {
@@ -456,7 +457,8 @@ int launch_cg_bwd(const VecCall& c, cudaStream_t s) {
   });
   if (!plan) return GELIB_CUDA_ERROR;
   if (plan->sched.triples.empty() || c.cg.ncells == 0) return GELIB_OK;
-  const int best = choose_layout(plan->cost, c.cg.ncells);
+  const int best = choose_layout(plan->cost, c.cg.ncells, pinned);
+  if (best < 0 && pinned >= 0) return fail(GELIB_INVALID, fn, "the pinned lane layout does not fit the call");
   if (best < 0) return -1;  // caller falls back to the strided kernels
   if (c.plan_only) return GELIB_OK;
   const BwdCfg cfg = kCfgs[best];

@@ -245,7 +245,8 @@ int launch_cg_fwd(const VecCall& c, cudaStream_t s) {
     for (const auto& p : *v) cell_floats += 2 * (2 * p.l + 1) * (ceil_div(p.n, 4) * 4);
   // floats; tiles may read up to 128 past the last row
   auto smem_floats = [&](int WC) { return (size_t)cell_floats * WC + 128 + 2 * WC * kMaxParts; };
-  std::vector<int> key = {1 /*family*/, c.vec_ok ? 1 : 0, (int)c.x.size(), (int)c.y.size(), (int)c.r.size()};
+  const int pinned = pinned_layout(false);
+  std::vector<int> key = {1 /*family*/, pinned, c.vec_ok ? 1 : 0, (int)c.x.size(), (int)c.y.size(), (int)c.r.size()};
   for (const auto& p : c.x) { key.push_back(p.l); key.push_back(p.n); }
   for (const auto& p : c.y) { key.push_back(p.l); key.push_back(p.n); }
   for (const auto& p : c.r) key.push_back(p.l);
@@ -279,7 +280,7 @@ int launch_cg_fwd(const VecCall& c, cudaStream_t s) {
     }
     // per layout: {first item, items, first of its job tables}; a job table for every number of jobs up to kMaxJobs
     p.tables.assign(3 * kNumCfgs, 0);
-    for (int i : layouts_used(p.cost)) {
+    for (int i : layouts_used(p.cost, pinned)) {
       const int ta = kCfgs[i].TA * kCfgs[i].WA, tb = 4 * kCfgs[i].NBL;
       const int first = (int)p.h_items.size();
       std::vector<long long> cost;
@@ -312,7 +313,8 @@ int launch_cg_fwd(const VecCall& c, cudaStream_t s) {
   });
   if (!plan) return GELIB_CUDA_ERROR;
   if (plan->sched.triples.empty() || c.cg.ncells == 0) return GELIB_OK;
-  const int best = choose_layout(plan->cost, c.cg.ncells);
+  const int best = choose_layout(plan->cost, c.cg.ncells, pinned);
+  if (best < 0 && pinned >= 0) return fail(GELIB_INVALID, fn, "the pinned lane layout does not fit the call");
   if (best < 0) return -1;  // caller falls back to the strided kernel
   if (c.plan_only) return GELIB_OK;
   const TileCfg cfg = kCfgs[best];

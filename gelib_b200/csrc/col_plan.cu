@@ -383,7 +383,8 @@ bool col_setup(const VecCall& c, bool backward, ColArgs* a, ColPlan* plan) {
       if ((uintptr_t)p.base % 16 || p.sb % 4 || p.sg0 % 4 || p.sg1 % 4 || p.sm % 4) two = false;
   // two columns share the records, coefficients and control of a step; with few columns warps matter more
   const long long columns = c.cg.ncells * n;
-  plan->cpl = two && columns >= 64 * 148 * 4 ? 2 : 1;
+  const int mode = col_mode();
+  plan->cpl = two && (mode == kColAuto ? columns >= 64 * 148 * 4 : mode == kColTwo) ? 2 : 1;
   // Calls that the other kernels do faster (measured, us, other kernel / this one):
   //   diagonal forward: with l >= 6 and full 64-channel slices diag_fwd_cell_kernel, which shares its operands between the
   //     warps of a block, fits more warps on an SM: maxl 8 x 128 channels, batch 2048 3018 / 3820; maxl 6 x 64 608 / 835,
@@ -394,7 +395,7 @@ bool col_setup(const VecCall& c, bool backward, ColArgs* a, ColPlan* plan) {
   //   its gradient of y: cg_narrow1_bwd_kernel under the same conditions and l >= 6: 65536 cells, maxl 6 x 16 5418 / 5609;
   //     but maxl 4 x 32, 5000 cells 356 / 331; 60000 cells, maxl 2 x 16 247 / 189; 4096 cells, maxl 6 x 16 638 / 370.
   // One column per lane (an odd channel count) does without what two share, so padding has to cost more before these win.
-  if (c.diag) {
+  if (c.diag && mode == kColAuto) {
     const int slices = (n + 63) / 64;
     if (!backward && max_la >= 6 && 8 * n >= 7 * 64 * slices) return false;
   }
@@ -405,7 +406,7 @@ bool col_setup(const VecCall& c, bool backward, ColArgs* a, ColPlan* plan) {
   const auto xs = sig_of(c.x), ys = sig_of(c.y), rs = sig_of(c.r);
   const bool diag = c.diag;
   plan->dev = get_plan(key, [&](DevicePlan& p) { build(p, xs, ys, rs, diag, backward, do_x, do_y); });
-  if (!c.diag && n > 1 && n <= 32) {  // reads the number of cells: another batch of the signature may go the other way
+  if (!c.diag && n > 1 && n <= 32 && mode == kColAuto) {  // reads the number of cells: another batch of the signature may go the other way
     int cw = 1;
     while (cw < n) cw *= 2;
     const long long narrow_warps = c.cg.ncells * cw / 32;
@@ -432,6 +433,10 @@ bool col_setup(const VecCall& c, bool backward, ColArgs* a, ColPlan* plan) {
   int walk = 0;  // as build() orders them
   while (!backward && walk < kMaxSplitLog && (warps << (walk + 1)) <= 148 * 12) walk++;
   plan->owned = backward && plan->cpl == 1 && warps <= (do_x && do_y ? 2 : 4) * 148;
+  if (mode != kColAuto) {
+    walk = !backward && mode == kColSplit ? kMaxSplitLog : 0;
+    plan->owned = backward && mode == kColSplit;
+  }
   if (plan->owned) walk = 1;
   a->accumulate = (c.flags & GELIB_OVERWRITE) ? 0 : 1;
 

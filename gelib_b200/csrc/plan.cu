@@ -40,7 +40,7 @@ bool upload(const std::vector<T>& h, T** d) {
 
 namespace {
 struct Options {
-  std::atomic<int> fwd{kFwdAuto}, bwd{kBwdAuto}, inject{0}, pair_tma{1}, narrow1{1}, col{1};
+  std::atomic<int> fwd{kFwdAuto}, bwd{kBwdAuto}, inject{0}, pair_tma{1}, narrow1{1}, col{kColAuto}, fwd_layout{-1}, bwd_layout{-1};
 };
 int parse_fwd(const char* v) {
   if (!v || !*v || !strcmp(v, "auto")) return kFwdAuto;
@@ -80,7 +80,8 @@ bool inject_timeout() { return options().inject.load(std::memory_order_relaxed) 
 bool pair_tma() { return options().pair_tma.load(std::memory_order_relaxed) != 0; }
 bool narrow1_enabled() { return options().narrow1.load(std::memory_order_relaxed) != 0; }
 
-bool col_enabled() { return options().col.load(std::memory_order_relaxed) != 0; }
+int col_mode() { return options().col.load(std::memory_order_relaxed); }
+int pinned_layout(bool backward) { return (backward ? options().bwd_layout : options().fwd_layout).load(std::memory_order_relaxed); }
 
 int set_option(const char* name, const char* value) {
   if (!name) return GELIB_INVALID;
@@ -102,7 +103,14 @@ int set_option(const char* name, const char* value) {
     return GELIB_OK;
   }
   if (!strcmp(name, "col")) {
-    o.col = !(value && !strcmp(value, "0"));
+    const char* names[] = {"auto", "0", "one", "two", "split"};
+    o.col = kColAuto;
+    for (int i = 0; i < 5; i++)
+      if (value && !strcmp(value, names[i])) o.col = i;
+    return GELIB_OK;
+  }
+  if (!strcmp(name, "fwd_layout") || !strcmp(name, "bwd_layout")) {
+    (name[0] == 'f' ? o.fwd_layout : o.bwd_layout) = value && *value >= '0' && *value <= '9' ? atoi(value) : -1;
     return GELIB_OK;
   }
   if (!strcmp(name, "pair_tma")) {
@@ -181,7 +189,8 @@ bool device_has_tcgen05() {
   return cc_major[dev] == 10;
 }
 
-int choose_layout(const std::vector<LayoutCost>& cost, long long ncells) {
+int choose_layout(const std::vector<LayoutCost>& cost, long long ncells, int pinned) {
+  if (pinned >= 0) return pinned < (int)cost.size() && cost[pinned].work > 0 ? pinned : -1;
   int shift = 0;
   while ((ncells >> shift) >= 16) shift++;
   const long long n = (ncells >> shift) << shift;
@@ -199,12 +208,12 @@ int choose_layout(const std::vector<LayoutCost>& cost, long long ncells) {
   return best;
 }
 
-std::vector<int> layouts_used(const std::vector<LayoutCost>& cost) {
+std::vector<int> layouts_used(const std::vector<LayoutCost>& cost, int pinned) {
   std::vector<bool> used(cost.size(), false);
   std::vector<int> v;
   for (int shift = 0; shift < 40; shift++)
     for (long long n = shift == 0 ? 1 : 8; n < 16; n++) {
-      const int i = choose_layout(cost, n << shift);
+      const int i = choose_layout(cost, n << shift, pinned);
       if (i >= 0 && !used[i]) {
         used[i] = true;
         v.push_back(i);

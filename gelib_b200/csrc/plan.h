@@ -35,8 +35,9 @@ DevicePlan* get_plan(const std::vector<int>& key, const std::function<void(Devic
 // Layout of the least estimated time for a number of cells, -1 when none fits.  The number is cut to its four leading bits
 // (the estimate is no finer), so that layouts_used can name every layout some batch size will choose: a plan holds the work
 // lists of all of them, and no later call of the signature, whatever its batch, builds or uploads anything.
-int choose_layout(const std::vector<LayoutCost>& cost, long long ncells);
-std::vector<int> layouts_used(const std::vector<LayoutCost>& cost);
+// With pinned >= 0 that layout is the only one.
+int choose_layout(const std::vector<LayoutCost>& cost, long long ncells, int pinned);
+std::vector<int> layouts_used(const std::vector<LayoutCost>& cost, int pinned);
 
 // Kernel families (each returns a status code; with c.plan_only they build their plan and return).
 int launch_cg_fwd(const VecCall& c, cudaStream_t s);
@@ -54,7 +55,12 @@ int launch_cg_strided_static(const VecCall& c, cudaStream_t s);  // forward, tab
 // at other batch sizes, and they have not planned it yet.
 int launch_col_fwd(const VecCall& c, cudaStream_t s, bool* plan_others);
 int launch_col_bwd(const VecCall& c, cudaStream_t s, bool* plan_others);
-bool col_enabled();  // option "col" (default on): tests compare the kernels
+// Option "col": by the rules of col_plan.cu, not at all ("0"), or, with every call that the column kernels can take, one or
+// two columns per lane with the walk in one piece ("one", "two"), or one column and the walk split over blocks ("split").
+// Tests pin what only large calls reach and compare the kernels.
+enum ColMode { kColAuto = 0, kColOff, kColOne, kColTwo, kColSplit };
+int col_mode();
+int pinned_layout(bool backward);  // options "fwd_layout" / "bwd_layout": lane layout of the FP32 kernels, -1 by the estimate
 int launch_diag_fwd(const VecCall& c, cudaStream_t s);
 int launch_diag_bwd(const VecCall& c, cudaStream_t s);
 int launch_diag_fwd_fast(const VecCall& c, cudaStream_t s);  // -1 when the call does not qualify

@@ -1,7 +1,8 @@
 """The column kernels (diagonal products, products with a one-channel x): every direction against the CPU oracle at the
-edges of their range -- column counts that do not fill a warp, few cells (the walk is split over blocks), pairs with more
-output l than one pass holds, types with gaps, truncated outputs, accumulation, broadcast operands, strided operands,
-grids -- and non-finite inputs."""
+edges of their range -- column counts that do not fill a warp, pairs with more output l than one pass holds, types with
+gaps, truncated outputs, accumulation, broadcast operands, strided operands, grids -- and non-finite inputs.  Each case runs
+by the rules ("auto": few cells, so mostly the walk split over blocks) and pinned to one and to two columns per lane with the
+walk in one piece, which the rules leave to calls too large for the oracle, and to the split walk."""
 import numpy as np
 import pytest
 import torch
@@ -20,6 +21,13 @@ def G():
     assert torch.cuda.is_available(), "these tests need a CUDA device"
     gelib_b200._lib.lib()
     return gelib_b200
+
+
+@pytest.fixture(params=["auto", "one", "two", "split"])
+def col(request, G):
+    G._lib.set_option("col", request.param)
+    yield request.param
+    G._lib.set_option("col", "auto")
 
 
 def parts(seed, B, tau, bcast=False):
@@ -43,6 +51,8 @@ CASES = [
     (True, 4, {1: 9, 4: 9}, {0: 9, 2: 9, 8: 9}, 6), (True, 3, U(3, 4), {12: 4, 20: 4}, -1), (True, 4700, U(1, 33), U(1, 33), 1),
     (False, 5, U(3, 1), U(3, 16), 3), (False, 33, U(6, 1), U(6, 16), 6), (False, 7, U(2, 1), U(4, 40), -1), (False, 300, U(2, 1), U(2, 7), 2),
     (False, 2, {0: 1, 7: 1}, {3: 65}, -1),
+    (True, 5, U(2, 34), U(2, 34), 2), (True, 2, {6: 48, 8: 48}, {0: 48, 7: 48}, 8), (False, 9, {0: 1, 5: 1}, U(4, 24), 5),
+    (True, 2, {9: 17}, {9: 17}, 4),  # beyond the column kernels: one cell per CTA
 ]
 
 
@@ -79,23 +89,25 @@ def check(G, oracle, diag, B, tx, ty, maxl, xb=False, yb=False):
 
 
 @pytest.mark.parametrize("diag,B,tx,ty,maxl", CASES)
-def test_products_and_gradients(G, oracle, diag, B, tx, ty, maxl):
+def test_products_and_gradients(G, oracle, col, diag, B, tx, ty, maxl):
     check(G, oracle, diag, B, tx, ty, maxl)
 
 
 @pytest.mark.parametrize("diag,tx,ty", [(True, U(3, 12), U(3, 12)), (True, U(2, 40), U(2, 40)), (False, U(2, 1), U(2, 16))])
 @pytest.mark.parametrize("xb,yb", [(True, False), (False, True)])
-def test_operand_broadcast_over_the_batch(G, oracle, diag, tx, ty, xb, yb):
+def test_operand_broadcast_over_the_batch(G, oracle, col, diag, tx, ty, xb, yb):
     check(G, oracle, diag, 9, tx, ty, 3, xb, yb)
 
 
-@pytest.mark.parametrize("diag", [True, False])
-def test_strided_rows_and_grids(G, oracle, diag):
-    """Operands cut out of larger tensors, on a contiguous grid and on one that is no arithmetic progression of cells."""
-    n, nx = 12, 12 if diag else 1
+@pytest.mark.parametrize("pad", [3, 4])
+@pytest.mark.parametrize("diag,n", [(True, 12), (True, 20), (False, 12)])
+def test_strided_rows_and_grids(G, oracle, col, diag, n, pad):
+    """Operands cut out of larger tensors (rows a multiple of 16 bytes apart or not), on a contiguous grid and on one that
+    is no arithmetic progression of cells and goes to the other kernels (with 20 channels: one cell per CTA)."""
+    nx = n if diag else 1
     for grid, cut in (((3,), False), ((3,), True), ((2, 3), False)):
         def make(seed, l, ch, odd):
-            t = crandn(seed, 4, *[k + (cut and i == 0) for i, k in enumerate(grid)], 2 * l + 1, ch + (3 if odd else 0)).cuda()
+            t = crandn(seed, 4, *[k + (cut and i == 0) for i, k in enumerate(grid)], 2 * l + 1, ch + (pad if odd else 0)).cuda()
             return t[:, :grid[0]][..., :ch] if odd or cut else t
         x = {l: make(l, l, nx, True) for l in range(3)}
         y = {l: make(10 + l, l, n, l == 1) for l in range(3)}
@@ -110,7 +122,15 @@ def test_strided_rows_and_grids(G, oracle, diag):
             assert rel_err(r[l].reshape(cells, 2 * l + 1, -1), want[l]) < TOL, (grid, cut, l)
         g = {l: torch.randn_like(t) for l, t in r.items()}
         yg = {l: torch.zeros(4, *grid, 2 * l + 1, n, dtype=torch.complex64, device="cuda") for l in y}
-        (vec(G, yg).addDiagCGproduct_back1 if diag else vec(G, yg).addCGproduct_back1)(vec(G, g), vec(G, x))
+        if diag:
+            xg = {l: torch.zeros(4, *grid, 2 * l + 1, n, dtype=torch.complex64, device="cuda") for l in x}
+            G.backend.SO3vec.addDiagCGproduct_back01(vec(G, xg), vec(G, yg), vec(G, g), vec(G, x), vec(G, y))
+            wx = {l: np.zeros((cells, 2 * l + 1, n), np.complex64) for l in x}
+            oracle.vec_cg_back0(wx, flat(g), flat(y), diag)
+            for l in wx:
+                assert rel_err(xg[l].reshape(cells, 2 * l + 1, -1), wx[l]) < TOL, (grid, cut, l)
+        else:
+            vec(G, yg).addCGproduct_back1(vec(G, g), vec(G, x))
         wy = {l: np.zeros((cells, 2 * l + 1, n), np.complex64) for l in y}
         oracle.vec_cg_back1(wy, flat(g), flat(x), diag)
         for l in wy:
@@ -118,9 +138,9 @@ def test_strided_rows_and_grids(G, oracle, diag):
 
 
 @pytest.mark.parametrize("l", [1, 4, 8])
-def test_an_infinity_stays_in_its_band(G, oracle, l):
+def test_an_infinity_stays_in_its_band(G, oracle, col, l):
     """x[m1] = inf reaches the rows that m1 couples to and no other."""
-    tx, ty = {l: 5}, {l: 5}
+    tx, ty = {l: 6}, {l: 6}
     x, y = parts(1, 3, tx), parts(50, 3, ty)
     x[l][1, 0, 2] = complex(float("inf"), 0.)
     tr = oracle.cg_type(tx, ty, 15, True)

@@ -338,6 +338,7 @@ def test_vec_backward_named_kernel(G, oracle, opt, B, tau_x, tau_y, maxl, tol, b
         assert rel_err(p - 1, 2 * w) < tol
 
 
+@pytest.mark.parametrize("kernel", ["column", "narrow"])
 @pytest.mark.parametrize("overwrite", [True, False])
 @pytest.mark.parametrize("B,lx,tau_y,maxl,bcast", [
     (5, 3, {0: 16, 1: 16, 2: 16, 3: 16}, 3, False),     # two cells per warp
@@ -345,9 +346,10 @@ def test_vec_backward_named_kernel(G, oracle, opt, B, tau_x, tau_y, maxl, tol, b
     (4, 4, {0: 32, 2: 32}, 6, False),                    # one cell per warp, truncated output
     (6, 2, {0: 8, 1: 8, 2: 8}, 2, True),                 # y broadcast over the batch
 ])
-def test_forward_for_single_channel_x(G, oracle, B, lx, tau_y, maxl, bcast, overwrite):
-    """The forward with a one-channel x (the narrow kernel) against the oracle, overwriting an output full of garbage
-    and accumulating on top of ones."""
+def test_forward_for_single_channel_x(G, oracle, opt, B, lx, tau_y, maxl, bcast, overwrite, kernel):
+    """The forward with a one-channel x (the column kernel, which takes small calls, and the narrow kernel) against the
+    oracle, overwriting an output full of garbage and accumulating on top of ones."""
+    opt("col", "auto" if kernel == "column" else "0")
     tau_x = {l: 1 for l in range(lx + 1)}
     x, y = _vec_inputs(tau_x, tau_y, B, 800)
     if bcast:
@@ -364,7 +366,7 @@ def test_forward_for_single_channel_x(G, oracle, B, lx, tau_y, maxl, bcast, over
         assert rel_err(p if overwrite else p - 1, w) < TOL
 
 
-@pytest.mark.parametrize("kernel", ["single-channel", "general"])
+@pytest.mark.parametrize("kernel", ["column", "single-channel", "general"])
 @pytest.mark.parametrize("B,lx,tau_y,maxl,bcast", [
     (5, 3, {0: 16, 1: 16, 2: 16, 3: 16}, 3, False),     # two cells per warp
     (3, 2, {1: 5, 2: 5}, 4, False),                      # channel count that is not a power of two, gaps in l
@@ -372,8 +374,10 @@ def test_forward_for_single_channel_x(G, oracle, B, lx, tau_y, maxl, bcast, over
     (6, 2, {0: 8, 1: 8, 2: 8}, 2, True),                 # y broadcast over the batch: its gradient is a sum over cells
 ])
 def test_gradient_of_y_for_single_channel_x(G, oracle, opt, B, lx, tau_y, maxl, bcast, kernel):
-    """back1 alone with a one-channel x (the first layer after spherical harmonics): the kernel that walks the band
-    once per (l1,l2) pair and the general narrow kernel must both give the oracle's gradient, on top of what yg holds."""
+    """back1 alone with a one-channel x (the first layer after spherical harmonics): the column kernel, the kernel that
+    walks the band once per (l1,l2) pair and the general narrow kernel must all give the oracle's gradient, on top of what
+    yg holds."""
+    opt("col", "auto" if kernel == "column" else "0")
     opt("narrow1", "1" if kernel == "single-channel" else "0")
     tau_x = {l: 1 for l in range(lx + 1)}
     x, y = _vec_inputs(tau_x, tau_y, B, 700)
@@ -548,9 +552,12 @@ def test_tcgen05_refuses_what_it_cannot_do(G, opt):
 
 # ---- the benchmark configurations' own layouts ----------------------------------------------------------------
 
-def test_diag_vector_maxl8_128_channels(G, oracle):
+@pytest.mark.parametrize("col", ["auto", "one", "two", "split", "0"])
+def test_diag_vector_maxl8_128_channels(G, oracle, opt, col):
     """DiagCGproduct of SO3vecs with parts l = 0..8, 128 channels each, truncated at 8 (369 triples): the layout of the
-    diagonal benchmark configuration, which takes the one-cell-per-CTA kernels with multi-chunk staging."""
+    diagonal benchmark configuration.  The column kernels in each of their forms, and ("0") the one-cell-per-CTA kernels
+    with multi-chunk staging; at that batch size the forward takes the latter and the backward two columns per lane."""
+    opt("col", col)
     B, tau = 2, {l: 128 for l in range(9)}
     x, y = _vec_inputs(tau, tau, B, 20)
     tau_r = oracle.cg_type(tau, tau, 8, True)

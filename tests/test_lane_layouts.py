@@ -1,5 +1,6 @@
 """The lane layouts of the FP32 product kernels: channel counts around the tile sizes of every layout, batches that do not
-fill a warp's cells, and calls small enough that several blocks share a cell (gradients added with atomics)."""
+fill a warp's cells, and calls small enough that several blocks share a cell (gradients added with atomics).  Small calls
+choose few of the layouts, so each is pinned once."""
 import numpy as np
 import pytest
 import torch
@@ -29,6 +30,32 @@ def test_uniform_vectors(G, oracle, n1, n2, B, lmax):
 @pytest.mark.parametrize("B", [2, 150])
 def test_ragged_vectors(G, oracle, tx, ty, maxl, B):
     run(G, oracle, B, tx, ty, maxl)
+
+
+# the layouts of the kernels: {n1 and n2 of a warp's tile, cells of a warp}, in their order
+FWD = [(16, 32, 1), (8, 32, 1), (16, 16, 2), (1, 16, 8), (8, 8, 8), (8, 8, 4), (4, 8, 8), (1, 4, 32), (16, 4, 8)]
+BWD = [(32, 32, 1), (16, 16, 2), (8, 8, 8), (8, 8, 4), (8, 16, 2), (1, 16, 8), (4, 4, 8), (16, 2, 8)]
+
+
+@pytest.fixture
+def pinned(G):
+    def pin(fwd, bwd):
+        for name, value in (("fwd", "simt"), ("bwd", "simt"), ("col", "0"), ("fwd_layout", fwd), ("bwd_layout", bwd)):
+            G._lib.set_option(name, value)
+
+    yield pin
+    for name in ("fwd", "bwd", "col", "fwd_layout", "bwd_layout"):
+        G._lib.set_option(name, "auto")
+
+
+@pytest.mark.parametrize("kernel,index", [("fwd", i) for i in range(len(FWD))] + [("bwd", i) for i in range(len(BWD))])
+@pytest.mark.parametrize("d1,d2", [(0, 0), (-1, 1), (1, -1), (1, 2)])
+def test_every_layout_around_its_tile(G, oracle, pinned, kernel, index, d1, d2):
+    """A pinned layout (a call that it does not fit would be refused), with cells that do not fill a warp."""
+    n1, n2, cells = (FWD if kernel == "fwd" else BWD)[index]
+    n1, n2 = max(5, n1 + d1), max(1, n2 + d2)  # a narrow x has kernels of its own
+    pinned(index if kernel == "fwd" else "auto", index if kernel == "bwd" else "auto")
+    run(G, oracle, cells + 3, {0: n1, 2: n1}, {1: n2, 2: n2}, 3)
 
 
 def run(G, oracle, B, tx, ty, maxl):

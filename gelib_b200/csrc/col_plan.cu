@@ -340,6 +340,26 @@ bool fill_part(const PartView& p, const CellGrid& cg, long long extra_floats, bo
   return true;
 }
 
+// One-channel x: whether the kernels of cg_narrow.cu / cg_narrow1_bwd.cu are faster.  Their lanes are padded to a power of
+// two of channels (cw) and they want a full chip; one column per lane does without what two columns share.  us, column
+// kernel / narrow kernel, maxl x channels, cells:
+//   forward, l <= 1: 1 x 12 2400 9.2 / 7.9, 24000 27 / 22; 300 cells 6.6 / 7.1.  l <= 3: 2 x 16 2400 21 / 19, 24000 90 / 63.
+//     From l = 4 on padding decides: 4 x 24 12000 331 / 394, 4 x 5 19200 416 / 522, 4 x 21 2400 95 / 119, 12000 495 / 473,
+//     6 x 21 909 / 1167 at 4800; without it 4 x 32 330 / 191 at 4800.
+//   gradient of y, one column per lane: l <= 1 1 x 11 2400 9.3 / 11.2, 24000 41 / 30; 1 x 21 12000 43 / 29; above, padding
+//     decides: 4 x 5 19200 191 / 397, 4 x 21 4800 208 / 346; 3 x 13 2400 41 / 76 but 4800 96 / 81, 4 x 31 2400 195 / 179, 12000 641 / 569.
+//   gradient of y, two columns: without padding l <= 1, l >= 6 and 32 channels lose: 6 x 16 24000 2389 / 2113, 3 x 32 12000
+//     286 / 265; but 2 x 16 24000 82 / 107, and with padding 6 x 24 4800 798 / 1231, 6 x 28 802 / 1258.
+bool narrow_wins(bool backward, int cpl, int n, int max_la, long long cells) {
+  int cw = 1;
+  while (cw < n) cw *= 2;
+  const long long warps = cells * cw / 32;
+  const bool padded = 4 * n <= 3 * cw;
+  if (!backward) return warps >= 148 * (max_la <= 1 ? 4 : 16) && !(max_la >= 4 && padded);
+  if (!narrow1_enabled() || warps < 148 * 16) return false;
+  return cpl == 1 ? max_la <= 1 || !padded : n == cw && (max_la <= 1 || max_la >= 6 || n == 32);
+}
+
 }  // namespace
 
 bool col_setup(const VecCall& c, bool backward, ColArgs* a, ColPlan* plan) {
@@ -385,16 +405,9 @@ bool col_setup(const VecCall& c, bool backward, ColArgs* a, ColPlan* plan) {
   const long long columns = c.cg.ncells * n;
   const int mode = col_mode();
   plan->cpl = two && (mode == kColAuto ? columns >= 64 * 148 * 4 : mode == kColTwo) ? 2 : 1;
-  // Calls that the other kernels do faster (measured, us, other kernel / this one):
-  //   diagonal forward: with l >= 6 and full 64-channel slices diag_fwd_cell_kernel, which shares its operands between the
-  //     warps of a block, fits more warps on an SM: maxl 8 x 128 channels, batch 2048 3018 / 3820; maxl 6 x 64 608 / 835,
-  //     maxl 6 x 128 1208 / 1265; but maxl 5 x 128 711 / 661, maxl 8 x 48, batch 1000 821 / 652.
-  //   one-channel x: cg_narrow_fwd_kernel when it fills the chip and wastes no lanes (its rows are padded to a power of two):
-  //     30000 cells, maxl 4 x 32 channels 900 / 1174; 16000, maxl 6 x 16 1274 / 1362; but 4096 cells 467 / 367, 1000 cells
-  //     357 / 151; 40000 cells, maxl 6 x 24 5043 / 4281.
-  //   its gradient of y: cg_narrow1_bwd_kernel under the same conditions and l >= 6: 65536 cells, maxl 6 x 16 5418 / 5609;
-  //     but maxl 4 x 32, 5000 cells 356 / 331; 60000 cells, maxl 2 x 16 247 / 189; 4096 cells, maxl 6 x 16 638 / 370.
-  // One column per lane (an odd channel count) does without what two share, so padding has to cost more before these win.
+  // Diagonal forward: with l >= 6 and full 64-channel slices diag_fwd_cell_kernel, which shares its operands between the
+  // warps of a block, fits more warps on an SM (us, that kernel / this one): maxl 8 x 128 channels, batch 2048 3018 / 3820;
+  // maxl 6 x 64 608 / 835, maxl 6 x 128 1208 / 1265; but maxl 5 x 128 711 / 661, maxl 8 x 48, batch 1000 821 / 652.
   if (c.diag && mode == kColAuto) {
     const int slices = (n + 63) / 64;
     if (!backward && max_la >= 6 && 8 * n >= 7 * 64 * slices) return false;
@@ -406,13 +419,9 @@ bool col_setup(const VecCall& c, bool backward, ColArgs* a, ColPlan* plan) {
   const auto xs = sig_of(c.x), ys = sig_of(c.y), rs = sig_of(c.r);
   const bool diag = c.diag;
   plan->dev = get_plan(key, [&](DevicePlan& p) { build(p, xs, ys, rs, diag, backward, do_x, do_y); });
-  if (!c.diag && n > 1 && n <= 32 && mode == kColAuto) {  // reads the number of cells: another batch of the signature may go the other way
-    int cw = 1;
-    while (cw < n) cw *= 2;
-    const long long narrow_warps = c.cg.ncells * cw / 32;
-    const bool padded = plan->cpl == 2 ? 4 * n <= 3 * cw : 5 * n <= 3 * cw;
-    if (!backward && narrow_warps >= 148 * 16 && !(max_la >= 4 && padded)) return false;
-    if (backward && narrow1_enabled() && narrow_warps >= 148 * 32 && (max_la >= 6 || plan->cpl == 1) && !padded) return false;
+  if (!c.diag && n > 1 && n <= 32 && mode == kColAuto) {
+    // the rule reads the number of cells: another batch of the signature may go the other way
+    if (narrow_wins(backward, plan->cpl, n, max_la, c.cg.ncells)) return false;
     plan->plan_others = plan->dev && plan->dev->first_use.exchange(false);
   }
   if (!plan->dev) return true;

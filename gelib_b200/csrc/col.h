@@ -20,10 +20,12 @@
 // the k rows that come kColRing later, so the bytes in flight do not depend on how short the steps are.  What the warps
 // of a block share is the walk itself: a chunk (row addresses, step records, coefficients stored twice for the packed
 // multiply-adds) is copied to shared memory one chunk ahead.
-// Gradient rows are added to global memory with red.  A row belongs to one lane of one block, so the sums have one order and
-// gradients are bitwise repeatable, except those of an operand that is broadcast over cells (stride 0).  Calls with few
-// columns split the walk over blocks; in the backward each of these takes everything that is added to one a block's rows
-// (an "owned" run, in which either part of a pair may be the larger one).
+// Gradient rows are added to global memory with red.  Unless an operand is broadcast over cells (stride 0) a row belongs to
+// one lane of one block, so the sums have one order and gradients are bitwise repeatable.  Calls with few columns split the
+// walk over blocks; in the backward by gradient rows ("owned": the blocks of a cluster walk everything that is added to the
+// rows of their group, in which either part of a pair may be the larger one, and sum at the end in the order of their ranks).
+// Diagonal products of more than 16 channels and one-channel x with more than 32, which no other kernel sums in one order,
+// may instead split by pairs, and then several blocks add to a row.
 // Why this form: diag_bwd_cell_kernel spends its time in four shared-memory atomics (compare-and-swap loops) per band
 // entry, which a lane that owns its column does not need.  Measured, backward of the diagonal product: maxl 8 x 128
 // channels, batch 2048 10.5 -> 4.8 ms; maxl 6 x 33, batch 4000 4.3 -> 1.1 ms; maxl 3 x 12, batch 500 49 -> 18 us (forward 32 ->
@@ -41,7 +43,9 @@ constexpr int kColBlockBwd = 11;                // a rows per block, backward (r
 constexpr int kColBlockFwd = 17;                // a rows per block, forward
 constexpr int kColChunkBytes = 13312;           // capacity of a chunk buffer
 constexpr int kColMaxSmem = 232448;
+constexpr int kColSumRows = 48;                 // gradient rows that the blocks of a cluster sum (owned walks)
 constexpr int kColSlots = 3 * kMaxParts;        // x parts, y parts, r (g) parts
+constexpr int kColFixedSmem = 16 * kColSlots + 2 * kColChunkBytes;  // part table, chunk buffers
 
 // Output l that a step of nl is worked on with (zero coefficients beyond nl): the body of a step is instantiated per block
 // size and for each of these numbers.  With both gradients the bodies are long and fetching them is what costs most, so
@@ -66,16 +70,18 @@ struct ColArgs {
   int b_rows;                      // rows of the largest b part
   int accumulate;                  // forward: add to r instead of storing
   const int4* blob;
-  const int* chunks;               // per split {first chunk, number of chunks, first record of the ring prologue}, then
-                                   // per chunk {offset, size} in int4 units
-  int nsplits;
+  const int* chunks;               // per run {first chunk, number of chunks, first record of the ring prologue, list of the
+                                   // rows that its group sums}, then per chunk {offset, size} in int4 units
+  int nsplits;                     // runs
+  int cluster, sum_rows;           // owned walks: blocks that sum rows together, rows of a lane's sums
 };
 
 struct ColPlan {
   DevicePlan* dev;
   int max_block;  // a rows of the largest block
   int cpl;        // columns per lane
-  bool owned;     // backward with few columns: one run per a block
+  bool owned;     // backward with few columns: the walk is cut by gradient rows
+  int warps;      // of a block, for an owned walk
   bool plan_others;  // first use of a signature that goes to other kernels at other batch sizes: they should plan it too
 };
 

@@ -20,6 +20,34 @@ __device__ __forceinline__ Row<CPL> to_row(const float2 (&v)[CPL]) {
   return r;
 }
 
+template <int CPL>
+__device__ __forceinline__ void add_slot(unsigned char* p, const float2 (&v)[CPL]) {
+  const Row<CPL> o = lds_row<CPL>(p);
+  float2 s[CPL];
+#pragma unroll
+  for (int c = 0; c < CPL; c++) {
+    unpack2(o.c[c], s[c].x, s[c].y);
+    s[c].x += v[c].x;
+    s[c].y += v[c].y;
+  }
+  sts_row<CPL>(p, to_row<CPL>(s));
+}
+
+// The row at p (shared memory) of block `rank` of the cluster.
+template <int CPL>
+__device__ __forceinline__ Row<CPL> lds_row_of(const unsigned char* p, int rank) {
+  uint32_t a;
+  asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a) : "r"((uint32_t)__cvta_generic_to_shared(p)), "r"(rank));
+  Row<CPL> v;
+#pragma unroll
+  for (int c = 0; c < CPL; c++) asm volatile("ld.shared::cluster.b64 %0, [%1];" : "=l"(v.c[c]) : "r"(a + 8 * c) : "memory");
+  return v;
+}
+__device__ __forceinline__ void cluster_sync() {
+  asm volatile("barrier.cluster.arrive.release;" ::: "memory");
+  asm volatile("barrier.cluster.wait.acquire;" ::: "memory");
+}
+
 // One step: an output row of a pair against the a block.  Entry i pairs a[i] with the b row at bptr - i rows.
 template <int K, int CPL, bool DOA, bool DOB, int NL, int NLMIN = NL - 1>
 __device__ __forceinline__ void bwd_step(Walk<CPL>& W, int st, const float2 (&a)[K][CPL], float2 (&ag)[K][CPL], float2 (&bg)[K][CPL],
@@ -76,8 +104,9 @@ __device__ __forceinline__ void bwd_step(Walk<CPL>& W, int st, const float2 (&a)
   W.coef += K * NL * 8;
 }
 
-// bval, bacc: byte offsets of the lane's slots of b row 0 (values, gradients).
-template <int K, int CPL, bool DOA, bool DOB>
+// bval, bacc: byte offsets of the lane's slots of b row 0 (values, gradients).  OWNED: the a rows' gradients are added to
+// slots from bacc on instead of to global memory.
+template <int K, int CPL, bool DOA, bool DOB, bool OWNED>
 __device__ __forceinline__ void bwd_segment(Walk<CPL>& W, const int4 h, int lb, uint32_t bval, uint32_t bacc) {
   constexpr int NLMAX = K < 6 ? K + 1 : kColMaxNl;  // six rows and more may be a part of a larger a part
   constexpr uint32_t kRow = Walk<CPL>::kRow;
@@ -90,18 +119,7 @@ __device__ __forceinline__ void bwd_segment(Walk<CPL>& W, const int4 h, int lb, 
   const int nsteps = h.x >> 16, nb = 2 * lb + 1;
   int br = h.y + lb;  // row of b that entry 0 meets
   auto leave = [&](int r, const float2 (&v)[CPL]) {
-    if ((unsigned)r < (unsigned)nb) {
-      unsigned char* p = W.smem + bacc + kRow * r;
-      const Row<CPL> o = lds_row<CPL>(p);
-      float2 s[CPL];
-#pragma unroll
-      for (int c = 0; c < CPL; c++) {
-        unpack2(o.c[c], s[c].x, s[c].y);
-        s[c].x += v[c].x;
-        s[c].y += v[c].y;
-      }
-      sts_row<CPL>(p, to_row<CPL>(s));
-    }
+    if ((unsigned)r < (unsigned)nb) add_slot<CPL>(W.smem + bacc + kRow * r, v);
   };
   const uint32_t steps = W.seg + 32;
   int next = *reinterpret_cast<const int*>(W.smem + steps);
@@ -135,7 +153,10 @@ __device__ __forceinline__ void bwd_segment(Walk<CPL>& W, const int4 h, int lb, 
     for (int i = 1; i < K; i++) leave(br - i, bg[i]);
   }
   W.seg = steps + 4 * ((nsteps + 3) & ~3);
-  if (DOA && W.ok) {
+  if constexpr (OWNED) {
+#pragma unroll
+    for (int i = 0; i < K; i++) add_slot<CPL>(W.smem + bacc + kRow * i, ag[i]);
+  } else if (DOA && W.ok) {
     const ColPart& p = W.A.grad[((h.x >> 8) & kColHalf1 ? kMaxParts : 0) + h.w];
     unsigned char* q = reinterpret_cast<unsigned char*>(p.base) + (unsigned long long)W.cell * p.cell_stride + 8ull * CPL * W.ch +
                        (unsigned long long)h.z * p.unit;
@@ -144,40 +165,32 @@ __device__ __forceinline__ void bwd_segment(Walk<CPL>& W, const int4 h, int lb, 
   }
 }
 
-// OWNED: a run of the walk holds everything that is added to the rows of one a block, and only those are computed.
-template <int KMAX, int CPL, bool DOX, bool DOY, int THREADS, bool OWNED>
-__global__ void __launch_bounds__(THREADS, 1) col_bwd_kernel(const __grid_constant__ ColArgs A) {
-  extern __shared__ __align__(16) unsigned char smem[];
-  constexpr uint32_t kRow = Walk<CPL>::kRow, kSets = OWNED ? 1 : 2;
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nwarps = blockDim.x >> 5;
-  // [part table][two chunk buffers][rings][b rows and, unless OWNED, their gradients, per warp]
-  const uint32_t bufs = 16 * kColSlots, rings = bufs + 2 * kColChunkBytes, slots = rings + nwarps * Walk<CPL>::kRing;
-  const uint32_t bval = slots + warp * kSets * kRow * A.b_rows + 8 * CPL * lane, bacc = bval + kRow * A.b_rows;
-  Walk<CPL> W(A, smem);
-  W.set_lane((blockIdx.x * nwarps + warp) * 32 + lane);
-  W.start(0, bufs, rings + warp * Walk<CPL>::kRing);
+// One run of the walk.
+template <int KMAX, int CPL, bool DOX, bool DOY, bool OWNED>
+__device__ __forceinline__ void walk_bwd(Walk<CPL>& W, uint32_t bufs, uint32_t ring, uint32_t bval, uint32_t bacc) {
+  constexpr uint32_t kRow = Walk<CPL>::kRow;
+  Row<CPL> zero;
+#pragma unroll
+  for (int c = 0; c < CPL; c++) zero.c[c] = 0ull;
+  W.start(0, bufs, ring);
   int f;
   do {
-    const int4 h = *reinterpret_cast<const int4*>(smem + W.seg), h1 = *reinterpret_cast<const int4*>(smem + W.seg + 16);
+    const int4 h = *reinterpret_cast<const int4*>(W.smem + W.seg), h1 = *reinterpret_cast<const int4*>(W.smem + W.seg + 16);
     const int kb = h.x & 255, nb = 2 * h1.y + 1;
     f = (h.x >> 8) & 255;
     const bool half1 = (f & kColHalf1) != 0;
     const bool do_a = OWNED || (half1 ? DOY : DOX), do_b = !OWNED && (half1 ? DOX : DOY);
     if (f & kColFirstOfB) {
       if (do_a) W.take_to(bval, nb);
-      if (do_b) {
-        Row<CPL> z;
-#pragma unroll
-        for (int c = 0; c < CPL; c++) z.c[c] = 0ull;
-        for (int r = 0; r < nb; r++) sts_row<CPL>(smem + bacc + kRow * r, z);
-      }
+      if (do_b)
+        for (int r = 0; r < nb; r++) sts_row<CPL>(W.smem + bacc + kRow * r, zero);
     }
-#define GELIB_COL_CASE(N)                                                                        \
-  if constexpr (N <= KMAX)                                                                       \
-    if (kb == N) {                                                                               \
-      if constexpr (OWNED) bwd_segment<N, CPL, true, false>(W, h, h1.y, bval, bacc);             \
-      else if (DOX == DOY || !half1) bwd_segment<N, CPL, DOX, DOY>(W, h, h1.y, bval, bacc);      \
-      else bwd_segment<N, CPL, DOY, DOX>(W, h, h1.y, bval, bacc);                                \
+#define GELIB_COL_CASE(N)                                                                          \
+  if constexpr (N <= KMAX)                                                                         \
+    if (kb == N) {                                                                                 \
+      if constexpr (OWNED) bwd_segment<N, CPL, true, false, true>(W, h, h1.y, bval, bacc + kRow * h1.z); \
+      else if (DOX == DOY || !half1) bwd_segment<N, CPL, DOX, DOY, false>(W, h, h1.y, bval, bacc); \
+      else bwd_segment<N, CPL, DOY, DOX, false>(W, h, h1.y, bval, bacc);                           \
     }
     if (kb <= 5) {
       GELIB_COL_CASE(1)
@@ -193,28 +206,91 @@ __global__ void __launch_bounds__(THREADS, 1) col_bwd_kernel(const __grid_consta
     }
 #undef GELIB_COL_CASE
     if (do_b && (f & kColLastOfB) && W.ok) {  // the gradient rows of the b part go to global memory
-      const ColPart& p = A.grad[(half1 ? 0 : kMaxParts) + h1.x];
+      const ColPart& p = W.A.grad[(half1 ? 0 : kMaxParts) + h1.x];
       unsigned char* q = reinterpret_cast<unsigned char*>(p.base) + (unsigned long long)W.cell * p.cell_stride + 8ull * CPL * W.ch;
-      for (int r = 0; r < nb; r++) red_row<CPL>(q + (unsigned long long)r * p.unit, lds_row<CPL>(smem + bacc + kRow * r));
+      for (int r = 0; r < nb; r++) red_row<CPL>(q + (unsigned long long)r * p.unit, lds_row<CPL>(W.smem + bacc + kRow * r));
     }
     if ((f & kColLastOfChunk) && !(f & kColLast)) W.next_chunk((f & kColDrain) != 0);
   } while (!(f & kColLast));
   cp_wait<0>();
 }
 
+// OWNED: the blocks of a cluster walk everything that is added to the gradient rows of their group, and only these are
+// computed.  Each lane sums in slots of its own; at the end the blocks share the rows out and add up each other's sums, in
+// the order of their ranks, through distributed shared memory.
+template <int KMAX, int CPL, bool DOX, bool DOY, int THREADS, bool OWNED>
+__global__ void __launch_bounds__(THREADS, 1) col_bwd_kernel(const __grid_constant__ ColArgs A) {
+  extern __shared__ __align__(16) unsigned char smem[];
+  constexpr uint32_t kRow = Walk<CPL>::kRow;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nwarps = blockDim.x >> 5;
+  // [part table][two chunk buffers][rings][b rows and their gradients (OWNED: sums), per warp]
+  const uint32_t bufs = 16 * kColSlots, rings = bufs + 2 * kColChunkBytes, slots = rings + nwarps * Walk<CPL>::kRing;
+  const uint32_t bval = slots + warp * kRow * (A.b_rows + (OWNED ? A.sum_rows : A.b_rows)) + 8 * CPL * lane;
+  const uint32_t bacc = bval + kRow * A.b_rows;
+  Walk<CPL> W(A, smem);
+  W.set_lane((blockIdx.x * nwarps + warp) * 32 + lane);
+  Row<CPL> zero;
+#pragma unroll
+  for (int c = 0; c < CPL; c++) zero.c[c] = 0ull;
+  bool work = true;
+  if constexpr (OWNED) {
+    for (int r = 0; r < A.sum_rows; r++) sts_row<CPL>(smem + bacc + kRow * r, zero);
+    work = __ldg(A.chunks + 4 * blockIdx.y + 1) > 0;  // a cluster may have more blocks than segments
+  }
+  if (work) walk_bwd<KMAX, CPL, DOX, DOY, OWNED>(W, bufs, rings + warp * Walk<CPL>::kRing, bval, bacc);
+  if constexpr (OWNED) {
+    const int rank = blockIdx.y % A.cluster;
+    const int4* list = A.blob + __ldg(A.chunks + 4 * blockIdx.y + 3);
+    const int rows = __ldg(&list[0].x);
+    if (A.cluster > 1) cluster_sync();
+    for (int r = rank; r < rows; r += A.cluster) {
+      float2 s[CPL];
+#pragma unroll
+      for (int c = 0; c < CPL; c++) s[c] = make_float2(0.f, 0.f);
+      for (int k = 0; k < A.cluster; k++) {
+        const Row<CPL> v = lds_row_of<CPL>(smem + bacc + kRow * r, k);
+#pragma unroll
+        for (int c = 0; c < CPL; c++) {
+          float re, im;
+          unpack2(v.c[c], re, im);
+          s[c].x += re;
+          s[c].y += im;
+        }
+      }
+      const int4 d = __ldg(&list[1 + r]);
+      const ColPart& p = A.grad[d.x];
+      unsigned char* q = reinterpret_cast<unsigned char*>(p.base) + (unsigned long long)W.cell * p.cell_stride + 8ull * CPL * W.ch;
+      if (W.ok) red_row<CPL>(q + (unsigned long long)d.y * p.unit, to_row<CPL>(s));
+    }
+    if (A.cluster > 1) cluster_sync();  // a block's slots stay until every block has read them
+  }
+}
+
 template <int KMAX, int CPL, bool DOX, bool DOY, int THREADS, bool OWNED = false>
-cudaError_t launch_bwd(const ColArgs& a, cudaStream_t s) {
-  const size_t fixed = 16 * kColSlots + 2 * kColChunkBytes;
-  const size_t per_warp = Walk<CPL>::kRow * (kColRing + (OWNED ? 1 : 2) * (size_t)a.b_rows);
+cudaError_t launch_bwd(const ColArgs& a, cudaStream_t s, int block_warps = 0) {
+  const size_t per_warp = Walk<CPL>::kRow * (kColRing + (size_t)a.b_rows + (OWNED ? a.sum_rows : a.b_rows));
   const unsigned warps = (a.nlanes + 31) / 32;
-  int nw = (int)std::min<size_t>(THREADS / 32, (kColMaxSmem - fixed) / per_warp);
-  nw = col_block_warps(warps, a.nsplits, nw);
-  const size_t smem = fixed + nw * per_warp;
+  int nw = (int)std::min<size_t>(THREADS / 32, (kColMaxSmem - kColFixedSmem) / per_warp);
+  nw = block_warps > 0 ? std::min(nw, block_warps) : col_block_warps(warps, a.nsplits, nw);
+  const size_t smem = kColFixedSmem + nw * per_warp;
   auto k = col_bwd_kernel<KMAX, CPL, DOX, DOY, THREADS, OWNED>;
   cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e != cudaSuccess) return e;
-  k<<<dim3((warps + nw - 1) / nw, a.nsplits), nw * 32, smem, s>>>(a);
-  return cudaGetLastError();
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3((warps + nw - 1) / nw, a.nsplits);
+  cfg.blockDim = nw * 32;
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = s;
+  cudaLaunchAttribute cluster;
+  cluster.id = cudaLaunchAttributeClusterDimension;
+  cluster.val.clusterDim.x = 1;
+  cluster.val.clusterDim.y = a.cluster;
+  cluster.val.clusterDim.z = 1;
+  if (OWNED) {
+    cfg.attrs = &cluster;
+    cfg.numAttrs = 1;
+  }
+  return cudaLaunchKernelEx(&cfg, k, a);
 }
 
 template <bool DOX, bool DOY>

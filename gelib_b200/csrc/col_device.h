@@ -65,7 +65,7 @@ __device__ __forceinline__ void red_row(unsigned char* p, const Row<CPL>& v) {
 
 // Header of a chunk: {byte offsets of the request list, the store list, the segments, the coefficients}, then
 // {address records, 0, 0, 0} and the address records.  A segment: {a rows | flags<<8 | steps<<16, d = m - mlo of the first
-// step, first a row, a part}, {b part, lb, 0, 0}, and one int per step (padded to four): nl | first entry of the band<<8 |
+// step, first a row, a part}, {b part, lb, first row of the sums (owned walks), 0}, and one int per step (padded to four): nl | first entry of the band<<8 |
 // last<<16.
 template <int CPL>
 struct Walk {
@@ -162,7 +162,7 @@ struct Walk {
   }
 
   __device__ __forceinline__ void fetch(int c) {  // copies chunk c into the buffer that is not in use
-    const int* t = A.chunks + 3 * A.nsplits + 2 * c;
+    const int* t = A.chunks + 4 * A.nsplits + 2 * c;
     const int off = __ldg(t), size = __ldg(t + 1);
     const uint32_t dst = (uint32_t)__cvta_generic_to_shared(smem) + buf0 + (which ^ 1) * kColChunkBytes;
     for (int e = threadIdx.x; e < size; e += blockDim.x)
@@ -175,7 +175,7 @@ struct Walk {
     which ^= 1;
     const uint32_t b = buf0 + which * kColChunkBytes;
     // the records' count lies in a word that another thread may have copied: it is read from global memory
-    const int* t = A.chunks + 3 * A.nsplits + 2 * chunk;
+    const int* t = A.chunks + 4 * A.nsplits + 2 * chunk;
     const int nrec = __ldg(&A.blob[__ldg(t) + 1].x);
     for (int e = threadIdx.x; e < nrec + 2; e += blockDim.x)
       if (e >= 2) {
@@ -207,7 +207,7 @@ struct Walk {
       const unsigned long long b = reinterpret_cast<unsigned long long>(p.base);
       *reinterpret_cast<uint4*>(smem + part_off + 16 * e) = make_uint4((unsigned)b, (unsigned)(b >> 32), p.unit, p.cell_stride);
     }
-    const int* sp = A.chunks + 3 * blockIdx.y;
+    const int* sp = A.chunks + 4 * blockIdx.y;
     chunk = __ldg(sp);
     chunk_end = chunk + __ldg(sp + 1);
     const int pro = __ldg(sp + 2);

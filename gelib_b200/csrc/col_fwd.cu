@@ -142,11 +142,11 @@ __global__ void __launch_bounds__(THREADS, 1) col_fwd_kernel(const __grid_consta
 
 template <int KMAX, int CPL, int THREADS>
 cudaError_t launch_fwd(const ColArgs& a, cudaStream_t s) {
-  const size_t fixed = 16 * kColSlots + 2 * kColChunkBytes, per_warp = Walk<CPL>::kRow * (kColRing + (size_t)a.b_rows);
+  const size_t per_warp = Walk<CPL>::kRow * (kColRing + (size_t)a.b_rows);
   const unsigned warps = (a.nlanes + 31) / 32;
-  int nw = (int)std::min<size_t>(THREADS / 32, (kColMaxSmem - fixed) / per_warp);
+  int nw = (int)std::min<size_t>(THREADS / 32, (kColMaxSmem - kColFixedSmem) / per_warp);
   nw = col_block_warps(warps, a.nsplits, nw);
-  const size_t smem = fixed + nw * per_warp;
+  const size_t smem = kColFixedSmem + nw * per_warp;
   auto k = col_fwd_kernel<KMAX, CPL, THREADS>;
   cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e != cudaSuccess) return e;

@@ -25,13 +25,23 @@ long long cell_stride(const PartView& p, const CellGrid& cg) {
   return any ? st : 0;
 }
 
-constexpr int kMaxSplitLog = 4;  // forward: at most 16 runs
+// How a walk is cut for the blocks that share a set of columns: into `groups` runs of pairs, or, with a cluster, by gradient
+// rows ("owned"): into groups of rows, each of whose walks is cut for the blocks of a cluster.
+struct Split {
+  int groups, cluster;
+};
+constexpr Split kSplitsFwd[] = {{1, 0}, {2, 0}, {4, 0}, {8, 0}, {16, 0}};
+constexpr Split kSplitsBwd[] = {{1, 0}, {999, 1}, {1, 2}, {1, 4}, {1, 8}, {2, 8}, {4, 8}, {8, 8}, {16, 8}, {2, 0}, {4, 0}, {8, 0}, {16, 0}};
+// Words of p.tables for a walk: {first word in h_jobs, runs, blocks of a cluster, most rows that a group sums, cost of the
+// longest run, cost of all}.
+constexpr int kTable = 6;
 
 struct Step {
   int m, nl, lo, hi;  // output row, output l, first and last entry of the band
 };
 struct Segment {
   int half, ai, bi, la, lb, mlo, kb;  // mlo, kb: first m1 and number of rows of the a block
+  int sum0 = 0;                       // owned walks: where the a block's rows lie among those that the group sums
   std::vector<Step> steps;
   std::vector<const Triple*> ls;      // the triples of the pair's l group, ascending l
   int flags = 0;
@@ -134,10 +144,10 @@ double cost_of(const std::vector<Segment>& v) {
   return c;
 }
 
-// Appends one walk to the plan (whose schedule and coefficients are there): `splits` runs of pairs, or owned runs.  Its place
-// goes to p.tables: {first word in h_jobs, runs}.
+// Appends one walk to the plan (whose schedule and coefficients are there) and describes it in p.tables.
 void build_walk(DevicePlan& p, const std::vector<PartSig>& xs, const std::vector<PartSig>& ys, const std::vector<PartSig>& rs,
-                bool backward, bool do_x, bool do_y, int splits, bool owned) {
+                bool backward, bool do_x, bool do_y, const Split& split) {
+  const bool owned = split.cluster > 0;
   Builder B{rs, backward, do_x, do_y, owned};
   std::map<std::pair<int, int>, std::vector<const Triple*>> pairs;
   for (const Triple& t : p.sched.triples) pairs[{t.xi, t.yi}].push_back(&t);
@@ -159,8 +169,26 @@ void build_walk(DevicePlan& p, const std::vector<PartSig>& xs, const std::vector
   };
 
   std::vector<std::vector<Segment>> runs;
+  std::vector<std::vector<int2>> sums;  // owned: per group, the gradient rows {slot, row} that its blocks sum
+  // contiguous runs of about equal cost
+  auto cut = [&](const std::vector<Segment>& all, int pieces) {
+    const double total = cost_of(all);
+    double done = 0;
+    size_t next = 0;
+    for (int sp = 0; sp < pieces && next < all.size(); sp++) {
+      std::vector<Segment> run;
+      const double until = total * (sp + 1) / pieces;
+      while (next < all.size() && (run.empty() || sp + 1 == pieces || done + 0.5 * all[next].cost <= until)) {
+        done += all[next].cost;
+        run.push_back(all[next++]);
+      }
+      runs.push_back(std::move(run));
+    }
+  };
   if (owned) {
-    // a run per block of rows of a part whose gradient is wanted: every pair of that part, with it as the a side
+    // A unit: a block of rows of a part whose gradient is wanted, with every pair of that part, it as the a side.
+    struct Unit { std::vector<Segment> segs; int slot, row0; double cost; };
+    std::vector<Unit> units;
     for (int half = 0; half < 2; half++) {
       if (half == 0 ? !do_x : !do_y) continue;
       const auto& as = half == 0 ? xs : ys;
@@ -168,22 +196,53 @@ void build_walk(DevicePlan& p, const std::vector<PartSig>& xs, const std::vector
       for (int ai = 0; ai < (int)as.size(); ai++) {
         int mlo = -as[ai].l;
         for (int kb : a_blocks(2 * as[ai].l + 1, max_block)) {
-          std::vector<Segment> run;
+          Unit u{{}, half * kMaxParts + ai, mlo + as[ai].l, 0};
           for (int bi = 0; bi < (int)bs.size(); bi++) {
             const auto* ts = triples(half, ai, bi);
             if (!ts) continue;
             Segment s = segment(half, ai, bi);
             s.mlo = mlo;
             s.kb = kb;
-            pair_segments(B, *ts, s, &run);
+            pair_segments(B, *ts, s, &u.segs);
           }
           mlo += kb;
-          if (!run.empty()) runs.push_back(std::move(run));
+          u.cost = cost_of(u.segs);
+          if (!u.segs.empty()) units.push_back(std::move(u));
         }
       }
     }
-    std::stable_sort(runs.begin(), runs.end(),  // the longest start first
-                     [](const std::vector<Segment>& u, const std::vector<Segment>& v) { return cost_of(u) > cost_of(v); });
+    // Groups of units, the longest unit to the group that has least so far; a group's walk is cut for the blocks of a cluster.
+    std::stable_sort(units.begin(), units.end(), [](const Unit& u, const Unit& v) { return u.cost > v.cost; });
+    const int most = std::min<int>(split.groups, (int)units.size());
+    std::vector<std::vector<Segment>> groups(most);
+    std::vector<double> load(most, 0.);
+    sums.resize(most);
+    for (Unit& u : units) {
+      const int kb = u.segs[0].kb;
+      int g = -1;
+      for (int k = 0; k < (int)groups.size(); k++)
+        if ((int)sums[k].size() + kb <= kColSumRows && (g < 0 || load[k] < load[g])) g = k;
+      if (g < 0) {  // no group has room for its rows
+        g = (int)groups.size();
+        groups.emplace_back();
+        load.push_back(0.);
+        sums.emplace_back();
+      }
+      for (Segment& s : u.segs) {
+        s.sum0 = (int)sums[g].size();
+        groups[g].push_back(std::move(s));
+      }
+      for (int i = 0; i < kb; i++) sums[g].push_back(make_int2(u.slot, u.row0 + i));
+      load[g] += u.cost;
+    }
+    for (auto& g : groups) {
+      std::stable_sort(g.begin(), g.end(), [](const Segment& s, const Segment& t) {  // the rows of a b part are fetched once
+        return s.half != t.half ? s.half < t.half : s.bi < t.bi;
+      });
+      const size_t first = runs.size();
+      cut(g, split.cluster);
+      runs.resize(first + split.cluster);  // fewer segments than blocks: the others only take part in the sums
+    }
   } else {
     // all segments in order: half, b part, a part, block of a rows, group of l, piece of m
     std::vector<Segment> all;
@@ -203,24 +262,16 @@ void build_walk(DevicePlan& p, const std::vector<PartSig>& xs, const std::vector
           }
         }
     }
-    // splits: contiguous runs of about equal cost
-    const double total = cost_of(all);
-    double done = 0;
-    size_t next = 0;
-    for (int sp = 0; sp < splits && next < all.size(); sp++) {
-      std::vector<Segment> run;
-      const double until = total * (sp + 1) / splits;
-      while (next < all.size() && (run.empty() || sp + 1 == splits || done + 0.5 * all[next].cost <= until)) {
-        done += all[next].cost;
-        run.push_back(all[next++]);
-      }
-      runs.push_back(std::move(run));
-    }
+    cut(all, split.groups);
   }
 
   std::vector<int> split_table, chunk_table;
-  int nchunks = 0;
-  for (auto& run : runs) {
+  int nchunks = 0, sum_rows = 0;
+  double longest = 0, total = 0;
+  for (size_t ri = 0; ri < runs.size(); ri++) {
+    auto& run = runs[ri];
+    longest = std::max(longest, cost_of(run));
+    total += cost_of(run);
     auto same_b = [](const Segment& s, const Segment& t) { return s.half == t.half && s.bi == t.bi; };
     for (size_t k = 0; k < run.size(); k++) {
       Segment& s = run[k];
@@ -257,6 +308,13 @@ void build_walk(DevicePlan& p, const std::vector<PartSig>& xs, const std::vector
     split_table.push_back((int)chunks.size());
     split_table.push_back((int)p.h_items.size());
     for (int j = 0; j < kColRing; j++) p.h_items.push_back(rec(j));
+    split_table.push_back((int)p.h_items.size());
+    if (owned) {
+      const auto& rows = sums[ri / split.cluster];
+      sum_rows = std::max(sum_rows, (int)rows.size());
+      p.h_items.push_back(make_int4((int)rows.size(), 0, 0, 0));
+      for (const int2& r : rows) p.h_items.push_back(make_int4(r.x, r.y, 0, 0));
+    }
     for (size_t ci = 0; ci < chunks.size(); ci++) {
       const Chunk& c = chunks[ci];
       const size_t row_end = ci + 1 < chunks.size() ? chunks[ci + 1].row_begin : B.rows.size();
@@ -275,7 +333,7 @@ void build_walk(DevicePlan& p, const std::vector<PartSig>& xs, const std::vector
       for (size_t q = c.from; q < c.to; q++) {
         const Segment& s = run[q];
         v.push_back(make_int4(s.kb | (s.flags << 8) | ((int)s.steps.size() << 16), s.steps[0].m - s.mlo, s.mlo + s.la, s.ai));
-        v.push_back(make_int4(s.bi, s.lb, 0, 0));
+        v.push_back(make_int4(s.bi, s.lb, s.sum0, 0));
         std::vector<int> w;
         for (const Step& st : s.steps) w.push_back(st.nl | (st.lo << 8) | (st.hi << 16));
         while (w.size() % 4) w.push_back(0);
@@ -311,8 +369,7 @@ void build_walk(DevicePlan& p, const std::vector<PartSig>& xs, const std::vector
       nchunks++;
     }
   }
-  p.tables.push_back((int)p.h_jobs.size());
-  p.tables.push_back((int)runs.size());
+  p.tables.insert(p.tables.end(), {(int)p.h_jobs.size(), (int)runs.size(), split.cluster, sum_rows, (int)longest, (int)total});
   p.h_jobs.insert(p.h_jobs.end(), split_table.begin(), split_table.end());
   p.h_jobs.insert(p.h_jobs.end(), chunk_table.begin(), chunk_table.end());
 }
@@ -321,12 +378,10 @@ void build_walk(DevicePlan& p, const std::vector<PartSig>& xs, const std::vector
 void build(DevicePlan& p, const std::vector<PartSig>& xs, const std::vector<PartSig>& ys, const std::vector<PartSig>& rs,
            bool diag, bool backward, bool do_x, bool do_y) {
   build_schedule(xs, ys, rs, diag, true, &p.sched);
-  if (backward) {
-    build_walk(p, xs, ys, rs, true, do_x, do_y, 1, false);
-    build_walk(p, xs, ys, rs, true, do_x, do_y, 1, true);
-  } else {
-    for (int k = 0; k <= kMaxSplitLog; k++) build_walk(p, xs, ys, rs, false, false, false, 1 << k, false);
-  }
+  if (backward)
+    for (const Split& sp : kSplitsBwd) build_walk(p, xs, ys, rs, true, do_x, do_y, sp);
+  else
+    for (const Split& sp : kSplitsFwd) build_walk(p, xs, ys, rs, false, false, false, sp);
   p.sched.coeffs.clear();  // they are in the walks
 }
 
@@ -338,6 +393,44 @@ bool fill_part(const PartView& p, const CellGrid& cg, long long extra_floats, bo
   out->unit = (unsigned)(4 * unit);
   out->cell_stride = (unsigned)(4 * cs);
   return true;
+}
+
+// The backward walk of the least estimated time, and the warps of a block for an owned one.  Fitted to 112 calls with every
+// owned walk each (maxl 1 .. 8, lopsided types, 2 .. 375 warps of columns; the choice loses 2 % on average, 28 % at worst): a
+// run takes 5 us and 2.5 ns per unit of its cost (2.8 with both gradients at once, which owned walks do not do), a little
+// more with every other warp on the SM, and a cluster's sums a microsecond and 40 ns a row.  120 of the 148 SMs hold clusters
+// of eight and 132 clusters of four; a second wave of clusters is never worth it, while blocks by themselves fill gaps.
+// Measured (us, diagonal products, both gradients): maxl 8 x 4 channels, batch 16 in one piece 564, a run per block of rows
+// 71, 64 runs in clusters of eight 29; x 16, batch 500 589, 298, 506; maxl 3 x 12, batch 100 35, 16, and 14 with 16 runs.
+// Runs of pairs that add to the same rows (the sums' order varies) are faster where the owned walk's second combination of
+// the g rows shows -- maxl 8 x 17, batch 192 55 against 171 -- and are open to calls that no kernel summed in one order.
+int choose_walk(const std::vector<int>& tables, long long warps, int b_rows, bool both, bool repeatable, int pinned, int* block_warps) {
+  int best = 0;
+  double best_time = 1e300;
+  const int walks = (int)tables.size() / kTable;
+  for (int k = 0; k < walks; k++) {
+    if (pinned >= 0 && k != std::min(pinned, walks - 1)) continue;
+    const int* t = &tables[kTable * k];
+    const int runs = t[1], cluster = t[2], slots = cluster == 0 ? 2 * b_rows : b_rows + t[3];
+    if (k > 0 && cluster == 0 && repeatable && pinned < 0) continue;
+    const int most = std::min(12, (kColMaxSmem - kColFixedSmem) / (256 * (kColRing + slots)));
+    const int blocks = cluster <= 2 ? 148 : cluster == 4 ? 132 : 120, sets = blocks / std::min(runs, blocks);
+    long long nw = std::max<long long>(2, (warps + sets - 1) / sets);
+    double cost = t[4];
+    if (nw > most || runs > blocks) {  // more than one wave
+      if (cluster > 1 && pinned < 0) continue;
+      nw = most;
+      cost = std::max(cost, (double)t[5] * ((warps + nw - 1) / nw) / blocks + 0.7 * cost);
+    }
+    const double time = 5.2 + 0.1 * (nw - 1) + (cluster > 1 ? 1 + 0.04 * t[3] : 0) +
+                        (cluster == 0 && both ? 2.8e-3 : 2.5e-3) * cost * (1 + 0.03 * (nw - 1));
+    if (time < best_time) {
+      best = k;
+      best_time = time;
+      *block_warps = cluster == 0 ? 0 : (int)nw;
+    }
+  }
+  return best;
 }
 
 // One-channel x: whether the kernels of cg_narrow.cu / cg_narrow1_bwd.cu are faster.  Their lanes are padded to a power of
@@ -433,25 +526,30 @@ bool col_setup(const VecCall& c, bool backward, ColArgs* a, ColPlan* plan) {
   a->n = (unsigned)(n / plan->cpl);
   a->nlanes = (unsigned)(c.cg.ncells * a->n);
   // With fewer warps than the chip holds, the walk is cut into runs that different blocks take: forward into runs of pairs;
-  // backward into one run per a block (owned), so that every gradient row is added to by one lane and the sums have one
-  // order.  The owned walk combines the g rows once per side and not once per pair, so with both gradients the whole walk
-  // wins earlier.  us, owned / whole, diagonal product of 15 channels: both gradients, 282 warps maxl 1 8.3 / 8.9, maxl 3
-  // 26 / 35, maxl 8 386 / 591; 375 warps 9.8 / 9.0, 37 / 35, 505 / 582; 563 warps 12 / 9, 40 / 35, 657 / 608.  One gradient,
-  // 563 warps 7.8 / 8.1, 23 / 30, 354 / 610; 703 warps 8.7 / 8.3, 30 / 33, 438 / 665; 938 warps 14 / 9, 42 / 33, 604 / 686.
+  // backward by gradient rows (owned), so that every row is added to by one lane and the sums have one order, or, where they
+  // need not, into runs of pairs.
   const long long warps = (a->nlanes + 31) / 32;
-  int walk = 0;  // as build() orders them
-  while (!backward && walk < kMaxSplitLog && (warps << (walk + 1)) <= 148 * 12) walk++;
-  plan->owned = backward && plan->cpl == 1 && warps <= (do_x && do_y ? 2 : 4) * 148;
-  if (mode != kColAuto) {
-    walk = !backward && mode == kColSplit ? kMaxSplitLog : 0;
-    plan->owned = backward && mode == kColSplit;
+  const std::vector<int>& tables = plan->dev->tables;
+  int walk = 0;
+  plan->warps = 0;
+  if (!backward) {
+    const int last = (int)tables.size() / kTable - 1;
+    if (mode == kColAuto)
+      while (walk < last && warps * kSplitsFwd[walk + 1].groups <= 148 * 12) walk++;
+    else if (mode >= kColSplit)
+      walk = std::min(last, mode - kColSplit);
+  } else if (plan->cpl == 1 && (mode == kColAuto || mode >= kColSplit)) {
+    const bool repeatable = n <= (c.diag ? 16 : 32);  // the kernels before these summed such calls in one order
+    walk = choose_walk(tables, warps, a->b_rows, do_x && do_y, repeatable, mode == kColAuto ? -1 : mode - kColSplit, &plan->warps);
   }
-  if (plan->owned) walk = 1;
+  plan->owned = backward && tables[kTable * walk + 2] > 0;
   a->accumulate = (c.flags & GELIB_OVERWRITE) ? 0 : 1;
 
   a->blob = plan->dev->items;
-  a->chunks = plan->dev->jobs + plan->dev->tables[2 * walk];
-  a->nsplits = plan->dev->tables[2 * walk + 1];
+  a->chunks = plan->dev->jobs + tables[kTable * walk];
+  a->nsplits = tables[kTable * walk + 1];
+  a->cluster = tables[kTable * walk + 2];
+  a->sum_rows = tables[kTable * walk + 3];
   return true;
 }
 

@@ -103,10 +103,11 @@ int set_option(const char* name, const char* value) {
     return GELIB_OK;
   }
   if (!strcmp(name, "col")) {
-    const char* names[] = {"auto", "0", "one", "two", "split"};
+    const char* names[] = {"auto", "0", "one", "two"};
     o.col = kColAuto;
-    for (int i = 0; i < 5; i++)
+    for (int i = 0; i < 4; i++)
       if (value && !strcmp(value, names[i])) o.col = i;
+    if (value && !strncmp(value, "split", 5) && atoi(value + 5) > 0) o.col = kColSplit + atoi(value + 5);
     return GELIB_OK;
   }
   if (!strcmp(name, "fwd_layout") || !strcmp(name, "bwd_layout")) {

@@ -56,9 +56,9 @@ int launch_cg_strided_static(const VecCall& c, cudaStream_t s);  // forward, tab
 int launch_col_fwd(const VecCall& c, cudaStream_t s, bool* plan_others);
 int launch_col_bwd(const VecCall& c, cudaStream_t s, bool* plan_others);
 // Option "col": by the rules of col_plan.cu, not at all ("0"), or, with every call that the column kernels can take, one or
-// two columns per lane with the walk in one piece ("one", "two"), or one column and the walk split over blocks ("split").
-// Tests pin what only large calls reach and compare the kernels.
-enum ColMode { kColAuto = 0, kColOff, kColOne, kColTwo, kColSplit };
+// two columns per lane with the walk in one piece ("one", "two"), or one column and the walk split over blocks in the k-th
+// of the plan's ways ("split1" ..).  Tests pin what only some batch sizes reach and compare the kernels.
+enum ColMode { kColAuto = 0, kColOff, kColOne, kColTwo, kColSplit /* + k */ };
 int col_mode();
 int pinned_layout(bool backward);  // options "fwd_layout" / "bwd_layout": lane layout of the FP32 kernels, -1 by the estimate
 int launch_diag_fwd(const VecCall& c, cudaStream_t s);

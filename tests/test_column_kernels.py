@@ -1,8 +1,8 @@
 """The column kernels (diagonal products, products with a one-channel x): every direction against the CPU oracle at the
 edges of their range -- column counts that do not fill a warp, pairs with more output l than one pass holds, types with
 gaps, truncated outputs, accumulation, broadcast operands, strided operands, grids -- and non-finite inputs.  Each case runs
-by the rules ("auto": few cells, so mostly the walk split over blocks) and pinned to one and to two columns per lane with the
-walk in one piece, which the rules leave to calls too large for the oracle, and to the split walk."""
+by the rules ("auto": few cells, so mostly the walk split over blocks), pinned to one and to two columns per lane with the
+walk in one piece, which the rules leave to calls too large for the oracle, and pinned to each way of splitting the walk."""
 import numpy as np
 import pytest
 import torch
@@ -23,7 +23,7 @@ def G():
     return gelib_b200
 
 
-@pytest.fixture(params=["auto", "one", "two", "split"])
+@pytest.fixture(params=["auto", "one", "two"] + ["split%d" % k for k in range(1, 13)])
 def col(request, G):
     G._lib.set_option("col", request.param)
     yield request.param
@@ -165,11 +165,13 @@ def test_an_infinity_stays_in_its_band(G, oracle, col, l):
 
 
 @pytest.mark.parametrize("diag,B,tx,ty,maxl", [
-    (True, 16, U(4, 8), U(4, 8), 4), (True, 500, U(3, 12), U(3, 12), 3), (True, 30, U(8, 16), U(8, 16), 8), (True, 40, U(3, 40), U(5, 40), 5),
+    (True, 16, U(4, 8), U(4, 8), 4), (True, 500, U(3, 12), U(3, 12), 3), (True, 30, U(8, 16), U(8, 16), 8), (True, 40, U(3, 15), U(5, 15), 5),
     (True, 4, U(3, 4), {9: 4, 12: 4, 20: 4}, -1), (False, 33, U(6, 1), U(6, 16), 6), (False, 500, U(4, 1), U(4, 8), 4),
 ])
-def test_gradients_are_repeatable(G, oracle, diag, B, tx, ty, maxl):
-    """Few columns: blocks share the walk, yet a gradient row is added to in one order."""
+def test_gradients_are_repeatable(G, oracle, col, diag, B, tx, ty, maxl):
+    """Few columns: blocks share the walk, yet a gradient row is added to in one order (but for splits by pairs, the last)."""
+    if col in ("split9", "split10", "split11", "split12"):
+        pytest.skip("several blocks add to a row")
     tr = oracle.cg_type(tx, ty, maxl, diag)
     x, y, g = cuda(parts(1, B, tx)), cuda(parts(100, B, ty)), cuda(parts(200, B, tr))
     x0, y0 = cuda(parts(300, B, tx)), cuda(parts(400, B, ty))

@@ -552,7 +552,7 @@ def test_tcgen05_refuses_what_it_cannot_do(G, opt):
 
 # ---- the benchmark configurations' own layouts ----------------------------------------------------------------
 
-@pytest.mark.parametrize("col", ["auto", "one", "two", "split", "0"])
+@pytest.mark.parametrize("col", ["auto", "one", "two", "split1", "split2", "split4", "split6", "0"])
 def test_diag_vector_maxl8_128_channels(G, oracle, opt, col):
     """DiagCGproduct of SO3vecs with parts l = 0..8, 128 channels each, truncated at 8 (369 triples): the layout of the
     diagonal benchmark configuration.  The column kernels in each of their forms, and ("0") the one-cell-per-CTA kernels

@@ -30,7 +30,7 @@ long long cell_stride(const PartView& p, const CellGrid& cg) {
 struct Split {
   int groups, cluster;
 };
-constexpr Split kSplitsFwd[] = {{1, 0}, {2, 0}, {4, 0}, {8, 0}, {16, 0}};
+constexpr Split kSplitsFwd[] = {{1, 0}, {2, 0}, {4, 0}, {8, 0}, {16, 0}, {32, 0}, {64, 0}};
 constexpr Split kSplitsBwd[] = {{1, 0}, {999, 1}, {1, 2}, {1, 4}, {1, 8}, {2, 8}, {4, 8}, {8, 8}, {16, 8}, {2, 0}, {4, 0}, {8, 0}, {16, 0}};
 // Words of p.tables for a walk: {first word in h_jobs, runs, blocks of a cluster, most rows that a group sums, cost of the
 // longest run, cost of all}.
@@ -527,7 +527,8 @@ bool col_setup(const VecCall& c, bool backward, ColArgs* a, ColPlan* plan) {
   a->nlanes = (unsigned)(c.cg.ncells * a->n);
   // With fewer warps than the chip holds, the walk is cut into runs that different blocks take: forward into runs of pairs;
   // backward by gradient rows (owned), so that every row is added to by one lane and the sums have one order, or, where they
-  // need not, into runs of pairs.
+  // need not, into runs of pairs.  Forward, us in 16 / 32 / 64 runs: maxl 8 x 16 channels, 30 cells 63 / 40 / 36, 128 cells
+  // 76 / 71 / 55; maxl 6 x 33, 4 cells 28 / 18 / 19; maxl 3 x 16, 30 cells 7.9 / 7.6 / 7.8.
   const long long warps = (a->nlanes + 31) / 32;
   const std::vector<int>& tables = plan->dev->tables;
   int walk = 0;

@@ -152,41 +152,57 @@ _TENSOR5 = struct.Struct("@P5i5q")
 assert _TENSOR5.size == ctypes.sizeof(Tensor5)
 
 
+_pack_into = _TENSOR5.pack_into
+_COMPLEX = torch.complex64
+
+
+def _resolved(buf, t, written):
+    """t.conj() only marks a view, and the kernels read memory.  The descriptor keeps the copy until the call has been issued;
+    after that the allocator hands its memory out in stream order."""
+    if written:
+        raise RuntimeError("GElib error: a conjugated view cannot be written to.")
+    t = t.resolve_conj()
+    buf.__dict__.setdefault("copies", []).append(t)
+    return t
+
+
 def _pack(buf, at, t, real, written):
     if not t.is_cuda:
         raise RuntimeError("gelib_b200 computes on CUDA tensors only (this build has no CPU path); got a %s tensor"
                            % t.device.type)
+    D = t.shape
+    d = len(D)
+    if d == 3 and not real and t.dtype is _COMPLEX:
+        if t.is_conj():
+            t = _resolved(buf, t, written)
+        b, m, n = D
+        sb, sm, sn = t.stride()
+        _pack_into(buf, at, t.data_ptr(), b, 1, 1, m, n, 2 * sb, 0, 0, 2 * sm, 2 * sn)
+        return
     if real:
         if t.dtype != torch.float32:
             raise RuntimeError("expected a float32 tensor")
         scale = 1
     else:
-        if t.dtype != torch.complex64:
+        if t.dtype != _COMPLEX:
             raise RuntimeError("expected a complex64 tensor (an SO3part)")
         scale = 2
         if t.is_conj():
-            # t.conj() only marks a view, and the kernels read memory.  The array keeps the copy until the call has been
-            # issued; after that the allocator hands its memory out in stream order.
-            if written:
-                raise RuntimeError("GElib error: a conjugated view cannot be written to.")
-            t = t.resolve_conj()
-            buf.__dict__.setdefault("copies", []).append(t)
-    D, S = t.shape, t.stride()
-    d = len(D)
-    if d == 3:
-        _TENSOR5.pack_into(buf, at, t.data_ptr(), D[0], 1, 1, D[1], D[2], scale * S[0], 0, 0, scale * S[1], scale * S[2])
-        return
+            t = _resolved(buf, t, written)
     if d < 3:
         raise RuntimeError("an SO3part has at least 3 dimensions (batch, 2l+1, channels)")
-    S = [scale * s for s in S]
-    if d == 4:
+    S = [scale * s for s in t.stride()]
+    if d == 3:
+        D = (D[0], 1, 1, D[1], D[2])
+        S = (S[0], 0, 0, S[1], S[2])
+    elif d == 4:
         D = (D[0], D[1], 1, D[2], D[3])
         S = (S[0], S[1], 0, S[2], S[3])
     elif d > 5:
         g, s = _fuse(D[1:d - 2], S[1:d - 2])
         D = (D[0], g, 1, D[d - 2], D[d - 1])
         S = (S[0], s, 0, S[d - 2], S[d - 1])
-    _TENSOR5.pack_into(buf, at, t.data_ptr(), *D, *S)
+    _pack_into(buf, at, t.data_ptr(), *D, *S)
 
 
 def descriptor(t, real=False, written=False):

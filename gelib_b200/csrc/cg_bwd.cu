@@ -319,16 +319,17 @@ __global__ void __launch_bounds__(256, 2) cg_bwd_kernel(const __grid_constant__ 
 
 struct BwdCfg {
   int TA, TBU, WA, WB;
+  double factor;  // measured time against the estimate
 };
 constexpr BwdCfg kCfgs[] = {
-    {4, 4, 8, 4},  // 32 x 32 channels (16 without vector loads), 1 cell per warp
-    {4, 2, 4, 4},  // 16 x 16, 2 cells
-    {4, 2, 2, 2},  //  8 x  8, 8 cells
-    {2, 2, 4, 2},  //  8 x  8, 4 cells
-    {2, 2, 4, 4},  //  8 x 16, 2 cells
-    {1, 2, 1, 4},  //  1 x 16, 8 cells
-    {2, 1, 2, 2},  //  4 x  4, 8 cells
-    {4, 1, 4, 1},  // 16 x  2, 8 cells
+    {4, 4, 8, 4, 1.0},   // 32 x 32 channels (16 without vector loads), 1 cell per warp
+    {4, 2, 4, 4, 1.0},   // 16 x 16, 2 cells
+    {4, 2, 2, 2, 1.7},   //  8 x  8, 8 cells
+    {2, 2, 4, 2, 1.0},   //  8 x  8, 4 cells
+    {2, 2, 4, 4, 1.05},  //  8 x 16, 2 cells
+    {1, 2, 1, 4, 0.8},   //  1 x 16, 8 cells
+    {2, 1, 2, 2, 1.05},  //  4 x  4, 8 cells
+    {4, 1, 4, 1, 1.3},   // 16 x  2, 8 cells
 };
 constexpr int kNumCfgs = sizeof(kCfgs) / sizeof(kCfgs[0]);
 
@@ -344,18 +345,29 @@ cudaError_t launch_cfg(const BwdArgs& a, dim3 grid, int threads, size_t smem, bo
 inline int ceil_div(int a, int b) { return (a + b - 1) / b; }
 inline int align4(int v) { return (v + 3) / 4 * 4; }
 
-// Whether the operands and gradients of wc cells, padded to ta x tb tiles, fit shared memory and the items' 16 bits.
-bool fits(const std::vector<PartSig>& xs, const std::vector<PartSig>& ys, int ta, int tb, int wc) {
+// Few cells: several blocks share a group of cells, each takes every splits-th round of slabs, and the rows are added to
+// global memory with atomics.  A block should still have two rounds.
+int splits_for(long long groups, const LayoutCost& c) {
+  int splits = 1;
+  while (splits < 16 && groups * splits * 2 <= 2 * 148 && c.items >= 2 * c.warps * splits * 2) splits *= 2;
+  return splits;
+}
+constexpr LayoutRule kRule = {8.8, splits_for};
+
+// Shared memory for the operands and gradients of wc cells, padded to ta x tb tiles; 0 when it is more than there is or the
+// padded counts leave the items' 16 bits.
+size_t smem_bytes(const std::vector<PartSig>& xs, const std::vector<PartSig>& ys, int ta, int tb, int wc) {
   size_t floats = 0;
   for (const auto& p : xs) {
-    if (ceil_div(p.n, ta) * ta > 65535) return false;
+    if (ceil_div(p.n, ta) * ta > 65535) return 0;
     floats += align4(2 * (2 * p.l + 1) * (ceil_div(p.n, ta) * ta));
   }
   for (const auto& p : ys) {
-    if (ceil_div(p.n, tb) * tb > 65535) return false;
+    if (ceil_div(p.n, tb) * tb > 65535) return 0;
     floats += align4(2 * (2 * p.l + 1) * (ceil_div(p.n, tb) * tb));
   }
-  return (6 * kMaxParts + 2 * floats) * wc * sizeof(float) <= 220 * 1024;
+  const size_t bytes = (6 * kMaxParts + 2 * floats) * wc * sizeof(float);
+  return bytes <= 220 * 1024 ? bytes : 0;
 }
 
 }  // namespace
@@ -393,11 +405,13 @@ int launch_cg_bwd(const VecCall& c, cudaStream_t s) {
     build_schedule(xs, ys, rs, false, true, &p.sched);
     std::vector<int> band;
     for (const Triple& t : p.sched.triples) band.push_back(band_size(t.l1, t.l2, t.l));
-    // The estimate of a layout's time: the instructions its warps execute.  Per band entry: 8 multiply-adds per complex
-    // number of the slab, the operand loads, the butterflies' shuffles and adds, and about five instructions per
-    // shared-memory atomic (they are compare-and-swap loops); per slab its loads.  The layouts differ in the padding of
-    // the channel counts and in how many multiply-adds share a butterfly; the work is spread over the warps the call can
-    // fill.  Measured (maxl 4 x 16 channels, batch 1000): 689 us with 8 x 16 channels per warp, 418 us with 16 x 16.
+    // The estimate of a layout's time: the instructions its warps issue, the latencies of staging a block's cells, and adding
+    // their rows up.  Per band entry: multiply-adds of the slab, operand loads, the butterflies' shuffles and adds, and the
+    // shared-memory atomics (compare-and-swap loops); per slab its loads.  The layouts differ in the padding of the channel
+    // counts, in how many multiply-adds share a butterfly and in the cells of a block.  The numbers are fitted to 1200 random
+    // calls with every layout each (up to 64 channels, l <= 5, 1 .. 4096 cells): the choice loses 2 % on average against the
+    // best layout.  Measured (maxl 4 x 16 channels, batch 1000): 689 us with 8 x 16 channels per warp, 418 us with 16 x 16;
+    // (maxl 3 x 9, batch 1368) 692 us with 8 x 8 and eight cells, 235 with 16 x 16.
     auto halving = [](int n, int e, int w, int* own) {  // shuffles of butterfly<n, e, w>, elements left per lane
       int sh = 0;
       for (int s = 1; s < w; s *= 2) {
@@ -409,25 +423,40 @@ int launch_cg_bwd(const VecCall& c, cudaStream_t s) {
     };
     for (const BwdCfg& f : kCfgs) {
       const int ta = f.TA * f.WA, tb = f.TBU * UB * f.WB, wc = 32 / (f.WA * f.WB);
-      LayoutCost lc{0, 0, wc};
-      if (fits(xs, ys, ta, tb, wc)) {
+      LayoutCost lc;
+      const size_t smem = smem_bytes(xs, ys, ta, tb, wc);
+      if (smem > 0) {
         int own_x, own_y;
         const int sh = halving(f.TA, 2, f.WB, &own_x) + halving(f.TBU, 2 * UB, f.WA, &own_y);
-        const double entry = 8.0 * f.TA * f.TBU * UB + f.TA + f.TBU + 2 * sh + 6 * (own_x + own_y) + 12, slab = 3.0 * f.TA * f.TBU + 30;
-        double items = 0;
+        const double entry = 0.6 * (8.0 * f.TA * f.TBU * UB + f.TA + f.TBU + 2 * sh + 12) + 13.0 * (own_x + own_y);
+        double work = 0;
         for (size_t i = 0; i < band.size(); i++) {
           const Triple& t = p.sched.triples[i];
-          const double tiles = (double)ceil_div(xs[t.xi].n, ta) * ceil_div(ys[t.yi].n, tb);
-          lc.work += tiles * (band[i] * entry + (2 * t.l + 1) * slab);
-          items += tiles * (2 * t.l + 1);
+          const long long tiles = (long long)ceil_div(xs[t.xi].n, ta) * ceil_div(ys[t.yi].n, tb);
+          work += (double)tiles * (band[i] * entry + (2 * t.l + 1) * (8.0 * f.TA * f.TBU + 115));
+          lc.items = (int)std::min(1LL << 30, lc.items + tiles * (2 * t.l + 1));
         }
-        lc.warps = std::min(128.0, std::max(8.0, items / 2));
+        lc.cells = wc;
+        lc.warps = std::max(1, std::min(8, lc.items));
+        lc.blocks = (int)std::min<size_t>(16 / lc.warps, 227 * 1024 / (smem + 1024));
+        lc.item = work / std::max(1, lc.items);
+        int rounds = 0, floats = 0;
+        auto part = [&](const PartSig& q, int tile) {
+          const int n = (2 * q.l + 1) * ceil_div(q.n, tile) * tile;
+          rounds += ceil_div(n, 32 * lc.warps);
+          floats += 2 * n;
+        };
+        for (const auto& q : xs) part(q, ta);
+        for (const auto& q : ys) part(q, tb);
+        lc.wait = 2750 + 1100.0 * rounds * wc;
+        lc.rest = 250.0 * floats * wc / (32 * lc.warps);
+        lc.factor = f.factor;
       }
       p.cost.push_back(lc);
     }
     struct It { int4 v0, v1; int cost; };
     p.tables.assign(2 * kNumCfgs, 0);  // per layout: {first entry of h_items, items}
-    for (int i : layouts_used(p.cost, pinned)) {
+    for (int i : layouts_used(p.cost, kRule, pinned)) {
       const int ta = kCfgs[i].TA * kCfgs[i].WA, tb = kCfgs[i].TBU * UB * kCfgs[i].WB;
       std::vector<It> its;
       for (const Triple& t : p.sched.triples) {
@@ -457,7 +486,7 @@ int launch_cg_bwd(const VecCall& c, cudaStream_t s) {
   });
   if (!plan) return GELIB_CUDA_ERROR;
   if (plan->sched.triples.empty() || c.cg.ncells == 0) return GELIB_OK;
-  const int best = choose_layout(plan->cost, c.cg.ncells, pinned);
+  const int best = choose_layout(plan->cost, kRule, c.cg.ncells, pinned);
   if (best < 0 && pinned >= 0) return fail(GELIB_INVALID, fn, "the pinned lane layout does not fit the call");
   if (best < 0) return -1;  // caller falls back to the strided kernels
   if (c.plan_only) return GELIB_OK;
@@ -496,15 +525,12 @@ int launch_cg_bwd(const VecCall& c, cudaStream_t s) {
   a.nitems = nitems;
   // a warp per slab when a cell has fewer than eight: idle warps would only cost residency (l1 = l2 = l = 2, 32 channels,
   // batch 1024, five slabs per cell: 38 -> 32 us)
-  const int nwarps = std::min(8, a.nitems);
+  const int nwarps = plan->cost[best].warps;
   a.offs_extra = c.offs_extra;
   a.do_x = c.xg.empty() ? 0 : 1;
   a.do_y = c.yg.empty() ? 0 : 1;
   const long long groups = (c.cg.ncells + WC - 1) / WC;
-  // Few cells: several blocks share a group of cells, each takes every splits-th round of slabs, and the rows are added
-  // to global memory with atomics.  A block should still have two rounds.
-  int splits = 1;
-  while (splits < 16 && groups * splits * 2 <= 2 * 148 && a.nitems >= 2 * nwarps * splits * 2) splits *= 2;
+  const int splits = splits_for(groups, plan->cost[best]);
   a.x_atomic = c.xg_bcast || splits > 1 ? 1 : 0;
   a.y_atomic = c.yg_bcast || splits > 1 ? 1 : 0;
 

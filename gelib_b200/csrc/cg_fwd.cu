@@ -192,20 +192,26 @@ __global__ void __launch_bounds__(128) cg_fwd_kernel(const __grid_constant__ Fwd
 
 struct TileCfg {
   int TA, WA, NBL;
+  double factor;  // measured time against the estimate
 };
 constexpr TileCfg kCfgs[] = {
-    {4, 4, 8},  // 16 x 32 channels, 1 cell per warp
-    {2, 4, 8},  //  8 x 32, 1 cell
-    {4, 4, 4},  // 16 x 16, 2 cells
-    {1, 1, 4},  //  1 x 16, 8 cells
-    {4, 2, 2},  //  8 x  8, 8 cells
-    {2, 4, 2},  //  8 x  8, 4 cells
-    {2, 2, 2},  //  4 x  8, 8 cells
-    {1, 1, 1},  //  1 x  4, 32 cells
-    {4, 4, 1},  // 16 x  4, 8 cells
+    {4, 4, 8, 1.0},   // 16 x 32 channels, 1 cell per warp
+    {2, 4, 8, 0.8},   //  8 x 32, 1 cell
+    {4, 4, 4, 0.95},  // 16 x 16, 2 cells
+    {1, 1, 4, 2.6},   //  1 x 16, 8 cells
+    {4, 2, 2, 1.0},   //  8 x  8, 8 cells
+    {2, 4, 2, 1.0},   //  8 x  8, 4 cells
+    {2, 2, 2, 2.1},   //  4 x  8, 8 cells
+    {1, 1, 1, 1.15},  //  1 x  4, 32 cells
+    {4, 4, 1, 0.8},   // 16 x  4, 8 cells
 };
 constexpr int kNumCfgs = sizeof(kCfgs) / sizeof(kCfgs[0]);
 constexpr int kMaxJobs = 16;
+int jobs_for(long long groups, const LayoutCost& c) {  // enough blocks to fill the machine several times over
+  const long long n = std::min<long long>(kMaxJobs, (16384 + groups - 1) / groups);
+  return std::max(1, (int)std::min<long long>(n, c.items / 4));
+}
+constexpr LayoutRule kRule = {2.25, jobs_for};
 
 template <int TA, int WA, int NBL>
 cudaError_t launch_cfg(const FwdArgs& a, dim3 grid, size_t smem, bool vec, cudaStream_t s) {
@@ -256,31 +262,42 @@ int launch_cg_fwd(const VecCall& c, cudaStream_t s) {
     build_schedule(xs, ys, rs, false, true, &p.sched);
     std::vector<int> band;
     for (const Triple& t : p.sched.triples) band.push_back(band_size(t.l1, t.l2, t.l));
-    // The estimate of a layout's time.  Per band entry a warp issues 16 multiply-adds and 2 multiplies for each of its TA
-    // rows, half a load per row and about 7 others; per output row it issues 2 TA stores (4 TA of half the size without
-    // 16-byte alignment), each of which occupies the load/store unit, which four schedulers share, once per 128-byte line
-    // it touches.  The work is spread over the warps the call can fill.  Layouts differ in the padding of the channel
-    // counts, in how many multiply-adds share the loads and in how many lines a store touches.  Measured (maxl 4 x 16
-    // channels, batch 1000): 521 us with 1 x 16 channels per warp row, 247 us with 16 x 16.
+    // The estimate of a layout's time: issue cycles, and the staging of a block's cells, whose loads are one round after the
+    // other.  A band entry has 16 multiply-adds per row of the tile and as many others, an output row its control and its
+    // stores, each of which occupies the load/store unit once per 128-byte line it touches.  Layouts differ in the
+    // padding of the channel counts, in how many multiply-adds share the loads, in the lines of a store and in the cells of
+    // a block.  The numbers are fitted to 1500 random calls with every layout each (up to 64 channels, l <= 5, 1 .. 4096
+    // cells): the choice loses 3 % on average against the best layout, more than 15 % in one call of 25.  Measured (maxl 4 x
+    // 16 channels, batch 1000): 521 us with 1 x 16 channels per warp row, 247 us with 16 x 16; (l = 0 x 32, batch 147) 9
+    // and 4 us.
     for (const TileCfg& f : kCfgs) {
       const int ta = f.TA * f.WA, tb = 4 * f.NBL, wc = 32 / (f.WA * f.NBL);
-      LayoutCost lc{0, 0, wc};
-      if (smem_floats(wc) * sizeof(float) <= 200 * 1024) {
-        const double entry = 18.5 * f.TA + 7, row = 6.0 * f.TA + 12 + 4.0 * (vec ? 2 : 4) * f.TA * wc * f.WA;
-        double items = 0;
+      LayoutCost lc;
+      const size_t smem = smem_floats(wc) * sizeof(float);
+      if (smem <= 200 * 1024) {
+        double work = 0;
         for (size_t i = 0; i < band.size(); i++) {
           const Triple& t = p.sched.triples[i];
-          const double tiles = (double)ceil_div(xs[t.xi].n, ta) * ceil_div(ys[t.yi].n, tb);
-          lc.work += tiles * (band[i] * entry + (2 * t.l + 1) * row);
-          items += tiles;
+          const long long tiles = (long long)ceil_div(xs[t.xi].n, ta) * ceil_div(ys[t.yi].n, tb);
+          work += (double)tiles * (band[i] * (16.5 * f.TA + 14.5) + (2 * t.l + 1) * (15.0 * f.TA + 5 + 3.1 * (vec ? 2 : 5.6) * f.TA * wc * f.WA));
+          lc.items = (int)std::min(1LL << 30, lc.items + tiles);
         }
-        lc.warps = std::min(64.0, std::max(4.0, items));
+        lc.cells = wc;
+        lc.warps = 4;
+        lc.blocks = (int)std::min<size_t>(f.TA == 4 ? 8 : f.TA == 2 ? 7 : 16, 227 * 1024 / (smem + 1024));
+        lc.item = work / std::max(1, lc.items);
+        int rounds = 0;
+        for (auto* v : {&xs, &ys})
+          for (const auto& q : *v) rounds += ceil_div((2 * q.l + 1) * q.n, 128);
+        lc.wait = 1150 + 650.0 * rounds * wc;
+        lc.each = 190;
+        lc.factor = f.factor;
       }
       p.cost.push_back(lc);
     }
     // per layout: {first item, items, first of its job tables}; a job table for every number of jobs up to kMaxJobs
     p.tables.assign(3 * kNumCfgs, 0);
-    for (int i : layouts_used(p.cost, pinned)) {
+    for (int i : layouts_used(p.cost, kRule, pinned)) {
       const int ta = kCfgs[i].TA * kCfgs[i].WA, tb = 4 * kCfgs[i].NBL;
       const int first = (int)p.h_items.size();
       std::vector<long long> cost;
@@ -313,7 +330,7 @@ int launch_cg_fwd(const VecCall& c, cudaStream_t s) {
   });
   if (!plan) return GELIB_CUDA_ERROR;
   if (plan->sched.triples.empty() || c.cg.ncells == 0) return GELIB_OK;
-  const int best = choose_layout(plan->cost, c.cg.ncells, pinned);
+  const int best = choose_layout(plan->cost, kRule, c.cg.ncells, pinned);
   if (best < 0 && pinned >= 0) return fail(GELIB_INVALID, fn, "the pinned lane layout does not fit the call");
   if (best < 0) return -1;  // caller falls back to the strided kernel
   if (c.plan_only) return GELIB_OK;
@@ -344,11 +361,8 @@ int launch_cg_fwd(const VecCall& c, cudaStream_t s) {
   a.cell_floats = off;
   const size_t smem = smem_floats(WC) * sizeof(float);
 
-  // ---- jobs: enough CTAs to fill the machine several times over
   const long long groups = (c.cg.ncells + WC - 1) / WC;
-  int njobs = 1;
-  if (groups < 16384) njobs = (int)std::min<long long>(kMaxJobs, (16384 + groups - 1) / groups);
-  njobs = std::max(1, std::min(njobs, nitems / 4));
+  const int njobs = jobs_for(groups, plan->cost[best]);
 
   a.cg = c.cg;
   a.triples = plan->triples;

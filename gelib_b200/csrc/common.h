@@ -92,9 +92,15 @@ int band_size(int l1, int l2, int l);  // number of (m1,m2) with |m1|<=l1, |m2|<
 
 // What the choice of a lane layout needs besides the number of cells.
 struct LayoutCost {
-  double work;  // warp instructions of one group of cells; 0: the layout does not fit shared memory
-  double warps; // warps that can share a group
-  int cells;    // cells of a group
+  int cells = 0;      // of a group; 0: the layout does not fit shared memory
+  int items = 0;      // work items of a group
+  int warps = 0;      // of a block
+  int blocks = 0;     // that an SM holds
+  double item = 0;    // issue cycles of an item
+  double wait = 0;    // cycles of a block that neighbours do not lengthen (the latency of staging)
+  double rest = 0;    // issue cycles of a block beside its items
+  double each = 0;    // cycles that starting an item takes
+  double factor = 1;  // measured time of the layout against the estimate
 };
 
 // Device-resident copy of a plan's tables.  Owned by the per-device cache; never freed before exit.

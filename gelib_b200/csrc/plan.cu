@@ -8,6 +8,7 @@
 // takes, so a signature that has run once builds and uploads nothing more.
 #include <algorithm>
 #include <atomic>
+#include <cmath>
 #include <cstdlib>
 #include <cstring>
 #include <map>
@@ -190,17 +191,24 @@ bool device_has_tcgen05() {
   return cc_major[dev] == 10;
 }
 
-int choose_layout(const std::vector<LayoutCost>& cost, long long ncells, int pinned) {
-  if (pinned >= 0) return pinned < (int)cost.size() && cost[pinned].work > 0 ? pinned : -1;
+int choose_layout(const std::vector<LayoutCost>& cost, const LayoutRule& rule, long long ncells, int pinned) {
+  if (pinned >= 0) return pinned < (int)cost.size() && cost[pinned].cells > 0 ? pinned : -1;
   int shift = 0;
   while ((ncells >> shift) >= 16) shift++;
   const long long n = (ncells >> shift) << shift;
   int best = -1;
   double best_time = 0;
   for (size_t i = 0; i < cost.size(); i++) {
-    if (cost[i].work <= 0) continue;
-    const double groups = (double)((n + cost[i].cells - 1) / cost[i].cells);
-    const double time = cost[i].work * groups / std::min(groups * cost[i].warps, 148.0 * 16);
+    const LayoutCost& c = cost[i];
+    if (c.cells == 0) continue;
+    const long long groups = (n + c.cells - 1) / c.cells;
+    const int split = rule.split(groups, c);
+    const double blocks = (double)groups * split;
+    // warps that share a scheduler
+    const double shared = std::min((double)c.blocks, std::ceil(blocks / 148)) * c.warps / 4;
+    const double rounds = std::ceil((double)c.items / (split * c.warps));
+    const double block = c.wait + c.rest * std::max(1.0, shared) + rounds * (c.each + c.item * std::max(rule.alone, shared));
+    const double time = c.factor * std::max(1.0, blocks / (148.0 * c.blocks)) * block;
     if (best < 0 || time < best_time * 0.999) {
       best = (int)i;
       best_time = time;
@@ -209,12 +217,12 @@ int choose_layout(const std::vector<LayoutCost>& cost, long long ncells, int pin
   return best;
 }
 
-std::vector<int> layouts_used(const std::vector<LayoutCost>& cost, int pinned) {
+std::vector<int> layouts_used(const std::vector<LayoutCost>& cost, const LayoutRule& rule, int pinned) {
   std::vector<bool> used(cost.size(), false);
   std::vector<int> v;
   for (int shift = 0; shift < 40; shift++)
     for (long long n = shift == 0 ? 1 : 8; n < 16; n++) {
-      const int i = choose_layout(cost, n << shift, pinned);
+      const int i = choose_layout(cost, rule, n << shift, pinned);
       if (i >= 0 && !used[i]) {
         used[i] = true;
         v.push_back(i);

@@ -35,9 +35,14 @@ DevicePlan* get_plan(const std::vector<int>& key, const std::function<void(Devic
 // Layout of the least estimated time for a number of cells, -1 when none fits.  The number is cut to its four leading bits
 // (the estimate is no finer), so that layouts_used can name every layout some batch size will choose: a plan holds the work
 // lists of all of them, and no later call of the signature, whatever its batch, builds or uploads anything.
-// With pinned >= 0 that layout is the only one.
-int choose_layout(const std::vector<LayoutCost>& cost, long long ncells, int pinned);
-std::vector<int> layouts_used(const std::vector<LayoutCost>& cost, int pinned);
+// With pinned >= 0 that layout is the only one.  `alone`: cycles between two issues of a warp that has its scheduler to itself;
+// `split`: blocks that share a group.
+struct LayoutRule {
+  double alone;
+  int (*split)(long long groups, const LayoutCost& c);
+};
+int choose_layout(const std::vector<LayoutCost>& cost, const LayoutRule& rule, long long ncells, int pinned);
+std::vector<int> layouts_used(const std::vector<LayoutCost>& cost, const LayoutRule& rule, int pinned);
 
 // Kernel families (each returns a status code; with c.plan_only they build their plan and return).
 int launch_cg_fwd(const VecCall& c, cudaStream_t s);

@@ -45,6 +45,7 @@
 #include <map>
 #include <string>
 
+#include "f32x2.h"
 #include "plan.h"
 #include "tc_common.h"
 #include "tma_maps.h"
@@ -123,27 +124,8 @@ __device__ __forceinline__ void cp_async_arrive(uint64_t* bar) {
   asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" ::"r"(smem_u32(bar)) : "memory");
 }
 
-// Packed single precision (two lanes of one 64-bit register per instruction): the combination H = sum_l c_l G_l
-// takes one instruction per complex number and slab instead of two.
-typedef unsigned long long f32x2;
-__device__ __forceinline__ f32x2 pack2(float a, float b) {
-  f32x2 r;
-  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
-  return r;
-}
-__device__ __forceinline__ void unpack2(f32x2 v, float& a, float& b) { asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(v)); }
-__device__ __forceinline__ f32x2 mul2(f32x2 a, f32x2 b) {
-  f32x2 r;
-  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
-  return r;
-}
-__device__ __forceinline__ f32x2 fma2(f32x2 a, f32x2 b, f32x2 c) {
-  f32x2 r;
-  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
-  return r;
-}
-
 // H = sum_l c_l G_l for the warp's 8 complex numbers, contracted with the conjugate of the other operand's 8.
+// Packed single precision takes one instruction per complex number and slab instead of two.
 template <int LM>
 __device__ __forceinline__ void contract(const f32x2 (&G)[kGroupSlabs][kCW], const float4 c, const float4 (&w)[kCW / 2], float& sr,
                                          float& si) {

@@ -13,8 +13,8 @@
 // block) and their gradients sit in registers.  The pair is walked by output row m: entry i of a step multiplies a[i]
 // with b[m - m1(i)].  The gradients of the b rows that a step touches are a window of registers that moves by one row per
 // step (the body is instantiated per block size, so everything in registers is indexed statically); a row is added to its
-// slot when it leaves the window.  There are no atomics in shared memory, no shuffles and no barriers in the loop, and one
-// read-modify-write per row and block instead of one per band entry.
+// slot when it leaves the window.  There are no atomics in shared memory and no shuffles, no barriers within a chunk of the
+// walk (below), and one read-modify-write per row and block instead of one per band entry.
 // Everything a warp reads from global memory -- b rows, a rows, the gradient rows g -- arrives through one stream of rows
 // (cp.async, 8 or 16 bytes per lane) in a ring of kColRing rows, whose order is the order of use: taking k rows requests
 // the k rows that come kColRing later, so the bytes in flight do not depend on how short the steps are.  What the warps
@@ -28,9 +28,12 @@
 // may instead split by pairs, and then several blocks add to a row.
 // Why this form: diag_bwd_cell_kernel spends its time in four shared-memory atomics (compare-and-swap loops) per band
 // entry, which a lane that owns its column does not need.  Measured, backward of the diagonal product: maxl 8 x 128
-// channels, batch 2048 10.5 -> 4.8 ms; maxl 6 x 33, batch 4000 4.3 -> 1.1 ms; maxl 3 x 12, batch 500 49 -> 18 us (forward 32 ->
-// 15 us).  Bound by instruction issue at two to three warps per scheduler: about 475 k warp instructions per 64 columns at
-// maxl 8; the largest stalls are instruction fetch (the unrolled bodies) and fixed-latency dependencies.
+// channels, batch 2048 10.5 -> 4.8 ms; maxl 6 x 33, batch 4000 4.3 -> 1.1 ms; maxl 3 x 12, batch 500 49 -> 29 us (forward 32 ->
+// 15 us).  At maxl 8 the backward holds two warps per scheduler -- 252 registers a thread and 25.6 KB of shared memory a warp
+// both end there -- and issues in 42 % of its cycles: 502 k warp instructions per 64 columns, whose largest stalls are
+// fixed-latency dependencies (1.3 cycles per issue) and shared memory (0.7).  The forward issues in 32 %: 345 k
+// instructions, dependencies 1.5, shared memory 1.3, instruction fetch of the unrolled bodies 1.1; its instances spill 84 to
+// 168 bytes a thread at 168, 128 and 128 registers, which its block sizes impose.
 #pragma once
 #include "plan.h"
 
@@ -55,7 +58,7 @@ constexpr int kColFixedSmem = 16 * kColSlots + 2 * kColChunkBytes;  // part tabl
 // forward, maxl 8 x 128 3.8 against 4.3 ms.
 constexpr int col_nl_padded(int nl, int kb, bool both) { return !both || kb < 6 ? (nl + 1) / 2 * 2 : nl <= 6 ? 6 : 10; }
 
-// Row (slot, v) of a column: base + v * unit + cell * cell_stride + channel * ch_stride, all in bytes.
+// Row (slot, v) of a lane: base + v * unit + cell * cell_stride + (lane of the cell) * ch_stride, all in bytes.
 struct ColPart {
   float* base;
   unsigned unit, cell_stride;
@@ -64,8 +67,7 @@ struct ColPart {
 struct ColArgs {
   ColPart part[kColSlots];         // x: 0.., y: kMaxParts.., r or g: 2 kMaxParts..  (v = row for x, y; complex offset for r)
   ColPart grad[2 * kMaxParts];     // xg: 0.., yg: kMaxParts..  (v = row)
-  unsigned ch_stride[3];           // bytes between channels of x, y, r: 8, or 0 for an operand of one channel
-  int nx, ny, nr;
+  unsigned ch_stride[3];           // bytes between lanes of x, y, r: 8 per column, or 0 for an operand of one channel
   unsigned n, nlanes;              // lanes per cell (channels / columns per lane), lanes in all
   int b_rows;                      // rows of the largest b part
   int accumulate;                  // forward: add to r instead of storing

@@ -1,27 +1,10 @@
 // Device side of the column kernels (see col.h).
 #pragma once
 #include "col.h"
+#include "f32x2.h"
 
 namespace gelib_b200 {
 namespace col {
-
-typedef unsigned long long f32x2;
-__device__ __forceinline__ f32x2 pack2(float a, float b) {
-  f32x2 r;
-  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
-  return r;
-}
-__device__ __forceinline__ void unpack2(f32x2 v, float& a, float& b) { asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(v)); }
-__device__ __forceinline__ f32x2 mul2(f32x2 a, f32x2 b) {
-  f32x2 r;
-  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
-  return r;
-}
-__device__ __forceinline__ f32x2 fma2(f32x2 a, f32x2 b, f32x2 c) {
-  f32x2 r;
-  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
-  return r;
-}
 
 template <int N>
 __device__ __forceinline__ void cp_wait() {
@@ -95,13 +78,12 @@ struct Walk {
     const int side = r.x / kMaxParts;
     return make_uint4((unsigned)b, (unsigned)(b >> 32), p.w, side == 0 ? A.ch_stride[0] : side == 1 ? A.ch_stride[1] : A.ch_stride[2]);
   }
-  // kShared: the row may be one number per cell (lane stride 0), which both columns of a lane get
-  template <bool kShared>
+  // A row may be one number per cell (lane stride 0), which both columns of a lane get.
   __device__ __forceinline__ void request(unsigned long long src, uint32_t lane_stride, uint32_t pos) const {
     const uint32_t dst = (uint32_t)__cvta_generic_to_shared(smem) + ring + (pos & (kRing - 1));
     if constexpr (CPL == 1) {
       asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(dst), "l"(src) : "memory");
-    } else if (kShared && lane_stride == 0) {
+    } else if (lane_stride == 0) {
       asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(dst), "l"(src) : "memory");
       asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(dst + 8), "l"(src) : "memory");
     } else {
@@ -128,7 +110,7 @@ struct Walk {
         }
 #pragma unroll
       for (int j = 0; j < 4; j++)
-        if (j0 + j < N && j0 + j < k) request<true>(ad[j], ls[j], pb + kRow * (j0 + j));
+        if (j0 + j < N && j0 + j < k) request(ad[j], ls[j], pb + kRow * (j0 + j));
     }
     req += 16 * k;
     pb += kRow * k;
@@ -219,7 +201,7 @@ struct Walk {
     pb = 8 * CPL * lane;
     for (int j = 0; j < kColRing; j++) {
       const uint4 q = resolve(__ldg(A.blob + pro + j));
-      request<true>(addr(q), q.w, pb + kRow * j);
+      request(addr(q), q.w, pb + kRow * j);
     }
   }
 

@@ -520,9 +520,6 @@ bool col_setup(const VecCall& c, bool backward, ColArgs* a, ColPlan* plan) {
   if (!plan->dev) return true;
   a->ch_stride[0] = x_shared ? 0 : 8 * plan->cpl;
   a->ch_stride[1] = a->ch_stride[2] = 8 * plan->cpl;
-  a->nx = (int)c.x.size();
-  a->ny = (int)c.y.size();
-  a->nr = (int)c.r.size();
   a->n = (unsigned)(n / plan->cpl);
   a->nlanes = (unsigned)(c.cg.ncells * a->n);
   // With fewer warps than the chip holds, the walk is cut into runs that different blocks take: forward into runs of pairs;
@@ -545,7 +542,6 @@ bool col_setup(const VecCall& c, bool backward, ColArgs* a, ColPlan* plan) {
   }
   plan->owned = backward && tables[kTable * walk + 2] > 0;
   a->accumulate = (c.flags & GELIB_OVERWRITE) ? 0 : 1;
-
   a->blob = plan->dev->items;
   a->chunks = plan->dev->jobs + tables[kTable * walk];
   a->nsplits = tables[kTable * walk + 1];

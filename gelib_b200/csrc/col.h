@@ -99,6 +99,9 @@ inline int col_block_warps(unsigned warps, int splits, int most) {
   return (int)(nw < 2 ? 2 : nw);
 }
 
+// False when the view's cells are no arithmetic progression or a stride does not fit.
+bool col_fill_part(const PartView& p, const CellGrid& cg, long long extra_floats, bool rows, ColPart* out);
+
 // Returns false when the call is not one the column kernels take; otherwise fills args and
 // plan (plan->dev == nullptr on a CUDA error).
 bool col_setup(const VecCall& c, bool backward, ColArgs* a, ColPlan* plan);

@@ -163,7 +163,7 @@ int launch_col_fwd(const VecCall& c, cudaStream_t s, bool* plan_others) {
   if (!col_setup(c, false, &a, &plan)) return -1;
   if (!plan.dev) return GELIB_CUDA_ERROR;
   *plan_others = plan.plan_others;
-  if (a.nsplits == 0) return GELIB_OK;
+  if (a.nsplits == 0 || c.plan_only) return GELIB_OK;
   cudaError_t e;
   if (plan.cpl == 1) e = col::launch_fwd<17, 1, 512>(a, s);
   else if (plan.max_block <= 9) e = col::launch_fwd<9, 2, 512>(a, s);

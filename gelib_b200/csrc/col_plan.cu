@@ -385,16 +385,6 @@ void build(DevicePlan& p, const std::vector<PartSig>& xs, const std::vector<Part
   p.sched.coeffs.clear();  // they are in the walks
 }
 
-bool fill_part(const PartView& p, const CellGrid& cg, long long extra_floats, bool rows, ColPart* out) {
-  const long long cs = cell_stride(p, cg);
-  const long long unit = rows ? p.sm : 2;
-  if (cs < 0 || 4 * cs > 0xffffffffLL || unit < 0 || 4 * unit > 0xffffffffLL) return false;
-  out->base = p.base + extra_floats;
-  out->unit = (unsigned)(4 * unit);
-  out->cell_stride = (unsigned)(4 * cs);
-  return true;
-}
-
 // The backward walk of the least estimated time, and the warps of a block for an owned one.  Fitted to 112 calls with every
 // owned walk each (maxl 1 .. 8, lopsided types, 2 .. 375 warps of columns; the choice loses 2 % on average, 28 % at worst): a
 // run takes 5 us and 2.5 ns per unit of its cost (2.8 with both gradients at once, which owned walks do not do), a little
@@ -455,6 +445,16 @@ bool narrow_wins(bool backward, int cpl, int n, int max_la, long long cells) {
 
 }  // namespace
 
+bool col_fill_part(const PartView& p, const CellGrid& cg, long long extra_floats, bool rows, ColPart* out) {
+  const long long cs = cell_stride(p, cg);
+  const long long unit = rows ? p.sm : 2;
+  if (cs < 0 || 4 * cs > 0xffffffffLL || unit < 0 || 4 * unit > 0xffffffffLL) return false;
+  out->base = p.base + extra_floats;
+  out->unit = (unsigned)(4 * unit);
+  out->cell_stride = (unsigned)(4 * cs);
+  return true;
+}
+
 bool col_setup(const VecCall& c, bool backward, ColArgs* a, ColPlan* plan) {
   if (c.x.empty() || c.y.empty() || c.r.empty() || !c.dense_channels || c.sph) return false;
   if (c.x.size() > (size_t)kMaxParts || c.y.size() > (size_t)kMaxParts || c.r.size() > (size_t)kMaxParts) return false;
@@ -475,19 +475,19 @@ bool col_setup(const VecCall& c, bool backward, ColArgs* a, ColPlan* plan) {
   plan->max_block = std::min(2 * max_la + 1, backward ? kColBlockBwd : kColBlockFwd);
   a->b_rows = 2 * max_lb + 1;
   for (size_t i = 0; i < c.x.size(); i++)
-    if (!fill_part(c.x[i], c.cg, 0, true, &a->part[i])) return false;
+    if (!col_fill_part(c.x[i], c.cg, 0, true, &a->part[i])) return false;
   for (size_t i = 0; i < c.y.size(); i++)
-    if (!fill_part(c.y[i], c.cg, 0, true, &a->part[kMaxParts + i])) return false;
+    if (!col_fill_part(c.y[i], c.cg, 0, true, &a->part[kMaxParts + i])) return false;
   for (size_t i = 0; i < c.r.size(); i++) {
     if (c.r[i].sm != 2LL * c.r[i].n) return false;  // the walk holds offsets of dense rows
     if ((2LL * c.r[i].l + 1) * c.r[i].n > 0x7fffffffLL) return false;
-    if (!fill_part(c.r[i], c.cg, 2LL * c.offs_extra, false, &a->part[2 * kMaxParts + i])) return false;
+    if (!col_fill_part(c.r[i], c.cg, 2LL * c.offs_extra, false, &a->part[2 * kMaxParts + i])) return false;
     a->part[2 * kMaxParts + i].unit = 8;
   }
   for (size_t i = 0; i < c.xg.size(); i++)
-    if (!fill_part(c.xg[i], c.cg, 0, true, &a->grad[i])) return false;
+    if (!col_fill_part(c.xg[i], c.cg, 0, true, &a->grad[i])) return false;
   for (size_t i = 0; i < c.yg.size(); i++)
-    if (!fill_part(c.yg[i], c.cg, 0, true, &a->grad[kMaxParts + i])) return false;
+    if (!col_fill_part(c.yg[i], c.cg, 0, true, &a->grad[kMaxParts + i])) return false;
   // two columns per lane: every access is 16 bytes (8 for an operand of one channel, which both columns share)
   const bool x_shared = nx == 1 && n > 1;
   bool two = n % 2 == 0 && c.offs_extra % 2 == 0;

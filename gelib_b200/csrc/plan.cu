@@ -41,7 +41,7 @@ bool upload(const std::vector<T>& h, T** d) {
 
 namespace {
 struct Options {
-  std::atomic<int> fwd{kFwdAuto}, bwd{kBwdAuto}, inject{0}, pair_tma{1}, narrow1{1}, col{kColAuto}, fwd_layout{-1}, bwd_layout{-1};
+  std::atomic<int> fwd{kFwdAuto}, bwd{kBwdAuto}, inject{0}, pair_tma{1}, narrow1{1}, col{kColAuto}, mir{kColAuto}, fwd_layout{-1}, bwd_layout{-1};
 };
 int parse_fwd(const char* v) {
   if (!v || !*v || !strcmp(v, "auto")) return kFwdAuto;
@@ -81,6 +81,7 @@ bool inject_timeout() { return options().inject.load(std::memory_order_relaxed) 
 bool pair_tma() { return options().pair_tma.load(std::memory_order_relaxed) != 0; }
 bool narrow1_enabled() { return options().narrow1.load(std::memory_order_relaxed) != 0; }
 
+int mir_mode() { return options().mir.load(std::memory_order_relaxed); }
 int col_mode() { return options().col.load(std::memory_order_relaxed); }
 int pinned_layout(bool backward) { return (backward ? options().bwd_layout : options().fwd_layout).load(std::memory_order_relaxed); }
 
@@ -109,6 +110,13 @@ int set_option(const char* name, const char* value) {
     for (int i = 0; i < 4; i++)
       if (value && !strcmp(value, names[i])) o.col = i;
     if (value && !strncmp(value, "split", 5) && atoi(value + 5) > 0) o.col = kColSplit + atoi(value + 5);
+    return GELIB_OK;
+  }
+  if (!strcmp(name, "mir")) {
+    const char* names[] = {"auto", "0", "one", "two"};
+    o.mir = kColAuto;
+    for (int i = 0; i < 4; i++)
+      if (value && !strcmp(value, names[i])) o.mir = i;
     return GELIB_OK;
   }
   if (!strcmp(name, "fwd_layout") || !strcmp(name, "bwd_layout")) {

@@ -58,6 +58,7 @@ int launch_cg_strided(const VecCall& c, int mode, cudaStream_t s);  // mode 0 fw
 int launch_cg_strided_static(const VecCall& c, cudaStream_t s);  // forward, tables in a static device array: no allocation
 // Diagonal products and one-channel x; -1 when the call does not qualify.  *plan_others: the signature goes to other kernels
 // at other batch sizes, and they have not planned it yet.
+int launch_mir_fwd(const VecCall& c, cudaStream_t s, bool* plan_others);
 int launch_col_fwd(const VecCall& c, cudaStream_t s, bool* plan_others);
 int launch_col_bwd(const VecCall& c, cudaStream_t s, bool* plan_others);
 // Option "col": by the rules of col_plan.cu, not at all ("0"), or, with every call that the column kernels can take, one or
@@ -65,6 +66,7 @@ int launch_col_bwd(const VecCall& c, cudaStream_t s, bool* plan_others);
 // of the plan's ways ("split1" ..).  Tests pin what only some batch sizes reach and compare the kernels.
 enum ColMode { kColAuto = 0, kColOff, kColOne, kColTwo, kColSplit /* + k */ };
 int col_mode();
+int mir_mode();  // option "mir": the mirrored-row kernels by their rules, not at all ("0"), or with one or two columns per lane
 int pinned_layout(bool backward);  // options "fwd_layout" / "bwd_layout": lane layout of the FP32 kernels, -1 by the estimate
 int launch_diag_fwd(const VecCall& c, cudaStream_t s);
 int launch_diag_bwd(const VecCall& c, cudaStream_t s);

@@ -9,6 +9,7 @@ and the backward pass reads the upstream gradient once for both input gradients.
 import torch
 
 from . import backend as gb
+from ._lib import native
 from .gelib_common import common_batch, of_class, plain
 from .SO3element import SO3element
 from .SO3irrep import SO3irrep
@@ -51,6 +52,9 @@ class SO3partArr_GatherFn(torch.autograd.Function):
         ctx.gmap, ctx.d = gmap, d
         with plain():
             ctx.xshape = list(x.shape)
+            r = gb.gather(x, gmap, d)
+            if r is not None:
+                return r.as_subclass(SO3partArr)
             shape = list(x.shape)
             shape[d + 1] = gmap.d_out()
             r = torch.zeros(shape, dtype=torch.complex64, device=x.device)
@@ -60,6 +64,9 @@ class SO3partArr_GatherFn(torch.autograd.Function):
     @staticmethod
     def backward(ctx, rg):
         with plain():
+            xg = gb.gather(rg, ctx.gmap, ctx.d, transposed=True)
+            if xg is not None:
+                return xg, None, None
             xg = torch.zeros(ctx.xshape, dtype=torch.complex64, device=rg.device)
             gb.SO3part.view(xg).add_gather_back(rg.as_subclass(torch.Tensor).contiguous(), ctx.gmap, ctx.d)
         return xg, None, None
@@ -83,6 +90,9 @@ def _product_forward_plain(ctx, x, y, l, diag):
     ctx.l = l
     ctx.diag = diag
     ctx.save_for_backward(x, y)
+    r = native().part_forward(x, y, l, diag)
+    if r is not None:
+        return r
     b = common_batch(x, y)
     if diag:
         assert x.size(-1) == y.size(-1)
@@ -103,6 +113,9 @@ def _product_forward_plain(ctx, x, y, l, diag):
 def _product_backward_plain(ctx, g):
     x, y = ctx.saved_tensors
     need_x, need_y = ctx.needs_input_grad[0], ctx.needs_input_grad[1]
+    done = native().part_backward(x, y, g, need_x, need_y, ctx.diag)
+    if done is not None:
+        return of_class(done[0], x) if need_x else None, of_class(done[-1], y) if need_y else None, None
     xg = of_class(torch.zeros_like(x), x) if need_x else None
     yg = of_class(torch.zeros_like(y), y) if need_y else None
     gv, xv, yv = gb.SO3part.view(g), gb.SO3part.view(x), gb.SO3part.view(y)

@@ -8,7 +8,8 @@ forward and one backward instead of one launch per triple (core/Gvec.hpp:311-389
 import torch
 
 from . import backend as gb
-from .gelib_common import common_batch, plain, zeros_like_all
+from ._lib import native
+from .gelib_common import common_batch, of_class, plain, zeros_like_all
 from .SO3part import SO3part, SO3partArr
 
 
@@ -20,6 +21,9 @@ def _vec_forward(ctx, k1, k2, maxl, args, diag, part_cls):
 def _vec_forward_plain(ctx, k1, k2, maxl, args, diag, part_cls):
     ctx.k1, ctx.k2, ctx.diag = k1, k2, diag
     ctx.save_for_backward(*args)
+    done = native().vec_forward(args[0:k1], args[k1:k1 + k2], maxl, diag)
+    if done is not None:
+        return tuple([p.as_subclass(part_cls) for p in done])
     xs, ys = [a.detach() for a in args[0:k1]], [a.detach() for a in args[k1:k1 + k2]]
     x, y = gb.SO3vec.view(xs), gb.SO3vec.view(ys)
     b = common_batch(xs[0], ys[0])
@@ -52,6 +56,10 @@ def _vec_backward_plain(ctx, gargs):
     # a side that needs no gradient (spherical harmonics of fixed points, say) is not computed at all
     grads = [None] * len(saved)
     first, last = 0 if need_x else k1, k1 + k2 if need_y else k1
+    done = native().vec_backward(saved[0:k1], saved[k1:k1 + k2], gargs, need_x, need_y, ctx.diag)
+    if done is not None:
+        grads[first:last] = [of_class(z, t) for z, t in zip(done, saved[first:last])]
+        return tuple([None, None, None] + grads)
     grads[first:last] = zeros_like_all(saved[first:last])
     x, y = gb.SO3vec.view(list(saved[0:k1])), gb.SO3vec.view(list(saved[k1:k1 + k2]))
     g = gb.SO3vec.view([a.as_subclass(torch.Tensor) for a in gargs])

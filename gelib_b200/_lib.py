@@ -101,6 +101,23 @@ def lib():
     return _lib
 
 
+_native = None
+
+
+def native():
+    """The native host side of the products (csrc/host.cpp).  Raises when it has not been built, like lib()."""
+    global _native
+    if _native is None:
+        lib()
+        try:
+            from . import _native as module
+        except ImportError as e:
+            raise RuntimeError("gelib_b200: %s cannot be loaded (%s). Build it with `python -m gelib_b200.build`."
+                               % (os.path.join(_HERE, "_native.so"), e))
+        _native = module
+    return _native
+
+
 def last_error():
     return lib().gelib_last_error().decode()
 

@@ -13,7 +13,7 @@ import functools
 import torch
 
 from . import _lib
-from ._lib import GELIB_FP64, GELIB_OVERWRITE, check, descriptor, descriptor_array, device_guard, lib, stream_of
+from ._lib import GELIB_FP64, GELIB_OVERWRITE, check, descriptor, descriptor_array, device_guard, lib, native, stream_of
 
 
 def _ints(v):
@@ -193,6 +193,14 @@ def _gather(r, x, gmap, d, transposed):
     with device_guard(r):
         return check(lib().gelib_add_gather(r.data_ptr(), x.data_ptr(), outer, n_out, n_in, inner, ptr.data_ptr(),
                                             col.data_ptr(), stream_of(r)))
+
+
+def gather(x, gmap, d, transposed=False):
+    """x gathered along array dimension d into a new tensor, by the native host side; None when x is not plain."""
+    if not x.is_cuda:
+        return None
+    n_in, n_out = (gmap.n_out, gmap.n_in) if transposed else (gmap.n_in, gmap.n_out)
+    return native().gather(x, *gmap.csr(x.device, transposed), n_in, n_out, d)
 
 
 MIX_MAX_CHANNELS = 64

@@ -4,16 +4,19 @@
 
 The library is a plain shared object (no Python or torch dependency); it is what a GElib build
 links instead of its own ``cuda/`` objects, and what ``gelib_b200._lib`` loads through ctypes.
+``_native.so``, built beside it, is the Python package's own: it links the library and torch.
 """
 import os
 import subprocess
 import sys
+import sysconfig
 from concurrent.futures import ThreadPoolExecutor
 
 HERE = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(HERE, "csrc")
 OBJ = os.path.join(CSRC, "build")
 LIB = os.path.join(HERE, "libgelib_b200.so")
+NATIVE = os.path.join(HERE, "_native.so")  # host side of the Python products (csrc/host.cpp), against torch's C++ library
 SOURCES = ["bank.cu", "plan.cu", "cg_fwd.cu", "cg_fwd_tc.cu", "cg_bwd.cu", "cg_bwd_pair.cu", "cg_bwd_tc.cu", "cg_narrow.cu", "cg_narrow1_bwd.cu", "cg_strided.cu", "col_plan.cu", "col_fwd.cu", "col_bwd.cu", "col_bwd_x.cu", "col_bwd_y.cu", "col_bwd_owned.cu", "mir_fwd.cu", "diag.cu", "diag_fwd.cu", "diag_bwd.cu", "spharm.cu", "probe.cu", "gather_apply.cu", "mix.cu", "cabi.cu"]
 HEADERS = ["common.h", "plan.h", "tc_common.h", "tma_maps.h", "col.h", "col_device.h", "mir.h", "f32x2.h", "col_bwd.cuh", os.path.join("..", "..", "include", "gelib_b200.h")]
 NVCC = os.environ.get("NVCC", "/usr/local/cuda/bin/nvcc")
@@ -27,7 +30,7 @@ def _newest(paths):
     return max(os.path.getmtime(p) for p in paths)
 
 
-def build(force=False, verbose=False):
+def build_library(force=False, verbose=False):
     srcs = [os.path.join(CSRC, s) for s in SOURCES]
     deps = srcs + [os.path.join(CSRC, h) for h in HEADERS] + [os.path.abspath(__file__)]
     if not force and os.path.exists(LIB) and os.path.getmtime(LIB) >= _newest(deps):
@@ -57,6 +60,30 @@ def build(force=False, verbose=False):
     if r.returncode != 0:
         raise RuntimeError("link failed:\n%s\n%s" % (r.stdout, r.stderr))
     return LIB
+
+
+def build_native(force=False, verbose=False):
+    src, header = os.path.join(CSRC, "host.cpp"), os.path.join(HERE, "..", "include", "gelib_b200.h")
+    if not force and os.path.exists(NATIVE) and os.path.getmtime(NATIVE) >= _newest([src, header, LIB, os.path.abspath(__file__)]):
+        return NATIVE
+    import torch
+    root = os.path.dirname(os.path.abspath(torch.__file__))
+    include = [os.path.join(root, "include"), os.path.join(root, "include", "torch", "csrc", "api", "include"),
+               os.path.join(os.path.dirname(os.path.dirname(NVCC)), "include"), sysconfig.get_paths()["include"]]
+    cmd = [os.environ.get("CXX", "g++"), "-O2", "-std=c++17", "-fPIC", "-shared", "-fvisibility=hidden"]
+    cmd += ["-D_GLIBCXX_USE_CXX11_ABI=%d" % torch._C._GLIBCXX_USE_CXX11_ABI] + ["-I" + i for i in include] + [src, "-o", NATIVE]
+    cmd += ["-L" + os.path.join(root, "lib"), "-lc10", "-lc10_cuda", "-ltorch_cpu", "-ltorch", "-ltorch_python"]
+    cmd += ["-L" + HERE, "-l:" + os.path.basename(LIB), "-Wl,-rpath,$ORIGIN"]
+    r = subprocess.run(cmd, capture_output=True, text=True)
+    if r.returncode != 0:
+        raise RuntimeError("g++ failed for host.cpp:\n%s\n%s" % (r.stdout, r.stderr))
+    return NATIVE
+
+
+def build(force=False, verbose=False):
+    path = build_library(force, verbose)
+    build_native(force, verbose)
+    return path
 
 
 if __name__ == "__main__":

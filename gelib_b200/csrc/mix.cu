@@ -6,10 +6,14 @@
 //
 // rows = every (cell, m) of the part; all arrays dense complex64.  In GElib this is torch.matmul per part
 // (python/src/gelib/SO3vec.py:174-177, python/src/gelib/SO3weights.py:22-85); with 16 channels the library GEMM runs at
-// a tenth of the memory rate, and the mixing of config 5's pipeline cost as much as a fifth of its product.  The
-// kernels here are bound by memory: a block stages tiles of rows (and the matrix) in shared memory with coalesced
-// asynchronous copies, one tile in flight while the other is worked on, and every thread forms one output element per pass; the weight gradient keeps one (i,j) sum per thread over
-// the block's rows and adds it to global memory once.
+// a tenth of the memory rate, and the mixing of a point cloud's first layer cost as much as a fifth of its product.
+//
+// Both kernels stage tiles of rows in shared memory (asynchronous copies, one tile in flight while the other is worked on) and
+// give a thread a tile of the result: 4 rows x 2 columns of the product, 4 x 4 entries of the weight gradient, so that a 16-byte
+// load feeds 11 (16) multiply-adds.  Measured against one output element (one (i,j) sum) per thread, us, product / adjoint /
+// weight gradient: 16 x 16 channels, 3.2 million rows 215 / 240 / 396 -> 217 / 214 / 245; 32 x 32, 400000 96 / 156 / 194 -> 96 /
+// 98 / 110; 8 x 8, 2 million 105 / 107 / 132 -> 55 / 55 / 77; 12 x 20, 500000 76 / 70 / 85 -> 47 / 49 / 62; 64 x 64, 100000 207 /
+// 213 / 241 -> 94 / 102 / 108.  At 16 channels the multiply-adds alone take 91 us and the memory 126.
 #include <cuda_pipeline.h>
 
 #include <algorithm>
@@ -21,151 +25,184 @@ namespace gelib_b200 {
 namespace {
 
 constexpr int kMixMaxN = 64;   // channels on either side
-constexpr int kTileRows = 64;  // rows per block and pass
+constexpr int kThreads = 256;
+constexpr int kRowsPerThread = 4;
 
-// `count` complex numbers from global to shared memory, asynchronously (8 bytes per copy; the caller commits).
-__device__ __forceinline__ void tile_copy_async(float2* dst, const float2* src, int count) {
-  for (int e = threadIdx.x; e < count; e += blockDim.x) __pipeline_memcpy_async(dst + e, src + e, 8);
+// How rows of n complex numbers are copied: 16 bytes at a time where they are aligned, `per` copies a row.
+struct RowCopy {
+  int per, shift;  // shift: of a power of two, else -1
+  bool wide;
+};
+
+// Copies `rows` rows to shared rows of `pitch` bytes, asynchronously.
+__device__ __forceinline__ void tile_copy_async(unsigned char* dst, int pitch, const float2* src, int rows, const RowCopy c) {
+  for (int e = threadIdx.x; e < rows * c.per; e += kThreads) {
+    const int row = c.shift >= 0 ? e >> c.shift : e / c.per, at = e - row * c.per;
+    if (c.wide) __pipeline_memcpy_async(dst + row * pitch + 16 * at, src + 2 * e, 16);
+    else __pipeline_memcpy_async(dst + row * pitch + 8 * at, src + e, 8);
+  }
 }
 
+// s += a b
+__device__ __forceinline__ void mac(float2& s, float ar, float ai, float br, float bi) {
+  s.x = fmaf(ar, br, s.x); s.x = fmaf(-ai, bi, s.x);
+  s.y = fmaf(ar, bi, s.y); s.y = fmaf(ai, br, s.y);
+}
+
+// r[row][j] = sum_k x[row][k] M[k][j], M = W (mode 0) or its adjoint (mode 1).  A thread has columns 2 tx, 2 tx + 1 of the rows
+// ty, ty + TY, ..; odd lengths are padded with zeros in shared memory.
 template <int MODE>
-__global__ void __launch_bounds__(256) mix_kernel(float2* __restrict__ r, const float2* __restrict__ x, const float2* __restrict__ W,
-                                                  long long rows, int nk, int nj, int w_cols) {
-  extern __shared__ float2 sm[];
-  float2* Ms = sm;                 // [nk][nj + 1]: the matrix the rows are multiplied by
-  float2* xs = sm + nk * (nj + 1); // [kTileRows][nk]
-  for (int e = threadIdx.x; e < nk * nj; e += blockDim.x) {
-    const int k = e / nj, j = e - k * nj;
-    float2 w;
+__global__ void __launch_bounds__(kThreads) mix_kernel(float2* __restrict__ r, const float2* __restrict__ x, const float2* __restrict__ W,
+                                                       long long rows, int nk, int nj, int w_cols, int ty_n, RowCopy copy_x, bool wide_r) {
+  extern __shared__ __align__(16) unsigned char sm[];
+  const int tx_n = (nj + 1) / 2, nk2 = (nk + 1) / 2, tile = ty_n * kRowsPerThread;
+  const int pitch = 16 * nk2 + 16;                        // bytes of a staged row of x
+  float4* Ms = reinterpret_cast<float4*>(sm);             // [2 nk2][tx_n]: two columns each
+  unsigned char* xs = sm + 32 * nk2 * tx_n;               // two tiles
+  for (int e = threadIdx.x; e < 4 * nk2 * tx_n; e += kThreads) {  // neighbouring threads read neighbouring weights
+    int k, j;
     if (MODE == 0) {
-      w = W[k * w_cols + j];       // W[i = k][j]
+      k = e / (2 * tx_n);
+      j = e - k * 2 * tx_n;
     } else {
-      w = W[j * w_cols + k];       // conj(W[i = j][j' = k])
-      w.y = -w.y;
+      j = e / (2 * nk2);
+      k = e - j * 2 * nk2;
     }
-    Ms[k * (nj + 1) + j] = w;
-  }
-  for (long long row0 = (long long)blockIdx.x * kTileRows; row0 < rows; row0 += (long long)gridDim.x * kTileRows) {
-    const int nr = (int)min((long long)kTileRows, rows - row0);
-    __syncthreads();
-    for (int e = threadIdx.x; e < nr * nk; e += blockDim.x) xs[e] = __ldcs(x + row0 * nk + e);
-    __syncthreads();
-    for (int e = threadIdx.x; e < nr * nj; e += blockDim.x) {
-      const int row = e / nj, j = e - row * nj;
-      const float2* xr = xs + row * nk;
-      float sr = 0.f, si = 0.f;
-#pragma unroll 4
-      for (int k = 0; k < nk; k++) {
-        const float2 a = xr[k], b = Ms[k * (nj + 1) + j];
-        sr = fmaf(a.x, b.x, sr); sr = fmaf(-a.y, b.y, sr);
-        si = fmaf(a.x, b.y, si); si = fmaf(a.y, b.x, si);
-      }
-      __stcs(r + row0 * nj + e, make_float2(sr, si));
+    float2 w = make_float2(0.f, 0.f);
+    if (k < nk && j < nj) {
+      w = MODE == 0 ? W[k * w_cols + j] : W[j * w_cols + k];
+      if (MODE == 1) w.y = -w.y;
     }
+    reinterpret_cast<float2*>(Ms)[k * 2 * tx_n + j] = w;
   }
-}
-
-// The same product for power-of-two channel counts up to 32 on both sides: the thread keeps its column of the matrix
-// in registers and walks the rows of the tile with 16-byte loads of x (two complex numbers per load).
-template <int MODE, int NK>
-__global__ void __launch_bounds__(256) mix_reg_kernel(float2* __restrict__ r, const float2* __restrict__ x,
-                                                      const float2* __restrict__ W, long long rows, int nj, int w_cols) {
-  extern __shared__ float2 sm[];  // two tiles [kTileRows][NK]: one is loaded while the other is worked on
-  const int j = threadIdx.x % nj, rg = threadIdx.x / nj, nrg = blockDim.x / nj;
-  float2 wc[NK];
-#pragma unroll
-  for (int k = 0; k < NK; k++) {
-    if (MODE == 0) {
-      wc[k] = W[k * w_cols + j];
-    } else {
-      wc[k] = W[j * w_cols + k];
-      wc[k].y = -wc[k].y;
-    }
-  }
-  const long long stride = (long long)gridDim.x * kTileRows;
-  long long row0 = (long long)blockIdx.x * kTileRows;
-  if (row0 < rows) tile_copy_async(sm, x + row0 * NK, (int)min((long long)kTileRows, rows - row0) * NK);
+  if (nk & 1)
+    for (int row = threadIdx.x; row < 2 * tile; row += kThreads) *reinterpret_cast<float2*>(xs + row * pitch + 8 * nk) = make_float2(0.f, 0.f);
+  const int tx = threadIdx.x % tx_n, ty = threadIdx.x / tx_n;
+  const bool works = ty < ty_n;
+  const long long stride = (long long)gridDim.x * tile;
+  long long row0 = (long long)blockIdx.x * tile;
+  if (row0 < rows) tile_copy_async(xs, pitch, x + row0 * nk, (int)min((long long)tile, rows - row0), copy_x);
   __pipeline_commit();
   for (int buf = 0; row0 < rows; row0 += stride, buf ^= 1) {
-    const int nr = (int)min((long long)kTileRows, rows - row0);
+    const int nr = (int)min((long long)tile, rows - row0);
     const long long next = row0 + stride;
-    if (next < rows) tile_copy_async(sm + (buf ^ 1) * kTileRows * NK, x + next * NK, (int)min((long long)kTileRows, rows - next) * NK);
+    if (next < rows) tile_copy_async(xs + (buf ^ 1) * tile * pitch, pitch, x + next * nk, (int)min((long long)tile, rows - next), copy_x);
     __pipeline_commit();
     __pipeline_wait_prior(1);
     __syncthreads();
-    const float2* xs = sm + buf * kTileRows * NK;
-    for (int row = rg; row < nr; row += nrg) {
-      const float4* xr = reinterpret_cast<const float4*>(xs + row * NK);
-      float sr = 0.f, si = 0.f, tr = 0.f, ti = 0.f;
+    if (works) {
+      float2 s[kRowsPerThread][2];
 #pragma unroll
-      for (int k = 0; k < NK / 2; k++) {
-        const float4 a = xr[k];
-        sr = fmaf(a.x, wc[2 * k].x, sr); sr = fmaf(-a.y, wc[2 * k].y, sr);
-        si = fmaf(a.x, wc[2 * k].y, si); si = fmaf(a.y, wc[2 * k].x, si);
-        tr = fmaf(a.z, wc[2 * k + 1].x, tr); tr = fmaf(-a.w, wc[2 * k + 1].y, tr);
-        ti = fmaf(a.z, wc[2 * k + 1].y, ti); ti = fmaf(a.w, wc[2 * k + 1].x, ti);
+      for (int i = 0; i < kRowsPerThread; i++) s[i][0] = s[i][1] = make_float2(0.f, 0.f);
+      const unsigned char* xr = xs + buf * tile * pitch + ty * pitch;
+      const float4* m = Ms + tx;
+#pragma unroll 4
+      for (int k = 0; k < nk2; k++) {  // rows past the end of the part read what the tile held before
+        const float4 w0 = m[2 * k * tx_n], w1 = m[(2 * k + 1) * tx_n];
+#pragma unroll
+        for (int i = 0; i < kRowsPerThread; i++) {
+          const float4 a = *reinterpret_cast<const float4*>(xr + i * ty_n * pitch + 16 * k);
+          mac(s[i][0], a.x, a.y, w0.x, w0.y);
+          mac(s[i][1], a.x, a.y, w0.z, w0.w);
+          mac(s[i][0], a.z, a.w, w1.x, w1.y);
+          mac(s[i][1], a.z, a.w, w1.z, w1.w);
+        }
       }
-      __stcs(r + (row0 + row) * nj + j, make_float2(sr + tr, si + ti));
+#pragma unroll
+      for (int i = 0; i < kRowsPerThread; i++) {
+        const int row = ty + i * ty_n;
+        if (row < nr) {
+          float2* p = r + (row0 + row) * nj + 2 * tx;
+          if (wide_r) {
+            __stcs(reinterpret_cast<float4*>(p), make_float4(s[i][0].x, s[i][0].y, s[i][1].x, s[i][1].y));
+          } else {
+            __stcs(p, s[i][0]);
+            if (2 * tx + 1 < nj) __stcs(p + 1, s[i][1]);
+          }
+        }
+      }
     }
     __syncthreads();  // the tile may be overwritten by the copy after next
   }
 }
 
-__global__ void __launch_bounds__(256) mix_back_w_kernel(float* __restrict__ Wg, const float2* __restrict__ x,
-                                                         const float2* __restrict__ g, long long rows, int ni, int nj,
-                                                         long long rows_per_block) {
-  extern __shared__ float2 sm[];      // two pairs of tiles [kTileRows][ni], [kTileRows][nj]
-  const int tile = kTileRows * (ni + nj);
+// The block's share of sum_row conj(x[row][i]) g[row][j].  Threads: tiles of 4 x 4 entries, times as many groups of rows as fit;
+// the groups' sums meet in shared memory, the blocks' in global memory.
+__global__ void __launch_bounds__(kThreads) mix_back_w_kernel(float* __restrict__ Wg, const float2* __restrict__ x, const float2* __restrict__ g,
+                                                              long long rows, int ni, int nj, long long rows_per_block, int tile_rows, RowCopy copy_x, RowCopy copy_g) {
+  extern __shared__ __align__(16) unsigned char sm[];
+  const int ti_n = (ni + 3) / 4, tj_n = (nj + 3) / 4, tiles = ti_n * tj_n, groups = kThreads / tiles;
+  const int px = 32 * ti_n + 16, pg = 32 * tj_n + 16, tile = tile_rows * (px + pg);
+  for (int e = threadIdx.x; e < 2 * tile / 16; e += kThreads) reinterpret_cast<float4*>(sm)[e] = make_float4(0.f, 0.f, 0.f, 0.f);  // padding
+  __syncthreads();
   const long long begin = (long long)blockIdx.x * rows_per_block, end = min(rows, begin + rows_per_block);
-  constexpr int kPairs = (kMixMaxN * kMixMaxN + 255) / 256;  // (i,j) sums per thread
-  float accr[kPairs], acci[kPairs];
-#pragma unroll
-  for (int p = 0; p < kPairs; p++) accr[p] = acci[p] = 0.f;
-  const int npairs = ni * nj;
   auto copy_tile = [&](int buf, long long row0) {
-    const int nr = (int)min((long long)kTileRows, end - row0);
-    tile_copy_async(sm + buf * tile, x + row0 * ni, nr * ni);
-    tile_copy_async(sm + buf * tile + kTileRows * ni, g + row0 * nj, nr * nj);
+    const int nr = (int)min((long long)tile_rows, end - row0);
+    tile_copy_async(sm + buf * tile, px, x + row0 * ni, nr, copy_x);
+    tile_copy_async(sm + buf * tile + tile_rows * px, pg, g + row0 * nj, nr, copy_g);
   };
   if (begin < end) copy_tile(0, begin);
   __pipeline_commit();
+  const int at = threadIdx.x % tiles, group = threadIdx.x / tiles, ti = at / tj_n, tj = at - ti * tj_n;
+  float2 s[4][4];
+#pragma unroll
+  for (int a = 0; a < 4; a++)
+#pragma unroll
+    for (int b = 0; b < 4; b++) s[a][b] = make_float2(0.f, 0.f);
   int buf = 0;
-  for (long long row0 = begin; row0 < end; row0 += kTileRows, buf ^= 1) {
-    const int nr = (int)min((long long)kTileRows, end - row0);
-    if (row0 + kTileRows < end) copy_tile(buf ^ 1, row0 + kTileRows);
+  for (long long row0 = begin; row0 < end; row0 += tile_rows, buf ^= 1) {
+    const int nr = (int)min((long long)tile_rows, end - row0);
+    if (row0 + tile_rows < end) copy_tile(buf ^ 1, row0 + tile_rows);
     __pipeline_commit();
     __pipeline_wait_prior(1);
     __syncthreads();
-    const float2* xs = sm + buf * tile;
-    const float2* gs = xs + kTileRows * ni;
+    if (group < groups) {
+      const unsigned char* xp = sm + buf * tile + 32 * ti;
+      const unsigned char* gp = sm + buf * tile + tile_rows * px + 32 * tj;
+#pragma unroll 2
+      for (int row = group; row < nr; row += groups) {
+        const float4 x0 = *reinterpret_cast<const float4*>(xp + row * px), x1 = *reinterpret_cast<const float4*>(xp + row * px + 16);
+        const float4 g0 = *reinterpret_cast<const float4*>(gp + row * pg), g1 = *reinterpret_cast<const float4*>(gp + row * pg + 16);
+        const float2 xv[4] = {{x0.x, x0.y}, {x0.z, x0.w}, {x1.x, x1.y}, {x1.z, x1.w}};
+        const float2 gv[4] = {{g0.x, g0.y}, {g0.z, g0.w}, {g1.x, g1.y}, {g1.z, g1.w}};
 #pragma unroll
-    for (int p = 0; p < kPairs; p++) {
-      const int pair = threadIdx.x + 256 * p;
-      if (pair < npairs) {
-        const int i = pair / nj, j = pair - i * nj;
-        float sr = accr[p], si = acci[p];
-        const float2* xa = xs + i;
-        const float2* gb = gs + j;
-#pragma unroll 8
-        for (int row = 0; row < nr; row++) {  // conj(x) g
-          const float2 a = xa[row * ni], b = gb[row * nj];
-          sr = fmaf(a.x, b.x, sr); sr = fmaf(a.y, b.y, sr);
-          si = fmaf(a.x, b.y, si); si = fmaf(-a.y, b.x, si);
-        }
-        accr[p] = sr;
-        acci[p] = si;
+        for (int a = 0; a < 4; a++)
+#pragma unroll
+          for (int b = 0; b < 4; b++) mac(s[a][b], xv[a].x, -xv[a].y, gv[b].x, gv[b].y);
       }
     }
     __syncthreads();  // the tiles may be overwritten by the copy after next
   }
+  float2* sums = reinterpret_cast<float2*>(sm);  // [group][tile][16]
+  if (group < groups) {
 #pragma unroll
-  for (int p = 0; p < kPairs; p++) {
-    const int pair = threadIdx.x + 256 * p;
-    if (pair < npairs) {
-      atomicAdd(Wg + 2 * pair, accr[p]);
-      atomicAdd(Wg + 2 * pair + 1, acci[p]);
-    }
+    for (int a = 0; a < 4; a++)
+#pragma unroll
+      for (int b = 0; b < 4; b++) sums[(group * tiles + at) * 16 + 4 * a + b] = s[a][b];
   }
+  __syncthreads();
+  for (int e = threadIdx.x; e < ni * nj; e += kThreads) {
+    const int i = e / nj, j = e - i * nj, at_e = (i / 4) * tj_n + j / 4, in = 4 * (i % 4) + j % 4;
+    float2 t = make_float2(0.f, 0.f);
+    for (int q = 0; q < groups; q++) {
+      const float2 v = sums[(q * tiles + at_e) * 16 + in];
+      t.x += v.x;
+      t.y += v.y;
+    }
+    atomicAdd(Wg + 2 * e, t.x);
+    atomicAdd(Wg + 2 * e + 1, t.y);
+  }
+}
+
+bool aligned(const void* p) { return reinterpret_cast<uintptr_t>(p) % 16 == 0; }
+RowCopy row_copy(const void* p, int n) {
+  RowCopy c;
+  c.wide = n % 2 == 0 && aligned(p);
+  c.per = c.wide ? n / 2 : n;
+  c.shift = -1;
+  for (int k = 0; k < 7; k++)
+    if (c.per == 1 << k) c.shift = k;
+  return c;
 }
 
 }  // namespace
@@ -175,30 +212,16 @@ int launch_mix(float* r, const float* x, const float* W, long long rows, int n_i
   if (n_in < 1 || n_out < 1 || n_in > kMixMaxN || n_out > kMixMaxN) return fail(GELIB_SKIPPED, fn, "more than 64 channels");
   if (rows <= 0) return GELIB_OK;
   const int nk = mode == 0 ? n_in : n_out, nj = mode == 0 ? n_out : n_in;  // contraction length, output channels
-  const size_t smem = ((size_t)nk * (nj + 1) + (size_t)kTileRows * nk) * sizeof(float2);
-  const unsigned blocks = (unsigned)std::min<long long>((rows + kTileRows - 1) / kTileRows, 148LL * 16);
-  cudaError_t e;
-  const bool pow2 = (nj & (nj - 1)) == 0 && nj <= 32;
-  if (pow2 && (nk == 16 || nk == 32)) {
-    const size_t smem_r = (size_t)2 * kTileRows * nk * sizeof(float2);
-    float2* rp = reinterpret_cast<float2*>(r);
-    const float2 *xp = reinterpret_cast<const float2*>(x), *wp = reinterpret_cast<const float2*>(W);
-    if (mode == 0 && nk == 16) mix_reg_kernel<0, 16><<<blocks, 256, smem_r, s>>>(rp, xp, wp, rows, nj, n_out);
-    else if (mode == 0) mix_reg_kernel<0, 32><<<blocks, 256, smem_r, s>>>(rp, xp, wp, rows, nj, n_out);
-    else if (nk == 16) mix_reg_kernel<1, 16><<<blocks, 256, smem_r, s>>>(rp, xp, wp, rows, nj, n_out);
-    else mix_reg_kernel<1, 32><<<blocks, 256, smem_r, s>>>(rp, xp, wp, rows, nj, n_out);
-    e = cudaSuccess;
-  } else if (mode == 0) {
-    e = cudaFuncSetAttribute(mix_kernel<0>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (e == cudaSuccess)
-      mix_kernel<0><<<blocks, 256, smem, s>>>(reinterpret_cast<float2*>(r), reinterpret_cast<const float2*>(x),
-                                              reinterpret_cast<const float2*>(W), rows, nk, nj, n_out);
-  } else {
-    e = cudaFuncSetAttribute(mix_kernel<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (e == cudaSuccess)
-      mix_kernel<1><<<blocks, 256, smem, s>>>(reinterpret_cast<float2*>(r), reinterpret_cast<const float2*>(x),
-                                              reinterpret_cast<const float2*>(W), rows, nk, nj, n_out);
-  }
+  const int tx_n = (nj + 1) / 2, nk2 = (nk + 1) / 2, pitch = 16 * nk2 + 16;
+  const int ty_n = std::min(kThreads / tx_n, 32768 / (kRowsPerThread * pitch));  // a tile of at most 32 KB
+  const int tile = ty_n * kRowsPerThread;
+  const size_t smem = (size_t)32 * nk2 * tx_n + (size_t)2 * tile * pitch;
+  const unsigned blocks = (unsigned)std::min<long long>((rows + tile - 1) / tile, 148LL * 8);
+  auto k = mode == 0 ? mix_kernel<0> : mix_kernel<1>;
+  cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  if (e == cudaSuccess)
+    k<<<blocks, kThreads, smem, s>>>(reinterpret_cast<float2*>(r), reinterpret_cast<const float2*>(x), reinterpret_cast<const float2*>(W), rows, nk,
+                                     nj, n_out, ty_n, row_copy(x, nk), nj % 2 == 0 && aligned(r));
   if (e == cudaSuccess) e = cudaGetLastError();
   if (e != cudaSuccess) return check_cuda(e, fn, "mixing kernel launch");
   count_launch();
@@ -209,15 +232,17 @@ int launch_mix_back_w(float* Wg, const float* x, const float* g, long long rows,
   static const char* fn = "SO3part_mix_back_w";
   if (n_in < 1 || n_out < 1 || n_in > kMixMaxN || n_out > kMixMaxN) return fail(GELIB_SKIPPED, fn, "more than 64 channels");
   if (rows <= 0) return GELIB_OK;
-  const long long want_blocks = std::min<long long>((rows + kTileRows - 1) / kTileRows, 148LL * 8);
+  const int ti_n = (n_in + 3) / 4, tj_n = (n_out + 3) / 4, tiles = ti_n * tj_n;
+  const int tile_rows = std::min(256, 32768 / (32 * (ti_n + tj_n) + 32) / 16 * 16);  // about 32 KB
+  const long long want_blocks = std::min<long long>((rows + tile_rows - 1) / tile_rows, 148LL * 3);
   long long rpb = (rows + want_blocks - 1) / want_blocks;
-  rpb = (rpb + kTileRows - 1) / kTileRows * kTileRows;
+  rpb = (rpb + tile_rows - 1) / tile_rows * tile_rows;
   const unsigned blocks = (unsigned)((rows + rpb - 1) / rpb);
-  const size_t smem = (size_t)2 * kTileRows * (n_in + n_out) * sizeof(float2);
+  const size_t smem = std::max((size_t)2 * tile_rows * (32 * (ti_n + tj_n) + 32), (size_t)kThreads / tiles * tiles * 128);
   cudaError_t e = cudaFuncSetAttribute(mix_back_w_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e == cudaSuccess)
-    mix_back_w_kernel<<<blocks, 256, smem, s>>>(Wg, reinterpret_cast<const float2*>(x), reinterpret_cast<const float2*>(g), rows,
-                                                n_in, n_out, rpb);
+    mix_back_w_kernel<<<blocks, kThreads, smem, s>>>(Wg, reinterpret_cast<const float2*>(x), reinterpret_cast<const float2*>(g), rows, n_in, n_out,
+                                                     rpb, tile_rows, row_copy(x, n_in), row_copy(g, n_out));
   if (e == cudaSuccess) e = cudaGetLastError();
   if (e != cudaSuccess) return check_cuda(e, fn, "weight gradient kernel launch");
   count_launch();

@@ -17,7 +17,7 @@ CSRC = os.path.join(HERE, "csrc")
 OBJ = os.path.join(CSRC, "build")
 LIB = os.path.join(HERE, "libgelib_b200.so")
 NATIVE = os.path.join(HERE, "_native.so")  # host side of the Python products (csrc/host.cpp), against torch's C++ library
-SOURCES = ["bank.cu", "plan.cu", "cg_fwd.cu", "cg_fwd_tc.cu", "cg_bwd.cu", "cg_bwd_pair.cu", "cg_bwd_tc.cu", "cg_narrow.cu", "cg_narrow1_bwd.cu", "cg_strided.cu", "col_plan.cu", "col_fwd.cu", "col_bwd.cu", "col_bwd_x.cu", "col_bwd_y.cu", "col_bwd_owned.cu", "mir_fwd.cu", "diag.cu", "diag_fwd.cu", "diag_bwd.cu", "spharm.cu", "probe.cu", "gather_apply.cu", "mix.cu", "cabi.cu"]
+SOURCES = ["bank.cu", "plan.cu", "cg_fwd.cu", "cg_fwd_tc.cu", "cg_bwd.cu", "cg_bwd_pair.cu", "cg_bwd_tc.cu", "cg_narrow.cu", "cg_narrow1_bwd.cu", "cg_strided.cu", "col_plan.cu", "col_fwd.cu", "col_bwd.cu", "col_bwd_x.cu", "col_bwd_y.cu", "col_bwd_owned.cu", "mir_fwd.cu", "mir_bwd.cu", "diag.cu", "diag_fwd.cu", "diag_bwd.cu", "spharm.cu", "probe.cu", "gather_apply.cu", "mix.cu", "cabi.cu"]
 HEADERS = ["common.h", "plan.h", "tc_common.h", "tma_maps.h", "col.h", "col_device.h", "mir.h", "f32x2.h", "col_bwd.cuh", os.path.join("..", "..", "include", "gelib_b200.h")]
 NVCC = os.environ.get("NVCC", "/usr/local/cuda/bin/nvcc")
 FLAGS = ["-O3", "-std=c++17", "-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo", "-Xcompiler", "-fPIC",

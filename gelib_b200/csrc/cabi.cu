@@ -251,12 +251,14 @@ int run_product(const char* fn, bool diag, int mode, int nr, const gelib_tensor5
   st = -1;
   if (c.dense_channels && !(mode == 0 && c.r_bcast) && !fp64 && col_mode() != kColOff) {
     bool plan_others = false, plan_column = false;
-    if (mode == 0) st = launch_mir_fwd(c, s, &plan_column);
+    st = mode == 0 ? launch_mir_fwd(c, s, &plan_column) : launch_mir_bwd(c, s, &plan_column);
     if (st == -1) st = mode == 0 ? launch_col_fwd(c, s, &plan_others) : launch_col_bwd(c, s, &plan_others);
     if (plan_others || plan_column) {  // should that fail, the call that needs the plan says so
       VecCall other = c;
       other.plan_only = true;
-      if (!plan_column || launch_col_fwd(other, s, &plan_others) == -1 || plan_others) run_kernels(other, mode, fp64, s);
+      int st_others = -1;
+      if (plan_column) st_others = mode == 0 ? launch_col_fwd(other, s, &plan_others) : launch_col_bwd(other, s, &plan_others);
+      if (st_others == -1 || plan_others) run_kernels(other, mode, fp64, s);
     }
   }
   return st == -1 ? run_kernels(c, mode, fp64, s) : st;

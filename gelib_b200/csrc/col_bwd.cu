@@ -15,7 +15,7 @@ int launch_col_bwd(const VecCall& c, cudaStream_t s, bool* plan_others) {
   if (!col_setup(c, true, &a, &plan)) return -1;
   if (!plan.dev) return GELIB_CUDA_ERROR;
   *plan_others = plan.plan_others;
-  if (a.nsplits == 0) return GELIB_OK;
+  if (a.nsplits == 0 || c.plan_only) return GELIB_OK;
   const bool do_x = !c.xg.empty(), do_y = !c.yg.empty();
   const cudaError_t e = plan.owned     ? col_launch_bwd_owned(a, plan, s)
                         : do_x && do_y ? col::launch_bwd_k<true, true>(a, plan, s)

@@ -32,6 +32,22 @@ struct MirArgs {
   int nitems;
 };
 
+// Backward, mir_bwd.cu.
+struct MirBwdArgs {
+  ColPart x[kMaxParts], yg[kMaxParts], g[kMaxParts];
+  unsigned char xl[kMaxParts];
+  int nx, nr;
+  int y_rows;            // most rows of a y part
+  int ring_bytes;        // of the item tables in shared memory
+  unsigned n, ncols;     // channels of a cell, columns in all
+  int xcells;            // most cells that the columns of a warp touch
+  const int4* items;     // per item {header, records, coefficients}
+  const int2* dir;       // per item {first int4, int4 units | place in the ring << 8}
+  int nitems;
+};
+// Flags of a backward item: only row m has the first entry, only row m + 1 the last; a row m alone; first and last of an l2.
+enum { kMirPrologue = 1, kMirEpilogue = 2, kMirSingle = 4, kMirFirstOfB = 8, kMirLastOfB = 16 };
+
 #ifdef __CUDACC__
 namespace mir {
 __device__ __forceinline__ uint32_t sptr(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
@@ -45,6 +61,7 @@ template <int N>
 __device__ __forceinline__ void cp_wait() {
   asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory");
 }
+__device__ __forceinline__ void cp_wait_all() { asm volatile("cp.async.wait_all;" ::: "memory"); }
 }  // namespace mir
 #endif
 

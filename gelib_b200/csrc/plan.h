@@ -59,6 +59,7 @@ int launch_cg_strided_static(const VecCall& c, cudaStream_t s);  // forward, tab
 // Diagonal products and one-channel x; -1 when the call does not qualify.  *plan_others: the signature goes to other kernels
 // at other batch sizes, and they have not planned it yet.
 int launch_mir_fwd(const VecCall& c, cudaStream_t s, bool* plan_others);
+int launch_mir_bwd(const VecCall& c, cudaStream_t s, bool* plan_others);
 int launch_col_fwd(const VecCall& c, cudaStream_t s, bool* plan_others);
 int launch_col_bwd(const VecCall& c, cudaStream_t s, bool* plan_others);
 // Option "col": by the rules of col_plan.cu, not at all ("0"), or, with every call that the column kernels can take, one or

@@ -124,3 +124,31 @@ def test_a_type_of_few_items_is_captured_at_another_batch(G, oracle, diag, n, ba
     f()
     for l in got:
         assert float((got[l] - r[l]).abs().max()) <= 1e-5 * float(r[l].abs().max())
+
+
+def test_row_pair_gradient_by_the_rule(G, oracle):
+    """Enough columns for the row-pair gradient to be taken by its rule, in the last cells of which the oracle is asked: the
+    choice of kernel changes nothing, and a first small call plans what the large one runs."""
+    n, lmax, B = 16, 3, 6100
+    tx, ty = U(lmax, 1), U(lmax, n)
+    tr = oracle.cg_type(tx, ty, lmax, False)
+    cells = slice(B - 3, B)
+
+    def call(B):
+        x, g = parts(1, B, tx), parts(20, B, tr)
+        dx, dg = cuda(x), cuda(g)
+        yg = {l: torch.zeros(B, 2 * l + 1, n, dtype=torch.complex64, device="cuda") for l in ty}
+        return (lambda: vec(G, yg).addCGproduct_back1(vec(G, dg), vec(G, dx))), yg, x, g
+
+    call(3)[0]()
+    f, yg, x, g = call(B)
+    torch.cuda.synchronize()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        f()
+    graph.replay()
+    torch.cuda.synchronize()
+    want = {l: np.zeros((3, 2 * l + 1, n), np.complex64) for l in ty}
+    oracle.vec_cg_back1(want, {l: np_c(t[cells]) for l, t in g.items()}, {l: np_c(t[cells]) for l, t in x.items()})
+    for l in want:
+        assert np.abs(np_c(yg[l][cells]) - want[l]).max() < 1e-5 * np.abs(want[l]).max()

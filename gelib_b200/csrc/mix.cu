@@ -10,10 +10,11 @@
 //
 // Both kernels stage tiles of rows in shared memory (asynchronous copies, one tile in flight while the other is worked on) and
 // give a thread a tile of the result: 4 rows x 2 columns of the product, 4 x 4 entries of the weight gradient, so that a 16-byte
-// load feeds 11 (16) multiply-adds.  Measured against one output element (one (i,j) sum) per thread, us, product / adjoint /
-// weight gradient: 16 x 16 channels, 3.2 million rows 215 / 240 / 396 -> 217 / 214 / 245; 32 x 32, 400000 96 / 156 / 194 -> 96 /
-// 98 / 110; 8 x 8, 2 million 105 / 107 / 132 -> 55 / 55 / 77; 12 x 20, 500000 76 / 70 / 85 -> 47 / 49 / 62; 64 x 64, 100000 207 /
-// 213 / 241 -> 94 / 102 / 108.  At 16 channels the multiply-adds alone take 91 us and the memory 126.
+// load feeds 11 (16) multiply-adds; products are summed in two halves, and 8, 16 and 32 channels on both sides have a body of
+// their own (16 x 16, 3.2 million rows: 240 us without).  Measured against one output element (one (i,j) sum) per thread, us,
+// product / adjoint / weight gradient: 16 x 16 channels, 3.2 million rows 214 / 238 / 396 -> 197 / 197 / 247; 32 x 32, 400000 96 /
+// 156 / 194 -> 98 / 99 / 110; 8 x 8, 2 million 104 / 104 / 132 -> 57 / 57 / 79; 12 x 20, 500000 76 / 70 / 85 -> 49 / 51 / 62; 64 x
+// 64, 100000 207 / 213 / 243 -> 106 / 115 / 108.  At 16 channels the multiply-adds alone take 91 us and the memory 126.
 #include <cuda_pipeline.h>
 
 #include <algorithm>
@@ -50,12 +51,13 @@ __device__ __forceinline__ void mac(float2& s, float ar, float ai, float br, flo
 }
 
 // r[row][j] = sum_k x[row][k] M[k][j], M = W (mode 0) or its adjoint (mode 1).  A thread has columns 2 tx, 2 tx + 1 of the rows
-// ty, ty + TY, ..; odd lengths are padded with zeros in shared memory.
-template <int MODE>
-__global__ void __launch_bounds__(kThreads) mix_kernel(float2* __restrict__ r, const float2* __restrict__ x, const float2* __restrict__ W,
-                                                       long long rows, int nk, int nj, int w_cols, int ty_n, RowCopy copy_x, bool wide_r) {
+// ty, ty + TY, ..; odd lengths are padded with zeros in shared memory.  N: both channel counts where they are known here.
+template <int MODE, int N>
+__global__ void __launch_bounds__(kThreads, 4) mix_kernel(float2* __restrict__ r, const float2* __restrict__ x, const float2* __restrict__ W,
+                                                       long long rows, int nk_arg, int nj_arg, int w_cols, int ty_n_arg, RowCopy copy_x, bool wide_r) {
   extern __shared__ __align__(16) unsigned char sm[];
-  const int tx_n = (nj + 1) / 2, nk2 = (nk + 1) / 2, tile = ty_n * kRowsPerThread;
+  const int nk = N > 0 ? N : nk_arg, nj = N > 0 ? N : nj_arg;
+  const int tx_n = (nj + 1) / 2, nk2 = (nk + 1) / 2, ty_n = N > 0 ? kThreads / tx_n : ty_n_arg, tile = ty_n * kRowsPerThread;
   const int pitch = 16 * nk2 + 16;                        // bytes of a staged row of x
   float4* Ms = reinterpret_cast<float4*>(sm);             // [2 nk2][tx_n]: two columns each
   unsigned char* xs = sm + 32 * nk2 * tx_n;               // two tiles
@@ -91,12 +93,12 @@ __global__ void __launch_bounds__(kThreads) mix_kernel(float2* __restrict__ r, c
     __pipeline_wait_prior(1);
     __syncthreads();
     if (works) {
-      float2 s[kRowsPerThread][2];
+      float2 s[kRowsPerThread][2], t[kRowsPerThread][2];  // sums over even and over odd k
 #pragma unroll
-      for (int i = 0; i < kRowsPerThread; i++) s[i][0] = s[i][1] = make_float2(0.f, 0.f);
+      for (int i = 0; i < kRowsPerThread; i++) s[i][0] = s[i][1] = t[i][0] = t[i][1] = make_float2(0.f, 0.f);
       const unsigned char* xr = xs + buf * tile * pitch + ty * pitch;
       const float4* m = Ms + tx;
-#pragma unroll 4
+#pragma unroll 2
       for (int k = 0; k < nk2; k++) {  // rows past the end of the part read what the tile held before
         const float4 w0 = m[2 * k * tx_n], w1 = m[(2 * k + 1) * tx_n];
 #pragma unroll
@@ -104,13 +106,18 @@ __global__ void __launch_bounds__(kThreads) mix_kernel(float2* __restrict__ r, c
           const float4 a = *reinterpret_cast<const float4*>(xr + i * ty_n * pitch + 16 * k);
           mac(s[i][0], a.x, a.y, w0.x, w0.y);
           mac(s[i][1], a.x, a.y, w0.z, w0.w);
-          mac(s[i][0], a.z, a.w, w1.x, w1.y);
-          mac(s[i][1], a.z, a.w, w1.z, w1.w);
+          mac(t[i][0], a.z, a.w, w1.x, w1.y);
+          mac(t[i][1], a.z, a.w, w1.z, w1.w);
         }
       }
 #pragma unroll
       for (int i = 0; i < kRowsPerThread; i++) {
         const int row = ty + i * ty_n;
+#pragma unroll
+        for (int c = 0; c < 2; c++) {
+          s[i][c].x += t[i][c].x;
+          s[i][c].y += t[i][c].y;
+        }
         if (row < nr) {
           float2* p = r + (row0 + row) * nj + 2 * tx;
           if (wide_r) {
@@ -217,7 +224,10 @@ int launch_mix(float* r, const float* x, const float* W, long long rows, int n_i
   const int tile = ty_n * kRowsPerThread;
   const size_t smem = (size_t)32 * nk2 * tx_n + (size_t)2 * tile * pitch;
   const unsigned blocks = (unsigned)std::min<long long>((rows + tile - 1) / tile, 148LL * 8);
-  auto k = mode == 0 ? mix_kernel<0> : mix_kernel<1>;
+  auto k = mode == 0 ? mix_kernel<0, 0> : mix_kernel<1, 0>;
+  if (nk == 8 && nj == 8) k = mode == 0 ? mix_kernel<0, 8> : mix_kernel<1, 8>;
+  if (nk == 16 && nj == 16) k = mode == 0 ? mix_kernel<0, 16> : mix_kernel<1, 16>;
+  if (nk == 32 && nj == 32) k = mode == 0 ? mix_kernel<0, 32> : mix_kernel<1, 32>;
   cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e == cudaSuccess)
     k<<<blocks, kThreads, smem, s>>>(reinterpret_cast<float2*>(r), reinterpret_cast<const float2*>(x), reinterpret_cast<const float2*>(W), rows, nk,

@@ -12,7 +12,7 @@
 // registers, asks those of the one after into the L2, and copies the tables of the third (cp.async).
 //
 // Measured against cg_narrow1_bwd_kernel and the column kernel, us: maxl 6 x 16, 65536 cells 5470 -> 4580; maxl 4 x 32,
-// 10000 592 -> 430; maxl 3 x 9, 44444 460 -> 327.  Bound by issue and latency: 96 k warp instructions per 32 columns at maxl 6, of
+// 10000 586 -> 480; maxl 3 x 9, 44444 461 -> 349.  Bound by issue and latency: 96 k warp instructions per 32 columns at maxl 6, of
 // which the band loops are 40 %, issued in 54 % of the cycles with 16 warps on an SM.  Without the request into the L2 5310, at 16 warps
 // instead of 20 4970, at 24, which spills, 5420; two columns per lane (187 registers, 11 warps) 6790.
 #include <algorithm>
@@ -140,10 +140,13 @@ __device__ __forceinline__ void prefetch_rows(const unsigned char* it, const uns
     default: break;                \
   }
 
+// Two levels: a pair's sums are kept apart and added to those of the pairs before it when the pair ends, as the column kernel sums;
+// with up to five l there is room for them (maxl 4 x 16: error against 64-bit sums 1.18e-7 in one level).
 // NLMAX: most output l of an item.  WARPS: warps that should share an SM; more of them cover the latency of the loads better,
 // and registers beyond these numbers bought nothing.
 template <int NLMAX, int WARPS>
 __global__ void __launch_bounds__(32, WARPS) mir_bwd_kernel(const __grid_constant__ MirBwdArgs A) {
+  constexpr bool TWO_LEVELS = NLMAX <= kMirTwoLevels;
   extern __shared__ __align__(16) unsigned char smem[];
   const int lane = threadIdx.x;
   unsigned col = blockIdx.x * 32 + lane;
@@ -154,7 +157,8 @@ __global__ void __launch_bounds__(32, WARPS) mir_bwd_kernel(const __grid_constan
   unsigned long long* ptr = reinterpret_cast<unsigned long long*>(smem);
   unsigned char* ring = smem + 256 * A.nr;
   unsigned char* yg = ring + A.ring_bytes + 8 * lane;
-  unsigned char* xs = ring + A.ring_bytes + kPitch * A.y_rows;
+  unsigned char* total = yg + (TWO_LEVELS ? kPitch * A.y_rows : 0);
+  unsigned char* xs = ring + A.ring_bytes + kPitch * A.y_rows * (TWO_LEVELS ? 2 : 1);
   const int xpitch = 8 * A.xcells;
 
   auto dir = [&](int i) { return i < A.nitems ? __ldg(A.dir + i) : make_int2(0, 0); };
@@ -208,7 +212,7 @@ __global__ void __launch_bounds__(32, WARPS) mir_bwd_kernel(const __grid_constan
     }
     const int lb = (h.w >> 8) & 255;
     if (flags & kMirFirstOfB)
-      for (int r = 0; r <= 2 * lb; r++) *reinterpret_cast<float2*>(yg + kPitch * r) = make_float2(0.f, 0.f);
+      for (int r = 0; r <= 2 * lb; r++) *reinterpret_cast<float2*>(yg + kPitch * r) = *reinterpret_cast<float2*>(total + kPitch * r) = make_float2(0.f, 0.f);
     Band B;
     B.cf = reinterpret_cast<const float4*>(it + 16 + 16 * nl);
     B.x = xs + xpitch * h.y;
@@ -218,11 +222,18 @@ __global__ void __launch_bounds__(32, WARPS) mir_bwd_kernel(const __grid_constan
     } else {
       GELIB_MIR_SWITCH(nl, GELIB_MIR_RUN)
     }
+    if (TWO_LEVELS && (flags & kMirLastOfPair))
+      for (int r = 0; r <= 2 * lb; r++) {
+        float2 *a = reinterpret_cast<float2*>(total + kPitch * r), *b = reinterpret_cast<float2*>(yg + kPitch * r);
+        const float2 u = *a, v = *b;
+        *a = make_float2(u.x + v.x, u.y + v.y);
+        *b = make_float2(0.f, 0.f);
+      }
     if ((flags & kMirLastOfB) && ok) {
       const ColPart& p = A.yg[h.w & 255];
       unsigned char* q = reinterpret_cast<unsigned char*>(p.base) + (unsigned long long)cell * p.cell_stride + 8ull * ch;
       for (int r = 0; r <= 2 * lb; r++) {
-        const float2 v = *reinterpret_cast<const float2*>(yg + kPitch * r);
+        const float2 v = *reinterpret_cast<const float2*>(total + kPitch * r);
         asm volatile("red.global.add.v2.f32 [%0], {%1, %2};" ::"l"(q + (unsigned long long)r * p.unit), "f"(v.x), "f"(v.y) : "memory");
       }
     }
@@ -307,6 +318,7 @@ void build_bwd(DevicePlan& p, const std::vector<PartSig>& xs, const std::vector<
           p.h_items.push_back(q);
         }
         const int size = (int)p.h_items.size() - last_header;
+        if (single && g + 1 == groups) p.h_items[last_header].x |= kMirLastOfPair << 16;
         p.h_jobs.push_back(last_header);
         p.h_jobs.push_back(size);
         sizes.push_back(size);
@@ -384,15 +396,15 @@ int launch_mir_bwd(const VecCall& c, cudaStream_t s, bool* plan_others) {
   a.ring_bytes = plan->tables[0];
   a.y_rows = plan->tables[1];
   const int nl = plan->tables[2];
-  const size_t smem = 256 * (size_t)a.nr + a.ring_bytes + mir::kPitch * (size_t)a.y_rows + 8 * (size_t)a.xcells * xrows;
+  const size_t smem = 256 * (size_t)a.nr + a.ring_bytes + mir::kPitch * (size_t)a.y_rows * (nl <= kMirTwoLevels ? 2 : 1) + 8 * (size_t)a.xcells * xrows;
   if (smem > kColMaxSmem) return -1;
-  // Where these kernels are faster: enough columns for several warps per scheduler, and enough work per row of g.  us, the others
+  // Where this kernel is faster: enough columns for several warps per scheduler, and enough work per row of g.  us, the others
   // (cg_narrow1_bwd_kernel, column kernel) / this one: maxl 6 x 16, 60000 columns 386 / 414, 100000 703 / 729, 400000 2162 / 1890;
-  // maxl 4 x 16, 60000 110 / 138, 100000 215 / 172, 400000 584 / 530; maxl 3 x 9, 60000 87 / 86, 100000 130 / 111, 400000 460 / 327;
-  // maxl 8 x 16, 100000 2083 / 1756; but maxl 2 x 16, 100000 33 / 44, maxl 6 x 4 (eight cells to a warp), 400000 3780 / 4496, and
-  // more than 32 channels, which the column kernel takes two to a lane, l <= 2 with l <= 7 x 40, 160000 338 / 405.
+  // maxl 3 x 9, 60000 87 / 86, 100000 130 / 113, 400000 461 / 349; maxl 4 x 21, 400000 907 / 748; maxl 4 x 32, 320000 586 / 480; maxl
+  // 8 x 16, 100000 2083 / 1756; but maxl 2 x 16, 100000 33 / 44, maxl 6 x 4 (eight cells to a warp), 400000 3780 / 4496, maxl 4 x 16,
+  // 400000 (two columns per lane there, none padded) 585 / 598, and more than 32 channels, l <= 2 with l <= 7 x 40, 160000 338 / 405.
   if (mode == kColAuto) {
-    if (n > 32 || nl < 4 || (nl > 5 && n < 8)) return -1;
+    if (n > 32 || nl < 4 || (nl > 5 && n < 8) || (nl <= 5 && (n == 8 || n == 16))) return -1;
     const bool first = plan->first_use.exchange(false);
     if (a.ncols < (nl == 6 || nl == 7 ? 128000u : 96000u)) return -1;
     *plan_others = first;

@@ -129,7 +129,7 @@ def test_a_type_of_few_items_is_captured_at_another_batch(G, oracle, diag, n, ba
 def test_row_pair_gradient_by_the_rule(G, oracle):
     """Enough columns for the row-pair gradient to be taken by its rule, in the last cells of which the oracle is asked: the
     choice of kernel changes nothing, and a first small call plans what the large one runs."""
-    n, lmax, B = 16, 3, 6100
+    n, lmax, B = 20, 3, 4900
     tx, ty = U(lmax, 1), U(lmax, n)
     tr = oracle.cg_type(tx, ty, lmax, False)
     cells = slice(B - 3, B)

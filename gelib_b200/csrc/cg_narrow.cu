@@ -1,5 +1,5 @@
 // Clebsch-Gordan product of a narrow x (a few channels, e.g. spherical harmonics with one channel per l) with a
-// y of up to 32 channels: forward and both gradients.
+// y of up to 32 channels: forward and both gradients.  (x with one channel mostly goes to mir_fwd.cu, mir_bwd.cu.)
 //
 // The tiled kernels (cg_fwd.cu, cg_bwd.cu) get their operand reuse from an n1 x n2 channel tile; with one or two
 // x channels there is no tile, and every multiply-add would need its own shared-memory operand.  Here the reuse

@@ -498,7 +498,7 @@ bool col_setup(const VecCall& c, bool backward, ColArgs* a, ColPlan* plan) {
   const long long columns = c.cg.ncells * n;
   const int mode = col_mode();
   plan->cpl = two && (mode == kColAuto ? columns >= 64 * 148 * 4 : mode == kColTwo) ? 2 : 1;
-  // Diagonal forward: with l >= 6 and full 64-channel slices diag_fwd_cell_kernel, which shares its operands between the
+  // Diagonal forward, where the mirrored-row kernel does not take it: with l >= 6 and full 64-channel slices diag_fwd_cell_kernel, which shares its operands between the
   // warps of a block, fits more warps on an SM (us, that kernel / this one): maxl 8 x 128 channels, batch 2048 3018 / 3820;
   // maxl 6 x 64 608 / 835, maxl 6 x 128 1208 / 1265; but maxl 5 x 128 711 / 661, maxl 8 x 48, batch 1000 821 / 652.
   if (c.diag && mode == kColAuto) {

@@ -1,4 +1,5 @@
-// Diagonal Clebsch-Gordan product, forward, one cell per CTA: the variant used for 17 or more channels.
+// Diagonal Clebsch-Gordan product, forward, one cell per CTA: the variant used for 17 or more channels by calls that the
+// mirrored-row and column kernels do not take.
 //
 // Same arithmetic and item structure as diag_fwd_kernel (diag.cu): an item is one (l1,l2) pair and one output
 // row index m; every product p = x[m1] y[m-m1] feeds the accumulators of all output l through a dense

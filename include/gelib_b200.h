@@ -236,7 +236,9 @@ double gelib_probe_fp32_tflops(float* scratch, int ctas, int reps, void* stream)
  * gradient of y for a one-channel x takes the kernel written for that shape, "0": the general narrow kernel);
  * name "col": "auto" | "0" | "one" | "two" | "split1", "split2", .. (diagonal products and products of a one-channel x take
  * the column kernels by rules on the type and the number of cells, not at all, or whenever they can: with one or two columns
- * per lane and the walk in one piece, or with the walk split over blocks in the k-th way, the last way for larger k);  names "fwd_layout", "bwd_layout": "auto" or the index of
+ * per lane and the walk in one piece, or with the walk split over blocks in the k-th way, the last way for larger k);  name "mir": "auto" | "0" | "one" | "two" (the
+ * mirrored-row and row-pair kernels of such products by rules, while "col" is "auto", not at all, or whenever they can, with one
+ * or two columns per lane);  names "fwd_layout", "bwd_layout": "auto" or the index of
  * a lane layout of the FP32 kernels (a call it does not fit is refused);  name "inject_timeout": "0" | "1" (tests:
  * one bounded device wait is made to run out).
  * Initial values: the environment variables GELIB_B200_FWD, GELIB_B200_BWD, GELIB_B200_PAIR_TMA,

@@ -18,8 +18,7 @@
 // Everything a warp reads from global memory -- b rows, a rows, the gradient rows g -- arrives through one stream of rows
 // (cp.async, 8 or 16 bytes per lane) in a ring of kColRing rows, whose order is the order of use: taking k rows requests
 // the k rows that come kColRing later, so the bytes in flight do not depend on how short the steps are.  What the warps
-// of a block share is the walk itself: a chunk (row addresses, step records, coefficients stored twice for the packed
-// multiply-adds) is copied to shared memory one chunk ahead.
+// of a block share is the walk itself: a chunk (row addresses, step records, coefficients) is copied to shared memory one chunk ahead.
 // Gradient rows are added to global memory with red.  Unless an operand is broadcast over cells (stride 0) a row belongs to
 // one lane of one block, so the sums have one order and gradients are bitwise repeatable.  Calls with few columns split the
 // walk over blocks; in the backward by gradient rows ("owned": the blocks of a cluster walk everything that is added to the
@@ -28,7 +27,7 @@
 // may instead split by pairs, and then several blocks add to a row.
 // Why this form: diag_bwd_cell_kernel spends its time in four shared-memory atomics (compare-and-swap loops) per band
 // entry, which a lane that owns its column does not need.  Measured, backward of the diagonal product: maxl 8 x 128
-// channels, batch 2048 10.5 -> 4.8 ms; maxl 6 x 33, batch 4000 4.3 -> 1.1 ms; maxl 3 x 12, batch 500 49 -> 29 us (forward 32 ->
+// channels, batch 2048 10.5 -> 4.7 ms; maxl 6 x 33, batch 4000 4.3 -> 1.0 ms; maxl 3 x 12, batch 500 49 -> 29 us (forward 32 ->
 // 15 us).  At maxl 8 the backward holds two warps per scheduler -- 252 registers a thread and 25.6 KB of shared memory a warp
 // both end there -- and issues in 42 % of its cycles: 502 k warp instructions per 64 columns, whose largest stalls are
 // fixed-latency dependencies (1.3 cycles per issue) and shared memory (0.7).  The forward issues in 32 %: 345 k

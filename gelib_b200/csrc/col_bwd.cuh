@@ -52,6 +52,7 @@ __device__ __forceinline__ void cluster_sync() {
 template <int K, int CPL, bool DOA, bool DOB, int NL, int NLMIN = NL - 1>
 __device__ __forceinline__ void bwd_step(Walk<CPL>& W, int st, const float2 (&a)[K][CPL], float2 (&ag)[K][CPL], float2 (&bg)[K][CPL],
                                          uint32_t bptr) {
+  constexpr int kCoefs = (NL + 3) / 4 * 4;
   cp_wait<kColRing - NL>();
   const int nl = st & 255, lo = (st >> 8) & 255, hi = (st >> 16) & 255;
   f32x2 g[NL][CPL];
@@ -72,12 +73,16 @@ __device__ __forceinline__ void bwd_step(Walk<CPL>& W, int st, const float2 (&a)
         if (4 * blk + e >= K) continue;
         f32x2 G[CPL];
 #pragma unroll
-        for (int j = 0; j < NL; j += 2) {
-          const ulonglong2 q = *reinterpret_cast<const ulonglong2*>(W.smem + W.coef + (i * NL + j) * 8);
+        for (int j = 0; j < NL; j += 4) {
+          const Coefs q = coefs<NL>(W.smem + W.coef + (i * kCoefs + j) * 4);
 #pragma unroll
           for (int c = 0; c < CPL; c++) {
-            G[c] = j == 0 ? mul2(q.x, g[0][c]) : fma2(q.x, g[j][c], G[c]);
-            G[c] = fma2(q.y, g[j + 1][c], G[c]);
+            G[c] = j == 0 ? mul2(q.c[0], g[0][c]) : fma2(q.c[0], g[j][c], G[c]);
+            G[c] = fma2(q.c[1], g[j + 1][c], G[c]);
+            if (j + 2 < NL) {
+              G[c] = fma2(q.c[2], g[j + 2][c], G[c]);
+              G[c] = fma2(q.c[3], g[j + 3][c], G[c]);
+            }
           }
         }
         float gr[CPL], gi[CPL];
@@ -101,7 +106,7 @@ __device__ __forceinline__ void bwd_step(Walk<CPL>& W, int st, const float2 (&a)
       }
     }
   }
-  W.coef += K * NL * 8;
+  W.coef += K * kCoefs * 4;
 }
 
 // bval, bacc: byte offsets of the lane's slots of b row 0 (values, gradients).  OWNED: the a rows' gradients are added to

@@ -46,6 +46,30 @@ __device__ __forceinline__ void red_row(unsigned char* p, const Row<CPL>& v) {
   }
 }
 
+// Coefficients of a step's next four output l, each twice for the packed multiply-adds.  They are paired in registers: read as
+// pairs they took the rate of shared memory (diagonal product, both gradients, maxl 8 x 128 channels, batch 2048 4919 -> 4697 us,
+// maxl 6 x 33, batch 4000 1073 -> 1015; gradient of y, maxl 8 x 128 4493 -> 4299).  For a step of two l nothing would be saved: the
+// walk holds its coefficients twice.
+struct Coefs {
+  f32x2 c[4];
+};
+template <int NL>
+__device__ __forceinline__ Coefs coefs(const unsigned char* p) {
+  Coefs q;
+  if constexpr (NL == 2) {
+    const ulonglong2 v = *reinterpret_cast<const ulonglong2*>(p);
+    q.c[0] = v.x;
+    q.c[1] = v.y;
+  } else {
+    const float4 v = *reinterpret_cast<const float4*>(p);
+    q.c[0] = pack2(v.x, v.x);
+    q.c[1] = pack2(v.y, v.y);
+    q.c[2] = pack2(v.z, v.z);
+    q.c[3] = pack2(v.w, v.w);
+  }
+  return q;
+}
+
 // Header of a chunk: {byte offsets of the request list, the store list, the segments, the coefficients}, then
 // {address records, 0, 0, 0} and the address records.  A segment: {a rows | flags<<8 | steps<<16, d = m - mlo of the first
 // step, first a row, a part}, {b part, lb, first row of the sums (owned walks), 0}, and one int per step (padded to four): nl | first entry of the band<<8 |

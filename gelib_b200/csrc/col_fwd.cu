@@ -11,6 +11,7 @@ template <int K, int CPL, int NL>
 __device__ __forceinline__ void fwd_step(Walk<CPL>& W, int st, const float2 (&a)[K][CPL], uint32_t bptr, bool add) {
   const int nl = st & 255, lo = (st >> 8) & 255, hi = (st >> 16) & 255;
   const unsigned span = hi - lo;
+  constexpr int kCoefs = (NL + 3) / 4 * 4;
   f32x2 acc[NL][CPL];
 #pragma unroll
   for (int j = 0; j < NL; j++)
@@ -36,18 +37,22 @@ __device__ __forceinline__ void fwd_step(Walk<CPL>& W, int st, const float2 (&a)
           }
         }
 #pragma unroll
-        for (int j = 0; j < NL; j += 2) {
-          const ulonglong2 q = *reinterpret_cast<const ulonglong2*>(W.smem + W.coef + (i * NL + j) * 8);
+        for (int j = 0; j < NL; j += 4) {
+          const Coefs q = coefs<NL>(W.smem + W.coef + (i * kCoefs + j) * 4);
 #pragma unroll
           for (int c = 0; c < CPL; c++) {
-            acc[j][c] = fma2(q.x, p[c], acc[j][c]);
-            acc[j + 1][c] = fma2(q.y, p[c], acc[j + 1][c]);
+            acc[j][c] = fma2(q.c[0], p[c], acc[j][c]);
+            acc[j + 1][c] = fma2(q.c[1], p[c], acc[j + 1][c]);
+            if (j + 2 < NL) {
+              acc[j + 2][c] = fma2(q.c[2], p[c], acc[j + 2][c]);
+              acc[j + 3][c] = fma2(q.c[3], p[c], acc[j + 3][c]);
+            }
           }
         }
       }
     }
   }
-  W.coef += K * NL * 8;
+  W.coef += K * kCoefs * 4;
   unsigned long long ad[NL];
 #pragma unroll
   for (int j = 0; j < NL; j++)

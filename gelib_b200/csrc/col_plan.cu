@@ -87,7 +87,7 @@ struct Builder {
     rows.resize(n0);
     int u = 2 + ((int)s.steps.size() + 3) / 4;
     for (const Step& st : s.steps) {
-      u += s.kb * nlp(st.nl, s.kb) / 2;
+      u += s.kb * ((nlp(st.nl, s.kb) + 3) / 4);
       if (!backward) *recs += st.nl;
     }
     return u + *recs;
@@ -123,7 +123,7 @@ void pair_segments(const Builder& B, const std::vector<const Triple*>& ts, Segme
       Step st{m, 0, std::max(0, m - s.lb - s.mlo), std::min(s.kb - 1, m + s.lb - s.mlo)};
       for (const Triple* t : s.ls) st.nl += t->l >= std::abs(m);
       if (st.hi < st.lo || st.nl == 0) continue;
-      const int need = 1 + s.kb * B.nlp(st.nl, s.kb) / 2 + st.nl;
+      const int need = 1 + s.kb * ((B.nlp(st.nl, s.kb) + 3) / 4) + st.nl;
       if (need > room || s.steps.empty() || st.m != s.steps.back().m + 1) {  // a new piece
         if (!s.steps.empty()) out->push_back(s);
         s.steps.clear();
@@ -344,17 +344,18 @@ void build_walk(DevicePlan& p, const std::vector<PartSig>& xs, const std::vector
       for (size_t q = c.from; q < c.to; q++) {
         const Segment& s = run[q];
         for (const Step& st : s.steps)
-          for (int i = 0; i < s.kb; i++)
-            for (int j = 0; j < B.nlp(st.nl, s.kb); j++) {
+          for (int i = 0; i < s.kb; i++) {
+            const int nlp = B.nlp(st.nl, s.kb);
+            for (int j = 0; j < (nlp == 2 ? 2 : (nlp + 3) / 4 * 4); j++) {
               float x = 0.f;
               if (i >= st.lo && i <= st.hi && j < st.nl) {
                 const Triple& t = *s.ls[s.ls.size() - st.nl + j];
                 const int ma = s.mlo + i;
                 x = B.coefficient(p.sched, t, st.m, s.half == 0 ? ma : st.m - ma);
               }
-              cf.push_back(x);
-              cf.push_back(x);
+              cf.insert(cf.end(), nlp == 2 ? 2 : 1, x);  // two l: each twice, for the packed multiply-adds
             }
+          }
       }
       for (size_t i = 0; i < cf.size(); i += 4) {
         int4 q;

@@ -23,6 +23,16 @@ namespace {
 
 using Tensors = std::vector<at::Tensor>;
 
+// A plain Python int of 32 bits.  Others are left to the Python code too: through ctypes the low 32 bits of a larger maxl count
+// (sys.maxsize: every l), and what is not an int is refused there.
+std::optional<int> plain_int(pybind11::handle h) {
+  if (!PyLong_CheckExact(h.ptr())) return std::nullopt;
+  int overflow = 0;
+  const long v = PyLong_AsLongAndOverflow(h.ptr(), &overflow);
+  if (overflow || v < INT_MIN || v > INT_MAX) return std::nullopt;
+  return static_cast<int>(v);
+}
+
 // The tensor in canonical form, core/Gpart.hpp:450-469 of GElib; false when it is not plain.
 bool describe(const at::Tensor& t, c10::Device device, gelib_tensor5* d) {
   if (!t.defined() || !t.is_cuda() || t.device() != device || t.scalar_type() != at::kComplexFloat || t.is_conj()) return false;
@@ -108,15 +118,16 @@ Tensors zeros_like_all(const Tensors& v) {
   return r;
 }
 
-std::optional<Tensors> vec_forward(const Tensors& x, const Tensors& y, int maxl, bool diag) {
-  if (x.empty() || y.empty() || !x[0].defined() || !x[0].is_cuda()) return std::nullopt;
+std::optional<Tensors> vec_forward(const Tensors& x, const Tensors& y, pybind11::handle max_l, bool diag) {
+  const auto maxl = plain_int(max_l);
+  if (!maxl || x.empty() || y.empty() || !x[0].defined() || !x[0].is_cuda()) return std::nullopt;
   const auto device = x[0].device();
   Vec dx, dy, dr;
   std::vector<int64_t> lead;
   if (!describe_all(x, device, &dx) || !describe_all(y, device, &dy) || !lead_dims(x[0], y[0], &lead)) return std::nullopt;
   const int cap = dx.l.back() + dy.l.back() + 1;
   std::vector<int> l(cap), n(cap);
-  const int k = gelib_SO3type_CGproduct(dx.size(), dx.l.data(), dx.n.data(), dy.size(), dy.l.data(), dy.n.data(), maxl, diag, cap, l.data(), n.data());
+  const int k = gelib_SO3type_CGproduct(dx.size(), dx.l.data(), dx.n.data(), dy.size(), dy.l.data(), dy.n.data(), *maxl, diag, cap, l.data(), n.data());
   if (k <= 0) return std::nullopt;
   c10::cuda::CUDAGuard guard(device);
   Tensors r;
@@ -156,15 +167,16 @@ std::optional<Tensors> vec_backward(const Tensors& x, const Tensors& y, const Te
   return r;
 }
 
-std::optional<at::Tensor> part_forward(const at::Tensor& x, const at::Tensor& y, int l, bool diag) {
-  if (!x.defined() || !x.is_cuda() || l < 0) return std::nullopt;
+std::optional<at::Tensor> part_forward(const at::Tensor& x, const at::Tensor& y, pybind11::handle out_l, bool diag) {
+  const auto l = plain_int(out_l);
+  if (!l || !x.defined() || !x.is_cuda() || *l < 0) return std::nullopt;
   const auto device = x.device();
   gelib_tensor5 dx, dy, dr;
   std::vector<int64_t> lead;
   if (!describe(x, device, &dx) || !describe(y, device, &dy) || !lead_dims(x, y, &lead)) return std::nullopt;
   if (diag && x.size(-1) != y.size(-1)) return std::nullopt;
   c10::cuda::CUDAGuard guard(device);
-  at::Tensor r = output(lead, l, diag ? x.size(-1) : x.size(-1) * y.size(-1), device);
+  at::Tensor r = output(lead, *l, diag ? x.size(-1) : x.size(-1) * y.size(-1), device);
   if (!describe(r, device, &dr)) return std::nullopt;
   void* s = stream_of(device);
   const auto f = diag ? gelib_SO3part_addDiagCGproduct : gelib_SO3part_addCGproduct;
@@ -195,9 +207,11 @@ std::optional<Tensors> part_backward(const at::Tensor& x, const at::Tensor& y, c
 }
 
 // x gathered along array dimension d (tensor dimension d + 1) by a map of n_in cells into n_out.
-std::optional<at::Tensor> gather(const at::Tensor& x0, const at::Tensor& row_ptr, const at::Tensor& col, int n_in, int n_out, int d) {
-  if (!x0.defined() || !x0.is_cuda() || x0.scalar_type() != at::kComplexFloat || x0.is_conj()) return std::nullopt;
+std::optional<at::Tensor> gather(const at::Tensor& x0, const at::Tensor& row_ptr, const at::Tensor& col, int n_in, int n_out, pybind11::handle dim) {
+  const auto array_dim = plain_int(dim);
+  if (!array_dim || !x0.defined() || !x0.is_cuda() || x0.scalar_type() != at::kComplexFloat || x0.is_conj()) return std::nullopt;
   const auto device = x0.device();
+  const int d = *array_dim;
   if (d < 0 || d + 1 >= x0.dim() || x0.size(d + 1) != n_in || row_ptr.device() != device || col.device() != device) return std::nullopt;
   c10::cuda::CUDAGuard guard(device);
   const at::Tensor x = x0.detach().contiguous();

@@ -101,6 +101,10 @@ inline int col_block_warps(unsigned warps, int splits, int most) {
 // False when the view's cells are no arithmetic progression or a stride does not fit.
 bool col_fill_part(const PartView& p, const CellGrid& cg, long long extra_floats, bool rows, ColPart* out);
 
+// One-channel x: whether the kernels of cg_narrow.cu / cg_narrow1_bwd.cu are faster than the column kernels, which take cpl
+// columns per lane; max_la: largest min(l1, l2).
+bool narrow_wins(bool backward, int cpl, int n, int max_la, long long cells);
+
 // Returns false when the call is not one the column kernels take; otherwise fills args and
 // plan (plan->dev == nullptr on a CUDA error).
 bool col_setup(const VecCall& c, bool backward, ColArgs* a, ColPlan* plan);

@@ -424,9 +424,20 @@ int choose_walk(const std::vector<int>& tables, long long warps, int b_rows, boo
   return best;
 }
 
-// One-channel x: whether the kernels of cg_narrow.cu / cg_narrow1_bwd.cu are faster.  Their lanes are padded to a power of
-// two of channels (cw) and they want a full chip; one column per lane does without what two columns share.  us, column
-// kernel / narrow kernel, maxl x channels, cells:
+}  // namespace
+
+bool col_fill_part(const PartView& p, const CellGrid& cg, long long extra_floats, bool rows, ColPart* out) {
+  const long long cs = cell_stride(p, cg);
+  const long long unit = rows ? p.sm : 2;
+  if (cs < 0 || 4 * cs > 0xffffffffLL || unit < 0 || 4 * unit > 0xffffffffLL) return false;
+  out->base = p.base + extra_floats;
+  out->unit = (unsigned)(4 * unit);
+  out->cell_stride = (unsigned)(4 * cs);
+  return true;
+}
+
+// The narrow kernels' lanes are padded to a power of two of channels (cw) and they want a full chip; one column per lane does
+// without what two columns share.  us, column kernel / narrow kernel, maxl x channels, cells:
 //   forward, l <= 1: 1 x 12 2400 9.2 / 7.9, 24000 27 / 22; 300 cells 6.6 / 7.1.  l <= 3: 2 x 16 2400 21 / 19, 24000 90 / 63.
 //     From l = 4 on padding decides: 4 x 24 12000 331 / 394, 4 x 5 19200 416 / 522, 4 x 21 2400 95 / 119, 12000 495 / 473,
 //     6 x 21 909 / 1167 at 4800; without it 4 x 32 330 / 191 at 4800.
@@ -442,18 +453,6 @@ bool narrow_wins(bool backward, int cpl, int n, int max_la, long long cells) {
   if (!backward) return warps >= 148 * (max_la <= 1 ? 4 : 16) && !(max_la >= 4 && padded);
   if (!narrow1_enabled() || warps < 148 * 16) return false;
   return cpl == 1 ? max_la <= 1 || !padded : n == cw && (max_la <= 1 || max_la >= 6 || n == 32);
-}
-
-}  // namespace
-
-bool col_fill_part(const PartView& p, const CellGrid& cg, long long extra_floats, bool rows, ColPart* out) {
-  const long long cs = cell_stride(p, cg);
-  const long long unit = rows ? p.sm : 2;
-  if (cs < 0 || 4 * cs > 0xffffffffLL || unit < 0 || 4 * unit > 0xffffffffLL) return false;
-  out->base = p.base + extra_floats;
-  out->unit = (unsigned)(4 * unit);
-  out->cell_stride = (unsigned)(4 * cs);
-  return true;
 }
 
 bool col_setup(const VecCall& c, bool backward, ColArgs* a, ColPlan* plan) {

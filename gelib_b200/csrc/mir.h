@@ -48,7 +48,7 @@ struct MirBwdArgs {
 // Flags of a backward item: only row m has the first entry, only row m + 1 the last; a row m alone; first and last of an l2;
 // last of a pair.
 enum { kMirPrologue = 1, kMirEpilogue = 2, kMirSingle = 4, kMirFirstOfB = 8, kMirLastOfB = 16, kMirLastOfPair = 32 };
-constexpr int kMirTwoLevels = 5;  // most output l of an item for which the sums of a pair are kept apart
+constexpr int kMirTwoLevels = 6;  // most output l of an item for which the sums of a pair are kept apart
 
 #ifdef __CUDACC__
 namespace mir {

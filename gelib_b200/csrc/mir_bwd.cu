@@ -141,7 +141,8 @@ __device__ __forceinline__ void prefetch_rows(const unsigned char* it, const uns
   }
 
 // Two levels: a pair's sums are kept apart and added to those of the pairs before it when the pair ends, as the column kernel sums;
-// with up to five l there is room for them (maxl 4 x 16: error against 64-bit sums 1.18e-7 in one level).
+// with up to six l there is room for them.  Error against 64-bit sums, in one level / in two / of the column kernel: maxl 4 x 16
+// 1.18e-7 / 0.78e-7 / 0.84e-7, maxl 5 x 16 1.03e-7 / 0.82e-7 / 0.91e-7 (a million columns 2.54 / 2.73 ms).
 // NLMAX: most output l of an item.  WARPS: warps that should share an SM; more of them cover the latency of the loads better,
 // and registers beyond these numbers bought nothing.
 template <int NLMAX, int WARPS>
@@ -396,6 +397,9 @@ int launch_mir_bwd(const VecCall& c, cudaStream_t s, bool* plan_others) {
   a.ring_bytes = plan->tables[0];
   a.y_rows = plan->tables[1];
   const int nl = plan->tables[2];
+  int max_la = 0;
+  for (const auto& p : c.x)
+    for (const auto& q : c.y) max_la = std::max(max_la, std::min(p.l, q.l));
   const size_t smem = 256 * (size_t)a.nr + a.ring_bytes + mir::kPitch * (size_t)a.y_rows * (nl <= kMirTwoLevels ? 2 : 1) + 8 * (size_t)a.xcells * xrows;
   if (smem > kColMaxSmem) return -1;
   // Where this kernel is faster: enough columns for several warps per scheduler, and enough work per row of g.  us, the others
@@ -404,6 +408,9 @@ int launch_mir_bwd(const VecCall& c, cudaStream_t s, bool* plan_others) {
   // 8 x 16, 100000 2083 / 1756; but maxl 2 x 16, 100000 33 / 44, maxl 6 x 4 (eight cells to a warp), 400000 3780 / 4496, maxl 4 x 16,
   // 400000 (two columns per lane there, none padded) 585 / 598, and more than 32 channels, l <= 2 with l <= 7 x 40, 160000 338 / 405.
   if (mode == kColAuto) {
+    // One level of sums only in the place of cg_narrow1_bwd_kernel, which has one too (maxl 6 x 16: error 2.1e-7 there, 1.14e-7 here);
+    // the column kernel, which sums in two, stays more accurate from seven l on (maxl 6 x 20 0.97e-7, maxl 8 x 20 1.09e-7 / 1.42e-7).
+    if (nl > kMirTwoLevels && !narrow_wins(true, n % 2 ? 1 : 2, n, max_la, 1LL << 40)) return -1;
     if (n > 32 || nl < 4 || (nl > 5 && n < 8) || (nl <= 5 && (n == 8 || n == 16))) return -1;
     const bool first = plan->first_use.exchange(false);
     if (a.ncols < (nl == 6 || nl == 7 ? 128000u : 96000u)) return -1;
@@ -413,8 +420,8 @@ int launch_mir_bwd(const VecCall& c, cudaStream_t s, bool* plan_others) {
   a.items = plan->items;
   a.dir = reinterpret_cast<const int2*>(plan->jobs);
   cudaError_t e;
-  if (nl <= 3) e = mir::launch_bwd<3, 32>(a, smem, s);
-  else if (nl <= 5) e = mir::launch_bwd<5, 28>(a, smem, s);
+  if (nl <= 5) e = mir::launch_bwd<5, 28>(a, smem, s);
+  else if (nl <= 6) e = mir::launch_bwd<6, 20>(a, smem, s);
   else if (nl <= 7) e = mir::launch_bwd<7, 20>(a, smem, s);
   else e = mir::launch_bwd<kMirMaxNl, 16>(a, smem, s);
   if (e != cudaSuccess) return check_cuda(e, fn, "row-pair backward kernel launch");

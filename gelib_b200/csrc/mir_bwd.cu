@@ -349,6 +349,35 @@ void build_bwd(DevicePlan& p, const std::vector<PartSig>& xs, const std::vector<
   p.tables = {16 * ring, most_b, most_nl};
 }
 
+// The number of columns from which the row-pair kernel takes a signature: nl output l in an item at most, max_la the largest
+// min(l1, l2).  0: never.  Measured with 1 million columns, the other kernel / this one, ms:
+//   up to five l, where the column kernel has two columns to a lane (even counts) it is the faster one: maxl 3 x 12 .61 / .70, x 20 .62
+//     / .68, maxl 4 x 12 1.31 / 1.74, x 20 1.33 / 1.58, x 28 1.34 / 1.51; but with one (odd counts) maxl 3 x 9 1.10 / .77, x 17 1.11 / .70, x
+//     15 .79 / .71, x 31 .68 / .67, maxl 4 x 17 2.13 / 1.78, x 23 2.13 / 1.65.  Below, and where cg_narrow1_bwd_kernel pads little, not: maxl 3 x
+//     5 1.10 / 1.28, maxl 4 x 9 2.10 / 2.24, x 15 1.62 / 1.84, x 31 1.42 / 1.56.  In the place of cg_narrow1_bwd_kernel at 32 channels the sums
+//     are more accurate (maxl 4: error 1.36e-7 / 0.77e-7): maxl 3 .65 / .62, maxl 4 1.36 / 1.31.
+//   six l: maxl 5 x 16 3.02 / 2.73, x 32 2.66 / 2.69, x 17 3.80 / 3.66, x 23 3.79 / 3.42; but x 9 3.76 / 4.54, x 12 3.11 / 3.62, x 20 3.08 / 3.28, x
+//     28 3.09 / 3.14, x 31 2.86 / 3.25.
+//   seven and eight, in the place of cg_narrow1_bwd_kernel only (mir_bwd_kernel): maxl 6 x 16 5.05 / 4.33, x 32 4.87 / 4.28, x 25 6.32 / 5.84, x
+//     31 5.24 / 4.96, x 8 5.66 / 5.95, but maxl 7 x 8, 330000 columns 4.78 / 3.83; maxl 6 x 15, with parts of four cells in a warp, 5.75 / 6.66;
+//     maxl 6 x 4 8.90 / 10.8.
+// The lines in columns: both kernels step by what fills the chip, which decides up to some 400000 columns (maxl 4 x 32: 150000 .21 / .31,
+// 200000 .39 / .34, 300000 .40 / .46, 420000 .59 / .60; maxl 5 x 16: 300000 .87 / .95, 420000 1.30 / 1.23); where the gain is larger it
+// starts earlier (maxl 3 x 9: 150000 .19 / .20, 200000 .24 / .21; maxl 4 x 17: 200000 .45 / .44; maxl 6 x 16: 112000 .66 / .73, 130000 .80 / .75;
+// maxl 7 x 16: 98000 1.17 / 1.10).
+unsigned row_pairs_from(int n, int nl, int max_la) {
+  const bool odd = n % 2 != 0, narrow = narrow_wins(true, odd ? 1 : 2, n, max_la, 1LL << 40);
+  if (n > 32 || nl < 4) return 0;
+  if (nl <= 5) {
+    if (max_la >= 6) return 0;  // a truncated product: little work per row of g (l up to 6, output up to 4, x 32: 130000 columns .43 / .54)
+    if (odd) return n >= 9 && (nl == 4 || (n > 16 && !narrow)) ? 200000 : 0;
+    return narrow ? 400000 : 0;
+  }
+  if (nl == 6) return (32 % n == 0 && n >= 16) || (odd && n > 16 && !narrow) ? 400000 : 0;
+  if (!narrow || n < 8 || (n < 16 && 32 % n != 0)) return 0;
+  return nl == 7 ? 128000 : 96000;
+}
+
 }  // namespace
 
 // Returns -1 when the call does not qualify.
@@ -402,18 +431,11 @@ int launch_mir_bwd(const VecCall& c, cudaStream_t s, bool* plan_others) {
     for (const auto& q : c.y) max_la = std::max(max_la, std::min(p.l, q.l));
   const size_t smem = 256 * (size_t)a.nr + a.ring_bytes + mir::kPitch * (size_t)a.y_rows * (nl <= kMirTwoLevels ? 2 : 1) + 8 * (size_t)a.xcells * xrows;
   if (smem > kColMaxSmem) return -1;
-  // Where this kernel is faster: enough columns for several warps per scheduler, and enough work per row of g.  us, the others
-  // (cg_narrow1_bwd_kernel, column kernel) / this one: maxl 6 x 16, 60000 columns 386 / 414, 100000 703 / 729, 400000 2162 / 1890;
-  // maxl 3 x 9, 60000 87 / 86, 100000 130 / 113, 400000 461 / 349; maxl 4 x 21, 400000 907 / 748; maxl 4 x 32, 320000 586 / 480; maxl
-  // 8 x 16, 100000 2083 / 1756; but maxl 2 x 16, 100000 33 / 44, maxl 6 x 4 (eight cells to a warp), 400000 3780 / 4496, maxl 4 x 16,
-  // 400000 (two columns per lane there, none padded) 585 / 598, and more than 32 channels, l <= 2 with l <= 7 x 40, 160000 338 / 405.
   if (mode == kColAuto) {
-    // One level of sums only in the place of cg_narrow1_bwd_kernel, which has one too (maxl 6 x 16: error 2.1e-7 there, 1.14e-7 here);
-    // the column kernel, which sums in two, stays more accurate from seven l on (maxl 6 x 20 0.97e-7, maxl 8 x 20 1.09e-7 / 1.42e-7).
-    if (nl > kMirTwoLevels && !narrow_wins(true, n % 2 ? 1 : 2, n, max_la, 1LL << 40)) return -1;
-    if (n > 32 || nl < 4 || (nl > 5 && n < 8) || (nl <= 5 && (n == 8 || n == 16))) return -1;
-    const bool first = plan->first_use.exchange(false);
-    if (a.ncols < (nl == 6 || nl == 7 ? 128000u : 96000u)) return -1;
+    const unsigned least = row_pairs_from(n, nl, max_la);
+    if (least == 0) return -1;
+    const bool first = plan->first_use.exchange(false);  // another batch of the signature goes to the others
+    if (a.ncols < least) return -1;
     *plan_others = first;
   }
   if (c.plan_only) return GELIB_OK;

@@ -70,3 +70,17 @@ def test_sums_are_no_less_accurate_than_without_the_row_pair_kernel(G, maxl, n, 
     call = Call(G, maxl, n, cols)
     want = call.in_64_bits(200)
     assert relative_error(call.gradient("auto"), want) < 1.03 * relative_error(call.gradient("0"), want)
+
+
+# every row is summed in one order, so that two runs of one kernel agree bit for bit
+@pytest.mark.parametrize("maxl,n,cols,taken", [
+    (3, 12, 100000, False), (3, 20, 400000, False), (3, 1, 100000, False), (3, 6, 400000, False), (3, 32, 130000, False),
+    (4, 5, 100000, False), (4, 12, 400000, False), (4, 15, 200000, False), (4, 20, 200000, False), (4, 32, 130000, False),
+    (5, 8, 200000, False), (5, 12, 200000, False), (5, 20, 200000, False), (6, 9, 200000, False), (6, 15, 200000, False), (6, 20, 130000, False),
+    (8, 15, 98000, False), (3, 9, 200000, True), (3, 17, 210000, True), (4, 23, 210000, True), (4, 32, 400000, True), (5, 16, 420000, True),
+    (6, 16, 130000, True), (6, 31, 130000, True), (7, 8, 98000, True), (8, 32, 98000, True)])
+def test_calls_that_the_row_pair_kernel_takes(G, maxl, n, cols, taken):
+    call = Call(G, maxl, n, cols)
+    auto, pinned, others = (call.gradient(mir) for mir in ("auto", "one", "0"))
+    assert all(torch.equal(a, b) for a, b in zip(auto, pinned if taken else others))
+    assert not all(torch.equal(a, b) for a, b in zip(pinned, others))

@@ -264,14 +264,14 @@ cudaError_t launch_bwd(const MirBwdArgs& a, size_t smem, cudaStream_t s) {
 namespace {
 
 // The items, in order.  Their directory is kept in h_jobs: {first int4, int4 units | place in the ring << 8}; any four neighbours
-// of the walk lie apart in the ring.  Words of tables: {bytes of the ring, most y rows, most output l of an item}.
+// of the walk lie apart in the ring.  Words of tables: {bytes of the ring, most y rows}.
 void build_bwd(DevicePlan& p, const std::vector<PartSig>& xs, const std::vector<PartSig>& ys, const std::vector<PartSig>& rs, bool diag) {
   build_schedule(xs, ys, rs, diag, false, &p.sched);
   std::map<std::pair<int, int>, std::vector<const Triple*>> pairs;  // by (yi, xi)
   for (const Triple& t : p.sched.triples) pairs[{t.yi, t.xi}].push_back(&t);
   std::vector<int> xrow(1, 0);
   for (const auto& q : xs) xrow.push_back(xrow.back() + 2 * q.l + 1);
-  int most_b = 0, most_nl = 0, last_yi = -1, last_header = -1;
+  int most_b = 0, last_yi = -1, last_header = -1;
   std::vector<int> sizes;
   for (auto& kv : pairs) {
     const int yi = kv.first.first, xi = kv.first.second, la = xs[xi].l, lb = ys[yi].l;
@@ -323,7 +323,6 @@ void build_bwd(DevicePlan& p, const std::vector<PartSig>& xs, const std::vector<
         p.h_jobs.push_back(last_header);
         p.h_jobs.push_back(size);
         sizes.push_back(size);
-        most_nl = std::max(most_nl, nl);
         most_b = std::max(most_b, 2 * lb + 1);
       }
     }
@@ -346,7 +345,7 @@ void build_bwd(DevicePlan& p, const std::vector<PartSig>& xs, const std::vector<
     if (fits) break;
   }
   for (size_t i = 0; i < sizes.size(); i++) p.h_jobs[2 * i + 1] |= place[i] << 8;
-  p.tables = {16 * ring, most_b, most_nl};
+  p.tables = {16 * ring, most_b};
 }
 
 // The number of columns from which the row-pair kernel takes a signature: nl output l in an item at most, max_la the largest
@@ -413,6 +412,17 @@ int launch_mir_bwd(const VecCall& c, cudaStream_t s, bool* plan_others) {
   a.n = (unsigned)n;
   a.ncols = (unsigned)(c.cg.ncells * n);
   a.xcells = 32 % n == 0 ? 32 / n : (30 + n) / n + 1;
+  int nl = 0, max_la = 0;  // most output l of an item, largest min(l1, l2)
+  for (const auto& p : c.x)
+    for (const auto& q : c.y) {
+      int ls = 0;
+      for (const auto& r : c.r) ls += r.l >= std::abs(p.l - q.l) && r.l <= p.l + q.l;
+      const int groups = (ls + kMirMaxNl - 1) / kMirMaxNl;
+      if (groups > 0) nl = std::max(nl, (ls + groups - 1) / groups);
+      max_la = std::max(max_la, std::min(p.l, q.l));
+    }
+  const unsigned least = mode == kColAuto ? row_pairs_from(n, nl, max_la) : 0;
+  if (mode == kColAuto && least == 0) return -1;
   std::vector<int> key = {22 /*family*/, c.diag, a.nx, (int)c.y.size(), a.nr, n};
   for (const auto& p : c.x) key.push_back(p.l);
   for (const auto& p : c.y) key.push_back(p.l);
@@ -425,15 +435,9 @@ int launch_mir_bwd(const VecCall& c, cudaStream_t s, bool* plan_others) {
   if (a.nitems == 0) return GELIB_OK;
   a.ring_bytes = plan->tables[0];
   a.y_rows = plan->tables[1];
-  const int nl = plan->tables[2];
-  int max_la = 0;
-  for (const auto& p : c.x)
-    for (const auto& q : c.y) max_la = std::max(max_la, std::min(p.l, q.l));
   const size_t smem = 256 * (size_t)a.nr + a.ring_bytes + mir::kPitch * (size_t)a.y_rows * (nl <= kMirTwoLevels ? 2 : 1) + 8 * (size_t)a.xcells * xrows;
   if (smem > kColMaxSmem) return -1;
   if (mode == kColAuto) {
-    const unsigned least = row_pairs_from(n, nl, max_la);
-    if (least == 0) return -1;
     const bool first = plan->first_use.exchange(false);  // another batch of the signature goes to the others
     if (a.ncols < least) return -1;
     *plan_others = first;

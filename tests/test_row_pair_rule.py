@@ -84,3 +84,18 @@ def test_calls_that_the_row_pair_kernel_takes(G, maxl, n, cols, taken):
     auto, pinned, others = (call.gradient(mir) for mir in ("auto", "one", "0"))
     assert all(torch.equal(a, b) for a, b in zip(auto, pinned if taken else others))
     assert not all(torch.equal(a, b) for a, b in zip(pinned, others))
+
+
+def test_a_signature_that_it_never_takes_gets_no_plan(G):
+    # device memory for a plan cannot be had during capture
+    call = Call(G, 3, 40, 100000)
+    want = call.gradient("0")
+    V = G.backend.SO3vec.view
+    yg = [torch.zeros_like(t) for t in call.y]
+    torch.cuda.synchronize()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        V(yg).addCGproduct_back1(V(call.g), V(call.x))
+    graph.replay()
+    torch.cuda.synchronize()
+    assert all(torch.equal(a, b) for a, b in zip(yg, want))

@@ -7,6 +7,7 @@ product on CPU tensors raises.
 """
 import contextlib
 import ctypes
+import importlib
 import os
 import struct
 import sys
@@ -109,11 +110,16 @@ def native():
     global _native
     if _native is None:
         lib()
+        why = None
         try:
-            from . import _native as module
+            module = importlib.import_module(__package__ + "._native")
+            if module.torch_version != torch.__version__:
+                why = "built for torch %s, this is %s" % (module.torch_version, torch.__version__)
         except ImportError as e:
+            why = e
+        if why is not None:
             raise RuntimeError("gelib_b200: %s cannot be loaded (%s). Build it with `python -m gelib_b200.build`."
-                               % (os.path.join(_HERE, "_native.so"), e))
+                               % (os.path.join(_HERE, "_native.so"), why))
         _native = module
     return _native
 

@@ -6,6 +6,7 @@ The library is a plain shared object (no Python or torch dependency); it is what
 links instead of its own ``cuda/`` objects, and what ``gelib_b200._lib`` loads through ctypes.
 ``_native.so``, built beside it, is the Python package's own: it links the library and torch.
 """
+import hashlib
 import os
 import subprocess
 import sys
@@ -28,6 +29,11 @@ PER_FILE = {"spharm.cu": ["-fmad=false"]}
 
 def _newest(paths):
     return max(os.path.getmtime(p) for p in paths)
+
+
+def _digest(path):
+    with open(path, "rb") as f:
+        return hashlib.sha256(f.read()).hexdigest()
 
 
 def build_library(force=False, verbose=False):
@@ -64,19 +70,26 @@ def build_library(force=False, verbose=False):
 
 def build_native(force=False, verbose=False):
     src, header = os.path.join(CSRC, "host.cpp"), os.path.join(HERE, "..", "include", "gelib_b200.h")
-    if not force and os.path.exists(NATIVE) and os.path.getmtime(NATIVE) >= _newest([src, header, LIB, os.path.abspath(__file__)]):
-        return NATIVE
     import torch
     root = os.path.dirname(os.path.abspath(torch.__file__))
     include = [os.path.join(root, "include"), os.path.join(root, "include", "torch", "csrc", "api", "include"),
                os.path.join(os.path.dirname(os.path.dirname(NVCC)), "include"), sysconfig.get_paths()["include"]]
     cmd = [os.environ.get("CXX", "g++"), "-O2", "-std=c++17", "-fPIC", "-shared", "-fvisibility=hidden"]
-    cmd += ["-D_GLIBCXX_USE_CXX11_ABI=%d" % torch._C._GLIBCXX_USE_CXX11_ABI] + ["-I" + i for i in include] + [src, "-o", NATIVE]
+    cmd += ["-DGELIB_TORCH_VERSION=\"%s\"" % torch.__version__, "-D_GLIBCXX_USE_CXX11_ABI=%d" % torch._C._GLIBCXX_USE_CXX11_ABI]
+    cmd += ["-I" + i for i in include] + [src, "-o", NATIVE]
     cmd += ["-L" + os.path.join(root, "lib"), "-lc10", "-lc10_cuda", "-ltorch_cpu", "-ltorch", "-ltorch_python"]
     cmd += ["-L" + HERE, "-l:" + os.path.basename(LIB), "-Wl,-rpath,$ORIGIN"]
+    # The file is tied to this torch and this Python; what it was made with, and its own digest, are kept beside the objects.
+    stamp, made_with = os.path.join(OBJ, "native.stamp"), "\n".join([sys.version] + cmd)
+    if not force and os.path.exists(NATIVE) and os.path.getmtime(NATIVE) >= _newest([src, header, LIB, os.path.abspath(__file__)]):
+        if os.path.exists(stamp) and open(stamp).read() == made_with + "\n" + _digest(NATIVE):
+            return NATIVE
     r = subprocess.run(cmd, capture_output=True, text=True)
     if r.returncode != 0:
         raise RuntimeError("g++ failed for host.cpp:\n%s\n%s" % (r.stdout, r.stderr))
+    os.makedirs(OBJ, exist_ok=True)
+    with open(stamp, "w") as f:
+        f.write(made_with + "\n" + _digest(NATIVE))
     return NATIVE
 
 

@@ -232,6 +232,7 @@ std::optional<at::Tensor> gather(const at::Tensor& x0, const at::Tensor& row_ptr
 }  // namespace
 
 PYBIND11_MODULE(_native, m) {
+  m.attr("torch_version") = GELIB_TORCH_VERSION;
   m.def("vec_forward", torch::wrap_pybind_function(&vec_forward));
   m.def("vec_backward", torch::wrap_pybind_function(&vec_backward));
   m.def("part_forward", torch::wrap_pybind_function(&part_forward));

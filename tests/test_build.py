@@ -1,0 +1,50 @@
+"""What `python -m gelib_b200.build` does about the native host side, whose file is tied to a torch and a Python.  Nothing is
+compiled here: the compiler is a stand-in that writes a file."""
+import os
+import sys
+import types
+
+import pytest
+import torch
+
+
+@pytest.fixture
+def builder(tmp_path, monkeypatch):
+    from gelib_b200 import build as b
+    calls = []
+
+    def run(cmd, **kw):
+        calls.append(cmd)
+        with open(b.NATIVE, "w") as f:
+            f.write("made by call %d" % len(calls))
+        return types.SimpleNamespace(returncode=0, stdout="", stderr="")
+
+    lib = tmp_path / "lib.so"
+    lib.write_text("")
+    os.utime(lib, (1, 1))
+    monkeypatch.setattr(b, "LIB", str(lib))
+    monkeypatch.setattr(b, "NATIVE", str(tmp_path / "_native.so"))
+    monkeypatch.setattr(b, "OBJ", str(tmp_path))
+    monkeypatch.setattr(b, "build_library", lambda *a: str(lib))
+    monkeypatch.setattr(b.subprocess, "run", run)
+    return types.SimpleNamespace(b=b, calls=calls, build=b.build)
+
+
+def test_an_up_to_date_file_is_kept(builder):
+    builder.build()
+    builder.build()
+    assert len(builder.calls) == 1
+
+
+@pytest.mark.parametrize("change", ["torch", "python", "file"])
+def test_a_file_for_another_torch_or_python_or_a_broken_one_is_built_again(builder, monkeypatch, change):
+    builder.build()
+    if change == "torch":
+        monkeypatch.setattr(torch, "__version__", "0.0")
+    if change == "python":
+        monkeypatch.setattr(sys, "version", "0.0")
+    if change == "file":
+        with open(builder.b.NATIVE, "w") as f:
+            f.write("broken")
+    builder.build()
+    assert len(builder.calls) == 2

@@ -8,6 +8,7 @@ links instead of its own ``cuda/`` objects, and what ``gelib_b200._lib`` loads t
 """
 import hashlib
 import os
+import shutil
 import subprocess
 import sys
 import sysconfig
@@ -68,12 +69,20 @@ def build_library(force=False, verbose=False):
     return LIB
 
 
+def _cuda_include():
+    """Beside the compiler, wherever NVCC names it: by path, by name, or through a link."""
+    found = shutil.which(NVCC) or NVCC
+    roots = [os.path.dirname(os.path.dirname(p)) for p in (found, os.path.realpath(found))]
+    places = [os.path.join(r, "include") for r in roots]
+    return next((p for p in places if os.path.exists(os.path.join(p, "cuda_runtime_api.h"))), places[0])
+
+
 def build_native(force=False, verbose=False):
     src, header = os.path.join(CSRC, "host.cpp"), os.path.join(HERE, "..", "include", "gelib_b200.h")
     import torch
     root = os.path.dirname(os.path.abspath(torch.__file__))
     include = [os.path.join(root, "include"), os.path.join(root, "include", "torch", "csrc", "api", "include"),
-               os.path.join(os.path.dirname(os.path.dirname(NVCC)), "include"), sysconfig.get_paths()["include"]]
+               _cuda_include(), sysconfig.get_paths()["include"]]
     cmd = [os.environ.get("CXX", "g++"), "-O2", "-std=c++17", "-fPIC", "-shared", "-fvisibility=hidden"]
     cmd += ["-DGELIB_TORCH_VERSION=\"%s\"" % torch.__version__, "-D_GLIBCXX_USE_CXX11_ABI=%d" % torch._C._GLIBCXX_USE_CXX11_ABI]
     cmd += ["-I" + i for i in include] + [src, "-o", NATIVE]

@@ -48,3 +48,13 @@ def test_a_file_for_another_torch_or_python_or_a_broken_one_is_built_again(build
             f.write("broken")
     builder.build()
     assert len(builder.calls) == 2
+
+
+def test_the_toolkits_headers_are_found_from_the_compilers_name_alone(builder, monkeypatch):
+    if not os.path.exists(builder.b.NVCC):
+        pytest.skip("no CUDA compiler here")
+    monkeypatch.setenv("PATH", os.path.dirname(builder.b.NVCC) + os.pathsep + os.environ["PATH"])
+    monkeypatch.setattr(builder.b, "NVCC", "nvcc")
+    builder.build()
+    include = [a[2:] for a in builder.calls[0] if a.startswith("-I")]
+    assert any(os.path.exists(os.path.join(d, "cuda_runtime_api.h")) for d in include), include

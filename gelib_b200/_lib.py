@@ -11,6 +11,7 @@ import importlib
 import os
 import struct
 import sys
+import warnings
 
 import torch
 
@@ -105,8 +106,16 @@ def lib():
 _native = None
 
 
+class _Declines:
+    """Stands in for the native host side: every function leaves the call to the Python code."""
+
+    def __getattr__(self, name):
+        return lambda *args: None
+
+
 def native():
-    """The native host side of the products (csrc/host.cpp).  Raises when it has not been built, like lib()."""
+    """The native host side of the products (csrc/host.cpp).  It only saves host time, so where it cannot be had -- no Python
+    headers to build it with, or made for another torch -- the Python code does its part, after a warning."""
     global _native
     if _native is None:
         lib()
@@ -118,8 +127,9 @@ def native():
         except ImportError as e:
             why = e
         if why is not None:
-            raise RuntimeError("gelib_b200: %s cannot be loaded (%s). Build it with `python -m gelib_b200.build`."
-                               % (os.path.join(_HERE, "_native.so"), why))
+            warnings.warn("gelib_b200: %s cannot be used (%s); products take more host time.  `python -m gelib_b200.build` builds it."
+                          % (os.path.join(_HERE, "_native.so"), why), RuntimeWarning, stacklevel=2)
+            module = _Declines()
         _native = module
     return _native
 

@@ -4,7 +4,8 @@
 
 The library is a plain shared object (no Python or torch dependency); it is what a GElib build
 links instead of its own ``cuda/`` objects, and what ``gelib_b200._lib`` loads through ctypes.
-``_native.so``, built beside it, is the Python package's own: it links the library and torch.
+``_native.so``, built beside it, is the Python package's own: it links the library and torch, and the
+package runs without it.
 """
 import hashlib
 import os
@@ -77,6 +78,21 @@ def _cuda_include():
     return next((p for p in places if os.path.exists(os.path.join(p, "cuda_runtime_api.h"))), places[0])
 
 
+def _native_lacks():
+    """What this machine lacks to build the native host side; None when it can."""
+    try:
+        import torch
+    except ImportError:
+        return "torch"
+    if torch.version.cuda is None:
+        return "a torch with CUDA"
+    include = os.path.join(os.path.dirname(os.path.abspath(torch.__file__)), "include")
+    for header, place in (("ATen/ATen.h", include), ("cuda_runtime_api.h", _cuda_include()), ("Python.h", sysconfig.get_paths()["include"])):
+        if not os.path.exists(os.path.join(place, header)):
+            return "%s in %s" % (header, place)
+    return None
+
+
 def build_native(force=False, verbose=False):
     src, header = os.path.join(CSRC, "host.cpp"), os.path.join(HERE, "..", "include", "gelib_b200.h")
     import torch
@@ -103,8 +119,14 @@ def build_native(force=False, verbose=False):
 
 
 def build(force=False, verbose=False):
+    """The library, which needs neither torch nor Python's headers, and the native host side where they are there."""
     path = build_library(force, verbose)
-    build_native(force, verbose)
+    lacks = _native_lacks()
+    if lacks is None:
+        build_native(force, verbose)
+    else:
+        sys.stderr.write("gelib_b200: %s is not built, for want of %s; products run without it, with more host time per call.\n"
+                         % (os.path.basename(NATIVE), lacks))
     return path
 
 

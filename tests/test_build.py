@@ -58,3 +58,21 @@ def test_the_toolkits_headers_are_found_from_the_compilers_name_alone(builder, m
     builder.build()
     include = [a[2:] for a in builder.calls[0] if a.startswith("-I")]
     assert any(os.path.exists(os.path.join(d, "cuda_runtime_api.h")) for d in include), include
+
+
+def test_the_library_is_built_where_pythons_headers_are_missing(builder, monkeypatch, capsys):
+    monkeypatch.setattr(builder.b.sysconfig, "get_paths", lambda: {"include": "/nonexistent"})
+    assert builder.build() == builder.b.LIB
+    assert builder.calls == [] and "Python.h" in capsys.readouterr().err
+
+
+@pytest.mark.parametrize("how", ["missing", "another torch"])
+def test_products_do_without_the_native_host_side(cabi, monkeypatch, how):
+    import gelib_b200 as G
+    module = None if how == "missing" else types.SimpleNamespace(torch_version="0.0")
+    monkeypatch.setitem(sys.modules, "gelib_b200._native", module)
+    monkeypatch.setattr(G._lib, "_native", None)
+    x = G.SO3vec.randn(2, {0: 2, 1: 2})
+    with pytest.warns(RuntimeWarning, match="_native.so"):
+        with pytest.raises(RuntimeError, match="CUDA"):  # what the Python code says about CPU tensors
+            x.CGproduct(x)

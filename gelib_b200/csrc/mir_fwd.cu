@@ -368,11 +368,15 @@ int launch_mir_fwd(const VecCall& c, cudaStream_t s, bool* plan_others) {
   // many of them (us, those / this one; 7 items at maxl 1, 23 at maxl 2): maxl 1 x 64, batch 468 14.5 / 10.2, 1562 16.4 / 18.5,
   // 4687 28 / 41; maxl 2 x 8, batch 12500 33 / 30; one-channel x, maxl 1 x 16, 1875 cells 13 / 10, 6250 13 / 19; maxl 2 x 16, 1875
   // 26 / 15, 25000 74 / 91, but, where the narrow kernel pads its lanes, maxl 2 x 7, 57142 140 / 109; maxl 3 x 32, 12500 174 / 164.
+  // The narrow kernel, for up to 32 channels of a one-channel x, is ahead earlier when there are least items or y has only
+  // l = 0, us at 36000 / 44000 / 62000 columns: maxl 1 x 16 7.7 / 7.6 / 7.8 against 6.2 / 7.6 / 9.8, l = 0 with l <= 2 x 16 6.3 / 6.8 / 7.0 against 5.6 /
+  // 7.2 / 9.3, l <= 4 with l = 0 x 16 9.7 / 10.5 / 10.5 against 8.2 / 10.8 / 13.2; but l = 0 with l <= 4 x 16 11.5 / 12.9 / 12.7 against 8.1 / 9.9 / 12.3.
   const bool pow2 = (n & (n - 1)) == 0;
   const bool few_items = a.nitems <= (one_channel && pow2 ? 24 : 8);
+  const bool narrow = one_channel && n <= 32 && (a.nitems <= 8 || a.yrows == 1);
   if (mode == kColAuto && few_items) {
     const bool first = plan->first_use.exchange(false);
-    if (columns > 64000) return -1;
+    if (columns > (narrow ? 40000 : 64000)) return -1;
     *plan_others = first;  // another batch of the signature goes there
   }
   if (c.plan_only) return GELIB_OK;

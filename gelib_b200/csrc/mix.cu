@@ -27,7 +27,6 @@ namespace {
 
 constexpr int kMixMaxN = 64;   // channels on either side
 constexpr int kThreads = 256;
-constexpr int kRowsPerThread = 4;
 
 // How rows of n complex numbers are copied: 16 bytes at a time where they are aligned, `per` copies a row.
 struct RowCopy {
@@ -51,16 +50,21 @@ __device__ __forceinline__ void mac(float2& s, float ar, float ai, float br, flo
 }
 
 // r[row][j] = sum_k x[row][k] M[k][j], M = W (mode 0) or its adjoint (mode 1).  A thread has columns 2 tx, 2 tx + 1 of the rows
-// ty, ty + TY, ..; odd lengths are padded with zeros in shared memory.  N: both channel counts where they are known here.
-template <int MODE, int N>
+// ty, ty + TY, ..; odd lengths are padded with zeros in shared memory.  R: rows per thread.  N: both channel counts where they are
+// known here.
+template <int MODE, int R, int N>
 __global__ void __launch_bounds__(kThreads, 4) mix_kernel(float2* __restrict__ r, const float2* __restrict__ x, const float2* __restrict__ W,
                                                        long long rows, int nk_arg, int nj_arg, int w_cols, int ty_n_arg, RowCopy copy_x, bool wide_r) {
   extern __shared__ __align__(16) unsigned char sm[];
   const int nk = N > 0 ? N : nk_arg, nj = N > 0 ? N : nj_arg;
-  const int tx_n = (nj + 1) / 2, nk2 = (nk + 1) / 2, ty_n = N > 0 ? kThreads / tx_n : ty_n_arg, tile = ty_n * kRowsPerThread;
+  const int tx_n = (nj + 1) / 2, nk2 = (nk + 1) / 2, ty_n = N > 0 ? kThreads / tx_n : ty_n_arg, tile = ty_n * R;
   const int pitch = 16 * nk2 + 16;                        // bytes of a staged row of x
   float4* Ms = reinterpret_cast<float4*>(sm);             // [2 nk2][tx_n]: two columns each
   unsigned char* xs = sm + 32 * nk2 * tx_n;               // two tiles
+  const long long stride = (long long)gridDim.x * tile;
+  long long row0 = (long long)blockIdx.x * tile;
+  if (row0 < rows) tile_copy_async(xs, pitch, x + row0 * nk, (int)min((long long)tile, rows - row0), copy_x);
+  __pipeline_commit();
   for (int e = threadIdx.x; e < 4 * nk2 * tx_n; e += kThreads) {  // neighbouring threads read neighbouring weights
     int k, j;
     if (MODE == 0) {
@@ -81,10 +85,6 @@ __global__ void __launch_bounds__(kThreads, 4) mix_kernel(float2* __restrict__ r
     for (int row = threadIdx.x; row < 2 * tile; row += kThreads) *reinterpret_cast<float2*>(xs + row * pitch + 8 * nk) = make_float2(0.f, 0.f);
   const int tx = threadIdx.x % tx_n, ty = threadIdx.x / tx_n;
   const bool works = ty < ty_n;
-  const long long stride = (long long)gridDim.x * tile;
-  long long row0 = (long long)blockIdx.x * tile;
-  if (row0 < rows) tile_copy_async(xs, pitch, x + row0 * nk, (int)min((long long)tile, rows - row0), copy_x);
-  __pipeline_commit();
   for (int buf = 0; row0 < rows; row0 += stride, buf ^= 1) {
     const int nr = (int)min((long long)tile, rows - row0);
     const long long next = row0 + stride;
@@ -93,16 +93,16 @@ __global__ void __launch_bounds__(kThreads, 4) mix_kernel(float2* __restrict__ r
     __pipeline_wait_prior(1);
     __syncthreads();
     if (works) {
-      float2 s[kRowsPerThread][2], t[kRowsPerThread][2];  // sums over even and over odd k
+      float2 s[R][2], t[R][2];  // sums over even and over odd k
 #pragma unroll
-      for (int i = 0; i < kRowsPerThread; i++) s[i][0] = s[i][1] = t[i][0] = t[i][1] = make_float2(0.f, 0.f);
+      for (int i = 0; i < R; i++) s[i][0] = s[i][1] = t[i][0] = t[i][1] = make_float2(0.f, 0.f);
       const unsigned char* xr = xs + buf * tile * pitch + ty * pitch;
       const float4* m = Ms + tx;
 #pragma unroll 2
       for (int k = 0; k < nk2; k++) {  // rows past the end of the part read what the tile held before
         const float4 w0 = m[2 * k * tx_n], w1 = m[(2 * k + 1) * tx_n];
 #pragma unroll
-        for (int i = 0; i < kRowsPerThread; i++) {
+        for (int i = 0; i < R; i++) {
           const float4 a = *reinterpret_cast<const float4*>(xr + i * ty_n * pitch + 16 * k);
           mac(s[i][0], a.x, a.y, w0.x, w0.y);
           mac(s[i][1], a.x, a.y, w0.z, w0.w);
@@ -111,7 +111,7 @@ __global__ void __launch_bounds__(kThreads, 4) mix_kernel(float2* __restrict__ r
         }
       }
 #pragma unroll
-      for (int i = 0; i < kRowsPerThread; i++) {
+      for (int i = 0; i < R; i++) {
         const int row = ty + i * ty_n;
 #pragma unroll
         for (int c = 0; c < 2; c++) {
@@ -133,19 +133,21 @@ __global__ void __launch_bounds__(kThreads, 4) mix_kernel(float2* __restrict__ r
   }
 }
 
-// The block's share of sum_row conj(x[row][i]) g[row][j].  Threads: tiles of 4 x 4 entries, times as many groups of rows as fit;
+// The block's share of sum_row conj(x[row][i]) g[row][j].  Threads: tiles of 4 x 4 entries, times groups of rows;
 // the groups' sums meet in shared memory, the blocks' in global memory.
 // FOLD, where at most two groups fit (more than 32 x 32 channels) and a thread's rows are many: every eight tiles it adds its sums
 // to those of the tiles before.  It takes registers for two blocks on an SM in place of three.  64 x 64 channels, 400000 rows: error
 // against 64-bit sums 8.5e-7 -> 4.2e-7, 347 -> 371 us.
 template <bool FOLD>
 __global__ void __launch_bounds__(kThreads) mix_back_w_kernel(float* __restrict__ Wg, const float2* __restrict__ x, const float2* __restrict__ g,
-                                                              long long rows, int ni, int nj, long long rows_per_block, int tile_rows, RowCopy copy_x, RowCopy copy_g) {
+                                                              long long rows, int ni, int nj, long long rows_per_block, int tile_rows, int groups, RowCopy copy_x, RowCopy copy_g) {
   extern __shared__ __align__(16) unsigned char sm[];
-  const int ti_n = (ni + 3) / 4, tj_n = (nj + 3) / 4, tiles = ti_n * tj_n, groups = kThreads / tiles;
+  const int ti_n = (ni + 3) / 4, tj_n = (nj + 3) / 4, tiles = ti_n * tj_n;
   const int px = 32 * ti_n + 16, pg = 32 * tj_n + 16, tile = tile_rows * (px + pg);
-  for (int e = threadIdx.x; e < 2 * tile / 16; e += kThreads) reinterpret_cast<float4*>(sm)[e] = make_float4(0.f, 0.f, 0.f, 0.f);  // padding
-  __syncthreads();
+  if ((ni | nj) & 3) {  // padding
+    for (int e = threadIdx.x; e < 2 * tile / 16; e += kThreads) reinterpret_cast<float4*>(sm)[e] = make_float4(0.f, 0.f, 0.f, 0.f);
+    __syncthreads();
+  }
   const long long begin = (long long)blockIdx.x * rows_per_block, end = min(rows, begin + rows_per_block);
   auto copy_tile = [&](int buf, long long row0) {
     const int nr = (int)min((long long)tile_rows, end - row0);
@@ -242,14 +244,22 @@ int launch_mix(float* r, const float* x, const float* W, long long rows, int n_i
   if (rows <= 0) return GELIB_OK;
   const int nk = mode == 0 ? n_in : n_out, nj = mode == 0 ? n_out : n_in;  // contraction length, output channels
   const int tx_n = (nj + 1) / 2, nk2 = (nk + 1) / 2, pitch = 16 * nk2 + 16;
-  const int ty_n = std::min(kThreads / tx_n, 32768 / (kRowsPerThread * pitch));  // a tile of at most 32 KB
-  const int tile = ty_n * kRowsPerThread;
+  const int most = std::min(kThreads / tx_n, 32768 / (4 * pitch));  // groups of rows; a tile of at most 32 KB
+  // Few rows: one to a thread, in tiles for two blocks on every SM.  More: four, in tiles for at least two.  us, tiles of full size and
+  // four rows a thread always / as here: 5 x 3 channels, 3000 rows 4.8 / 3.1, 30000 5.0 / 4.0, 100000 5.8 / 5.0; 32 x 16, 3000 5.7 / 3.7; 32 x 32, 7000
+  // 5.7 / 4.6; 16 x 8, 7000 rows with four rows a thread 4.3, with one 3.7; 14000 3.9, 4.2.
+  const int R = rows <= 10000 ? 1 : 4;
+  const int ty_n = (int)std::min<long long>(most, (rows + R * 296 - 1) / (R * 296));
+  const int tile = ty_n * R;
   const size_t smem = (size_t)32 * nk2 * tx_n + (size_t)2 * tile * pitch;
   const unsigned blocks = (unsigned)std::min<long long>((rows + tile - 1) / tile, 148LL * 8);
-  auto k = mode == 0 ? mix_kernel<0, 0> : mix_kernel<1, 0>;
-  if (nk == 8 && nj == 8) k = mode == 0 ? mix_kernel<0, 8> : mix_kernel<1, 8>;
-  if (nk == 16 && nj == 16) k = mode == 0 ? mix_kernel<0, 16> : mix_kernel<1, 16>;
-  if (nk == 32 && nj == 32) k = mode == 0 ? mix_kernel<0, 32> : mix_kernel<1, 32>;
+  auto k = mode == 0 ? mix_kernel<0, 4, 0> : mix_kernel<1, 4, 0>;
+  if (R == 1) k = mode == 0 ? mix_kernel<0, 1, 0> : mix_kernel<1, 1, 0>;
+  else if (ty_n == kThreads / tx_n) {  // the bodies of one channel count take that many groups
+    if (nk == 8 && nj == 8) k = mode == 0 ? mix_kernel<0, 4, 8> : mix_kernel<1, 4, 8>;
+    if (nk == 16 && nj == 16) k = mode == 0 ? mix_kernel<0, 4, 16> : mix_kernel<1, 4, 16>;
+    if (nk == 32 && nj == 32) k = mode == 0 ? mix_kernel<0, 4, 32> : mix_kernel<1, 4, 32>;
+  }
   cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e == cudaSuccess)
     k<<<blocks, kThreads, smem, s>>>(reinterpret_cast<float2*>(r), reinterpret_cast<const float2*>(x), reinterpret_cast<const float2*>(W), rows, nk,
@@ -265,18 +275,23 @@ int launch_mix_back_w(float* Wg, const float* x, const float* g, long long rows,
   if (n_in < 1 || n_out < 1 || n_in > kMixMaxN || n_out > kMixMaxN) return fail(GELIB_SKIPPED, fn, "more than 64 channels");
   if (rows <= 0) return GELIB_OK;
   const int ti_n = (n_in + 3) / 4, tj_n = (n_out + 3) / 4, tiles = ti_n * tj_n;
-  const int tile_rows = std::min(256, 32768 / (32 * (ti_n + tj_n) + 32) / 16 * 16);  // about 32 KB
+  // Tiles of about 32 KB; smaller ones, down to 64 rows, where there would be fewer than a block per SM.
+  const long long share = std::max<long long>(64, (rows / 148 + 15) / 16 * 16);
+  const int tile_rows = (int)std::min<long long>(std::min(256, 32768 / (32 * (ti_n + tj_n) + 32) / 16 * 16), share);
   const bool fold = kThreads / tiles <= 2;
   const long long want_blocks = std::min<long long>((rows + tile_rows - 1) / tile_rows, 148LL * (fold ? 2 : 3));
   long long rpb = (rows + want_blocks - 1) / want_blocks;
   rpb = (rpb + tile_rows - 1) / tile_rows * tile_rows;
   const unsigned blocks = (unsigned)((rows + rpb - 1) / rpb);
-  const size_t smem = std::max((size_t)2 * tile_rows * (32 * (ti_n + tj_n) + 32), (size_t)kThreads / tiles * tiles * 128);
+  // As many groups as fit, of at least four rows: their sums are added one after the other.  With the tiles above, us: 5 x 3 channels, 300
+  // rows 7.3 -> GROUPS.
+  const int groups = (int)std::min<long long>(kThreads / tiles, std::max<long long>(1, rpb / 4));
+  const size_t smem = std::max((size_t)2 * tile_rows * (32 * (ti_n + tj_n) + 32), (size_t)groups * tiles * 128);
   auto k = fold ? mix_back_w_kernel<true> : mix_back_w_kernel<false>;
   cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e == cudaSuccess)
     k<<<blocks, kThreads, smem, s>>>(Wg, reinterpret_cast<const float2*>(x), reinterpret_cast<const float2*>(g), rows, n_in, n_out, rpb,
-                                     tile_rows, row_copy(x, n_in), row_copy(g, n_out));
+                                     tile_rows, groups, row_copy(x, n_in), row_copy(g, n_out));
   if (e == cudaSuccess) e = cudaGetLastError();
   if (e != cudaSuccess) return check_cuda(e, fn, "weight gradient kernel launch");
   count_launch();

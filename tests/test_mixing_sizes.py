@@ -35,3 +35,25 @@ def test_wide_weight_gradients_are_as_accurate_as_narrow_ones(gb):
 
     narrow = error(32)
     assert error(48) < 1.15 * narrow and error(64) < 1.15 * narrow
+
+
+# several tiles and a partial last one for every block; few rows, and both sides of the lines
+SIZES = [(200003, 16, 16), (40001, 64, 64), (310007, 8, 8), (80021, 32, 32), (70001, 16, 32), (70001, 32, 16), (300011, 5, 3), (150001, 33, 31),
+         (1, 7, 9), (295, 5, 3), (297, 32, 4), (9999, 5, 3), (10000, 16, 8), (10001, 16, 8), (10001, 64, 2), (30011, 3, 5), (9473, 12, 20)]
+
+
+@pytest.mark.parametrize("aligned", [True, False])
+@pytest.mark.parametrize("rows,n_in,n_out", SIZES)
+def test_several_tiles_per_block(gb, rows, n_in, n_out, aligned):
+    off = 0 if aligned else 1  # eight bytes off a 16-byte boundary
+
+    def operand(seed, n):
+        return crand(seed, rows * n + off)[off:].view(rows, n)
+
+    x, w, g = operand(1, n_in), crand(2, n_in, n_out), operand(3, n_out)
+    # an element's error is at most the number of its roundings, 2 n + 1, times half an ulp of the terms' absolute sum
+    for got, a, b in ((gb.mix(x, w), wide(x), wide(w)), (gb.mix(g, w, adjoint=True), wide(g), wide(w).conj().T)):
+        bound = (2 * a.size(1) + 1) * 2.0 ** -24 * 2 ** 0.5 * (a.abs() @ b.abs())
+        assert bool(((wide(got) - a @ b).abs() <= bound).all())
+    # a tile left out or taken twice shows by more than a percent; sums of 32-bit numbers in random order by some 1e-6
+    assert relative_error(gb.mix_back_w(x, g, n_in, n_out), wide(x).conj().T @ wide(g)) < 1e-5

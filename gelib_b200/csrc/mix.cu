@@ -50,14 +50,14 @@ __device__ __forceinline__ void mac(float2& s, float ar, float ai, float br, flo
 }
 
 // r[row][j] = sum_k x[row][k] M[k][j], M = W (mode 0) or its adjoint (mode 1).  A thread has columns 2 tx, 2 tx + 1 of the rows
-// ty, ty + TY, ..; odd lengths are padded with zeros in shared memory.  R: rows per thread.  N: both channel counts where they are
-// known here.
-template <int MODE, int R, int N>
+// ty, ty + TY, ..; odd lengths are padded with zeros in shared memory.  R: rows per thread.  NK, NJ: the
+// channel counts where they are known here.
+template <int MODE, int R, int NK, int NJ>
 __global__ void __launch_bounds__(kThreads, 4) mix_kernel(float2* __restrict__ r, const float2* __restrict__ x, const float2* __restrict__ W,
                                                        long long rows, int nk_arg, int nj_arg, int w_cols, int ty_n_arg, RowCopy copy_x, bool wide_r) {
   extern __shared__ __align__(16) unsigned char sm[];
-  const int nk = N > 0 ? N : nk_arg, nj = N > 0 ? N : nj_arg;
-  const int tx_n = (nj + 1) / 2, nk2 = (nk + 1) / 2, ty_n = N > 0 ? kThreads / tx_n : ty_n_arg, tile = ty_n * R;
+  const int nk = NK > 0 ? NK : nk_arg, nj = NJ > 0 ? NJ : nj_arg;
+  const int tx_n = (nj + 1) / 2, nk2 = (nk + 1) / 2, ty_n = NK > 0 ? kThreads / tx_n : ty_n_arg, tile = ty_n * R;
   const int pitch = 16 * nk2 + 16;                        // bytes of a staged row of x
   float4* Ms = reinterpret_cast<float4*>(sm);             // [2 nk2][tx_n]: two columns each
   unsigned char* xs = sm + 32 * nk2 * tx_n;               // two tiles
@@ -244,7 +244,7 @@ int launch_mix(float* r, const float* x, const float* W, long long rows, int n_i
   if (rows <= 0) return GELIB_OK;
   const int nk = mode == 0 ? n_in : n_out, nj = mode == 0 ? n_out : n_in;  // contraction length, output channels
   const int tx_n = (nj + 1) / 2, nk2 = (nk + 1) / 2, pitch = 16 * nk2 + 16;
-  const int most = std::min(kThreads / tx_n, 32768 / (4 * pitch));  // groups of rows; a tile of at most 32 KB
+  const int most = std::min(kThreads / tx_n, 35000 / (4 * pitch));  // groups of rows; a tile of at most 34 KB
   // Few rows: one to a thread, in tiles for two blocks on every SM.  More: four, in tiles for at least two.  us, tiles of full size and
   // four rows a thread always / as here: 5 x 3 channels, 3000 rows 4.8 / 3.1, 30000 5.0 / 4.0, 100000 5.8 / 5.0; 32 x 16, 3000 5.7 / 3.7; 32 x 32, 7000
   // 5.7 / 4.6; 16 x 8, 7000 rows with four rows a thread 4.3, with one 3.7; 14000 3.9, 4.2.
@@ -253,12 +253,12 @@ int launch_mix(float* r, const float* x, const float* W, long long rows, int n_i
   const int tile = ty_n * R;
   const size_t smem = (size_t)32 * nk2 * tx_n + (size_t)2 * tile * pitch;
   const unsigned blocks = (unsigned)std::min<long long>((rows + tile - 1) / tile, 148LL * 8);
-  auto k = mode == 0 ? mix_kernel<0, 4, 0> : mix_kernel<1, 4, 0>;
-  if (R == 1) k = mode == 0 ? mix_kernel<0, 1, 0> : mix_kernel<1, 1, 0>;
-  else if (ty_n == kThreads / tx_n) {  // the bodies of one channel count take that many groups
-    if (nk == 8 && nj == 8) k = mode == 0 ? mix_kernel<0, 4, 8> : mix_kernel<1, 4, 8>;
-    if (nk == 16 && nj == 16) k = mode == 0 ? mix_kernel<0, 4, 16> : mix_kernel<1, 4, 16>;
-    if (nk == 32 && nj == 32) k = mode == 0 ? mix_kernel<0, 4, 32> : mix_kernel<1, 4, 32>;
+  auto k = mode == 0 ? mix_kernel<0, 4, 0, 0> : mix_kernel<1, 4, 0, 0>;
+  if (R == 1) k = mode == 0 ? mix_kernel<0, 1, 0, 0> : mix_kernel<1, 1, 0, 0>;
+  else if (ty_n == kThreads / tx_n) {  // the bodies of known channel counts take that many groups
+#define GELIB_MIX_BODY(a, b) if (nk == a && nj == b) k = mode == 0 ? mix_kernel<0, 4, a, b> : mix_kernel<1, 4, a, b>;
+    GELIB_MIX_BODY(8, 8) GELIB_MIX_BODY(16, 16) GELIB_MIX_BODY(32, 32) GELIB_MIX_BODY(16, 32) GELIB_MIX_BODY(32, 16)
+#undef GELIB_MIX_BODY
   }
   cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e == cudaSuccess)

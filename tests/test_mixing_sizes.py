@@ -57,3 +57,25 @@ def test_several_tiles_per_block(gb, rows, n_in, n_out, aligned):
         assert bool(((wide(got) - a @ b).abs() <= bound).all())
     # a tile left out or taken twice shows by more than a percent; sums of 32-bit numbers in random order by some 1e-6
     assert relative_error(gb.mix_back_w(x, g, n_in, n_out), wide(x).conj().T @ wide(g)) < 1e-5
+
+
+def test_two_channels_are_summed_in_one_chain(gb):
+    # fma in double rounded to float: the chain of four multiply-adds, and two halves of two added at the end
+    x, w = crand(1, 200000, 2), crand(2, 2, 16)
+    a, b = torch.view_as_real(x).double(), torch.view_as_real(w).double()
+
+    def fma(p, q, s):
+        return (p * q + s).float().double()
+
+    def mac(re, im, k):
+        xr, xi, wr, wi = a[:, k, None, 0], a[:, k, None, 1], b[k, :, 0], b[k, :, 1]
+        return fma(-xi, wi, fma(xr, wr, re)), fma(xi, wr, fma(xr, wi, im))
+
+    zero = torch.zeros(200000, 16, dtype=torch.float64, device="cuda")
+    first = mac(zero, zero, 0)
+    chain = torch.complex(*mac(*first, 1))
+    second = mac(zero, zero, 1)
+    halves = torch.complex((first[0] + second[0]).float().double(), (first[1] + second[1]).float().double())
+    want = wide(x) @ wide(w)
+    assert relative_error(chain, want) < relative_error(halves, want)
+    assert relative_error(gb.mix(x, w), want) < 1.01 * relative_error(chain, want)

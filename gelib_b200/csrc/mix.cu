@@ -10,11 +10,11 @@
 //
 // Both kernels stage tiles of rows in shared memory (asynchronous copies, one tile in flight while the other is worked on) and
 // give a thread a tile of the result: 4 rows x 2 columns of the product, 4 x 4 entries of the weight gradient, so that a 16-byte
-// load feeds 11 (16) multiply-adds; products are summed in two halves, and 8, 16 and 32 channels on both sides have a body of
-// their own (16 x 16, 3.2 million rows: 240 us without).  Measured against one output element (one (i,j) sum) per thread, us,
-// product / adjoint / weight gradient: 16 x 16 channels, 3.2 million rows 214 / 238 / 396 -> 197 / 197 / 247; 32 x 32, 400000 96 /
-// 156 / 194 -> 98 / 99 / 110; 8 x 8, 2 million 104 / 104 / 132 -> 57 / 57 / 79; 12 x 20, 500000 76 / 70 / 85 -> 49 / 51 / 62; 64 x
-// 64, 100000 207 / 213 / 243 -> 106 / 115 / 108.  At 16 channels the multiply-adds alone take 91 us and the memory 126.
+// load feeds 11 (16) multiply-adds; products are summed in two halves, and 8, 16 and 32 channels on both sides, and 16 with 32, have a
+// body of their own (us without / with: 16 x 16, 3.2 million rows 240 / 197; 1.6 million, 16 x 32 221 / 200, 32 x 16 223 / 175).  Measured
+// against one output element (one (i,j) sum) per thread, us, product / adjoint / weight gradient: 16 x 16 channels, 3.2 million rows
+// 214 / 238 / 396 -> 197 / 197 / 247; 32 x 32, 400000 96 / 156 / 194 -> 93 / 95 / 104; 8 x 8, 2 million 104 / 104 / 132 -> 57 / 57 / 79; 12 x 20, 500000
+// 76 / 70 / 85 -> 49 / 51 / 62; 64 x 64, 100000 197 / 198 / 235 -> 100 / 100 / 98.  At 16 channels the multiply-adds alone take 91 us and the memory 126.
 #include <cuda_pipeline.h>
 
 #include <algorithm>
@@ -137,8 +137,8 @@ __global__ void __launch_bounds__(kThreads, 4) mix_kernel(float2* __restrict__ r
 // The block's share of sum_row conj(x[row][i]) g[row][j].  Threads: tiles of 4 x 4 entries, times groups of rows;
 // the groups' sums meet in shared memory, the blocks' in global memory.
 // FOLD, where at most two groups fit (more than 32 x 32 channels) and a thread's rows are many: every eight tiles it adds its sums
-// to those of the tiles before.  It takes registers for two blocks on an SM in place of three.  64 x 64 channels, 400000 rows: error
-// against 64-bit sums 8.5e-7 -> 4.2e-7, 347 -> 371 us.
+// to those of the tiles before.  It takes registers for two blocks on an SM in place of three.  400000 rows, error against 64-bit sums
+// and us without / with: 64 x 64 channels 8.4e-7 / 4.2e-7, 347 / 342; 48 x 48 8.5e-7 / 4.9e-7, 275 / 283.
 template <bool FOLD>
 __global__ void __launch_bounds__(kThreads) mix_back_w_kernel(float* __restrict__ Wg, const float2* __restrict__ x, const float2* __restrict__ g,
                                                               long long rows, int ni, int nj, long long rows_per_block, int tile_rows, int groups, RowCopy copy_x, RowCopy copy_g) {
@@ -247,8 +247,9 @@ int launch_mix(float* r, const float* x, const float* W, long long rows, int n_i
   const int tx_n = (nj + 1) / 2, nk2 = (nk + 1) / 2, pitch = 16 * nk2 + 16;
   const int most = std::min(kThreads / tx_n, 35000 / (4 * pitch));  // groups of rows; a tile of at most 34 KB
   // Few rows: one to a thread, in tiles for two blocks on every SM.  More: four, in tiles for at least two.  us, tiles of full size and
-  // four rows a thread always / as here: 5 x 3 channels, 3000 rows 4.8 / 3.1, 30000 5.0 / 4.0, 100000 5.8 / 5.0; 32 x 16, 3000 5.7 / 3.7; 32 x 32, 7000
-  // 5.7 / 4.6; 16 x 8, 7000 rows with four rows a thread 4.3, with one 3.7; 14000 3.9, 4.2.
+  // four rows a thread always / as here: 5 x 3 channels, 3000 rows 4.9 / 3.2, 30000 4.7 / 3.7, 100000 5.9 / 5.1; 32 x 16, 3000 5.8 / 3.6;
+  // 64 x 4, 3000 6.8 / 3.8; 16 x 8, 7000 4.3 / 3.1.  Mean over 37 pairs of counts, against full tiles: 7000 rows, one row a thread 0.83, four 0.88;
+  // 14000 rows 0.99 and 0.90.
   const int R = rows <= 10000 ? 1 : 4;
   const int ty_n = (int)std::min<long long>(most, (rows + R * 296 - 1) / (R * 296));
   const int tile = ty_n * R;
@@ -286,8 +287,8 @@ int launch_mix_back_w(float* Wg, const float* x, const float* g, long long rows,
   long long rpb = (rows + want_blocks - 1) / want_blocks;
   rpb = (rpb + tile_rows - 1) / tile_rows * tile_rows;
   const unsigned blocks = (unsigned)((rows + rpb - 1) / rpb);
-  // As many groups as fit, of at least four rows: their sums are added one after the other.  With the tiles above, us: 5 x 3 channels, 300
-  // rows 7.3 -> GROUPS.
+  // As many groups as fit, of at least four rows: their sums are added one after the other.  With the tiles above, us, zeroing of the
+  // result included: 5 x 3 channels, 300 rows 7.0 -> 4.8, 3000 6.8 -> 4.7; 16 x 8, 3000 6.3 -> 5.6.
   const int groups = (int)std::min<long long>(kThreads / tiles, std::max<long long>(1, rpb / 4));
   const size_t smem = std::max((size_t)2 * tile_rows * (32 * (ti_n + tj_n) + 32), (size_t)groups * tiles * 128);
   auto k = fold ? mix_back_w_kernel<true> : mix_back_w_kernel<false>;

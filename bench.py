@@ -217,36 +217,11 @@ def cpu_baseline(tx, ty, maxl, B, diag, budget_s=15.0):
                                     "%.1f ms measured, extrapolated linearly" % (B1, B, t1 * 1e3)}
 
 
-def run_reference(args, tx, ty, maxl, B, diag, desc):
-    """--impl reference: the reference's CPU path for the same config, on the host cores.  GElib itself cannot be
-    compiled here (its cnine submodule is not vendored), so this arm times the CPU oracle, which restates the
-    reference's loops, with every host thread, each step on a bounded slice of the batch."""
-    rank = int(os.environ.get("RANK", "0"))
-    if rank != 0:
-        return
-    from oracle import oracle as O
-    O.build()
-    nt = host_threads()
-    Bs = max(nt, 8) * 4
-    times = []
-    for i in range(args.warmup + args.steps):
-        t = cpu_fwd_bwd(O, tx, ty, maxl, Bs, diag, nt)
-        if i >= args.warmup:
-            times.append(t)
-    ms = statistics.mean(times) * 1e3 * B / Bs
-    cb = {"value": ms, "unit": "ms", "cores": nt, "kind": "port",
-          "sample": "oracle on %d of %d batch rows per step, extrapolated linearly" % (Bs, B)}
-    print(json.dumps({"impl": "reference", "kind": "port", "extrapolated": True, "measured_rows": Bs,
-                      "measured_ms_per_step": statistics.mean(times) * 1e3, "cores": nt,
-                      "metric": "cg_product_fwd_bwd_ms_per_call", "value": ms, "unit": "ms",
-                      "n_gpus": args.gpus, "steps": args.steps, "warmup": args.warmup, "ms_per_step": ms,
-                      "higher_is_better": False, "scaling": "strong" if args.workload == "cfg5" else "weak",
-                      "vs_baseline": None, "dtype": "f32", "data": "synthetic",
-                      "config": {"workload": "%s: %s; per-GPU batch %d, global batch %d" % (
-                          (args.workload, desc, B // args.gpus, B) if args.workload == "cfg5"
-                          else (args.workload, desc, B, B * args.gpus))},
-                      "cpu_baseline": cb,
-                      "e2e": {"value": ms, "unit": "ms", "h2d_bytes_per_step": 0, "d2h_bytes_per_step": 0}}))
+def run_reference():
+    """--impl reference: GElib itself, which cannot be built here.  Nothing of this repository is timed in its place."""
+    if int(os.environ.get("RANK", "0")) == 0:
+        print(json.dumps({"impl": "reference", "unavailable": "GElib cannot be built: its headers include cnine, a git submodule that is not "
+                                                              "vendored and has no pinned commit"}))
 
 
 # ---- GPU arm -----------------------------------------------------------------------------------------------------
@@ -275,7 +250,7 @@ def main():
     if args.batch:
         B = args.batch
     if args.impl == "reference":
-        return run_reference(args, tx, ty, maxl, B, diag, desc)
+        return run_reference()
     strong = args.workload == "cfg5"   # its points are split evenly over the ranks; every other workload is weak
     if strong:
         B = B // max(1, int(os.environ.get("WORLD_SIZE", "1")))

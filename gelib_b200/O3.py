@@ -13,7 +13,7 @@ the running offset of that loop (core/Gvec.hpp:311-321 with O(3) indices).
 import torch
 
 from . import backend as gb
-from .gelib_common import common_batch
+from .gelib_common import common_batch, output_memory
 from .SO3element import SO3element
 from .SO3irrep import SO3irrep
 
@@ -211,7 +211,7 @@ def _part_forward(ctx, x, y, mu, diag):
     ctx.save_for_backward(x, y)
     b = common_batch(x, y)
     n = x.size(-1) if diag else x.size(-1) * y.size(-1)
-    r = torch.empty([b, 2 * mu[0] + 1, n], dtype=torch.complex64, device=x.device)
+    r = output_memory(_plain(x), _plain(y))([b, 2 * mu[0] + 1, n], dtype=torch.complex64, device=x.device)
     rb, xb, yb = gb.SO3part.view(r), gb.SO3part.view(_plain(x)), gb.SO3part.view(_plain(y))
     done = (rb.add_DiagCGproduct if diag else rb.add_CGproduct)(xb, yb, overwrite=True)
     if not done:
@@ -286,7 +286,8 @@ def _vec_forward(ctx, k1, k2, maxl, xmus, ymus, args, diag):
     rtype = (O3type(dict(zip(xmus, xn))).DiagCGproduct if diag else O3type(dict(zip(xmus, xn))).CGproduct)(
         O3type(dict(zip(ymus, yn))), maxl).get_parts()
     b = common_batch(xs[0], ys[0])
-    rparts = {mu: torch.empty([b, 2 * mu[0] + 1, n], dtype=torch.complex64, device=xs[0].device) for mu, n in rtype.items()}
+    memory = output_memory(*xs, *ys)
+    rparts = {mu: memory([b, 2 * mu[0] + 1, n], dtype=torch.complex64, device=xs[0].device) for mu, n in rtype.items()}
     calls = _sector_calls(xmus, xn, ymus, yn, rtype, maxl, diag)
     ctx.calls, ctx.k1, ctx.k2, ctx.diag, ctx.rmus = calls, k1, k2, diag, list(rtype)
     ctx.save_for_backward(*args)

@@ -10,7 +10,7 @@ import torch
 
 from . import backend as gb
 from ._lib import native
-from .gelib_common import common_batch, of_class, plain
+from .gelib_common import common_batch, of_class, output_memory, plain
 from .SO3element import SO3element
 from .SO3irrep import SO3irrep
 
@@ -102,7 +102,7 @@ def _product_forward_plain(ctx, x, y, l, diag):
         grid = [max(a, c) for a, c in zip(gx, gy)]
     else:
         grid = gx if len(gx) > len(gy) else gy
-    r = torch.empty([b] + grid + [2 * l + 1, n], dtype=torch.complex64, device=x.device)
+    r = output_memory(x, y)([b] + grid + [2 * l + 1, n], dtype=torch.complex64, device=x.device)
     xb, yb, rb = gb.SO3part.view(x.detach()), gb.SO3part.view(y.detach()), gb.SO3part.view(r)
     done = (rb.add_DiagCGproduct if diag else rb.add_CGproduct)(xb, yb, overwrite=True)
     if not done:  # a skipped call computes nothing: the reference's output is its zero-initialised tensor

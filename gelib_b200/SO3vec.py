@@ -9,7 +9,7 @@ import torch
 
 from . import backend as gb
 from ._lib import native
-from .gelib_common import common_batch, of_class, plain, zeros_like_all
+from .gelib_common import common_batch, of_class, output_memory, plain, zeros_like_all
 from .SO3part import SO3part, SO3partArr
 
 
@@ -33,7 +33,8 @@ def _vec_forward_plain(ctx, k1, k2, maxl, args, diag, part_cls):
         grid = [max(a, c) for a, c in zip(gx, gy)]
     else:
         grid = gx if len(gx) > len(gy) else gy
-    rparts = [torch.empty([b] + grid + [2 * l + 1, n], dtype=torch.complex64, device=xs[0].device)
+    memory = output_memory(*xs, *ys)
+    rparts = [memory([b] + grid + [2 * l + 1, n], dtype=torch.complex64, device=xs[0].device)
               for l, n in tau.get_parts().items()]
     r = gb.SO3vec.view(rparts)
     done = (r.addDiagCGproduct if diag else r.addCGproduct)(x, y, overwrite=True)
@@ -159,8 +160,8 @@ class SO3vec_SpharmCGproductFn(torch.autograd.Function):
         tx = gb.SO3type({l: 1 for l in range(lmax_x + 1)})
         y = gb.SO3vec.view(ys)
         tau = tx.CGproduct(y.get_tau(), maxl)
-        rparts = [torch.empty([X.size(0), 2 * l + 1, n], dtype=torch.complex64, device=X.device)
-                  for l, n in tau.get_parts().items()]
+        memory = output_memory(X, *ys)
+        rparts = [memory([X.size(0), 2 * l + 1, n], dtype=torch.complex64, device=X.device) for l, n in tau.get_parts().items()]
         if not gb.SO3vec.view(rparts).addCGproduct_spharm(X, lmax_x, y, overwrite=True):
             for p in rparts:
                 p.zero_()

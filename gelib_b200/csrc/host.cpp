@@ -93,10 +93,10 @@ bool call(F f) {
 
 void* stream_of(c10::Device device) { return c10::cuda::getCurrentCUDAStream(device.index()).stream(); }
 
-// Batch and grid of a product; false when the batches do not fit.
+// Batch and grid of a product; false when the batches do not fit, or an operand is empty (the kernels then write nothing).
 bool lead_dims(const at::Tensor& x, const at::Tensor& y, std::vector<int64_t>* lead) {
   const int64_t bx = x.size(0), by = y.size(0);
-  if (bx > 1 && by > 1 && bx != by) return false;
+  if ((bx > 1 && by > 1 && bx != by) || x.numel() == 0 || y.numel() == 0) return false;
   lead->push_back(std::max(bx, by));
   const int64_t gx = x.dim() - 3, gy = y.dim() - 3;
   for (int64_t k = 1; k <= std::max(gx, gy); k++)  // size-1 grid dimensions are broadcast against the other operand's

@@ -30,3 +30,9 @@ def common_batch(x, y):
     if x.size(0) > 1 and y.size(0) > 1:
         assert x.size(0) == y.size(0)
     return max(x.size(0), y.size(0))
+
+
+def output_memory(*operands):
+    """torch.empty for the output of a product that writes all of it; torch.zeros when an operand is empty: the product then has
+    no cells and writes nothing, and the reference's output is its zero-initialised tensor."""
+    return torch.zeros if any(t.numel() == 0 for t in operands) else torch.empty

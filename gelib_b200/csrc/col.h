@@ -28,8 +28,8 @@
 // Why this form: diag_bwd_cell_kernel spends its time in four shared-memory atomics (compare-and-swap loops) per band
 // entry, which a lane that owns its column does not need.  Measured, backward of the diagonal product: maxl 8 x 128
 // channels, batch 2048 10.5 -> 4.7 ms; maxl 6 x 33, batch 4000 4.3 -> 1.0 ms; maxl 3 x 12, batch 500 49 -> 29 us (forward 32 ->
-// 15 us).  At maxl 8 the backward holds two warps per scheduler -- 252 registers a thread and 25.6 KB of shared memory a warp
-// both end there -- and issues in 42 % of its cycles: 502 k warp instructions per 64 columns, whose largest stalls are
+// 15 us).  At maxl 8 the backward holds two warps per scheduler -- 242 registers a thread and 25.6 KB of shared memory a warp
+// both end there -- and issues in 43 % of its cycles: 494 k warp instructions per 64 columns, whose largest stalls are
 // fixed-latency dependencies (1.3 cycles per issue) and shared memory (0.7).  The forward issues in 32 %: 345 k
 // instructions, dependencies 1.5, shared memory 1.3, instruction fetch of the unrolled bodies 1.1; its instances spill 84 to
 // 168 bytes a thread at 168, 128 and 128 registers, which its block sizes impose.

@@ -1,5 +1,5 @@
-// Mirrored-row forward kernel: products in which every channel of the output has its own pair of input columns (column = (cell,
-// channel), see col.h), for calls with enough columns to fill the chip.
+// Mirrored-row and row-pair kernels: products in which every channel of the output has its own pair of input columns (column =
+// (cell, channel), see col.h).  Forward (mir_fwd.cu), at every batch except for types of a handful of items on many columns:
 //
 //   r_l[m] (+)= sum_{m1} C_l[m1, m-m1] x_l1[m1] y_l2[m-m1],     C_l[-m1,-m2] = (-1)^(l1+l2-l) C_l[m1,m2]
 //
@@ -9,6 +9,8 @@
 // entry 0, which meets itself, is halved.
 // The inner loop runs over the band with every operand in shared memory and is instantiated per number of output l only, so the
 // code is small, nothing is padded to a block size, and nothing is computed outside the band.
+// The gradient of y for a one-channel x (mir_bwd.cu), on a full chip and where it measured faster, walks items of two
+// neighbouring rows in the same manner.
 #pragma once
 #include "col.h"
 
@@ -32,7 +34,7 @@ struct MirArgs {
   int nitems;
 };
 
-// Backward, mir_bwd.cu.
+// Gradient of y.
 struct MirBwdArgs {
   ColPart x[kMaxParts], yg[kMaxParts], g[kMaxParts];
   unsigned char xl[kMaxParts];

@@ -11,10 +11,10 @@
 // The loop is instantiated per number of output l.  While it works on an item a warp loads the g rows of the next into
 // registers, asks those of the one after into the L2, and copies the tables of the third (cp.async).
 //
-// Measured against cg_narrow1_bwd_kernel and the column kernel, us: maxl 6 x 16, 65536 cells 5470 -> 4580; maxl 4 x 32,
-// 10000 586 -> 480; maxl 3 x 9, 44444 461 -> 349.  Bound by issue and latency: 96 k warp instructions per 32 columns at maxl 6, of
-// which the band loops are 40 %, issued in 54 % of the cycles with 16 warps on an SM.  Without the request into the L2 5310, at 16 warps
-// instead of 20 4970, at 24, which spills, 5420; two columns per lane (187 registers, 11 warps) 6790.
+// Measured, a million columns, against cg_narrow1_bwd_kernel: maxl 6 x 16 5.05 -> 4.33 ms, maxl 6 x 32 4.87 -> 4.28; against the column
+// kernel: maxl 3 x 9 1.10 -> .77, maxl 5 x 16 3.02 -> 2.73 (row_pairs_from).  Bound by issue and latency: 106 k warp instructions per 32
+// columns at maxl 6, of which the band loops are 40 %, issued in 58 % of the cycles.  Measured on maxl 6 x 16, 65536 cells, 4580 us: without the request into the L2
+// 5310, at 16 warps instead of 20 4970, at 24, which spills, 5420; two columns per lane (187 registers, 11 warps) 6790.
 #include <algorithm>
 #include <cstring>
 #include <map>
